@@ -74,6 +74,8 @@ typedef struct MskMoeCfg {
   int32_t stop_after;    /* measuring aid: 0 = whole step; 1/2/3 = return after sort / gate-up GEMM / down GEMM */
   int32_t flat_shares;   /* non-zero (with n_tokens * top_k <= 256 and paths 1, 2): the last rounds of the weight stream
                             are cut into equal shares per CTA instead of whole units (see msk_moe_share_pieces) */
+  int32_t host_inputs;   /* non-zero: x of the call lies in pinned host memory, so it is read once by all CTAs together
+                            and not once by each (results do not depend on it) */
 } MskMoeCfg;
 
 /* ---- prepare-time repack (lossless; replaces the four layouts built by
@@ -85,9 +87,9 @@ int msk_moe_packed_bytes(const MskMoeCfg* cfg, size_t* host_w13_bytes, size_t* h
 /* w13: uint8 [local_count, 2I, H/2] (two E2M1 codes per byte, low nibble = even k; rows
  * [gate 0..I-1; up I..2I-1]); w13_sf: E4M3 bytes [local_count, 2I, H/16];
  * w2: uint8 [local_count, H, I/2]; w2_sf: [local_count, H, I/16].
- * Output: tiles of 128 rows x 256 K, each 16 KiB of bit-permuted codes followed by
- * 2 KiB of scale bytes, ordered [expert][row tile][gate|up][k stage] for w13 and
- * [expert][row tile][k stage] for w2. Bit and byte permutation only. */
+ * Output: blocks of 8 rows x 256 K, each 1024 bytes of codes followed by 128 scale bytes, ordered
+ * [expert][pair of 128-row tiles][8-row slice][tile of the pair][k block]; a pair is (gate j, up j) of w13,
+ * (2j, 2j + 1) of w2. Byte permutation only. */
 int msk_moe_repack(const MskMoeCfg* cfg, const void* w13, const void* w13_sf, const void* w2, const void* w2_sf,
                    void* packed13, void* packed2, void* stream);
 

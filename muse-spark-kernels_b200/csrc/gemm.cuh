@@ -2,8 +2,8 @@
 //
 // D[128 weight rows, N tokens] = W_tile[128, K] * X_tile[N, K]^T, weights on the MMA M side.
 // Per CTA (768 threads, one CTA per SM):
-//   warp 0       weight producer: 1-D bulk async copies (TMA engine) of packed NVFP4 tiles,
-//                two tiles (a "pair") per K stage, into a shared-memory ring;
+//   warp 0       weight producer: one 3-D TMA box of packed NVFP4 octet blocks per K stage (the two
+//                tiles of a "pair"), into a shared-memory ring;
 //   warps 1, 3   MMA issuers (one per tile of the pair): tcgen05.mma kind::f16, A from TMEM,
 //                B from shared memory, FP32 accumulators in TMEM; warp 1 owns the TMEM allocation;
 //   warp 2       activation gather: cp.async of the token rows of the tile (through the
@@ -118,7 +118,8 @@ struct PhaseParams {
 };
 
 struct GemmParams {
-  CUtensorMap tmap_act[2];   // TMA_B only, per phase: [rows, K] f16, box 64 x N, 128-byte swizzle (64-byte aligned: first member)
+  CUtensorMap tmap_w[2];     // packed weights, per phase: a K stage of a pair as one 3-D box (64-byte aligned: first members)
+  CUtensorMap tmap_act[2];   // TMA_B only, per phase: [rows, K] f16, box 64 x N, 128-byte swizzle
   PhaseParams ph[2];         // [0] gate/up, [1] down; a single-phase launch uses its own entry only
   const __nv_bfloat16* post_norm_w;  // phase 1, nullable
   int32_t* cnt;              // [local_count]      sort tables in global memory: read here, or written by CTA 0
@@ -468,6 +469,25 @@ __device__ __forceinline__ bool grid_counter_wait(const unsigned int* ctr, unsig
   }
 }
 
+// The same without sleeping between the polls: for a single waiting warp per SM whose wake-up is on the critical
+// path of the step.
+__device__ __forceinline__ bool grid_counter_spin(const unsigned int* ctr, unsigned int target, volatile int* abort_word) {
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t polls = 0;
+  while (true) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+    if (v >= target) return true;
+    if ((++polls & 63u) == 0u) {
+      if (*abort_word != 0) return false;
+      if (globaltimer_ns() - t0 > MSK_WAIT_LIMIT_NS) {
+        *abort_word = 1;
+        return false;
+      }
+    }
+  }
+}
+
 template <int N, int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_constant__ GemmParams p) {
   using C = GemmCfg<N>;
@@ -514,6 +534,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     ctl.last_flag[0] = ctl.last_flag[1] = 0;
     ctl.fin_n = 0;
     fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&p.tmap_w[PH_FIRST]);
+    if (TMA_B) prefetch_tensormap(&p.tmap_act[PH_FIRST]);
   }
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, TMEM_COLS);

@@ -10,6 +10,7 @@
     const int g = (didx >> 2) & 1;
     const int kh = didx >> 3;
     const int row = (warp & 3) * 32 + lane;
+    const uint32_t row_off = static_cast<uint32_t>((2 * (row >> 3) + g) * OCT_BYTES + (row & 7) * 16);
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t a_tmem = tmem + lane_base + C::A_BASE + g * C::A_GROUP_COLS;
     uint32_t it = 0;
@@ -68,12 +69,11 @@
           if (!MSK_WAIT(&ctl.raw_full[slot], par, abortw)) { ok = false; break; }
           if (it == 0 && tid == 256) MSK_TR(TR_FIRST_RAW);
           if (lane == 0 && (didx == 0 || didx == 15)) MSK_TRD(didx ? 5 : 0, tri, 5);
-          const uint32_t tile = smem_u32(ring + slot * C::STAGE_BYTES + g * TILE_BYTES);
-          const uint32_t tile_row = tile + row * 16;
+          const uint32_t tile_row = smem_u32(ring + slot * C::STAGE_BYTES) + row_off;   // this row in its octet block
           uint32_t sfa[4];
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(sfa[0]), "=r"(sfa[1]), "=r"(sfa[2]), "=r"(sfa[3])
-                       : "r"(tile + TILE_CODE_BYTES + row * 16));
+                       : "r"(tile_row + OCT_CODE_BYTES));
           {
             // this warp's slot of the stage: K half kh = chunks 4*kh .. 4*kh+3
 #pragma unroll
@@ -82,7 +82,7 @@
               uint32_t q[4];
               asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                            : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
-                           : "r"(tile_row + chunk * 2048));
+                           : "r"(tile_row + chunk * 128));
               const uint32_t sfw = kh ? (c < 2 ? sfa[2] : sfa[3]) : (c < 2 ? sfa[0] : sfa[1]);
               uint32_t o[16];
               decode_chunk(q, (c & 1) ? (sfw >> 16) : sfw, o);

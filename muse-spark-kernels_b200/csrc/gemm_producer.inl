@@ -1,6 +1,6 @@
 // Role body of moe_gemm_kernel (included inside the kernel): weight producer, warp 0.
 // One lane streams the two packed tiles of every K stage of every piece of this CTA into the
-// shared-memory ring with 1-D bulk async copies that complete on the stage's mbarrier. With both
+// shared-memory ring, one 3-D box (layout.cuh) per stage that completes on the stage's mbarrier. With both
 // phases in one launch the stream runs on from the last gate/up stage into the first down stage.
 //
 // The ring is the only look-ahead. Asking L2 for stages further ahead (cp.async.bulk.prefetch.L2 from
@@ -19,10 +19,7 @@
         MSK_PHASE_SETUP;
         while (ok && pieces.next(base, ks0, ks1)) {
           const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
-          const size_t tile0 =
-              (static_cast<size_t>(ui.expert) * (2 * pp.n_pairs) + 2 * ui.pair) * static_cast<size_t>(nst_total);
-          const uint8_t* g0 = pp.w + tile0 * TILE_BYTES;
-          const uint8_t* g1 = g0 + static_cast<size_t>(nst_total) * TILE_BYTES;
+          const int oct0 = (ui.expert * pp.n_pairs + ui.pair) * TILE_OCTETS;   // first octet of the pair
           for (int ks = ks0; ks < ks1; ++ks, ++it) {
             const uint32_t slot = it % NST, par = (it / NST) & 1u;
 #ifdef MSK_TRACE_DETAIL
@@ -31,8 +28,7 @@
             if (!MSK_WAIT(&ctl.raw_empty[slot], par ^ 1u, abortw)) { ok = false; break; }
             uint8_t* dst = ring + slot * C::STAGE_BYTES;
             mbar_arrive_expect_tx(&ctl.raw_full[slot], 2 * TILE_BYTES);
-            bulk_g2s(dst, g0 + static_cast<size_t>(ks) * TILE_BYTES, TILE_BYTES, &ctl.raw_full[slot], pol);
-            bulk_g2s(dst + TILE_BYTES, g1 + static_cast<size_t>(ks) * TILE_BYTES, TILE_BYTES, &ctl.raw_full[slot], pol);
+            tma_load_3d(dst, &p.tmap_w[phase], 0, 2 * ks, oct0, &ctl.raw_full[slot], pol);
             if (it == 0) MSK_TR(TR_FIRST_BULK);
             if (TMA_B) {
               // activation tile of the stage: four boxes of 64 K x N rows, rows row0.. of the sorted matrix.
@@ -65,10 +61,9 @@
         int left = NST + 1, b2, k0, k1;
         while (left > 0 && pi.next(b2, k0, k1)) {
           const UnitInfo u2 = decode_unit(b2, tile_start, nx.n_pairs, p.nloc, N);
-          const size_t t0 = (static_cast<size_t>(u2.expert) * (2 * nx.n_pairs) + 2 * u2.pair) * static_cast<size_t>(nst2);
+          const int oct0 = (u2.expert * nx.n_pairs + u2.pair) * TILE_OCTETS;
           const int take = min(left, k1 - k0);
-          prefetch_l2(nx.w + (t0 + k0) * TILE_BYTES, static_cast<uint32_t>(take) * TILE_BYTES);
-          prefetch_l2(nx.w + (t0 + nst2 + k0) * TILE_BYTES, static_cast<uint32_t>(take) * TILE_BYTES);
+          for (int j = 0; j < take; ++j) tma_prefetch_3d(&p.tmap_w[1], 0, 2 * (k0 + j), oct0);
           left -= take;
         }
       }

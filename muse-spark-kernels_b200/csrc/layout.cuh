@@ -1,12 +1,21 @@
 // Packed NVFP4 tile layout and the in-register decode that goes with it.
 //
-// One tile = 128 weight rows x 256 K (one K stage):
-//   bytes [0, 16384)      codes: 16-byte chunk c (0..7) of row r at (c*128 + r)*16; a chunk
-//                         holds K [32c, 32c+32) of the stage, two E2M1 codes per byte in the
-//                         source order (low nibble = even k);
-//   bytes [16384, 18432)  scales: row r's sixteen E4M3 bytes at 16384 + r*16, byte j = block j.
-// Thread r of a 128-thread group owns row r, so every 16-byte shared-memory read of a
-// quarter-warp is 128 contiguous bytes. The repack is a pure byte permutation.
+// The unit of the layout is the octet block: 8 weight rows x 256 K, 1152 bytes:
+//   bytes [0, 1024)     codes: 16-byte chunk c (0..7) of row r (0..7) at c*128 + r*16; a chunk holds
+//                       K [32c, 32c+32) of the block, two E2M1 codes per byte in the source order (low
+//                       nibble = even k);
+//   bytes [1024, 1152)  scales: row r's sixteen E4M3 bytes at 1024 + r*16, byte j = 16-element block j.
+// Blocks lie in memory as [expert][pair j][octet o 0..15][K block ks][gu 0..1]: pair j is the two 128-row
+// tiles that share a unit of work (gate tile j and up tile j of w13; row tiles 2j and 2j+1 of w2), and block
+// (o, gu) holds rows 8o .. 8o+7 of tile gu. Two shapes of access are contiguous enough for one copy each:
+//   * a K stage of a pair (256 rows x 256 K): the 32 blocks of one ks, a 3-D box {1152 bytes, 2, 16};
+//   * a row slice (8 + 8 rows, any run of K blocks): the blocks of one octet follow one another.
+// What matters is the number of copies: measured on B200 (148 CTAs, ring of 36,864-byte stages) boxes stream
+// at 7.09 TB/s, contiguous stages at 7.12, the same stage as 32 separate copies of 1152 bytes at 5.5.
+// A thread that owns a weight row reads 16-byte chunks: the eight rows of a quarter-warp are 128
+// contiguous bytes; a warp that reads the four-byte words of a chunk for an mma.sync operand (lane =
+// row * 4 + word) reads the same 128 bytes. Neither has bank conflicts. The repack is a pure byte
+// permutation.
 //
 // Decode (per 16-byte chunk: 32 codes, two scale blocks): the hardware converts
 //   cvt.rn.f16x2.e2m1x2  one byte  -> two F16 code values {0, .5, 1, 1.5, 2, 3, 4, 6} (signed)
@@ -31,9 +40,11 @@ namespace msk {
 
 constexpr int KS = 256;                                   // K elements per stage
 constexpr int TILE_ROWS = 128;                            // weight rows per tile (= MMA M)
-constexpr int TILE_CODE_BYTES = TILE_ROWS * KS / 2;       // 16384
-constexpr int TILE_SF_BYTES = TILE_ROWS * KS / 16;        // 2048
-constexpr int TILE_BYTES = TILE_CODE_BYTES + TILE_SF_BYTES;  // 18432
+constexpr int OCT_ROWS = 8;                               // rows of an octet block
+constexpr int OCT_CODE_BYTES = OCT_ROWS * KS / 2;         // 1024
+constexpr int OCT_BYTES = OCT_CODE_BYTES + OCT_ROWS * KS / 16;  // 1152
+constexpr int TILE_OCTETS = TILE_ROWS / OCT_ROWS;         // 16
+constexpr int TILE_BYTES = TILE_OCTETS * OCT_BYTES;       // 18432: the bytes of one tile in a K stage
 
 #ifdef __CUDACC__
 // One chunk: four words (32 codes) and the low 16 bits of `sf2` (the scale bytes of its two

@@ -13,75 +13,95 @@
 #include "../../include/msk_moe.h"
 #include "route_sort.cuh"
 #include "gemm.cuh"
+#include "few.cuh"
 #include "router_gemm.cuh"
 
 namespace msk {
 
 // ------------------------------------------------------------ repack kernels
-// Tile order inside a packed buffer: ((expert * tiles_per_expert) + row_tile') * n_stages + ks,
-// where for w13 row_tile' = 2*j + (0 gate | 1 up) and the source rows are gu*I + j*128 + r;
-// for w2 row_tile' = row tile and the source rows are row_tile*128 + r.
+// Octet blocks (layout.cuh) in the order [expert][pair][octet][ks][gu]. Source rows of block (pair j,
+// octet o, gu): w13 gu*I + j*128 + o*8 .. +7, w2 (2j + gu)*128 + o*8 .. +7.
 struct RepackGeom {
   int rows_total;       // source rows per expert (2I or H)
   int K;                // source K
-  int tiles_per_expert; // rows_total / 128
+  int n_pairs;          // rows_total / 256
   int n_stages;         // K / 256
-  int interleave_I;     // I for w13 (gate/up interleave), 0 for w2
+  int interleave_I;     // I for w13 (gate tile j with up tile j), 0 for w2 (row tiles 2j and 2j + 1)
 };
 
-__device__ __forceinline__ int source_row(const RepackGeom& g, int tile_in_expert, int r) {
-  if (g.interleave_I > 0) {
-    const int j = tile_in_expert >> 1, gu = tile_in_expert & 1;
-    return gu * g.interleave_I + j * 128 + r;
-  }
-  return tile_in_expert * 128 + r;
+// First source row (over all experts) of octet-gu number og = ((expert * n_pairs + pair) * 16 + o) * 2 + gu.
+__device__ __forceinline__ long long source_row(const RepackGeom& g, long long og) {
+  const int gu = static_cast<int>(og & 1), o = static_cast<int>((og >> 1) & 15);
+  const long long ep = og >> 5;
+  const int pair = static_cast<int>(ep % g.n_pairs);
+  const long long e = ep / g.n_pairs;
+  const int row = g.interleave_I > 0 ? gu * g.interleave_I + pair * 128 + o * OCT_ROWS
+                                     : (2 * pair + gu) * 128 + o * OCT_ROWS;
+  return e * g.rows_total + row;
 }
 
-// One thread per 16 output bytes (a code chunk or a row's scale bytes).
+// One warp per (octet, gu): 8 source rows of K/2 code bytes and K/16 scale bytes. Bound by memory: both sides
+// move whole 32-byte sectors. Lane = (row r, 16-byte piece c of four): a warp reads 64 contiguous bytes of
+// each of the eight rows and writes four full 128-byte lines, eight such steps (4 KB) in flight. The form
+// this replaces gave each thread one 16-byte piece with the rows running along the lanes (16 useful bytes
+// of every 32-byte sector on the source side): 128 experts of 4096 x 1536, both matrices, 535 us in and
+// 722 us back out.
 template <bool INVERSE>
 __global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf, uint8_t* packed, RepackGeom g,
-                                                     long long n_tiles) {
-  const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const long long per_tile = 128 * 9;  // 8 code chunks + 1 scale chunk per row
-  if (gid >= n_tiles * per_tile) return;
-  const long long tile = gid / per_tile;
-  const int rem = static_cast<int>(gid % per_tile);
-  const int part = rem / 128, r = rem % 128;  // part 0..7 = code chunk, 8 = scales
-  const int ks = static_cast<int>(tile % g.n_stages);
-  const long long t2 = tile / g.n_stages;
-  const int tile_in_expert = static_cast<int>(t2 % g.tiles_per_expert);
-  const long long e = t2 / g.tiles_per_expert;
-  const long long srow = e * g.rows_total + source_row(g, tile_in_expert, r);
-  uint8_t* ptile = packed + tile * TILE_BYTES;
-  if (part < 8) {
-    uint4* src = reinterpret_cast<uint4*>(codes + srow * (g.K / 2) + ks * (KS / 2) + part * 16);
-    uint4* dst = reinterpret_cast<uint4*>(ptile + (part * 128 + r) * 16);
-    if (!INVERSE) *dst = *src; else *src = *dst;
-  } else {
-    uint4* src = reinterpret_cast<uint4*>(sf + srow * (g.K / 16) + ks * (KS / 16));
-    uint4* dst = reinterpret_cast<uint4*>(ptile + TILE_CODE_BYTES + r * 16);
-    if (!INVERSE) *dst = *src; else *src = *dst;
+                                                     long long n_og) {
+  const long long og = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (og >= n_og) return;
+  const int lane = threadIdx.x & 31, r = lane >> 2, c4 = lane & 3;
+  const long long srow = source_row(g, og) + r;
+  uint8_t* block = packed + ((og >> 1) * g.n_stages * 2 + (og & 1)) * OCT_BYTES;   // K block 0; the next one 2 * OCT_BYTES on
+  {
+    uint4* src = reinterpret_cast<uint4*>(codes + srow * (g.K / 2)) + c4;
+    // chunk i*4 + c4 of the row: K block (i*4 + c4) / 8, chunk (i*4 + c4) % 8 inside it
+    uint4* dst = reinterpret_cast<uint4*>(block + c4 * 128 + r * 16);
+    const int n = g.n_stages * 2;                       // steps of four chunks (128 K)
+    for (int i0 = 0; i0 < n; i0 += 8) {
+      uint4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j;
+        if (i < n) {
+          const size_t at = static_cast<size_t>(i >> 1) * (2 * OCT_BYTES / 16) + (i & 1) * 32;
+          v[j] = INVERSE ? __ldcs(dst + at) : __ldcs(src + i * 4);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j;
+        if (i < n) {
+          const size_t at = static_cast<size_t>(i >> 1) * (2 * OCT_BYTES / 16) + (i & 1) * 32;
+          if (INVERSE) __stcs(src + i * 4, v[j]); else __stcs(dst + at, v[j]);
+        }
+      }
+    }
+  }
+  uint4* src = reinterpret_cast<uint4*>(sf + srow * (g.K / 16));
+  uint4* dst = reinterpret_cast<uint4*>(block + OCT_CODE_BYTES + r * 16);
+  for (int ks = c4; ks < g.n_stages; ks += 4) {
+    if (INVERSE) __stcs(src + ks, __ldcs(dst + ks * (2 * OCT_BYTES / 16)));
+    else __stcs(dst + ks * (2 * OCT_BYTES / 16), __ldcs(src + ks));
   }
 }
 
 // Packed tiles -> BF16 e2m1*e4m3 matrices, through the decode routine of the GEMM kernel (the
 // F16 products are exact and convert to BF16 without rounding).
 __global__ void __launch_bounds__(128) dequant_packed_kernel(const uint8_t* packed, __nv_bfloat16* out, RepackGeom g,
-                                                             long long n_tiles) {
-  const long long tile = blockIdx.x;
-  if (tile >= n_tiles) return;
-  const int r = threadIdx.x;
-  const int ks = static_cast<int>(tile % g.n_stages);
-  const long long t2 = tile / g.n_stages;
-  const int tile_in_expert = static_cast<int>(t2 % g.tiles_per_expert);
-  const long long e = t2 / g.tiles_per_expert;
-  const long long srow = e * g.rows_total + source_row(g, tile_in_expert, r);
-  const uint8_t* ptile = packed + tile * TILE_BYTES;
-  const uint4 sfw = *reinterpret_cast<const uint4*>(ptile + TILE_CODE_BYTES + r * 16);
+                                                             long long n_og) {
+  // a block per 16 octet-gus of one K block: thread = (octet-gu, row)
+  const int ks = static_cast<int>(blockIdx.x % g.n_stages);
+  const long long og = (blockIdx.x / g.n_stages) * 16 + (threadIdx.x >> 3);
+  if (og >= n_og) return;
+  const int r = threadIdx.x & 7;
+  const uint8_t* block = packed + ((og >> 1) * g.n_stages * 2 + ks * 2 + (og & 1)) * OCT_BYTES;
+  const uint4 sfw = *reinterpret_cast<const uint4*>(block + OCT_CODE_BYTES + r * 16);
   const uint32_t sfa[4] = {sfw.x, sfw.y, sfw.z, sfw.w};
-  __nv_bfloat16* orow = out + srow * g.K + ks * KS;
+  __nv_bfloat16* orow = out + (source_row(g, og) + r) * g.K + ks * KS;
   for (int chunk = 0; chunk < 8; ++chunk) {
-    const uint4 qv = *reinterpret_cast<const uint4*>(ptile + (chunk * 128 + r) * 16);
+    const uint4 qv = *reinterpret_cast<const uint4*>(block + chunk * 128 + r * 16);
     const uint32_t q[4] = {qv.x, qv.y, qv.z, qv.w};
     const uint32_t sw = sfa[chunk >> 1] >> ((chunk & 1) * 16);
     uint32_t o[16];
@@ -642,8 +662,8 @@ typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint3
                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static int encode_act_map(CUtensorMap* map, const void* base, size_t rows, int K, int box_rows,
-                          CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_FLOAT16) {
+static int encode_map(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const void* base, const cuuint64_t* dims,
+                      const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
   static TensorMapEncodeFn fn = nullptr;
   if (fn == nullptr) {
     void* ptr = nullptr;
@@ -653,14 +673,19 @@ static int encode_act_map(CUtensorMap* map, const void* base, size_t rows, int K
     if (qres != cudaDriverEntryPointSuccess || ptr == nullptr) return static_cast<int>(cudaErrorNotSupported);
     fn = reinterpret_cast<TensorMapEncodeFn>(ptr);
   }
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  const CUresult r = fn(map, dtype, static_cast<cuuint32_t>(rank), const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(cudaErrorInvalidValue);
+}
+
+static int encode_act_map(CUtensorMap* map, const void* base, size_t rows, int K, int box_rows,
+                          CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_FLOAT16) {
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
   const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t estr[2] = {1u, 1u};
-  const CUresult r = fn(map, dtype, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : static_cast<int>(cudaErrorInvalidValue);
+  return encode_map(map, dtype, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // Experiment switch (environment variable MSK_FUSED_PLAIN): launch the one-launch kernel without the
@@ -723,14 +748,101 @@ static int launch_gemm_fused(int N, const GemmParams& p, int grid, cudaStream_t 
   }
 }
 
+// ---- the few-token kernel (few.cuh): shapes it takes, its shared memory and its dealing of work
+struct FewPlan {
+  int n_slots, slot_kb, part_bytes, n_light, w_light, w_heavy;
+  int xb_off, ys_off, part_off, ctl_off, smem;
+};
+
+// Tokens up to which the few-token kernel is the faster one (H4096 I1536 E128 top-8, us inside the launch, against
+// the tcgen05 kernel): 1 token 28 / 40, 2: 44 / 43 (but 7 us less outside it), 3: 53 / 52, 4: 71 / 65, 8: 121 / 108:
+// from four tokens on the decode work in its warps sets the pace, not the latencies it saves. With the pre-expert
+// norm the alternative is three launches, and the line lies higher.
+constexpr int FEW_BEST_TOKENS = 3, FEW_BEST_TOKENS_PRENORM = 6;
+
+// False when the step does not fit: more than eight tokens, or token rows and owned output rows that leave
+// less than two K blocks per warp (74 KB in flight per SM).
+static bool few_plan(const MskMoeCfg* c, int T, bool given_ids, int grid, FewPlan* f) {
+  if (T > FEW_TOKENS || T * c->top_k > FEW_ENTRIES) return false;
+  const int groups = c->hidden / (2 * OCT_ROWS), own = (groups + grid - 1) / grid;
+  const int x_bytes = T * (c->hidden * 2 + 64), ys_bytes = T * c->top_k * own * 64;
+  // rows of a tile: one per token when the top-k is taken here; given ids may repeat an expert
+  f->part_bytes = 128 * ((std::min(FEW_TOKENS, given_ids ? T * c->top_k : T) + 1) / 2);
+  const int parts = FEW_WARPS * 2 * f->part_bytes;
+  const int left = 227 * 1024 - x_bytes - ys_bytes - parts - static_cast<int>(sizeof(FewCtl));
+  const int ring_kb = left < 0 ? 0 : left / (FEW_WARPS * FEW_KB_BYTES);   // K blocks a warp's ring can hold
+  if (ring_kb < 2) return false;
+  f->slot_kb = ring_kb >= 4 ? 2 : 1;
+  f->n_slots = ring_kb >= 4 ? 2 : ring_kb;
+  f->xb_off = FEW_WARPS * f->n_slots * f->slot_kb * FEW_KB_BYTES;
+  f->ys_off = f->xb_off + x_bytes;
+  f->part_off = f->ys_off + ys_bytes;
+  f->ctl_off = f->part_off + parts;
+  f->smem = f->ctl_off + static_cast<int>(sizeof(FewCtl));
+  // gate/up units per super-round: a CTA with one group more of output rows streams that many bytes less of
+  // gate/up weights; the smallest pair of weights within 4 % of that ratio
+  const int extra = groups % grid;
+  f->n_light = extra == 0 ? grid : grid - extra;
+  f->w_light = f->w_heavy = 1;
+  // (one token has few units per team, and they go round the teams evenly only when every CTA has as many)
+  if (T == 1) {
+    f->n_light = grid;
+  } else if (extra != 0) {
+    const double unit = 2.0 * (c->hidden / KS), group = 2.0 * (c->inter / KS), per_cta = (c->inter / 8 * unit + groups * group) / grid;
+    const double light = per_cta - (groups / grid) * group, heavy = per_cta - own * group;
+    if (heavy <= 0.1 * light) {
+      f->w_heavy = 0;
+    } else {
+      for (int wh = 1; wh <= 6; ++wh) {
+        const int wl = static_cast<int>(light / heavy * wh + 0.5);
+        f->w_light = wl;
+        f->w_heavy = wh;
+        if (std::fabs(wl * heavy / (wh * light) - 1.0) <= 0.04) break;
+      }
+    }
+  }
+  return true;
+}
+
+static int launch_few(const FewParams& p, int grid, int smem, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(moe_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    attr_set[dev] = true;
+  }
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(static_cast<unsigned>(grid));
+  lc.blockDim = dim3(FEW_THREADS);
+  lc.dynamicSmemBytes = static_cast<size_t>(smem);
+  lc.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;   // its CTAs wait for one another: all resident, or the launch fails
+  at[0].val.cooperative = fused_plain_launch() ? 0 : 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&lc, moe_few_kernel, p));
+}
+
 static RepackGeom geom13(const MskMoeCfg* c) {
-  return RepackGeom{2 * c->inter, c->hidden, 2 * c->inter / 128, c->hidden / KS, c->inter};
+  return RepackGeom{2 * c->inter, c->hidden, c->inter / 128, c->hidden / KS, c->inter};
 }
 static RepackGeom geom2(const MskMoeCfg* c) {
-  return RepackGeom{c->hidden, c->inter, c->hidden / 128, c->inter / KS, 0};
+  return RepackGeom{c->hidden, c->inter, c->hidden / 256, c->inter / KS, 0};
 }
-static long long n_tiles_of(const MskMoeCfg* c, const RepackGeom& g) {
-  return static_cast<long long>(c->local_count) * g.tiles_per_expert * g.n_stages;
+static long long n_og_of(const MskMoeCfg* c, const RepackGeom& g) {   // octet-gus: 8-row slices of all experts
+  return static_cast<long long>(c->local_count) * g.n_pairs * 2 * TILE_OCTETS;
+}
+
+// Tensor maps of the packed weights: 8-byte elements, [block 144][K blocks * 2][octets of all experts], box
+// {144, 2, 16} = the 36,864 bytes of one K stage of a pair.
+static int encode_weight_map(CUtensorMap* map, const MskMoeCfg* c, const RepackGeom& g, const void* packed) {
+  const cuuint64_t dims[3] = {OCT_BYTES / 8, static_cast<cuuint64_t>(g.n_stages) * 2, static_cast<cuuint64_t>(n_og_of(c, g) / 2)};
+  const cuuint64_t strides[2] = {OCT_BYTES, static_cast<cuuint64_t>(g.n_stages) * 2 * OCT_BYTES};
+  const cuuint32_t box[3] = {OCT_BYTES / 8, 2, TILE_OCTETS};
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, packed, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 template <int N>
@@ -768,8 +880,8 @@ int msk_moe_packed_bytes(const MskMoeCfg* cfg, size_t* host_w13_bytes, size_t* h
   const int rc = check_cfg(cfg);
   if (rc != MSK_OK) return rc;
   if (host_w13_bytes == nullptr || host_w2_bytes == nullptr) return MSK_ERR_NULL;
-  *host_w13_bytes = static_cast<size_t>(n_tiles_of(cfg, geom13(cfg))) * TILE_BYTES;
-  *host_w2_bytes = static_cast<size_t>(n_tiles_of(cfg, geom2(cfg))) * TILE_BYTES;
+  *host_w13_bytes = static_cast<size_t>(n_og_of(cfg, geom13(cfg))) * (cfg->hidden / KS) * OCT_BYTES;
+  *host_w2_bytes = static_cast<size_t>(n_og_of(cfg, geom2(cfg))) * (cfg->inter / KS) * OCT_BYTES;
   return MSK_OK;
 }
 
@@ -783,9 +895,8 @@ static int repack_common(const MskMoeCfg* cfg, void* w13, void* w13_sf, void* w2
     return MSK_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const RepackGeom g13 = geom13(cfg), g2 = geom2(cfg);
-  const long long n13 = n_tiles_of(cfg, g13), n2 = n_tiles_of(cfg, g2);
-  const long long th13 = n13 * 128 * 9, th2 = n2 * 128 * 9;
-  const unsigned b13 = static_cast<unsigned>((th13 + 255) / 256), b2 = static_cast<unsigned>((th2 + 255) / 256);
+  const long long n13 = n_og_of(cfg, g13), n2 = n_og_of(cfg, g2);
+  const unsigned b13 = static_cast<unsigned>((n13 + 7) / 8), b2 = static_cast<unsigned>((n2 + 7) / 8);
   if (!inverse) {
     repack_kernel<false><<<b13, 256, 0, st>>>(static_cast<uint8_t*>(w13), static_cast<uint8_t*>(w13_sf),
                                               static_cast<uint8_t*>(packed13), g13, n13);
@@ -820,11 +931,11 @@ int msk_moe_dequant_packed(const MskMoeCfg* cfg, const void* packed13, const voi
   if (!aligned16(packed13) || !aligned16(packed2) || !aligned16(dq13) || !aligned16(dq2)) return MSK_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const RepackGeom g13 = geom13(cfg), g2 = geom2(cfg);
-  const long long n13 = n_tiles_of(cfg, g13), n2 = n_tiles_of(cfg, g2);
-  dequant_packed_kernel<<<static_cast<unsigned>(n13), 128, 0, st>>>(static_cast<const uint8_t*>(packed13),
-                                                                    static_cast<__nv_bfloat16*>(dq13), g13, n13);
-  dequant_packed_kernel<<<static_cast<unsigned>(n2), 128, 0, st>>>(static_cast<const uint8_t*>(packed2),
-                                                                   static_cast<__nv_bfloat16*>(dq2), g2, n2);
+  const long long n13 = n_og_of(cfg, g13), n2 = n_og_of(cfg, g2);
+  dequant_packed_kernel<<<static_cast<unsigned>(n13 / 16 * g13.n_stages), 128, 0, st>>>(
+      static_cast<const uint8_t*>(packed13), static_cast<__nv_bfloat16*>(dq13), g13, n13);
+  dequant_packed_kernel<<<static_cast<unsigned>(n2 / 16 * g2.n_stages), 128, 0, st>>>(
+      static_cast<const uint8_t*>(packed2), static_cast<__nv_bfloat16*>(dq2), g2, n2);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -835,9 +946,9 @@ int msk_moe_router_logits(const MskMoeCfg* cfg, const void* x, const float* rout
   if (!x || !router_w || !logits) return MSK_ERR_NULL;
   if (n_tokens < 0) return MSK_ERR_SHAPE;
   if (n_tokens == 0) return MSK_OK;
-  dim3 grid(static_cast<unsigned>(n_tokens), static_cast<unsigned>((cfg->n_experts + 7) / 8));
-  router_logits_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), router_w, logits, cfg->hidden, cfg->n_experts);
+  auto* kern = aligned16(x) && aligned16(router_w) ? router_logits_kernel<true> : router_logits_kernel<false>;
+  kern<<<static_cast<unsigned>(cfg->n_experts), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(x), router_w, logits, n_tokens, cfg->hidden, cfg->n_experts);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1060,6 +1171,34 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   p.evict_first = 1;
   p.post_norm_w = static_cast<const __nv_bfloat16*>(post_norm_w);
   p.eps = cfg->post_norm_eps;
+  FewPlan few;
+  if (plan.path == 0 && n_tokens <= (pre_norm_w != nullptr ? FEW_BEST_TOKENS_PRENORM : FEW_BEST_TOKENS) &&
+      few_plan(cfg, n_tokens, logits == nullptr, plan.grid, &few)) {
+    FewParams f{};
+    f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
+    f.gs13 = gs13; f.gs2 = gs2;
+    f.x = static_cast<const __nv_bfloat16*>(x);
+    f.pre_w = static_cast<const __nv_bfloat16*>(pre_norm_w); f.pre_eps = pre_norm_eps;
+    f.post_w = static_cast<const __nv_bfloat16*>(post_norm_w); f.post_eps = cfg->post_norm_eps;
+    f.xs = xs; f.inter = inter; f.y = y; f.out = static_cast<__nv_bfloat16*>(out);
+    f.logits = logits; f.bias = bias; f.ids_in = topk_ids; f.tw_in = topk_weights; f.ids_out = ids_out; f.tw_out = tw_out;
+    f.cnt = cnt; f.off = off; f.perm = perm; f.inv = inv; f.status = status;
+    f.ctl = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
+    f.tile_done = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4352);
+    f.norm_part = partial; f.trace = trace;
+    f.H = cfg->hidden; f.I = cfg->inter; f.T = n_tokens; f.E = cfg->n_experts; f.k = cfg->top_k;
+    f.lo = cfg->local_start; f.nloc = cfg->local_count; f.mode = cfg->routing_mode; f.route_scale = cfg->route_scale;
+    f.route = logits != nullptr ? 1 : 2;
+    f.share_x = cfg->host_inputs != 0 && pre_norm_w == nullptr ? 1 : 0;
+    f.inv_oct1 = static_cast<uint32_t>(((1ull << 32) + cfg->inter / 8 - 1) / (cfg->inter / 8));
+    f.n_slots = few.n_slots; f.slot_kb = few.slot_kb; f.part_bytes = few.part_bytes; f.part_off = few.part_off;
+    f.n_light = few.n_light; f.w_light = few.w_light; f.w_heavy = few.w_heavy;
+    f.xb_off = few.xb_off; f.ys_off = few.ys_off; f.ctl_off = few.ctl_off;
+    if (ev) { cudaEventRecord(ev[0], st); cudaEventRecord(ev[1], st); cudaEventRecord(ev[5], st); }
+    const int e = launch_few(f, plan.grid, few.smem, st);
+    if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); cudaEventRecord(ev[4], st); }
+    return e;
+  }
   PhaseParams& g13 = p.ph[0];
   PhaseParams& g2 = p.ph[1];
   g13.w = static_cast<const uint8_t*>(packed13); g13.gs = gs13; g13.act = xs; g13.outp = inter;
@@ -1069,6 +1208,11 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.partial = partial + round_up(partial_floats(cfg) * 4, 256) / 4;
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
+  {
+    int e = encode_weight_map(&p.tmap_w[0], cfg, geom13(cfg), packed13);
+    if (e == 0) e = encode_weight_map(&p.tmap_w[1], cfg, geom2(cfg), packed2);
+    if (e != 0) return e;
+  }
 
   if (plan.path != 1 && plan.path != 4) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
@@ -1423,6 +1567,9 @@ int msk_moe_forward_static(const MskMoeCfg* cfg, const void* packed13, const voi
   p.ph[0].K = cfg->hidden; p.ph[0].out_ld = cfg->inter; p.ph[0].n_pairs = cfg->inter / 128;
   p.ph[1].w = static_cast<const uint8_t*>(packed2); p.ph[1].gs = gs2; p.ph[1].act = inter; p.ph[1].outp = y;
   p.ph[1].K = cfg->inter; p.ph[1].out_ld = cfg->hidden; p.ph[1].n_pairs = cfg->hidden / 256;
+  e = encode_weight_map(&p.tmap_w[0], cfg, geom13(cfg), packed13);
+  if (e == 0) e = encode_weight_map(&p.tmap_w[1], cfg, geom2(cfg), packed2);
+  if (e != 0) return e;
   e = launch_gemm_n<0>(16, p, grid, st, 1);
   if (e != 0) return e;
   e = launch_gemm_n<1>(16, p, grid, st, 1);

