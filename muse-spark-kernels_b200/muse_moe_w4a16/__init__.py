@@ -13,6 +13,7 @@ py/03_kernel_fn.py:18-45). Extensions, all optional:
   pre_norm_w (bf16 [H]) may be present  -> the layer callers' pre-expert RMS norm is applied to x first
 There is no CPU path: tensors must be CUDA tensors and the native library must load.
 """
+import copy
 import ctypes
 
 import torch
@@ -208,52 +209,52 @@ def kernel_fn(data, state, return_routing=False, out=None):
           or tuple(out.shape) != (T, cfg.hidden)):
         raise RuntimeError("muse_moe_w4a16.kernel_fn: out must be a contiguous CUDA bfloat16 [T, H] tensor")
     logits = _logits(data, state, x, T)
-    if state.get("pre_norm_w") is not None:
-        # the layer callers' pre-expert RMS norm, fused into the kernel that copies the token rows
-        if logits is None:
-            ids = data["topk_ids"].to(torch.int32).contiguous()
-            tw = data["topk_weights"].to(torch.float32).contiguous()
-        else:
-            ids = torch.empty((T, cfg.top_k), dtype=torch.int32, device=x.device)
-            tw = torch.empty((T, cfg.top_k), dtype=torch.float32, device=x.device)
-        _lib.check(lib.msk_moe_forward_prenorm(ctypes.byref(cfg), _lib.ptr(state["packed13"]), _lib.ptr(state["packed2"]),
-                                               _lib.ptr(state["gs13"]), _lib.ptr(state["gs2"]),
-                                               _lib.ptr(state["post_norm_w"]), _lib.ptr(state["pre_norm_w"]),
-                                               ctypes.c_float(state["pre_norm_eps"]), _lib.ptr(x), _lib.ptr(logits),
-                                               _lib.ptr(state["route_bias"]), _lib.ptr(ids), _lib.ptr(tw), _lib.ptr(out),
-                                               _lib.ptr(state["workspace"]), state["workspace_bytes"], T, _stream()),
-                   "msk_moe_forward_prenorm")
-        return (out, ids, tw) if return_routing else out
     if logits is None:
         ids = data["topk_ids"].to(torch.int32).contiguous()
         tw = data["topk_weights"].to(torch.float32).contiguous()
-        _lib.check(lib.msk_moe_forward(ctypes.byref(cfg), _lib.ptr(state["packed13"]), _lib.ptr(state["packed2"]),
-                                       _lib.ptr(state["gs13"]), _lib.ptr(state["gs2"]), _lib.ptr(state["post_norm_w"]),
-                                       _lib.ptr(x), _lib.ptr(ids), _lib.ptr(tw), _lib.ptr(out),
-                                       _lib.ptr(state["workspace"]), state["workspace_bytes"], T, _stream()),
-                   "msk_moe_forward")
     else:
         ids = torch.empty((T, cfg.top_k), dtype=torch.int32, device=x.device)
         tw = torch.empty((T, cfg.top_k), dtype=torch.float32, device=x.device)
-        _lib.check(lib.msk_moe_forward_logits(ctypes.byref(cfg), _lib.ptr(state["packed13"]), _lib.ptr(state["packed2"]),
-                                              _lib.ptr(state["gs13"]), _lib.ptr(state["gs2"]),
-                                              _lib.ptr(state["post_norm_w"]), _lib.ptr(x), _lib.ptr(logits),
-                                              _lib.ptr(state["route_bias"]), _lib.ptr(ids), _lib.ptr(tw), _lib.ptr(out),
-                                              _lib.ptr(state["workspace"]), state["workspace_bytes"], T, _stream()),
-                   "msk_moe_forward_logits")
+    _forward(state, cfg, lib, x.data_ptr(), None if logits is None else logits.data_ptr(), ids.data_ptr(), tw.data_ptr(),
+             out.data_ptr(), T)
     if return_routing:
         return out, ids, tw
     return out
 
 
+def _addr(t):
+    return None if t is None else t.data_ptr()
+
+
+def _forward(state, cfg, lib, x, logits, ids, tw, out, T):
+    """The library call of a step, on addresses. ctypes takes plain integers for pointers; building a
+    c_void_p for each of them cost a third of the call."""
+    st = torch._C._cuda_getCurrentRawStream(state["packed13"].device.index)
+    ref, ws = ctypes.byref(cfg), state["workspace"].data_ptr()
+    w13, w2, gs13, gs2 = state["packed13"].data_ptr(), state["packed2"].data_ptr(), state["gs13"].data_ptr(), state["gs2"].data_ptr()
+    post, bias, pre = _addr(state["post_norm_w"]), _addr(state["route_bias"]), state.get("pre_norm_w")
+    if pre is not None:   # the layer callers' pre-expert RMS norm, fused into the kernel that reads the token rows
+        rc = lib.msk_moe_forward_prenorm(ref, w13, w2, gs13, gs2, post, pre.data_ptr(), state["pre_norm_eps"], x, logits, bias,
+                                         ids, tw, out, ws, state["workspace_bytes"], T, st)
+    elif logits is None:
+        rc = lib.msk_moe_forward(ref, w13, w2, gs13, gs2, post, x, ids, tw, out, ws, state["workspace_bytes"], T, st)
+    else:
+        rc = lib.msk_moe_forward_logits(ref, w13, w2, gs13, gs2, post, x, logits, bias, ids, tw, out, ws,
+                                        state["workspace_bytes"], T, st)
+    if rc != 0:
+        _lib.check(rc, "msk_moe_forward")
+
+
 class GraphedStep:
     """kernel_fn for a fixed token count, captured once into a CUDA graph over static device buffers
-    (how the decode layer consumes the module: its steps are graph replays). Calling it copies the
-    inputs into the static buffers, replays the graph on the current stream and returns the static
-    output tensor, which the next call overwrites. Device inputs are copied tensor by tensor; host
-    inputs are first packed into one pinned staging block (a ring of them, each guarded by an
-    event) so that they reach the device in a single asynchronous copy. Inputs: hidden_states and
-    either router_logits or topk_ids + topk_weights, whichever `like` holds."""
+    (how the decode layer consumes the module: its steps are graph replays). Calling it runs the step on
+    the current stream and returns the static output tensor, which the next call overwrites. Host inputs
+    are first packed into one pinned staging block (a ring of them, each guarded by an event) so that
+    they reach the device in a single asynchronous copy, and the graph is replayed. Device inputs of the
+    types the kernels read are used where they lie: the step's launches are issued on them directly,
+    because copying them into the static buffers first put two copies and their gaps (8 us) in front of a
+    one-token step of 30; others are copied tensor by tensor and the graph is replayed. Inputs:
+    hidden_states and either router_logits or topk_ids + topk_weights, whichever `like` holds."""
 
     STAGES = 4
 
@@ -275,6 +276,13 @@ class GraphedStep:
         self.turn = 0
         for k in self.keys:
             self.static[k].copy_(like[k])
+        self.T = like["hidden_states"].shape[0]
+        self.shapes = {k: self.static[k].shape for k in self.keys}
+        self.routed = "topk_ids" in self.keys
+        self.direct = self.routed or "router_logits" in self.keys
+        k = state["cfg"].top_k
+        self.ids = torch.empty((self.T, k), dtype=torch.int32, device=dev)
+        self.tw = torch.empty((self.T, k), dtype=torch.float32, device=dev)
         side = torch.cuda.Stream(dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):                      # warm-up outside the capture
@@ -284,7 +292,29 @@ class GraphedStep:
         with torch.cuda.graph(self.graph):
             self.out = kernel_fn(self.static, state)
 
+    _READ_AS = {"hidden_states": torch.bfloat16, "router_logits": torch.float32, "topk_ids": torch.int32,
+                "topk_weights": torch.float32}
+
+    def _usable(self, data):
+        """Device tensors that the kernels can read as they are (aligned rows on this device)."""
+        dev = self.out.device
+        for k in self.keys:
+            t = data[k]
+            if (t.device != dev or t.dtype != self._READ_AS[k] or t.shape != self.shapes[k] or not t.is_contiguous()
+                    or t.data_ptr() % 16):
+                return False
+        return True
+
     def __call__(self, data):
+        if self.direct and self._usable(data):
+            state = self.state
+            if self.routed:
+                logits, ids, tw = None, data["topk_ids"].data_ptr(), data["topk_weights"].data_ptr()
+            else:
+                logits, ids, tw = data["router_logits"].data_ptr(), self.ids.data_ptr(), self.tw.data_ptr()
+            _forward(state, state["cfg"], state["lib"].lib, data["hidden_states"].data_ptr(), logits, ids, tw,
+                     self.out.data_ptr(), self.T)
+            return self.out
         if all(not data[k].is_cuda for k in self.keys):
             i = self.turn
             self.turn = (i + 1) % self.STAGES
@@ -325,7 +355,8 @@ class HostMappedStep:
 
     def __init__(self, state, like):
         self.state = state
-        cfg = state["cfg"]
+        cfg = self.cfg = copy.deepcopy(state["cfg"])
+        cfg.host_inputs = 1
         dev = state["packed13"].device
         if state.get("pre_norm_w") is not None:
             raise RuntimeError("HostMappedStep: states with a pre-expert norm are not supported")
@@ -365,7 +396,7 @@ class HostMappedStep:
 
     def _launch(self, i):
         state, inp = self.state, self.inputs[i]
-        cfg, lib = state["cfg"], state["lib"].lib
+        cfg, lib = self.cfg, state["lib"].lib
         args = (ctypes.byref(cfg), _lib.ptr(state["packed13"]), _lib.ptr(state["packed2"]), _lib.ptr(state["gs13"]),
                 _lib.ptr(state["gs2"]), _lib.ptr(state["post_norm_w"]), _lib.ptr(inp["hidden_states"]))
         tail = (_lib.ptr(self.outs[i]), _lib.ptr(state["workspace"]), state["workspace_bytes"], self.T, _stream())
