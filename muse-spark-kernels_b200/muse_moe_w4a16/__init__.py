@@ -115,6 +115,17 @@ def _make_state(cfg, packed13, packed2, gs13, gs2, post_norm_w, pre_norm_w, pre_
     }
 
 
+# Order of the packed weights in a saved state. States saved before the number was kept hold tiles of 128 rows x
+# 256 K ([expert][tile][K block][8 chunks of codes, then the scales][row][16 bytes]); 2 is the octet blocks that the
+# kernels read now.
+PACKED_LAYOUT = 2
+
+
+def _octet_blocks(tiles, cfg, K):
+    """Packed weights of a state saved in 128-row tiles, in the order of the octet blocks (a byte permutation)."""
+    return tiles.view(cfg.local_count, -1, 2, K // 256, 9, 16, 8, 16).permute(0, 1, 5, 3, 2, 4, 6, 7).reshape(-1)
+
+
 _SD_TENSORS = ("packed13", "packed2", "gs13", "gs2", "post_norm_w", "pre_norm_w", "router", "route_bias")
 
 
@@ -127,12 +138,14 @@ def state_dict(state):
     sd = {k: state[k] for k in _SD_TENSORS if state.get(k) is not None}
     sd["config"] = {name: getattr(cfg, name) for name, _ in MskMoeCfg._fields_}
     sd["pre_norm_eps"] = state["pre_norm_eps"]
+    sd["packed_layout"] = PACKED_LAYOUT
     return sd
 
 
 def load_state_dict(sd, device=None):
     """Inverse of state_dict: a ready state on `device` (default: where the tensors are). No repack runs;
-    the packed tiles are taken as they are, so kernel_fn gives the same bits as on the state they came from."""
+    the packed weights are taken as they are (those saved in another order are put in order first), so kernel_fn
+    gives the same bits as on the state they came from."""
     lib = _lib.load()
     cfg = MskMoeCfg(**sd["config"])
     t = {k: (sd[k] if device is None else sd[k].to(device)) for k in _SD_TENSORS if sd.get(k) is not None}
@@ -142,6 +155,12 @@ def load_state_dict(sd, device=None):
     _lib.check(lib.msk_moe_packed_bytes(ctypes.byref(cfg), ctypes.byref(b13), ctypes.byref(b2)), "msk_moe_packed_bytes")
     if t["packed13"].numel() != b13.value or t["packed2"].numel() != b2.value:
         raise RuntimeError("muse_moe_w4a16.load_state_dict: packed weights do not match the configuration")
+    layout = sd.get("packed_layout", 1)
+    if layout not in (1, PACKED_LAYOUT):
+        raise RuntimeError("muse_moe_w4a16.load_state_dict: packed weights in an unknown order (%r)" % (layout,))
+    if layout == 1:
+        t["packed13"] = _octet_blocks(t["packed13"], cfg, cfg.hidden)
+        t["packed2"] = _octet_blocks(t["packed2"], cfg, cfg.inter)
     return _make_state(cfg, t["packed13"].contiguous(), t["packed2"].contiguous(), t["gs13"], t["gs2"],
                        t.get("post_norm_w"), t.get("pre_norm_w"), sd.get("pre_norm_eps", 1e-5), t.get("router"),
                        t.get("route_bias"))
@@ -229,7 +248,7 @@ def _addr(t):
 def _forward(state, cfg, lib, x, logits, ids, tw, out, T):
     """The library call of a step, on addresses. ctypes takes plain integers for pointers; building a
     c_void_p for each of them cost a third of the call."""
-    st = torch._C._cuda_getCurrentRawStream(state["packed13"].device.index)
+    st = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     ref, ws = ctypes.byref(cfg), state["workspace"].data_ptr()
     w13, w2, gs13, gs2 = state["packed13"].data_ptr(), state["packed2"].data_ptr(), state["gs13"].data_ptr(), state["gs2"].data_ptr()
     post, bias, pre = _addr(state["post_norm_w"]), _addr(state["route_bias"]), state.get("pre_norm_w")
@@ -306,7 +325,7 @@ class GraphedStep:
         return True
 
     def __call__(self, data):
-        if self.direct and self._usable(data):
+        if self.direct and self._usable(data) and torch._C._cuda_getDevice() == self.out.device.index:
             state = self.state
             if self.routed:
                 logits, ids, tw = None, data["topk_ids"].data_ptr(), data["topk_weights"].data_ptr()

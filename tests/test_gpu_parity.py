@@ -774,6 +774,31 @@ def test_state_dict_round_trip_skips_the_repack(cuda_dev):
     assert torch.equal(back["w13"], w["w13"]) and torch.equal(back["w2_sf"], w["w2_sf"].view(torch.uint8))
 
 
+def test_state_saved_in_128_row_tiles_loads(cuda_dev):
+    """A saved state without a layout number holds tiles of 128 rows x 256 K: loading puts them in the order the
+    kernels read. The tiles are built here from the original weights."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E = 768, 512, 3
+    w = inputs.make_weights(H, I, E, 41, cuda_dev)
+    st = m.prepare(w, n_experts=E, top_k=2, max_tokens=16)
+
+    def tiles(codes, sf, first_rows):   # rows of each tile in the order of the tiles
+        rows = torch.cat([torch.arange(r, r + 128) for r in first_rows]).to(cuda_dev)
+        c = codes.view(torch.uint8)[:, rows].view(E, len(first_rows), 128, -1, 8, 16).permute(0, 1, 3, 4, 2, 5)
+        s = sf.view(torch.uint8)[:, rows].view(E, len(first_rows), 128, -1, 1, 16).permute(0, 1, 3, 4, 2, 5)
+        return torch.cat([c, s], dim=3).reshape(-1)
+
+    sd = m.state_dict(st)
+    assert sd.pop("packed_layout") == 2
+    sd["packed13"] = tiles(w["w13"], w["w13_sf"], [g * I + j * 128 for j in range(I // 128) for g in (0, 1)])
+    sd["packed2"] = tiles(w["w2"], w["w2_sf"], [j * 128 for j in range(H // 128)])
+    st2 = m.load_state_dict(sd)
+    assert torch.equal(st2["packed13"], st["packed13"]) and torch.equal(st2["packed2"], st["packed2"])
+    sd["packed_layout"] = 3
+    with pytest.raises(RuntimeError):
+        m.load_state_dict(sd)
+
+
 def test_prefill_moe_runs_the_prefill_layer_call_site(cuda_dev):
     """The prefill layer's expert step (muse_prefill_layer/py/04_moe_forward.py:6-52 followed by its
     combine): un-normed pooler rows, local ids with -1, routing weights in; pre-expert norm, both
