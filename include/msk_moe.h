@@ -88,7 +88,7 @@ int msk_moe_packed_bytes(const MskMoeCfg* cfg, size_t* host_w13_bytes, size_t* h
  * [gate 0..I-1; up I..2I-1]); w13_sf: E4M3 bytes [local_count, 2I, H/16];
  * w2: uint8 [local_count, H, I/2]; w2_sf: [local_count, H, I/16].
  * Output: blocks of 8 rows x 256 K, each 1024 bytes of codes followed by 128 scale bytes, ordered
- * [expert][pair of 128-row tiles][8-row slice][tile of the pair][k block]; a pair is (gate j, up j) of w13,
+ * [expert][pair of 128-row tiles][k block][8-row slice][tile of the pair]; a pair is (gate j, up j) of w13,
  * (2j, 2j + 1) of w2. Byte permutation only. */
 int msk_moe_repack(const MskMoeCfg* cfg, const void* w13, const void* w13_sf, const void* w2, const void* w2_sf,
                    void* packed13, void* packed2, void* stream);

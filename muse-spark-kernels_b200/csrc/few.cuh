@@ -7,7 +7,7 @@
 //
 // Twelve working warps, one CTA per SM. A warp streams its part of a unit through a private ring of small bulk
 // copies that its own lane 0 issues, and keeps the accumulators in registers. A gate/up unit (8 gate + 8 up rows
-// over all of K, one contiguous piece of memory) is the work of a team of two warps, half of K each; they meet
+// over all of K) is the work of a team of two warps, half of K each; they meet
 // once per unit, where one of them adds the two partials and runs the epilogue while the other goes on. A
 // down unit (16 rows) is one warp's. So at most six units of a CTA are open at a time and the tiles of `inter`
 // complete one after the other, before the last weights have arrived.
@@ -519,22 +519,27 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
         begun = true;
         if (is.gate()) {
           const int u = is.unit(deal), t = static_cast<int>(__umulhi(static_cast<uint32_t>(u), p.inv_oct1));
-          src = p.w13 + ((static_cast<size_t>(ctl.tile_expert[t]) * oct1 + (u - t * oct1)) * n_kb1 + kb_a) * FEW_KB_BYTES;
+          const int o = u - t * oct1;
+          src = p.w13 + (static_cast<size_t>(ctl.tile_expert[t]) * (oct1 >> 4) + (o >> 4)) * n_kb1 * STAGE_W_BYTES + kb_a * STAGE_W_BYTES +
+                (o & 15) * FEW_KB_BYTES;
           is_left = kb_b - kb_a;
         } else if (is.j < n_down) {
           const int t = is.j / n_own, g = is.j - t * n_own;
-          src = p.w2 + (static_cast<size_t>(ctl.tile_expert[t]) * groups + first_group + g * n_ctas) * n_kb2 * FEW_KB_BYTES;
+          const int grp = first_group + g * n_ctas;
+          src = p.w2 + (static_cast<size_t>(ctl.tile_expert[t]) * (groups >> 4) + (grp >> 4)) * n_kb2 * STAGE_W_BYTES +
+                (grp & 15) * FEW_KB_BYTES;
           is_left = n_kb2;
         } else {
           return;
         }
       }
-      const int n = min(slot_kb, is_left) * FEW_KB_BYTES;
+      const int n = min(slot_kb, is_left);
       if (lane == 0) {
-        mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(n));
-        bulk_g2s(ring + slot * slot_bytes, src, static_cast<uint32_t>(n), &full[slot], pol);
+        mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(n * FEW_KB_BYTES));
+        for (int i = 0; i < n; ++i)
+          bulk_g2s(ring + slot * slot_bytes + i * FEW_KB_BYTES, src + i * STAGE_W_BYTES, FEW_KB_BYTES, &full[slot], pol);
       }
-      src += n;
+      src += n * STAGE_W_BYTES;
       is_left -= slot_kb;
     };
     for (int i = 0; i < p.n_slots; ++i) issue(i);

@@ -2,7 +2,7 @@
 //
 // D[128 weight rows, N tokens] = W_tile[128, K] * X_tile[N, K]^T, weights on the MMA M side.
 // Per CTA (768 threads, one CTA per SM):
-//   warp 0       weight producer: one 3-D TMA box of packed NVFP4 octet blocks per K stage (the two
+//   warp 0       weight producer: one bulk copy of packed NVFP4 octet blocks per K stage (the two
 //                tiles of a "pair"), into a shared-memory ring;
 //   warps 1, 3   MMA issuers (one per tile of the pair): tcgen05.mma kind::f16, A from TMEM,
 //                B from shared memory, FP32 accumulators in TMEM; warp 1 owns the TMEM allocation;
@@ -118,8 +118,7 @@ struct PhaseParams {
 };
 
 struct GemmParams {
-  CUtensorMap tmap_w[2];     // packed weights, per phase: a K stage of a pair as one 3-D box (64-byte aligned: first members)
-  CUtensorMap tmap_act[2];   // TMA_B only, per phase: [rows, K] f16, box 64 x N, 128-byte swizzle
+  CUtensorMap tmap_act[2];   // TMA_B only, per phase: [rows, K] f16, box 64 x N, 128-byte swizzle (64-byte aligned: first member)
   PhaseParams ph[2];         // [0] gate/up, [1] down; a single-phase launch uses its own entry only
   const __nv_bfloat16* post_norm_w;  // phase 1, nullable
   int32_t* cnt;              // [local_count]      sort tables in global memory: read here, or written by CTA 0
@@ -535,10 +534,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     ctl.fin_n = 0;
     fence_mbar_init();
   }
-  if (warp == 0 && lane == 0) {
-    prefetch_tensormap(&p.tmap_w[PH_FIRST]);
-    if (TMA_B) prefetch_tensormap(&p.tmap_act[PH_FIRST]);
-  }
+  if (TMA_B && warp == 0 && lane == 0) prefetch_tensormap(&p.tmap_act[PH_FIRST]);
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, TMEM_COLS);
     tmem_relinquish();

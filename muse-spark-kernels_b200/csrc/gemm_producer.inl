@@ -1,6 +1,6 @@
 // Role body of moe_gemm_kernel (included inside the kernel): weight producer, warp 0.
 // One lane streams the two packed tiles of every K stage of every piece of this CTA into the
-// shared-memory ring, one 3-D box (layout.cuh) per stage that completes on the stage's mbarrier. With both
+// shared-memory ring, one contiguous copy (layout.cuh) per stage that completes on the stage's mbarrier. With both
 // phases in one launch the stream runs on from the last gate/up stage into the first down stage.
 //
 // The ring is the only look-ahead. Asking L2 for stages further ahead (cp.async.bulk.prefetch.L2 from
@@ -19,7 +19,7 @@
         MSK_PHASE_SETUP;
         while (ok && pieces.next(base, ks0, ks1)) {
           const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
-          const int oct0 = (ui.expert * pp.n_pairs + ui.pair) * TILE_OCTETS;   // first octet of the pair
+          const uint8_t* wsrc = pp.w + static_cast<size_t>(ui.expert * pp.n_pairs + ui.pair) * nst_total * STAGE_W_BYTES;
           for (int ks = ks0; ks < ks1; ++ks, ++it) {
             const uint32_t slot = it % NST, par = (it / NST) & 1u;
 #ifdef MSK_TRACE_DETAIL
@@ -27,8 +27,8 @@
 #endif
             if (!MSK_WAIT(&ctl.raw_empty[slot], par ^ 1u, abortw)) { ok = false; break; }
             uint8_t* dst = ring + slot * C::STAGE_BYTES;
-            mbar_arrive_expect_tx(&ctl.raw_full[slot], 2 * TILE_BYTES);
-            tma_load_3d(dst, &p.tmap_w[phase], 0, 2 * ks, oct0, &ctl.raw_full[slot], pol);
+            mbar_arrive_expect_tx(&ctl.raw_full[slot], STAGE_W_BYTES);
+            bulk_g2s(dst, wsrc + static_cast<size_t>(ks) * STAGE_W_BYTES, STAGE_W_BYTES, &ctl.raw_full[slot], pol);
             if (it == 0) MSK_TR(TR_FIRST_BULK);
             if (TMA_B) {
               // activation tile of the stage: four boxes of 64 K x N rows, rows row0.. of the sorted matrix.
@@ -61,9 +61,9 @@
         int left = NST + 1, b2, k0, k1;
         while (left > 0 && pi.next(b2, k0, k1)) {
           const UnitInfo u2 = decode_unit(b2, tile_start, nx.n_pairs, p.nloc, N);
-          const int oct0 = (u2.expert * nx.n_pairs + u2.pair) * TILE_OCTETS;
+          const uint8_t* src = nx.w + (static_cast<size_t>(u2.expert * nx.n_pairs + u2.pair) * nst2 + k0) * STAGE_W_BYTES;
           const int take = min(left, k1 - k0);
-          for (int j = 0; j < take; ++j) tma_prefetch_3d(&p.tmap_w[1], 0, 2 * (k0 + j), oct0);
+          bulk_prefetch_l2(src, static_cast<uint32_t>(take) * STAGE_W_BYTES);
           left -= take;
         }
       }

@@ -5,13 +5,13 @@
 //                       K [32c, 32c+32) of the block, two E2M1 codes per byte in the source order (low
 //                       nibble = even k);
 //   bytes [1024, 1152)  scales: row r's sixteen E4M3 bytes at 1024 + r*16, byte j = 16-element block j.
-// Blocks lie in memory as [expert][pair j][octet o 0..15][K block ks][gu 0..1]: pair j is the two 128-row
+// Blocks lie in memory as [expert][pair j][K block ks][octet o 0..15][gu 0..1]: pair j is the two 128-row
 // tiles that share a unit of work (gate tile j and up tile j of w13; row tiles 2j and 2j+1 of w2), and block
-// (o, gu) holds rows 8o .. 8o+7 of tile gu. Two shapes of access are contiguous enough for one copy each:
-//   * a K stage of a pair (256 rows x 256 K): the 32 blocks of one ks, a 3-D box {1152 bytes, 2, 16};
-//   * a row slice (8 + 8 rows, any run of K blocks): the blocks of one octet follow one another.
-// What matters is the number of copies: measured on B200 (148 CTAs, ring of 36,864-byte stages) boxes stream
-// at 7.09 TB/s, contiguous stages at 7.12, the same stage as 32 separate copies of 1152 bytes at 5.5.
+// (o, gu) holds rows 8o .. 8o+7 of tile gu. Two shapes of access are contiguous:
+//   * a K stage of a pair (256 rows x 256 K): the 32 blocks of one ks, 36,864 bytes, one copy;
+//   * a K block of a row slice (8 + 8 rows): the two blocks of one octet, 2,304 bytes.
+// What matters is the number of copies: measured on B200 (148 CTAs, ring of 36,864-byte stages) contiguous
+// stages stream at 7.12 TB/s, the same stage as 32 separate copies of 1152 bytes at 5.5.
 // A thread that owns a weight row reads 16-byte chunks: the eight rows of a quarter-warp are 128
 // contiguous bytes; a warp that reads the four-byte words of a chunk for an mma.sync operand (lane =
 // row * 4 + word) reads the same 128 bytes. Neither has bank conflicts. The repack is a pure byte
@@ -45,6 +45,7 @@ constexpr int OCT_CODE_BYTES = OCT_ROWS * KS / 2;         // 1024
 constexpr int OCT_BYTES = OCT_CODE_BYTES + OCT_ROWS * KS / 16;  // 1152
 constexpr int TILE_OCTETS = TILE_ROWS / OCT_ROWS;         // 16
 constexpr int TILE_BYTES = TILE_OCTETS * OCT_BYTES;       // 18432: the bytes of one tile in a K stage
+constexpr int STAGE_W_BYTES = 2 * TILE_BYTES;             // 36864: a K stage of a pair
 
 #ifdef __CUDACC__
 // One chunk: four words (32 codes) and the low 16 bits of `sf2` (the scale bytes of its two

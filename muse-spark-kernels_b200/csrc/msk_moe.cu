@@ -19,7 +19,7 @@
 namespace msk {
 
 // ------------------------------------------------------------ repack kernels
-// Octet blocks (layout.cuh) in the order [expert][pair][octet][ks][gu]. Source rows of block (pair j,
+// Octet blocks (layout.cuh) in the order [expert][pair][ks][octet][gu]. Source rows of block (pair j,
 // octet o, gu): w13 gu*I + j*128 + o*8 .. +7, w2 (2j + gu)*128 + o*8 .. +7.
 struct RepackGeom {
   int rows_total;       // source rows per expert (2I or H)
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf
   if (og >= n_og) return;
   const int lane = threadIdx.x & 31, r = lane >> 2, c4 = lane & 3;
   const long long srow = source_row(g, og) + r;
-  uint8_t* block = packed + ((og >> 1) * g.n_stages * 2 + (og & 1)) * OCT_BYTES;   // K block 0; the next one 2 * OCT_BYTES on
+  uint8_t* block = packed + (og >> 5) * g.n_stages * STAGE_W_BYTES + (og & 31) * OCT_BYTES;   // K block 0; the next one STAGE_W_BYTES on
   {
     uint4* src = reinterpret_cast<uint4*>(codes + srow * (g.K / 2)) + c4;
     // chunk i*4 + c4 of the row: K block (i*4 + c4) / 8, chunk (i*4 + c4) % 8 inside it
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf
       for (int j = 0; j < 8; ++j) {
         const int i = i0 + j;
         if (i < n) {
-          const size_t at = static_cast<size_t>(i >> 1) * (2 * OCT_BYTES / 16) + (i & 1) * 32;
+          const size_t at = static_cast<size_t>(i >> 1) * (STAGE_W_BYTES / 16) + (i & 1) * 32;
           v[j] = INVERSE ? __ldcs(dst + at) : __ldcs(src + i * 4);
         }
       }
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf
       for (int j = 0; j < 8; ++j) {
         const int i = i0 + j;
         if (i < n) {
-          const size_t at = static_cast<size_t>(i >> 1) * (2 * OCT_BYTES / 16) + (i & 1) * 32;
+          const size_t at = static_cast<size_t>(i >> 1) * (STAGE_W_BYTES / 16) + (i & 1) * 32;
           if (INVERSE) __stcs(src + i * 4, v[j]); else __stcs(dst + at, v[j]);
         }
       }
@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf
   uint4* src = reinterpret_cast<uint4*>(sf + srow * (g.K / 16));
   uint4* dst = reinterpret_cast<uint4*>(block + OCT_CODE_BYTES + r * 16);
   for (int ks = c4; ks < g.n_stages; ks += 4) {
-    if (INVERSE) __stcs(src + ks, __ldcs(dst + ks * (2 * OCT_BYTES / 16)));
-    else __stcs(dst + ks * (2 * OCT_BYTES / 16), __ldcs(src + ks));
+    if (INVERSE) __stcs(src + ks, __ldcs(dst + ks * (STAGE_W_BYTES / 16)));
+    else __stcs(dst + ks * (STAGE_W_BYTES / 16), __ldcs(src + ks));
   }
 }
 
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128) dequant_packed_kernel(const uint8_t* pack
   const long long og = (blockIdx.x / g.n_stages) * 16 + (threadIdx.x >> 3);
   if (og >= n_og) return;
   const int r = threadIdx.x & 7;
-  const uint8_t* block = packed + ((og >> 1) * g.n_stages * 2 + ks * 2 + (og & 1)) * OCT_BYTES;
+  const uint8_t* block = packed + ((og >> 5) * g.n_stages + ks) * STAGE_W_BYTES + (og & 31) * OCT_BYTES;
   const uint4 sfw = *reinterpret_cast<const uint4*>(block + OCT_CODE_BYTES + r * 16);
   const uint32_t sfa[4] = {sfw.x, sfw.y, sfw.z, sfw.w};
   __nv_bfloat16* orow = out + (source_row(g, og) + r) * g.K + ks * KS;
@@ -836,15 +836,6 @@ static long long n_og_of(const MskMoeCfg* c, const RepackGeom& g) {   // octet-g
   return static_cast<long long>(c->local_count) * g.n_pairs * 2 * TILE_OCTETS;
 }
 
-// Tensor maps of the packed weights: 8-byte elements, [block 144][K blocks * 2][octets of all experts], box
-// {144, 2, 16} = the 36,864 bytes of one K stage of a pair.
-static int encode_weight_map(CUtensorMap* map, const MskMoeCfg* c, const RepackGeom& g, const void* packed) {
-  const cuuint64_t dims[3] = {OCT_BYTES / 8, static_cast<cuuint64_t>(g.n_stages) * 2, static_cast<cuuint64_t>(n_og_of(c, g) / 2)};
-  const cuuint64_t strides[2] = {OCT_BYTES, static_cast<cuuint64_t>(g.n_stages) * 2 * OCT_BYTES};
-  const cuuint32_t box[3] = {OCT_BYTES / 8, 2, TILE_OCTETS};
-  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, packed, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
-}
-
 template <int N>
 static int launch_router_hilo(const CUtensorMap& mw, const CUtensorMap& mx, float* logits, int32_t* status, int T, int E,
                               int H, cudaStream_t st) {
@@ -1208,11 +1199,6 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.partial = partial + round_up(partial_floats(cfg) * 4, 256) / 4;
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
-  {
-    int e = encode_weight_map(&p.tmap_w[0], cfg, geom13(cfg), packed13);
-    if (e == 0) e = encode_weight_map(&p.tmap_w[1], cfg, geom2(cfg), packed2);
-    if (e != 0) return e;
-  }
 
   if (plan.path != 1 && plan.path != 4) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
@@ -1567,9 +1553,6 @@ int msk_moe_forward_static(const MskMoeCfg* cfg, const void* packed13, const voi
   p.ph[0].K = cfg->hidden; p.ph[0].out_ld = cfg->inter; p.ph[0].n_pairs = cfg->inter / 128;
   p.ph[1].w = static_cast<const uint8_t*>(packed2); p.ph[1].gs = gs2; p.ph[1].act = inter; p.ph[1].outp = y;
   p.ph[1].K = cfg->inter; p.ph[1].out_ld = cfg->hidden; p.ph[1].n_pairs = cfg->hidden / 256;
-  e = encode_weight_map(&p.tmap_w[0], cfg, geom13(cfg), packed13);
-  if (e == 0) e = encode_weight_map(&p.tmap_w[1], cfg, geom2(cfg), packed2);
-  if (e != 0) return e;
   e = launch_gemm_n<0>(16, p, grid, st, 1);
   if (e != 0) return e;
   e = launch_gemm_n<1>(16, p, grid, st, 1);

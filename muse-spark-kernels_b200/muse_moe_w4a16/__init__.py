@@ -123,7 +123,7 @@ PACKED_LAYOUT = 2
 
 def _octet_blocks(tiles, cfg, K):
     """Packed weights of a state saved in 128-row tiles, in the order of the octet blocks (a byte permutation)."""
-    return tiles.view(cfg.local_count, -1, 2, K // 256, 9, 16, 8, 16).permute(0, 1, 5, 3, 2, 4, 6, 7).reshape(-1)
+    return tiles.view(cfg.local_count, -1, 2, K // 256, 9, 16, 8, 16).permute(0, 1, 3, 5, 2, 4, 6, 7).reshape(-1)
 
 
 _SD_TENSORS = ("packed13", "packed2", "gs13", "gs2", "post_norm_w", "pre_norm_w", "router", "route_bias")
