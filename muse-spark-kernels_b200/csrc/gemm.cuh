@@ -6,8 +6,8 @@
 //                tiles of a "pair"), into a shared-memory ring;
 //   warps 1, 3   MMA issuers (one per tile of the pair): tcgen05.mma kind::f16, A from TMEM,
 //                B from shared memory, FP32 accumulators in TMEM; warp 1 owns the TMEM allocation;
-//   warp 2       activation gather: cp.async of the token rows of the tile (through the
-//                permutation for the gate/up GEMM) into the K-major core-matrix layout;
+//   warp 2       activations: cp.async gather of the token rows of the tile (through the permutation for
+//                the gate/up GEMM) into the K-major core-matrix layout, or TMA boxes of sorted rows;
 //   warps 4-7    epilogue (gemm_epilogue.inl): TMEM accumulators -> SwiGLU / scale -> global,
 //                or split-K partials (token tiles up to 64; for 128 the accumulators are single-
 //                buffered and the sixteen dequant warps, idle by then, share the epilogue);
@@ -84,7 +84,7 @@ struct GemmCfg {
   static constexpr int NSLOT = N <= 32 ? 3 : 2;
   static constexpr int SLOT_COLS = 64;
   static constexpr int A_GROUP_COLS = NSLOT * SLOT_COLS;
-  // Token tiles of 64 and more fetch the activation operand with TMA (2-D boxes of 64 K x N rows,
+  // Token tiles of 64 and more fetch the activation operand with TMA (2-D boxes of 64 K x 16 to N rows,
   // 128-byte swizzle) from rows that are contiguous in sorted order (the sorted F16 copy of the token
   // rows for the gate/up GEMM, `inter` for the down GEMM); narrower tiles gather rows through the
   // permutation with cp.async (gemm_gather.inl). Gathering the wide tiles' rows with cp.async as well
@@ -118,7 +118,8 @@ struct PhaseParams {
 };
 
 struct GemmParams {
-  CUtensorMap tmap_act[2];   // TMA_B only, per phase: [rows, K] f16, box 64 x N, 128-byte swizzle (64-byte aligned: first member)
+  CUtensorMap tmap_act[2][4];   // TMA_B only, per phase: [rows, K] f16, boxes 64 x (16 << i) up to 64 x N, 128-byte swizzle
+                                // (64-byte aligned: first member)
   PhaseParams ph[2];         // [0] gate/up, [1] down; a single-phase launch uses its own entry only
   const __nv_bfloat16* post_norm_w;  // phase 1, nullable
   int32_t* cnt;              // [local_count]      sort tables in global memory: read here, or written by CTA 0
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     ctl.fin_n = 0;
     fence_mbar_init();
   }
-  if (TMA_B && warp == 0 && lane == 0) prefetch_tensormap(&p.tmap_act[PH_FIRST]);
+  if (TMA_B && warp == 2 && lane < 4 && (16 << lane) <= N) prefetch_tensormap(&p.tmap_act[PH_FIRST][lane]);
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, TMEM_COLS);
     tmem_relinquish();

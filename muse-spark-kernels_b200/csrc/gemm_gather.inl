@@ -1,5 +1,5 @@
-// Role body of moe_gemm_kernel (included inside the kernel): activation gather, warp 2.
-// Copies the token rows of the piece (x rows through the permutation for phase 0, sorted inter
+// Role body of moe_gemm_kernel (included inside the kernel): activations, warp 2.
+// Narrow token tiles: copies the token rows of the piece (x rows through the permutation for phase 0, sorted inter
 // rows for phase 1) with 16-byte cp.async into the K-major core-matrix layout of the B operand:
 // element (n, k) at (n/8)*B_SBO + (k/8)*B_LBO + (n%8)*16 + (k%8)*2. Eight lanes write one
 // 128-byte core matrix, so shared-memory writes are conflict free. A stage is published a few
@@ -118,4 +118,30 @@
       // a CTA without work in this phase still takes part in nothing it has to wait for
     }
     drain();
+    } else if (lane == 0) {
+      // Wide token tiles: four boxes per K stage, rows row0.. of the sorted matrix, no higher than the tile's
+      // rows need (16, 32, 64 or 128: a tensor map each). The copies of a stage stay four; only their bytes
+      // shrink. (Whole 32-row boxes put side by side, more copies per stage, were slower than full height.) A full
+      // box of 128 rows is 64 KB a stage beside 36 KB of weights; an expert with 48 tokens needs half of it.
+      const uint64_t keep = policy_evict_last();  // token rows are re-read by every pair of the expert
+      uint32_t it = 0;
+      bool ok = true;
+      MSK_PHASES {
+        MSK_PHASE_SETUP;
+        if (MODE == 1) pdl_wait();  // inter comes from the gate/up GEMM
+        while (ok && pieces.next(base, ks0, ks1)) {
+          const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
+          const int h = ui.rows <= 16 ? 0 : ui.rows <= 32 ? 1 : ui.rows <= 64 ? 2 : 3;
+          const CUtensorMap* map = &p.tmap_act[phase][h];
+          for (int ks = ks0; ks < ks1; ++ks, ++it) {
+            const uint32_t slot = it % NST, par = (it / NST) & 1u;
+            if (!MSK_WAIT(&ctl.b_empty[slot], par ^ 1u, abortw)) { ok = false; break; }
+            uint8_t* dstB = ring + slot * C::STAGE_BYTES + 2 * TILE_BYTES;
+            mbar_arrive_expect_tx(&ctl.b_full[slot], static_cast<uint32_t>(4 * 64 * 2 * 16) << h);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) tma_load_2d(dstB + j * (N * 128), map, ks * KS + j * 64, ui.row0, &ctl.b_full[slot], keep);
+          }
+        }
+        if (!ok) break;
+      }
     }

@@ -10,8 +10,6 @@
 // prefetch occupies the copy engine of the SM for as long as the copy it anticipates.
     if (lane == 0) {
       const uint64_t pol = p.evict_first ? policy_evict_first() : policy_evict_last();
-      const uint64_t keep = policy_evict_last();  // token rows are re-read by every pair of the expert
-      (void)keep;
       uint32_t it = 0;
       int tri = 0;
       bool ok = true;
@@ -30,19 +28,6 @@
             mbar_arrive_expect_tx(&ctl.raw_full[slot], STAGE_W_BYTES);
             bulk_g2s(dst, wsrc + static_cast<size_t>(ks) * STAGE_W_BYTES, STAGE_W_BYTES, &ctl.raw_full[slot], pol);
             if (it == 0) MSK_TR(TR_FIRST_BULK);
-            if (TMA_B) {
-              // activation tile of the stage: four boxes of 64 K x N rows, rows row0.. of the sorted matrix.
-              // (Fetching only the 32-row groups a tile's rows lie in, with a second tensor map of 64 x 32
-              // boxes, halves the bytes of a sparsely filled tile and was slower: 256 tokens 351 against
-              // 307 us. More copies per stage cost more than the bytes they save.)
-              if (MODE == 1 && it == 0) pdl_wait();  // inter comes from the gate/up GEMM
-              if (!MSK_WAIT(&ctl.b_empty[slot], par ^ 1u, abortw)) { ok = false; break; }
-              uint8_t* dstB = dst + 2 * TILE_BYTES;
-              mbar_arrive_expect_tx(&ctl.b_full[slot], C::B_STAGE_BYTES);
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                tma_load_2d(dstB + j * (N * 128), &p.tmap_act[phase], ks * KS + j * 64, ui.row0, &ctl.b_full[slot], keep);
-            }
             MSK_TRD(2, tri, 1);
           }
         }

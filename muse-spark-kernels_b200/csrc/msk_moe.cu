@@ -1323,10 +1323,11 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     }
     if (e != 0) return e;
     if (tma_b) {
-      e = encode_act_map(&p.tmap_act[0], xs, r_max, cfg->hidden, plan.N);
-      if (e != 0) return e;
-      e = encode_act_map(&p.tmap_act[1], inter, r_max, cfg->inter, plan.N);
-      if (e != 0) return e;
+      for (int i = 0; (16 << i) <= plan.N; ++i) {
+        e = encode_act_map(&p.tmap_act[0][i], xs, r_max, cfg->hidden, 16 << i);
+        if (e == 0) e = encode_act_map(&p.tmap_act[1][i], inter, r_max, cfg->inter, 16 << i);
+        if (e != 0) return e;
+      }
     }
   }
   if (ev) cudaEventRecord(ev[5], st);
