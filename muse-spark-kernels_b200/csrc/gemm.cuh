@@ -134,7 +134,6 @@ struct GemmParams {
   int evict_first;
   int handover;              // two launches: gate/up units count per token tile (tile_done), down units wait for their
                              // tile's count instead of for the whole gate/up grid (see gemm_gather.inl)
-  int y_bf16;                // phase 1, token tile 128: y rows as BF16 instead of FP32
   // Phase 0 with route != 0 (at most 256 entries): every CTA derives the sort tables in its prologue.
   // route 1: top-k of `logits` first (CTA 0 writes ids_out / tw_out); route 2: ids_in given.
   int route;
@@ -328,51 +327,84 @@ __device__ __forceinline__ __half inter_value(float v) {
   return __float2half_rn(fminf(fmaxf(r, -65504.f), 65504.f));
 }
 
-// Epilogue of a whole unit for the thread that owns TMEM lane `row`: columns [c_beg, c_end) of the
-// accumulators at d_tmem (lane base included). Phase 0 reads gate (tile 0) and up (tile 1) and
-// writes bf16(silu(g) * u) into inter; phase 1 writes the rows of `tile` scaled by gs (and
-// 1 + post_norm_w) into y. (Used by the wide token tile, whose dequant warps share the epilogue.)
-template <int N>
-__device__ __forceinline__ void epilogue_columns(const GemmParams& p, const PhaseParams& pp, int phase,
-                                                 const UnitInfo& ui, uint32_t d_tmem, int row, int c_beg, int c_end,
-                                                 int tile) {
+// Two SwiGLU values as inter_value gives them, packed (first one in the low half). For the wide token tile, where
+// the dequant warps do this between two units of work: the quotient by reciprocal and the roundings two at a time,
+// 13 instructions a value instead of 30.
+__device__ __forceinline__ uint32_t inter_pair(uint32_t g0, uint32_t u0, uint32_t g1, uint32_t u1, float gs) {
+  const float a0 = __uint_as_float(g0) * gs, a1 = __uint_as_float(g1) * gs;
+  const float v0 = __fdividef(a0, 1.0f + __expf(-a0)) * (__uint_as_float(u0) * gs);
+  const float v1 = __fdividef(a1, 1.0f + __expf(-a1)) * (__uint_as_float(u1) * gs);
+  const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
+  const __half2 h = __floats2half2_rn(__low2float(b), __high2float(b));
+  const __half2 c = __hmin2(__hmax2(h, __half2half2(__ushort_as_half(0xFBFF))), __half2half2(__ushort_as_half(0x7BFF)));   // +-65504
+  return *reinterpret_cast<const uint32_t*>(&c);
+}
+
+// Epilogue of a unit of the 128-token tile for the thread that owns TMEM lane `row`: four warps share a lane quarter.
+// Phase 0: quarter `part` of the columns, gate (tile 0) and up (tile 1) -> bf16(silu(g) * u) into inter; phase 1: half
+// `part >> 1` of the columns of tile `part & 1` -> rows scaled by gs (and 1 + post_norm_w) into y as BF16, as the
+// reference's wide-tile build keeps them. The tensor core stands still from the last MMA of a unit until
+// release() hands the accumulators back: before that, the first half of this thread's values is only brought
+// down to packed results and the second half into registers; the rest of the arithmetic and all stores run
+// beside the next unit's MMAs. (Both halves as raw values would need 64 registers beside the main loop's: 80 are there.)
+template <typename Release>
+__device__ __forceinline__ void epilogue_wide(const GemmParams& p, const PhaseParams& pp, int phase, const UnitInfo& ui,
+                                              uint32_t d_tmem, int row, int part, Release release) {
+  constexpr int N = 128;
   const float gsc = pp.gs[ui.expert];
+  size_t ld = static_cast<size_t>(pp.out_ld);
+  asm volatile("" : "+l"(ld));   // or its multiples are kept in registers through the main loop
+  const int c_beg = phase == 0 ? part * (N / 4) : (part >> 1) * (N / 2);
+  const int n = ui.rows - c_beg;   // rows of this thread's columns
+  if (n <= 0) {
+    release();
+    return;
+  }
   if (phase == 0) {
-    __half* outp = static_cast<__half*>(pp.outp) + static_cast<size_t>(ui.row0) * pp.out_ld + ui.pair * 128 + row;
-    for (int c0 = c_beg; c0 < c_end; c0 += 16) {
-      if (c0 >= ui.rows) break;
-      uint32_t r0[16], r1[16];
-      tmem_ld16(d_tmem + c0, r0);
-      tmem_ld16(d_tmem + N + c0, r1);
-      tmem_wait_ld();
+    uint32_t a[16], b[16], first[8];
+    tmem_ld16(d_tmem + c_beg, a);
+    tmem_ld16(d_tmem + N + c_beg, b);
+    tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (c0 + j < ui.rows) {
-          const float v = silu_f(__uint_as_float(r0[j]) * gsc) * (__uint_as_float(r1[j]) * gsc);
-          outp[static_cast<size_t>(c0 + j) * pp.out_ld] = inter_value(v);
-        }
-      }
+    for (int j = 0; j < 8; ++j) first[j] = inter_pair(a[2 * j], b[2 * j], a[2 * j + 1], b[2 * j + 1], gsc);
+    tmem_ld16(d_tmem + c_beg + 16, a);
+    tmem_ld16(d_tmem + N + c_beg + 16, b);
+    tmem_wait_ld();
+    release();
+    __half* outp = static_cast<__half*>(pp.outp) + static_cast<size_t>(ui.row0 + c_beg) * ld + ui.pair * 128 + row;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t h = j < 8 ? first[j & 7] : inter_pair(a[2 * (j & 7)], b[2 * (j & 7)], a[2 * (j & 7) + 1], b[2 * (j & 7) + 1], gsc);
+      if (2 * j < n) *outp = __ushort_as_half(static_cast<unsigned short>(h));
+      outp += ld;
+      if (2 * j + 1 < n) *outp = __ushort_as_half(static_cast<unsigned short>(h >> 16));
+      outp += ld;
     }
   } else {
-    const int col = (2 * ui.pair + tile) * 128 + row;
+    const int col = (2 * ui.pair + (part & 1)) * 128 + row;
     float osc = gsc;
     if (p.post_norm_w != nullptr) osc *= 1.0f + __bfloat162float(p.post_norm_w[col]);
-    float* outp = static_cast<float*>(pp.outp) + static_cast<size_t>(ui.row0) * pp.out_ld + col;
-    __nv_bfloat16* outb = static_cast<__nv_bfloat16*>(pp.outp) + static_cast<size_t>(ui.row0) * pp.out_ld + col;
-    for (int c0 = c_beg; c0 < c_end; c0 += 32) {
-      if (c0 >= ui.rows) break;
-      uint32_t r[32];
-      tmem_ld32(d_tmem + tile * N + c0, r);
-      tmem_wait_ld();
-      if (p.y_bf16) {   // wide token tiles: y rows in BF16, as the reference's wide-tile build keeps them
+    const uint32_t src = d_tmem + (part & 1) * N + c_beg;
+    uint32_t a[32], first[16];
+    auto pack = [osc](uint32_t lo, uint32_t hi) -> uint32_t {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(lo) * osc, __uint_as_float(hi) * osc);
+      return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    tmem_ld32(src, a);
+    tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < ui.rows) outb[static_cast<size_t>(c0 + j) * pp.out_ld] = __float2bfloat16_rn(__uint_as_float(r[j]) * osc);
-      } else {
+    for (int j = 0; j < 16; ++j) first[j] = pack(a[2 * j], a[2 * j + 1]);
+    tmem_ld32(src + 32, a);
+    tmem_wait_ld();
+    release();
+    unsigned short* outp = static_cast<unsigned short*>(pp.outp) + static_cast<size_t>(ui.row0 + c_beg) * ld + col;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < ui.rows) outp[static_cast<size_t>(c0 + j) * pp.out_ld] = __uint_as_float(r[j]) * osc;
-      }
+    for (int j = 0; j < 32; ++j) {
+      const uint32_t h = j < 16 ? first[j & 15] : pack(a[2 * (j & 15)], a[2 * (j & 15) + 1]);
+      if (2 * j < n) *outp = static_cast<unsigned short>(h);
+      outp += ld;
+      if (2 * j + 1 < n) *outp = static_cast<unsigned short>(h >> 16);
+      outp += ld;
     }
   }
 }
@@ -661,7 +693,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
   // the others. They are dealt fewer down units, the way the one-launch kernel deals its second phase
   // (phase1_skew), with the block order reversed so that "heavy" means "started last". Only the balance
   // depends on that order, not the result.
-  const bool chained_skew = MODE == 1 && p.handover != 0;
+  const bool chained_skew = MODE == 1 && !TMA_B && p.handover != 0;
   const int deal_index = chained_skew ? static_cast<int>(n_ctas) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
   volatile int* abortw = &ctl.abort_word;
 #define MSK_WAIT(bar, par, ab) (N >= 64 ? mbar_wait_inline((bar), (par), (ab)) : mbar_wait((bar), (par), (ab)))

@@ -34,29 +34,25 @@
     // their operands ready, and the bubble between two units is the drain alone, not the drain plus
     // a refill of the decode pipeline.
     bool owe_drain = false;
-    UnitInfo owed_ui;
+    int owed_base = 0;
     uint32_t owed_unit_i = 0;
     MSK_PHASES {
       MSK_PHASE_SETUP;
       auto drain = [&]() -> bool {
+        const UnitInfo owed_ui = decode_unit(owed_base, tile_start, pp.n_pairs, p.nloc, N);
         if (!MSK_WAIT(&ctl.d_full[0], owed_unit_i & 1u, abortw)) return false;
         tc_fence_after();
         if (tid == 256) { if (owed_unit_i == 0) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); }
-        if (phase == 0) {
-          const int part = kh * 2 + g;  // 0..3: a quarter of the token columns, gate and up of this lane
-          epilogue_columns<N>(p, pp, phase, owed_ui, tmem + lane_base, row, part * (N / 4), (part + 1) * (N / 4), 0);
-        } else {
-          epilogue_columns<N>(p, pp, phase, owed_ui, tmem + lane_base, row, kh * (N / 2), (kh + 1) * (N / 2), g);
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.d_empty[0]);
+        epilogue_wide(p, pp, phase, owed_ui, tmem + lane_base, row, kh * 2 + g, [&]() {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.d_empty[0]);
+        });
         if (tid == 256 && owed_unit_i == 0) MSK_TR(TR_FIRST_EPI_DONE);
         owe_drain = false;
         return true;
       };
       for (; ok && pieces.next(base, ks0, ks1); ++unit_i) {
-        const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
         for (int ks = ks0; ks < ks1 && ok; ++ks, ++it) {
           const uint32_t slot = it % NST, par = (it / NST) & 1u;
 #ifdef MSK_TRACE_DETAIL
@@ -128,7 +124,7 @@
         if (pending) retire();  // the accumulators need every slot of the piece
         if (NDBUF == 1) {
           owe_drain = true;
-          owed_ui = ui;
+          owed_base = base;
           owed_unit_i = unit_i;
         }
       }

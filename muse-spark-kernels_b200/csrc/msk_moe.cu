@@ -1331,7 +1331,6 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     }
   }
   if (ev) cudaEventRecord(ev[5], st);
-  p.y_bf16 = plan.N == 128 ? 1 : 0;  // the wide tile: half the y bytes written and read back
   // Tile hand-over: the down GEMM's CTAs start on the SMs the gate/up CTAs leave (programmatic launch) and
   // would then wait for that whole grid, whose last CTAs run a unit longer than the others (the units do not
   // divide evenly): a tenth of the gate/up time with every SM but a few idle. Instead each down unit waits
@@ -1370,8 +1369,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     lc.attrs = at;
     lc.numAttrs = 1;
     const bool wide = n_tokens >= COMBINE_WIDE_TOKENS;
+    // the wide tile keeps y in BF16: half the bytes written and read back
     const bool narrow_rows = cfg->hidden <= COMBINE_THREADS * 2 * 4;   // two float4 slots per thread hold a row
-    auto* kern = p.y_bf16 ? (narrow_rows ? combine_kernel<8, true, 2, 2> : combine_kernel<4, true, 2>)
+    auto* kern = plan.N == 128 ? (narrow_rows ? combine_kernel<8, true, 2, 2> : combine_kernel<4, true, 2>)
                           : (wide ? combine_kernel<2, false, 2> : combine_kernel<4, false, 1>);
     e = static_cast<int>(cudaLaunchKernelEx(&lc, kern, static_cast<const float*>(y),
                                             static_cast<const int32_t*>(inv), topk_weights,
