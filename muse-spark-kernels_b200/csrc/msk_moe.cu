@@ -849,15 +849,23 @@ static int launch_router_hilo(const CUtensorMap& mw, const CUtensorMap& mx, floa
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3(static_cast<unsigned>((E + 127) / 128), static_cast<unsigned>((T + N - 1) / N));
+  // as many CTAs per tile (of K) as the machine has room for: one wave
+  const int tiles = ((E + 127) / 128) * ((T + N - 1) / N);
+  int split = 8;
+  while (split > 1 && (split * tiles > DEFAULT_CTAS || split > H / RG_KSTEP)) split /= 2;
+  lc.gridDim = dim3(static_cast<unsigned>(split), static_cast<unsigned>((E + 127) / 128), static_cast<unsigned>((T + N - 1) / N));
   lc.blockDim = dim3(RG_THREADS);
   lc.dynamicSmemBytes = smem;
   lc.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = static_cast<unsigned>(split);
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   lc.attrs = at;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   return static_cast<int>(cudaLaunchKernelEx(&lc, router_hilo_kernel<N>, mw, mx, logits, status, T, E, H));
 }
 
@@ -952,7 +960,8 @@ int msk_moe_router_logits_hilo(const MskMoeCfg* cfg, const void* x, const void* 
   if (n_tokens < 0) return MSK_ERR_SHAPE;
   if (n_tokens == 0) return MSK_OK;
   if (n_tokens < 16) return MSK_ERR_SHAPE;   // fewer tokens than the narrowest MMA tile: use msk_moe_router_logits
-  const int N = n_tokens >= 128 ? 128 : n_tokens >= 64 ? 64 : n_tokens >= 32 ? 32 : 16;
+  // (below 2048 tokens tiles of 64 fill the machine better: eight CTAs per tile)
+  const int N = n_tokens >= 2048 ? 128 : n_tokens >= 64 ? 64 : n_tokens >= 32 ? 32 : 16;
   CUtensorMap mw, mx;
   int e = encode_act_map(&mw, router_hilo, static_cast<size_t>(2) * cfg->n_experts, cfg->hidden, 128,
                          CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);

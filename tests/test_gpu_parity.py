@@ -906,6 +906,13 @@ def test_router_logits_gemm_on_the_hi_lo_pair(cuda_dev, T, E, H):
     assert len(set(rows.tolist())) <= max(1, T // 50)
 
 
+@pytest.mark.parametrize("T,E,H", [(64, 130, 256),      # four K steps: four CTAs of one step; two tiles of experts
+                                   (65, 8, 768),        # twelve steps over eight CTAs
+                                   (2051, 128, 256)])   # 128-token tiles, the last with three tokens
+def test_router_logits_split_over_a_cluster(cuda_dev, T, E, H):
+    test_router_logits_gemm_on_the_hi_lo_pair(cuda_dev, T, E, H)
+
+
 def test_kernel_fn_with_router_weight_uses_the_gemm_from_sixteen_tokens(cuda_dev):
     """weights["router"]: few tokens take the FP32 matvec, 16 and more the hi + lo GEMM; both feed the
     same routing and expert kernels, and the output matches the oracle on the routing the module used."""
