@@ -248,23 +248,107 @@ __global__ void __launch_bounds__(64) convert_rows_kernel(const __nv_bfloat16* _
 }
 
 // ---------------------------------------------------------------- combine
-// One block per token: out[t] = bf16( sum over slots in index order of
-// w[t,s] * norm_s * y[inv[t,s]] ), norm_s = rsqrt(mean(y^2) + eps) when the post-expert
-// norm is on (y already carries 1 + post_norm_w), else 1
+// out[t] = bf16( sum over slots in index order of w[t,s] * norm_s * y[inv[t,s]] ), norm_s =
+// rsqrt(mean(y^2) + eps) when the post-expert norm is on (y already carries 1 + post_norm_w), else 1
 // (muse_moe_w4a16/cuda/moe.cu:2604-2766; muse_decode_layer/py/04_triton_kernels.py:616-632).
-// The block sum of squares is a fixed shuffle tree followed by a fixed-order sum of the
-// eight warp partials, so the result does not depend on scheduling.
+// Slots without a local route (inv < 0) are squeezed out first, keeping their order, so an expert-parallel rank
+// that owns one or two of a token's eight routes reads only those rows, and a token without any
+// local route only gets zeros. Bound by memory for many tokens (8192 tokens, eight rows each: 0.6 GB).
 constexpr int COMBINE_THREADS = 512;
 constexpr int COMBINE_MAX_F4 = 4;   // float4 per thread per row: H <= 8192
 constexpr int COMBINE_WIDE_TOKENS = 512;  // from here on two blocks per SM, two slots per group
 
+// Eight consecutive y values of a row, FP32 or BF16 (the 128-token tile), in registers while in flight.
+template <bool YB> struct YOct;
+template <> struct YOct<false> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* y, size_t at) {
+    a = __ldcs(reinterpret_cast<const float4*>(y + at));
+    b = __ldcs(reinterpret_cast<const float4*>(y + at) + 1);
+  }
+  __device__ __forceinline__ void add_to(float (&acc)[8], float w) const {
+    acc[0] += a.x * w; acc[1] += a.y * w; acc[2] += a.z * w; acc[3] += a.w * w;
+    acc[4] += b.x * w; acc[5] += b.y * w; acc[6] += b.z * w; acc[7] += b.w * w;
+  }
+};
+template <> struct YOct<true> {
+  uint4 a;
+  __device__ __forceinline__ void load(const float* y, size_t at) {
+    a = __ldcs(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(y) + at));
+  }
+  __device__ __forceinline__ void add_to(float (&acc)[8], float w) const {
+    const uint32_t v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[2 * i] += __uint_as_float(v[i] << 16) * w;
+      acc[2 * i + 1] += __uint_as_float(v[i] & 0xFFFF0000u) * w;
+    }
+  }
+};
+
+// Without the post-expert norm the columns do not depend on one another: a warp per (token, C * 256 columns), G rows of
+// them in flight, no block-wide step. G = 8, C = 1 where most of a token's routes are local (8192 tokens of eight rows:
+// 106 us with a block per token, 98 with this); with two or fewer expected, G = 2, C = 4, or the warps would spend
+// their time on the table (8192 tokens of H = 7168 with one local route each: 68 us with a block per token, 78 with G = 8,
+// C = 1, 47 with G = 2, C = 4).
+constexpr int COMBINE_COLS_WARPS = 4;
+template <bool YB, int G, int C>
+__global__ void __launch_bounds__(COMBINE_COLS_WARPS * 32)
+    combine_cols_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv, const float* __restrict__ tw,
+                        __nv_bfloat16* __restrict__ out, int T, int H, int k) {
+  const int lane = threadIdx.x & 31, chunks = (H + C * 256 - 1) / (C * 256);
+  const long long item = static_cast<long long>(blockIdx.x) * COMBINE_COLS_WARPS + (threadIdx.x >> 5);
+  const int t = static_cast<int>(item / chunks), col = static_cast<int>(item % chunks) * (C * 256) + lane * 8;
+  pdl_wait();  // y and inv come from the kernels before this one
+  if (t >= T) return;
+  const int q = lane < k ? inv[static_cast<size_t>(t) * k + lane] : -1;
+  const float w = lane < k ? tw[static_cast<size_t>(t) * k + lane] : 0.f;
+  unsigned have = __ballot_sync(0xffffffffu, q >= 0);
+  float acc[C][8] = {};
+  while (have != 0u) {
+    YOct<YB> v[G][C];
+    float wv[G];
+    const int n = min(__popc(have), G);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (g < n) {
+        const int s = __ffs(have) - 1;
+        have &= have - 1u;
+        wv[g] = __shfl_sync(0xffffffffu, w, s);
+        const size_t at = static_cast<size_t>(__shfl_sync(0xffffffffu, q, s)) * H + col;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          if (col + c * 256 < H) v[g][c].load(y, at + c * 256);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {   // slot order
+      if (g < n) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          if (col + c * 256 < H) v[g][c].add_to(acc[c], wv[g]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if (col + c * 256 >= H) break;
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(acc[c][2 * i], acc[c][2 * i + 1]);
+      o[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * H + col + c * 256) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// With the post-expert norm: one block per token. The block sum of squares is a fixed shuffle tree followed by a
+// fixed-order sum of the warp partials, so the result does not depend on scheduling.
 // G = slots whose rows are loaded together (one memory latency per group instead of one per
 // slot; the sums still run in slot order). G = 4 for few tokens (latency), G = 2 with two blocks
 // per SM for many (one block's loads overlap the other's reduction and stores); BF16 rows need
-// half the registers while in flight, so they get G = 4 and two blocks per SM. Slots without a
-// local route (inv < 0) are squeezed out first, keeping their order, so an expert-parallel rank
-// that owns one or two of a token's eight routes pays for one group, and a token without any
-// local route only writes zeros.
+// half the registers while in flight, so they get G = 4 and two blocks per SM.
 // Four consecutive y values of a row as they sit in registers while their group is in flight:
 // FP32 (16 bytes) or BF16 (8 bytes, for the wide token tile), expanded when used.
 template <bool YB> struct YQuad;
@@ -292,9 +376,11 @@ template <> struct YQuad<true> {
 // the registers per row in flight, which is what lets all eight rows of a token be loaded at once).
 template <int G, bool YB, int MINB, int NF4 = COMBINE_MAX_F4>
 __global__ void __launch_bounds__(COMBINE_THREADS, MINB)
-    combine_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv, const float* __restrict__ tw,
-                   __nv_bfloat16* __restrict__ out, int H, int k, int post_norm, float eps) {
-  __shared__ float wsum[G][COMBINE_THREADS / 32];
+    combine_norm_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv, const float* __restrict__ tw,
+                   __nv_bfloat16* __restrict__ out, int H, int k, float eps) {
+  constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
+  static_assert(G == 1 << LG, "two, four or eight rows together");
+  __shared__ __align__(16) float wsum[G][COMBINE_THREADS / 32];
   __shared__ int s_q[MAX_TOP_K];
   __shared__ float s_w[MAX_TOP_K];
   __shared__ int s_n;
@@ -338,30 +424,42 @@ __global__ void __launch_bounds__(COMBINE_THREADS, MINB)
         if (q[g] >= 0 && i * COMBINE_THREADS + tid < n4) v[g][i].load(y, r, i * COMBINE_THREADS + tid);
       }
     }
-    if (post_norm) {
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
+    for (int g = 0; g < G; ++g) {
+      if (s0 + g >= nv) continue;
 #pragma unroll
-        for (int i = 0; i < NF4; ++i) {
-          const float4 f = v[g][i].get();
-          ss[g] += f.x * f.x + f.y * f.y + f.z * f.z + f.w * f.w;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
+      for (int i = 0; i < NF4; ++i) {
+        const float4 f = v[g][i].get();
+        ss[g] += f.x * f.x + f.y * f.y + f.z * f.z + f.w * f.w;
       }
-      __syncthreads();  // wsum of the previous group fully read
-      if (lane == 0) {
+    }
+    // G sums over the warp at once: in each of the first steps a lane passes on half of its sums and keeps the other
+    // half (xor 16, 8, 4, 2, 1 for every sum, as in G separate trees, but in G + 4 - LG shuffles instead of 5 * G)
+    int o = 16;
 #pragma unroll
-        for (int g = 0; g < G; ++g) wsum[g][warp] = ss[g];
+    for (int h = G / 2; h >= 1; h >>= 1, o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int g = 0; g < h; ++g) {
+        const float keep = up ? ss[g + h] : ss[g], send = up ? ss[g] : ss[g + h];
+        ss[g] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
-      __syncthreads();
+    }
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float tot = 0.f;
+    for (int r = 16 >> LG; r > 0; r >>= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], r);
+    if (s0 > 0) __syncthreads();  // wsum of the previous group fully read
+    if ((lane & ((32 >> LG) - 1)) == 0) wsum[lane >> (5 - LG)][warp] = ss[0];
+    __syncthreads();
 #pragma unroll
-        for (int w = 0; w < COMBINE_THREADS / 32; ++w) tot += wsum[g][w];  // fixed order
-        wgt[g] *= rsqrtf(tot / static_cast<float>(H) + eps);
+    for (int g = 0; g < G; ++g) {
+      if (s0 + g >= nv) continue;
+      float tot = 0.f;
+#pragma unroll
+      for (int w = 0; w < COMBINE_THREADS / 128; ++w) {  // fixed order
+        const float4 f = reinterpret_cast<const float4*>(wsum[g])[w];
+        tot += f.x; tot += f.y; tot += f.z; tot += f.w;
       }
+      wgt[g] *= rsqrtf(tot / static_cast<float>(H) + eps);
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {  // slot order within the group
@@ -1115,6 +1213,37 @@ int msk_moe_workspace_view(const MskMoeCfg* cfg, void* workspace, int which, voi
   return MSK_OK;
 }
 
+// y_bf16: the 128-token tile keeps y in BF16 (half the bytes written and read back).
+static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, const int32_t* inv, const float* tw, void* out,
+                          int n_tokens, bool post_norm, int pdl, cudaStream_t st) {
+  cudaLaunchConfig_t lc{};
+  lc.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = pdl;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  const int H = static_cast<int>(cfg->hidden), k = static_cast<int>(cfg->top_k);
+  if (!post_norm) {
+    const bool few_local = static_cast<long long>(k) * cfg->local_count <= 2LL * cfg->n_experts;   // two or fewer of a token's routes expected
+    const int cols = few_local ? 1024 : 256;
+    const long long items = static_cast<long long>(n_tokens) * ((H + cols - 1) / cols);
+    lc.gridDim = dim3(static_cast<unsigned>((items + COMBINE_COLS_WARPS - 1) / COMBINE_COLS_WARPS));
+    lc.blockDim = dim3(COMBINE_COLS_WARPS * 32);
+    auto* kern = y_bf16 ? (few_local ? combine_cols_kernel<true, 2, 4> : combine_cols_kernel<true, 8, 1>)
+                        : (few_local ? combine_cols_kernel<false, 2, 4> : combine_cols_kernel<false, 8, 1>);
+    return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, n_tokens, H, k));
+  }
+  lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
+  lc.blockDim = dim3(COMBINE_THREADS);
+  const bool wide = n_tokens >= COMBINE_WIDE_TOKENS;
+  const bool narrow_rows = H <= COMBINE_THREADS * 2 * 4;   // two float4 slots per thread hold a row
+  auto* kern = y_bf16 ? (narrow_rows ? combine_norm_kernel<8, true, 2, 2> : combine_norm_kernel<4, true, 2>)
+                      : (wide ? combine_norm_kernel<2, false, 2> : combine_norm_kernel<4, false, 1>);
+  return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, H, k, cfg->post_norm_eps));
+}
+
 // ev, when given, holds 6 events: [0] before the step, [1] after routing + sort, [5] after the row copy,
 // [2] after the gate/up GEMM, [3] after the down GEMM, [4] after the combine.
 static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* packed2, const float* gs13,
@@ -1367,27 +1496,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (cfg->stop_after == 3) return MSK_OK;
   }
 
-  {
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
-    lc.blockDim = dim3(COMBINE_THREADS);
-    lc.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    const bool wide = n_tokens >= COMBINE_WIDE_TOKENS;
-    // the wide tile keeps y in BF16: half the bytes written and read back
-    const bool narrow_rows = cfg->hidden <= COMBINE_THREADS * 2 * 4;   // two float4 slots per thread hold a row
-    auto* kern = plan.N == 128 ? (narrow_rows ? combine_kernel<8, true, 2, 2> : combine_kernel<4, true, 2>)
-                          : (wide ? combine_kernel<2, false, 2> : combine_kernel<4, false, 1>);
-    e = static_cast<int>(cudaLaunchKernelEx(&lc, kern, static_cast<const float*>(y),
-                                            static_cast<const int32_t*>(inv), topk_weights,
-                                            static_cast<__nv_bfloat16*>(out), static_cast<int>(cfg->hidden),
-                                            static_cast<int>(cfg->top_k), post_norm_w != nullptr ? 1 : 0,
-                                            cfg->post_norm_eps));
-  }
+  e = launch_combine(cfg, plan.N == 128, y, inv, topk_weights, out, n_tokens, post_norm_w != nullptr, pdl, st);
   if (ev) cudaEventRecord(ev[4], st);
   return e;
 }
@@ -1567,10 +1676,7 @@ int msk_moe_forward_static(const MskMoeCfg* cfg, const void* packed13, const voi
   if (e != 0) return e;
   e = launch_gemm_n<1>(16, p, grid, st, 1);
   if (e != 0) return e;
-  combine_kernel<4, false, 1><<<static_cast<unsigned>(n_tokens), COMBINE_THREADS, 0, st>>>(
-      y, inv, topk_weights, static_cast<__nv_bfloat16*>(out), cfg->hidden, cfg->top_k, post_norm_w != nullptr ? 1 : 0,
-      cfg->post_norm_eps);
-  return static_cast<int>(cudaGetLastError());
+  return launch_combine(cfg, false, y, inv, topk_weights, out, n_tokens, post_norm_w != nullptr, 0, st);
 }
 
 int msk_moe_share_pieces(int n_base, int n_stages, int shares, int flat, int cta, int heavy, int skip, int* host_out,
@@ -1662,7 +1768,7 @@ int msk_moe_attrs(int which, int token_tile, int* host_out) {
       }
       break;
     }
-    case 4: e = cudaFuncGetAttributes(&a, combine_kernel<4, false, 1>); break;
+    case 4: e = cudaFuncGetAttributes(&a, combine_norm_kernel<4, false, 1>); break;
     default: return MSK_ERR_SHAPE;
   }
   if (e != cudaSuccess) return static_cast<int>(e);
