@@ -1090,18 +1090,7 @@ int msk_moe_route(const MskMoeCfg* cfg, const float* logits, const float* bias, 
 
 static int launch_sort(const MskMoeCfg* cfg, const int32_t* ids, int n_tokens, int32_t* cnt, int32_t* off,
                        int32_t* perm, int32_t* inv, cudaStream_t st, const __nv_bfloat16* x = nullptr,
-                       __half* xh = nullptr, int32_t* blk = nullptr, const void* pre_w = nullptr, float pre_eps = 0.f) {
-  const int n_entries = n_tokens * cfg->top_k;
-  if (blk != nullptr && xh == nullptr && n_entries >= SORT_MULTI_MIN) {
-    // many entries: the same stable sort on several CTAs (count, scan, scatter)
-    const int nb = SORT_MULTI_BLOCKS;
-    sort_multi_count_kernel<<<nb, SORT_THREADS, sizeof(SortSmem), st>>>(ids, n_entries, cfg->local_start,
-                                                                        cfg->local_count, blk);
-    sort_multi_scan_kernel<<<1, MAX_LOCAL_EXPERTS, 0, st>>>(blk, nb, cfg->local_count, cnt, off);
-    sort_multi_scatter_kernel<<<nb, SORT_THREADS, sizeof(SortSmem), st>>>(ids, n_entries, cfg->local_start,
-                                                                          cfg->local_count, blk, perm, inv);
-    return static_cast<int>(cudaGetLastError());
-  }
+                       __half* xh = nullptr, const void* pre_w = nullptr, float pre_eps = 0.f) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1125,6 +1114,28 @@ static int launch_sort(const MskMoeCfg* cfg, const int32_t* ids, int n_tokens, i
                                              static_cast<int>(cfg->local_start), static_cast<int>(cfg->local_count),
                                              cnt, off, perm, inv, x, xh, n_tokens, static_cast<int>(cfg->hidden),
                                              static_cast<const __nv_bfloat16*>(pre_w), pre_eps));
+}
+
+// Top-k (when logits are given; otherwise ids is only read) and sort on several CTAs (route_sort.cuh).
+static int launch_sort_multi(const MskMoeCfg* cfg, const float* logits, const float* bias, int32_t* ids, float* tw, int n_tokens,
+                             int32_t* cnt, int32_t* off, int32_t* perm, int32_t* inv, int32_t* blk, cudaStream_t st) {
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(static_cast<unsigned>(std::min(SORT_MULTI_BLOCKS, (n_tokens + SORT_MULTI_TOKENS - 1) / SORT_MULTI_TOKENS)));
+  lc.blockDim = dim3(SORT_THREADS);
+  lc.dynamicSmemBytes = sizeof(SortSmem);
+  lc.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  const int k = static_cast<int>(cfg->top_k), lo = static_cast<int>(cfg->local_start), nloc = static_cast<int>(cfg->local_count);
+  const int e = static_cast<int>(cudaLaunchKernelEx(&lc, sort_multi_count_kernel, logits, bias, ids, tw, n_tokens,
+                                                    static_cast<int>(cfg->n_experts), k, static_cast<int>(cfg->routing_mode),
+                                                    cfg->route_scale, lo, nloc, blk));
+  if (e != 0) return e;
+  return static_cast<int>(cudaLaunchKernelEx(&lc, sort_multi_scatter_kernel, static_cast<const int32_t*>(ids), n_tokens, k, lo,
+                                             nloc, static_cast<const int32_t*>(blk), cnt, off, perm, inv));
 }
 
 constexpr int FUSED_ROUTE_MAX_TOKENS = 32;  // up to here one CTA routes and sorts in a single launch
@@ -1408,6 +1419,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (logits != nullptr && n_tokens <= FUSED_ROUTE_MAX_TOKENS) {
     e = launch_route_sort(cfg, logits, bias, ids_out, tw_out, n_tokens, cnt, off, perm, inv, st, xin, xh_in_sort,
                           pre_norm_w, pre_norm_eps);
+  } else if (n_tokens > FUSED_ROUTE_MAX_TOKENS && n_tokens * cfg->top_k >= SORT_MULTI_MIN) {
+    e = launch_sort_multi(cfg, logits, bias, const_cast<int32_t*>(topk_ids), tw_out, n_tokens, cnt, off, perm, inv,
+                          reinterpret_cast<int32_t*>(b + k.sort_blk), st);
   } else {
     if (logits != nullptr) {
       route_topk_kernel<<<static_cast<unsigned>((n_tokens + 7) / 8), 256, 0, st>>>(
@@ -1415,8 +1429,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
       e = static_cast<int>(cudaGetLastError());
       if (e != 0) return e;
     }
-    e = launch_sort(cfg, topk_ids, n_tokens, cnt, off, perm, inv, st, xin, xh_in_sort,
-                    reinterpret_cast<int32_t*>(b + k.sort_blk), pre_norm_w, pre_norm_eps);
+    e = launch_sort(cfg, topk_ids, n_tokens, cnt, off, perm, inv, st, xin, xh_in_sort, pre_norm_w, pre_norm_eps);
   }
   if (e != 0) return e;
   if (ev) cudaEventRecord(ev[1], st);

@@ -333,17 +333,21 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_kernel(const int32_t* __res
   sort_entries_block(sm, ids, n, lo, nloc, cnt, off, perm, inv);
 }
 
-// ---- the same stable sort on several CTAs, for many entries (prefill, expert-parallel chunks)
-// CTA b owns the contiguous entry range [b chunk, (b + 1) chunk). Three launches:
-//   count    per-CTA per-expert counts                                   -> blk[b][e]
-//   scan     one CTA: exclusive prefix over (expert, CTA) in that order  -> cnt, off, blk[b][e] = first
-//            sorted position of CTA b's entries of expert e
-//   scatter  each CTA ranks its entries as the single-CTA sort does (warps own ascending
-//            sub-ranges, in-warp rank by match/popc) on top of its bases
+// ---- top-k and the same stable sort on several CTAs, for many entries
+// CTA b owns a contiguous range of tokens, and with it of entries. Two launches:
+//   count    [top-k of its tokens,] per-CTA per-expert counts            -> blk[b][e]
+//   scatter  every CTA sums the counts of all CTAs itself (64 KB of L2 reads, all independent): its first sorted
+//            position of every expert is the exclusive prefix over (expert, CTA) in that order; then
+//            it ranks its entries as the single-CTA sort does (warps own ascending sub-ranges,
+//            in-warp rank by match/popc) on top of that. CTA 0 writes cnt and off.
 // Entries of one expert keep ascending entry order across CTAs, warps and lanes: the same
-// permutation as the single-CTA sort, bit for bit.
-constexpr int SORT_MULTI_MIN = 16384;    // entries from which several CTAs sort
+// permutation as the single-CTA sort, bit for bit. (With one CTA for the scan, whose loop over the 64 CTAs was a
+// chain of dependent loads and stores, a launch of its own for the top-k, and one CTA sorting everything below 16384
+// entries, the tables of 256, 777 and 8192 tokens took 13, 19 and 19 us; now 12, 14 and 15. At 64 tokens, 512
+// entries, one CTA behind the top-k kernel is the faster form: 9 against 12 us.)
+constexpr int SORT_MULTI_MIN = 1024;     // entries from which several CTAs sort
 constexpr int SORT_MULTI_BLOCKS = 64;
+constexpr int SORT_MULTI_TOKENS = 8;     // tokens per CTA while that makes fewer CTAs
 
 // Pass 1 of a CTA over its range: sm.wcnt[w][e] = entries of expert e in warp w's sub-range.
 __device__ __forceinline__ void sort_count_range(SortSmem& sm, const int32_t* ids, int beg, int end, int lo, int nloc,
@@ -365,15 +369,24 @@ __device__ __forceinline__ void sort_count_range(SortSmem& sm, const int32_t* id
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const int32_t* __restrict__ ids, int n, int lo,
-                                                                        int nloc, int32_t* __restrict__ blk) {
+__global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const float* __restrict__ logits,
+                                                                        const float* __restrict__ bias, int32_t* ids,
+                                                                        float* wts, int T, int E, int k, int mode,
+                                                                        float scale, int lo, int nloc, int32_t* blk) {
   extern __shared__ __align__(16) unsigned char sort_smem_raw[];
   SortSmem& sm = *reinterpret_cast<SortSmem*>(sort_smem_raw);
-  const int per = (n + gridDim.x - 1) / gridDim.x;
-  const int beg = min(n, static_cast<int>(blockIdx.x) * per), end = min(n, beg + per);
+  const int per = (T + gridDim.x - 1) / gridDim.x, t0 = min(T, static_cast<int>(blockIdx.x) * per), t1 = min(T, t0 + per);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (logits != nullptr) {
+    for (int t = t0 + warp; t < t1; t += SORT_WARPS)
+      route_token_dispatch(logits + static_cast<size_t>(t) * E, bias, ids + static_cast<size_t>(t) * k,
+                           wts + static_cast<size_t>(t) * k, E, k, mode, scale, lane);
+    __syncthreads();  // the ids are read back below by other threads of this CTA
+  }
   int wbeg, wend;
-  sort_count_range(sm, ids, beg, end, lo, nloc, wbeg, wend);
-  const int tid = threadIdx.x;
+  sort_count_range(sm, ids, t0 * k, t1 * k, lo, nloc, wbeg, wend);
   if (tid < nloc) {
     int acc = 0;
     for (int w = 0; w < SORT_WARPS; ++w) acc += sm.wcnt[w][tid];
@@ -381,56 +394,58 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const in
   }
 }
 
-__global__ void __launch_bounds__(MAX_LOCAL_EXPERTS) sort_multi_scan_kernel(int32_t* __restrict__ blk, int n_blocks,
-                                                                            int nloc, int32_t* __restrict__ cnt,
-                                                                            int32_t* __restrict__ off) {
-  __shared__ int wsum[MAX_LOCAL_EXPERTS / 32];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int total = 0;
-  if (tid < nloc) {
-    for (int b = 0; b < n_blocks; ++b) {
-      const int c = blk[b * MAX_LOCAL_EXPERTS + tid];
-      blk[b * MAX_LOCAL_EXPERTS + tid] = total;
-      total += c;
-    }
-    cnt[tid] = total;
-  }
-  int incl = total;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) wsum[warp] = incl;
-  __syncthreads();
-  int ex = incl - total;
-  for (int w = 0; w < warp; ++w) ex += wsum[w];
-  if (tid < nloc) {
-    off[tid] = ex;
-    if (tid == nloc - 1) off[nloc] = ex + total;
-    for (int b = 0; b < n_blocks; ++b) blk[b * MAX_LOCAL_EXPERTS + tid] += ex;
-  }
-}
-
-__global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const int32_t* __restrict__ ids, int n, int lo,
-                                                                          int nloc, const int32_t* __restrict__ blk,
+__global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const int32_t* __restrict__ ids, int T, int k,
+                                                                          int lo, int nloc,
+                                                                          const int32_t* __restrict__ blk,
+                                                                          int32_t* __restrict__ cnt,
+                                                                          int32_t* __restrict__ off,
                                                                           int32_t* __restrict__ perm,
                                                                           int32_t* __restrict__ inv) {
   extern __shared__ __align__(16) unsigned char sort_smem_raw[];
   SortSmem& sm = *reinterpret_cast<SortSmem*>(sort_smem_raw);
-  const int per = (n + gridDim.x - 1) / gridDim.x;
-  const int beg = min(n, static_cast<int>(blockIdx.x) * per), end = min(n, beg + per);
-  int wbeg, wend;
-  sort_count_range(sm, ids, beg, end, lo, nloc, wbeg, wend);
+  const int per = (T + gridDim.x - 1) / gridDim.x, t0 = min(T, static_cast<int>(blockIdx.x) * per), t1 = min(T, t0 + per);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < nloc) {   // exclusive prefix over the warps, and this CTA's base of the expert
-    int acc = 0;
-    for (int w = 0; w < SORT_WARPS; ++w) {
-      const int c = sm.wcnt[w][tid];
-      sm.wcnt[w][tid] = acc;
-      acc += c;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  int before = 0, total = 0;   // entries of expert tid in the CTAs before this one, and in all
+  if (tid < nloc) {
+#pragma unroll 16
+    for (int b = 0; b < static_cast<int>(gridDim.x); ++b) {
+      const int c = __ldg(blk + b * MAX_LOCAL_EXPERTS + tid);
+      before += b < static_cast<int>(blockIdx.x) ? c : 0;
+      total += c;
     }
-    sm.tot[tid] = blk[blockIdx.x * MAX_LOCAL_EXPERTS + tid];
+  }
+  int wbeg, wend;
+  sort_count_range(sm, ids, t0 * k, t1 * k, lo, nloc, wbeg, wend);
+  if (tid < MAX_LOCAL_EXPERTS) {
+    if (tid < nloc) {   // exclusive prefix over the warps
+      int acc = 0;
+      for (int w = 0; w < SORT_WARPS; ++w) {
+        const int c = sm.wcnt[w][tid];
+        sm.wcnt[w][tid] = acc;
+        acc += c;
+      }
+    }
+    int incl = total;   // exclusive scan of the totals over the experts (8 warps x 32)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) sm.wsum[warp] = incl;
+    sm.tot[tid] = incl - total;
+  }
+  __syncthreads();
+  if (tid < MAX_LOCAL_EXPERTS) {
+    int ex = sm.tot[tid];
+    for (int w = 0; w < warp; ++w) ex += sm.wsum[w];
+    sm.tot[tid] = ex + before;
+    if (blockIdx.x == 0 && tid < nloc) {
+      cnt[tid] = total;
+      off[tid] = ex;
+      if (tid == nloc - 1) off[nloc] = ex + total;
+    }
   }
   __syncthreads();
   for (int base = wbeg; base < wend; base += 32) {
