@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
   constexpr int PH_FIRST = MODE == 1 ? 1 : 0, PH_LAST = MODE == 0 ? 0 : 1;
   constexpr bool FUSED = MODE == 2;
   constexpr bool TMA_B = C::TMA_B;
-  static_assert(!(FUSED && (TMA_B || NDBUF == 1)), "the one-launch mode is built for the narrow token tiles");
+  static_assert(!(FUSED && NDBUF == 1), "the one-launch mode is built for token tiles up to 64");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* ring = smem;                                        // NST x [tile g0 | tile g1 | B]
   GemmCtrl& ctl = *reinterpret_cast<GemmCtrl*>(smem + NST * C::STAGE_BYTES + C::LUT_BYTES);
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
   //    GEMM fill up during the tail of the gate/up GEMM.
   //  * MODE 2 is the whole step: it reads its inputs next, so it waits here.
   if ((MODE == 0 && p.route == 0) || FUSED) pdl_wait();
-  if (FUSED) {
+  if (FUSED && !TMA_B) {   // (the 64-token tile reads the sorted copy made by the kernel before)
     // F16 copy of the token rows, a slice per CTA; the gather warps wait for all slices (stage 1 of
     // the grid counter) before their first read
     const int n8 = p.T * (p.ph[0].K / 8);
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (FUSED && tid == 0) atomicAdd(p.grid_bar, 1u);  // this CTA's slice of the F16 rows is in memory
+  if (FUSED && !TMA_B && tid == 0) atomicAdd(p.grid_bar, 1u);  // this CTA's slice of the F16 rows is in memory
 
   const uint32_t tmem = ctl.tmem_base;
   if (tid == 0) MSK_TR(TR_SETUP);
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     if (tid == 0) MSK_TR(TR_FOLD_END);
   }
   if (tid == 0) MSK_TR(TR_END);
-  if (FUSED && tid == 0 && ctl.abort_word == 0) {
+  if (FUSED && !TMA_B && tid == 0 && ctl.abort_word == 0) {
     // the last CTA to leave puts the grid counters back to zero for the next launch
     const unsigned int old = atomicAdd(p.grid_bar + 1, 1u);
     if (old == n_ctas - 1u) {

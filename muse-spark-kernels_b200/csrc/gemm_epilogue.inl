@@ -151,6 +151,7 @@
           // this unit's columns of inter are complete; count it for its token tile, whose down units (the
           // second phase of this launch, or the down GEMM launched behind it) wait for the count to reach
           // the number of gate/up pairs
+          if (TMA_B) fence_proxy_async_all();   // its readers are bulk copies
           __threadfence();
           if (!epi_sync()) { ok = false; break; }
           if (finish && tid == 128) { atomicAdd(p.tile_done + ui.tile, 1u); MSK_TRD(3, tri, 7); }

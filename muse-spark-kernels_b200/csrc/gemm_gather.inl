@@ -129,10 +129,24 @@
       MSK_PHASES {
         MSK_PHASE_SETUP;
         if (MODE == 1) pdl_wait();  // inter comes from the gate/up GEMM
+        int last_tile = -1;
+        (void)last_tile;
         while (ok && pieces.next(base, ks0, ks1)) {
           const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
           const int h = ui.rows <= 16 ? 0 : ui.rows <= 32 ? 1 : ui.rows <= 64 ? 2 : 3;
           const CUtensorMap* map = &p.tmap_act[phase][h];
+          if (FUSED && phase == 1) {   // the gate/up units of this token tile, as above
+            if (ui.tile != last_tile) {
+              if (!grid_counter_wait(p.tile_done + ui.tile, static_cast<unsigned>(p.ph[0].n_pairs), abortw)) { ok = false; break; }
+              fence_proxy_async_all();   // ordinary stores of other SMs, about to be read by bulk copies
+              last_tile = ui.tile;
+            }
+            const unsigned seen = atomicAdd(p.tile_seen + ui.tile, 1u);
+            if (seen == static_cast<unsigned>(pp.n_pairs) - 1u) {
+              atomicExch(p.tile_done + ui.tile, 0u);
+              atomicExch(p.tile_seen + ui.tile, 0u);
+            }
+          }
           for (int ks = ks0; ks < ks1; ++ks, ++it) {
             const uint32_t slot = it % NST, par = (it / NST) & 1u;
             if (!MSK_WAIT(&ctl.b_empty[slot], par ^ 1u, abortw)) { ok = false; break; }

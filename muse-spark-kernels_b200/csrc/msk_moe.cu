@@ -651,6 +651,7 @@ struct Plan {
   int path;      // 0 one launch, 1 chain of launches, 2 row copy + routing gate/up kernel + combining down kernel
   int flat;      // equal shares of the flat (base unit, K stage) list
   int grid;
+  bool both;     // both GEMMs in one launch: path 4, and the 64-token tile of path 1
 };
 
 static Plan make_plan(const MskMoeCfg* c, int T) {
@@ -699,9 +700,15 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   // down units, tile by tile, and the kernel makes its own F16 copy of the token rows), then the combine.
   // Measured at H4096 I1536 E128 (stamped runs): 16 / 32 / 64 / 128 tokens 176 / 227 / 253 / 268 us against
   // 186 / 240 / 258 / 270 for two GEMM launches with the per-tile hand-over between them. Same bits.
-  if (p.path == 1 && p.N <= 32 && p.flat == 0 && c->stop_after == 0 && p.grid <= sm_count() &&
+  const bool resident = p.flat == 0 && c->stop_after == 0 && p.grid <= sm_count();
+  if (p.path == 1 && p.N <= 32 && resident &&
       (c->decode_path == 4 || (c->decode_path == 0 && T >= BOTH_GEMMS_MIN_TOKENS)))
     p.path = 4;
+  // The 64-token tile keeps the row copy in front of the GEMMs and shares one launch between them as well, unless the
+  // chain is asked for: 256 tokens 279 us against 287. For the 128-token tile the same was built and
+  // slower (777 tokens 556 against 524 us, 8192 tokens 2890 against 2764): its units are long, few CTAs stand idle
+  // between the two launches, and the decode warps, which drain the accumulators there, lose more to the hand-over.
+  p.both = p.path == 4 || (p.path == 1 && p.N == 64 && resident && c->decode_path != 1);
   return p;
 }
 
@@ -842,6 +849,7 @@ static int launch_gemm_fused(int N, const GemmParams& p, int grid, cudaStream_t 
   switch (N) {
     case 16: return launch_gemm<16, 2>(p, grid, st, 0);
     case 32: return launch_gemm<32, 2>(p, grid, st, 0);
+    case 64: return launch_gemm<64, 2>(p, grid, st, 0);
     default: return MSK_ERR_SHAPE;
   }
 }
@@ -1412,7 +1420,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   int e = 0;
   // narrow token tiles read an F16 copy of x; for few tokens the sorting CTA makes it
   const bool tma_b = plan.N >= 64;  // GemmCfg<N>::TMA_B
-  const bool both_gemms = plan.path == 4 && pre_norm_w == nullptr;   // the pre-expert norm needs the row-copy kernel
+  const bool both_gemms = plan.both && (tma_b || pre_norm_w == nullptr);   // narrow tiles: the pre-expert norm needs the row-copy kernel
   const bool convert_in_sort = !tma_b && !both_gemms && n_tokens <= FUSED_ROUTE_MAX_TOKENS;
   const __nv_bfloat16* xin = convert_in_sort ? static_cast<const __nv_bfloat16*>(x) : nullptr;
   __half* xh_in_sort = convert_in_sort ? xs : nullptr;
@@ -1435,19 +1443,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (ev) cudaEventRecord(ev[1], st);
   if (cfg->stop_after == 1) return MSK_OK;
 
-  if (both_gemms) {
-    p.route = 0; p.fold = 0; p.flat = 0;
-    p.x_bf16 = static_cast<const __nv_bfloat16*>(x);
-    p.T = n_tokens;
-    p.grid_bar = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
-    p.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);
-    p.tile_seen = p.tile_done + max_tiles(cfg, cfg->max_tokens);
-    if (ev) cudaEventRecord(ev[5], st);
-    e = launch_gemm_fused(plan.N, p, plan.grid, st);
-    if (e != 0) return e;
-    if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); }
-  } else {
-  if (!convert_in_sort) {
+  if (!convert_in_sort && (tma_b || !both_gemms)) {
     // F16 copy of the token rows: sorted (expert-major) for the TMA tiles, plain [T, H] otherwise
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(static_cast<unsigned>(tma_b ? n_tokens * cfg->top_k : n_tokens));
@@ -1482,6 +1478,17 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     }
   }
   if (ev) cudaEventRecord(ev[5], st);
+  if (both_gemms) {
+    p.route = 0; p.fold = 0; p.flat = 0;
+    p.x_bf16 = static_cast<const __nv_bfloat16*>(x);
+    p.T = n_tokens;
+    p.grid_bar = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
+    p.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);
+    p.tile_seen = p.tile_done + max_tiles(cfg, cfg->max_tokens);
+    e = launch_gemm_fused(plan.N, p, plan.grid, st);
+    if (e != 0) return e;
+    if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); }
+  } else {
   // Tile hand-over: the down GEMM's CTAs start on the SMs the gate/up CTAs leave (programmatic launch) and
   // would then wait for that whole grid, whose last CTAs run a unit longer than the others (the units do not
   // divide evenly): a tenth of the gate/up time with every SM but a few idle. Instead each down unit waits
@@ -1490,9 +1497,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   // keep a producing one off the machine), whole units (a cut unit would be counted once per piece) and
   // both launches of the step. Narrow token tiles only, where the gather warp does the waiting: measured at
   // H4096 I1536 E128, 16 / 32 / 64 / 128 tokens take 187 / 242 / 257 / 270 us with it against 190 / 248 /
-  // 266 / 274 without. With the wide tiles, whose weight producer also fetches the activation tiles and so
-  // would stand still at every new token tile, the same hand-over was slower (256 tokens 326 against 320 us,
-  // 8192 tokens 2.62 against 2.58 ms) and is not built.
+  // 266 / 274 without. With the 128-token tile the same hand-over was slower (8192 tokens 2.62 against 2.58 ms) and is
+  // not built; the 64-token tile shares one launch between its GEMMs.
   p.handover = (pdl != 0 && !tma_b && plan.flat == 0 && plan.grid <= sm_count() && cfg->stop_after == 0) ? 1 : 0;
   if (handover_env_off()) p.handover = 0;
   p.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);

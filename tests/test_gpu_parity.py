@@ -396,6 +396,29 @@ def test_top_k_and_sort_on_several_ctas(cuda_dev, T, E, k, lo, nloc):
     _check_forward(out, ref, parts, views)
 
 
+@pytest.mark.parametrize("tile,path,post,H,I", [(64, 0, False, 512, 256), (64, 1, True, 768, 512), (128, 0, True, 512, 256),
+                                                (128, 0, False, 768, 512)])
+def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
+    """The 64- and 128-token tiles around the heights of their activation boxes and the columns of their epilogue
+    warps, the narrower one in one launch and in two, twice on one state; tokens with up to 12 routes for the combine."""
+    m, inputs, _lib, orc = _mods()
+    counts = [1, 15, 16, 17, 32, 33, 48, 0, 64, 65, 127, 128, 129]
+    T, E = 131, len(counts)
+    w = inputs.make_weights(H, I, E, 61, cuda_dev, post_norm=post)
+    st = m.prepare(w, n_experts=E, top_k=E, max_tokens=T, token_tile=tile, decode_path=path)
+    g = torch.Generator(device=cuda_dev).manual_seed(67)
+    ids = torch.stack([torch.where(torch.randperm(T, generator=g, device=cuda_dev) < c, e, -1) for e, c in enumerate(counts)], 1)
+    ids = ids.to(torch.int32).contiguous()
+    tw = torch.rand((T, E), generator=g, device=cuda_dev)
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    for _ in range(2):
+        out = m.kernel_fn({"hidden_states": x, "topk_ids": ids, "topk_weights": tw}, st)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        ref, parts = orc.moe_forward(x, ids, tw, w, return_parts=True)
+        _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
 def test_graphed_step_with_pinned_host_inputs(cuda_dev):
     """GraphedStep (static buffers + CUDA graph) returns what kernel_fn returns, bit for bit, for
     device inputs and for pinned host inputs, call after call."""
