@@ -70,7 +70,40 @@
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(sfa[0]), "=r"(sfa[1]), "=r"(sfa[2]), "=r"(sfa[3])
                        : "r"(tile_row + OCT_CODE_BYTES));
-          {
+          if constexpr (N == 128) {
+            // The 128-token tile has two slots per tile, a K stage in all, and between the MMAs that free a slot and those
+            // that use it again lie the decode that is left, the stores and the hand-over: two of the four
+            // chunks are decoded before the wait (one: 777 tokens 467 us, two: 444, three: 467; 3012 tokens at
+            // the layer shape 600, 533, 600 in a long run). With the accumulators of the 64-token tile the A ring is
+            // not what the MMAs wait for (256 tokens 279, 281, 288 us), so it keeps the form below.
+            uint32_t o[2][16];
+            auto decode = [&](int c, uint32_t (&d)[16]) {
+              uint32_t q[4];
+              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
+                           : "r"(tile_row + (kh * 4 + c) * 128));
+              const uint32_t sfw = kh ? (c < 2 ? sfa[2] : sfa[3]) : (c < 2 ? sfa[0] : sfa[1]);
+              decode_chunk(q, (c & 1) ? (sfw >> 16) : sfw, d);
+            };
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              decode(c, o[c]);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(o[c][j]));   // here, not behind the wait
+            }
+            if (!MSK_WAIT(&ctl.a_empty[g][as], apar ^ 1u, abortw)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (c >= 2) decode(c, o[c & 1]);
+              tmem_st16(a_tmem + as * C::SLOT_COLS + c * 16, o[c & 1]);
+            }
+            pending_slot = as;
+            retire();   // right behind the stores: the MMAs of this half can start
+            if (it == 0 && tid == 256) MSK_TR(TR_FIRST_AFULL);
+            as += 2;
+            if (as >= NSLOT) { as -= NSLOT; apar ^= 1u; }
+          } else {
             // this warp's slot of the stage: K half kh = chunks 4*kh .. 4*kh+3
 #pragma unroll
             for (int c = 0; c < 4; ++c) {

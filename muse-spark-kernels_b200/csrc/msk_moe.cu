@@ -663,12 +663,14 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     p.N = c->token_tile;
   } else {
     const double rpe = static_cast<double>(T) * c->top_k / c->n_experts;  // mean tokens per expert
-    // measured at H4096 I1536 E128 (us a step with 16 / 32 / 64-token tiles; the narrow ones with both GEMMs
-    // in one launch): T = 160 (rpe 10): 281 / 313 / 307; T = 192 (rpe 12): 301 / 321 / 311; T = 256 (rpe 16):
-    // 381 / 334 / 317; T = 384: 526 / 372 / 338; T = 512 (rpe 32): 648 / 510 / 352. The 16-token tile is the
-    // fastest per K stage and wins while most experts fit one tile; past that the 64-token tile does; the
+    // measured at H4096 I1536 E128 (us a step with 16 / 64 / 128-token tiles, near-even routing): T = 160 (rpe 10):
+    // 268 / 281 / 370; T = 192 (rpe 12): 313 / 302 / 390; T = 512 (rpe 32): - / 352 / 428; T = 640 (rpe 40): - / 374 /
+    // 440; T = 900 (rpe 56): - / 450 / 466; T = 1024 (rpe 64): - / 594 / 504. The 16-token tile is the fastest per K stage
+    // and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The host does not
+    // know the counts, and the less even they are the lower that line lies: with a few experts taking most tokens
+    // T = 512 takes 322 / 330 and T = 640 428 / 424, with a random router T = 777 (rpe 49) 536 / 524 in all. The
     // 32-token tile never wins at these shapes (it stays selectable with cfg.token_tile)
-    p.N = rpe <= 12 ? 16 : rpe <= 32 ? 64 : 128;
+    p.N = rpe <= 12 ? 16 : rpe <= 40 ? 64 : 128;
   }
   const long long rows = static_cast<long long>(T) * c->top_k;
   // Flat shares are an option, off by default: measured on B200 a cut unit's pieces cost about 6 us of
