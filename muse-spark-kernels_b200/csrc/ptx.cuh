@@ -153,33 +153,6 @@ __device__ __forceinline__ bool mbar_wait_short(uint64_t* bar, uint32_t parity, 
   return mbar_wait(bar, parity, abort_word);
 }
 
-// Bounded wait that polls without parking: for hand-overs whose wake-up latency is the pace of the kernel.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
-  const uint32_t addr = smem_u32(bar);
-  uint64_t t0 = 0;
-  uint32_t polls = 0;
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((++polls & 1023u) == 0u) {
-      if (*abort_word != 0) return false;
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > MSK_WAIT_LIMIT_NS) {
-        *abort_word = 1;
-        return false;
-      }
-    }
-  }
-}
-
 // Non-blocking probe of a phase (mbarrier.test_wait): true when the phase has completed. Unlike
 // try_wait it never suspends the thread, so it tells whether a wait that follows will have to wait.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
@@ -220,11 +193,6 @@ __device__ __forceinline__ int ld_acquire_cta(const int* p) {
 }
 __device__ __forceinline__ void st_release_cta(int* p, int v) {
   asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 
 // ----------------------------------------------------- bulk copy (TMA, 1-D)
