@@ -346,7 +346,8 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     R = T * k
     plan = moe.plan(state, T)
     one_launch = plan[1] == 0 and T <= 32 and R <= 256
-    both_gemms = plan[1] == 4     # sort launch(es), both GEMMs in one launch, combine
+    # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine
+    both_gemms = plan[1] == 4 or (plan[0] == 64 and not plan[2] and state["cfg"].decode_path != 1)
     step_bytes = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(steps)) / steps
     step_flops = inputs.algorithmic_flops(H, I, R)
     if one_launch:
@@ -355,12 +356,12 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": alg * NCU_TRAFFIC_RATIO,
                 "traffic_source": "ncu dram bytes of a weight-streaming GEMM capture / its algorithmic bytes (1.015), scaled",
-                "kernel": "moe_gemm_kernel<N,2> (whole step in one launch)",
+                "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if T <= 3 else "moe_gemm_kernel<N,2>"),
                 "peak_source": peaks["source"] + " (burst copy)"}
     elif both_gemms:
-        # both GEMMs in one launch: the touched experts' tiles of both, x read and converted, inter written and
-        # read back, y written
-        alg = mean_touched * (3 * I * H * 0.5625 + 8) + 4.0 * T * H + 4.0 * R * I + 4.0 * R * H
+        # both GEMMs in one launch: the touched experts' tiles of both, x read and converted (64-token tile: the sorted
+        # rows read), inter written and read back, y written
+        alg = mean_touched * (3 * I * H * 0.5625 + 8) + (2.0 * R * H if plan[0] == 64 else 4.0 * T * H) + 4.0 * R * I + 4.0 * R * H
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": alg * NCU_TRAFFIC_RATIO,
@@ -387,10 +388,10 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
         launches = 1
     elif plan[1] == 2 and T <= 32 and R <= 256:
         launches = 3      # row copy, gate/up kernel (routes, sorts), down kernel (combines)
-    elif both_gemms:      # [top-k +] sort (one launch up to 32 tokens), both GEMMs, combine
-        launches = 3 if T <= 32 else 4
-    else:                 # [top-k +] sort (one launch up to 32 tokens, three from 16384 entries), row copy, two GEMMs, combine
-        launches = 4 if T <= 32 else 6 + (2 if T * k >= 16384 else 0)
+    elif both_gemms:      # top-k and sort (one launch up to 32 tokens, two beyond), [row copy,] both GEMMs, combine
+        launches = (3 if T <= 32 else 4) + (1 if plan[0] == 64 else 0)
+    else:                 # top-k and sort, row copy (in the sort launch up to 32 tokens), two GEMMs, combine
+        launches = 4 if T <= 32 else 6
     return {
         "workload": spec["name"], "tokens": T, "steps": steps, "ms_per_step": total_ms / steps,
         "value": T / sec, "unit": UNIT,
@@ -688,9 +689,9 @@ def run_ep(args, spec, dev):
             "e2e": {"value": T * world * args.steps / (ms_e2e * 1e-3), "unit": UNIT,
                     "h2d_bytes_per_step": (T * H * 2 + T * E * 4) * world, "d2h_bytes_per_step": T * H * 2 * world,
                     "ms_per_step": ms_e2e / args.steps},
-            # per rank and step: top-k, the final rank-order sum, and per chunk the sort (three launches from
-            # 16384 entries on), the F16 row copy, two GEMMs and the combine
-            "gpu_launches": (2 + sum(7 if m * T * k >= 16384 else 5 for m in mod.sizes)) * args.steps * world,
+            # per rank and step: top-k, the final rank-order sum, and per chunk the sort (two launches from
+            # 1024 entries on), the F16 row copy, two GEMMs and the combine
+            "gpu_launches": (2 + sum(6 if m * T * k >= 1024 else 5 for m in mod.sizes)) * args.steps * world,
             "ep_parity_max_rel": ep_parity, "ep_parity_tokens_per_rank": CHECK,
             "single_gpu_same_shape_ms": float(single_ms.item()),
             "scaling_efficiency": float(single_ms.item()) / step_ms,
