@@ -108,22 +108,29 @@ struct FewCtl {
   uint8_t tile_rows[FEW_ENTRIES];
 };
 
-// Bounded wait for a mailbox to be emptied (one lane).
-__device__ __forceinline__ bool mail_wait_empty(int* box, volatile int* abort_word) {
-  uint64_t t0 = 0;
-  uint32_t polls = 0;
-  while (ld_acquire_cta(box) != 0) {
-    if ((++polls & 1023u) == 0u) {
-      if (*abort_word != 0) return false;
+// Waits of a whole warp. Every lane polls for itself (and so acquires what the barrier publishes), but the warp
+// has one outcome: lanes that gave up one by one would leave the others behind in full-warp instructions, and
+// without lane 0 a copy would start on a barrier that expects no bytes.
+__device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word)) != 0;
+}
+
+// Lane 0 puts `value` into a mailbox once it is empty (a bounded wait); the outcome goes to the whole warp.
+__device__ __forceinline__ bool warp_mail_post(int* box, int value, volatile int* abort_word, int lane) {
+  int ok = 1;
+  if (lane == 0) {
+    uint64_t t0 = 0;
+    uint32_t polls = 0;
+    while (ld_acquire_cta(box) != 0) {
+      if ((++polls & 1023u) != 0u) continue;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;
-      if (now - t0 > MSK_WAIT_LIMIT_NS) {
-        *abort_word = 1;
-        return false;
-      }
+      if (now - t0 > MSK_WAIT_LIMIT_NS) *abort_word = 1;
+      if (*abort_word != 0) { ok = 0; break; }
     }
+    if (ok) st_release_cta(box, value);
   }
-  return true;
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
 // Which gate/up units a CTA takes. CTAs below n_light take w_light units in every super-round, the others
@@ -552,7 +559,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
     it.start(deal, n_gate, warp);
     int slot = 0;
     uint32_t par = 0;
-    bool ok = ctl.abort_word == 0;
+    bool ok = __all_sync(0xffffffffu, *abortw == 0);
     const uint4 no_x[8] = {};
     uint8_t* parts = smem + p.part_off + (2 * team * FEW_TEAM) * p.part_bytes;
     uint32_t n_unit = 0;
@@ -563,7 +570,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       const uint8_t* xk = xb + ctl.row_x[row0 + min(r, rows - 1)] + q * 16 + kb_a * (KS * 2);
       float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
       for (int kb = kb_a; kb < kb_b; kb += slot_kb) {
-        if (!mbar_wait(&full[slot], par, abortw)) { ok = false; break; }
+        if (!warp_mbar_wait(&full[slot], par, abortw)) { ok = false; break; }
         const uint8_t* w = ring + slot * slot_bytes;
         for (int b = min(slot_kb, kb_b - kb); b > 0; --b, xk += KS * 2, w += FEW_KB_BYTES)
           few_block<false>(d0, d1, w, w + OCT_BYTES, xk, no_x, lane);
@@ -574,14 +581,14 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       if (!ok) break;
       // the team meets: the warps take turns in adding the four partials (in K order) and finishing the unit
       const uint32_t pb = n_unit & 1u, pp = (n_unit >> 1) & 1u;
-      if (!mbar_wait(&ctl.part_empty[team][pb], pp ^ 1u, abortw)) { ok = false; break; }
+      if (!warp_mbar_wait(&ctl.part_empty[team][pb], pp ^ 1u, abortw)) { ok = false; break; }
       uint8_t* pbuf = parts + pb * FEW_TEAM * p.part_bytes + (q * 8 + r) * 16;
       if (2 * q < rows)
         *reinterpret_cast<float4*>(pbuf + part * p.part_bytes) = make_float4(d0[0] + d1[0], d0[1] + d1[1], d0[2] + d1[2], d0[3] + d1[3]);
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.part_full[team][pb]);
       if (part == static_cast<int>(n_unit % FEW_TEAM)) {
-        if (!mbar_wait(&ctl.part_full[team][pb], pp, abortw)) { ok = false; break; }
+        if (!warp_mbar_wait(&ctl.part_full[team][pb], pp, abortw)) { ok = false; break; }
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         if (2 * q < rows) {
 #pragma unroll
@@ -596,11 +603,8 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
         if (2 * q < rows) dst[0] = inter_value(silu_f(s.x * gs) * (s.z * gs));
         if (2 * q + 1 < rows) dst[p.I] = inter_value(silu_f(s.y * gs) * (s.w * gs));
         __syncwarp();
-        if (lane == 0) {   // the box is empty unless the signalling warp lags a whole unit behind
-          if (!mail_wait_empty(&ctl.mail[team], abortw)) ok = false;
-          st_release_cta(&ctl.mail[team], t + 1);
-        }
-        __syncwarp();
+        // (the box is empty unless the signalling warp lags a whole unit behind)
+        if (!warp_mail_post(&ctl.mail[team], t + 1, abortw, lane)) { ok = false; break; }
       }
     }
     if (tid == 0) MSK_TR(TR_LAST_DFULL);
@@ -623,7 +627,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       for (int c = 0; c < 8; ++c) xn[c] = __ldcg(reinterpret_cast<const uint4*>(xk + c * 64));
       float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
       for (int kb = 0; kb < n_kb2; kb += slot_kb) {
-        if (!mbar_wait(&full[slot], par, abortw)) { ok = false; break; }
+        if (!warp_mbar_wait(&full[slot], par, abortw)) { ok = false; break; }
         const uint8_t* w = ring + slot * slot_bytes;
         for (int b = 0; b < min(slot_kb, n_kb2 - kb); ++b, w += FEW_KB_BYTES) {
           uint4 xc[8];

@@ -441,3 +441,27 @@ def test_timeline_stamp_slots_follow_the_kernel_enum():
     for name, slot in timeline.STAMPS:
         assert slots[name] == slot, name
     assert {n for n, _ in timeline.STAMPS} == set(slots)
+
+
+def _kernel_body(name, kernel):
+    """Source text of a kernel, comments and string literals left out."""
+    src = open(os.path.join(ROOT, "muse-spark-kernels_b200", "csrc", name)).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    at = src.index("{", src.index(")", src.index(kernel + "(")))
+    depth = 0
+    for i in range(at, len(src)):
+        depth += {"{": 1, "}": -1}.get(src[i], 0)
+        if depth == 0:
+            return src[at:i + 1]
+    raise AssertionError(kernel)
+
+
+def test_few_token_kernel_gives_up_a_warp_at_a_time():
+    """A bounded wait of moe_few_kernel that runs out must send the whole warp the same way: the kernel body
+    waits on its barriers and mailboxes through the warp-wide forms only, and those end in a warp vote or a
+    broadcast."""
+    body = _kernel_body("few.cuh", "moe_few_kernel")
+    waits = re.findall(r"\b\w*mbar_(?:try_)?wait\w*|\b\w*mail_\w+", body)
+    assert len(waits) >= 5 and set(waits) == {"warp_mbar_wait", "warp_mail_post"}
+    assert "__all_sync" in _kernel_body("few.cuh", "bool warp_mbar_wait")
+    assert "__shfl_sync" in _kernel_body("few.cuh", "bool warp_mail_post").split("return")[-1]

@@ -784,6 +784,36 @@ def test_bounded_wait_runs_out_cleanly_and_the_state_recovers(cuda_dev):
         assert m.read_status(st) == 0
 
 
+@pytest.mark.parametrize("T,post", [(1, False), (2, True)])
+def test_few_token_kernel_gives_up_cleanly_and_recovers(cuda_dev, T, post):
+    """A tile counter of the few-token kernel left one short (what a step that gave up can leave behind): the down units'
+    wait for that tile runs out (one second), the kernel comes back by itself with the time-out status, the
+    context stays usable, and after reinit_workspace the state gives the clean bits again."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1024, 2048, 16, 8     # every team has gate/up units to do before its first down unit
+    w = inputs.make_weights(H, I, E, 8, cuda_dev, post_norm=post)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
+    g = torch.Generator(device=cuda_dev).manual_seed(4)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    clean = m.kernel_fn(data, st).clone()
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    ptr = ctypes.c_void_p()
+    _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 8, ctypes.byref(ptr)),
+               "view")
+    tile0 = ptr.value - st["workspace"].data_ptr() + 4352     # per-tile counters of the few-token paths
+    st["workspace"][tile0:tile0 + 4].fill_(255)               # -1: the tile's last unit will not complete it
+    m.kernel_fn(data, st)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 1
+    m.reinit_workspace(st)
+    for _ in range(2):
+        assert torch.equal(m.kernel_fn(data, st), clean)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+
+
 def test_state_dict_round_trip_skips_the_repack(cuda_dev):
     """state_dict() / load_state_dict(): the packed tiles, scales and configuration are enough to
     rebuild a state; kernel_fn on the rebuilt state gives the same bits."""
