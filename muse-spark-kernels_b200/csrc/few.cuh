@@ -115,6 +115,16 @@ __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word)) != 0;
 }
 
+// Lane 0 waits for a counter in global memory; the barrier behind the broadcast, which orders no memory by itself,
+// passes on to the other lanes what lane 0 acquired.
+__device__ __forceinline__ bool warp_counter_wait(const unsigned int* ctr, unsigned int target, volatile int* abort_word, int lane) {
+  int ok = 1;
+  if (lane == 0) ok = grid_counter_spin(ctr, target, abort_word) ? 1 : 0;
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();
+  return ok != 0;
+}
+
 // Lane 0 puts `value` into a mailbox once it is empty (a bounded wait); the outcome goes to the whole warp.
 __device__ __forceinline__ bool warp_mail_post(int* box, int value, volatile int* abort_word, int lane) {
   int ok = 1;
@@ -404,9 +414,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
     const int xw = warp - FEW_ROUTE_WARPS, wpr = p.T == 1 ? XW : p.T == 2 ? XW / 2 : 1;
     const int i_first = (xw % wpr) * 32 + lane, i_step = wpr * 32, n16 = p.H / 8;
     if (p.share_x) {
-      int go = 1;
-      if (lane == 0) go = grid_counter_spin(p.ctl + 2, static_cast<unsigned int>(n_ctas), abortw);
-      go = __shfl_sync(0xffffffffu, go, 0);
+      const bool go = warp_counter_wait(p.ctl + 2, static_cast<unsigned int>(n_ctas), abortw, lane);
       for (int t = xw / wpr; t < p.T && go; t += XW / wpr) {
         const uint4* src = reinterpret_cast<const uint4*>(p.xs + static_cast<size_t>(t) * p.H);
         uint4* dst = reinterpret_cast<uint4*>(xb + t * x_stride);
@@ -620,9 +628,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
         o1 *= 1.0f + __bfloat162float(p.post_w[col + 128]);
       }
       const uint8_t* xk = reinterpret_cast<const uint8_t*>(p.inter + static_cast<size_t>(row0 + min(r, rows - 1)) * p.I) + q * 16;
-      int go = 1;
-      if (lane == 0) go = grid_counter_spin(p.tile_done + t, static_cast<unsigned int>(oct1), abortw);
-      if (!__shfl_sync(0xffffffffu, go, 0)) { ok = false; break; }
+      if (!warp_counter_wait(p.tile_done + t, static_cast<unsigned int>(oct1), abortw, lane)) { ok = false; break; }
 #pragma unroll
       for (int c = 0; c < 8; ++c) xn[c] = __ldcg(reinterpret_cast<const uint4*>(xk + c * 64));
       float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};

@@ -67,6 +67,7 @@
                             : grid_counter_wait(p.tile_done + ui.tile, static_cast<unsigned>(p.ph[0].n_pairs), abortw);
           }
           go = __shfl_sync(0xffffffffu, go, 0);
+          __syncwarp();   // the shuffle orders no memory: the other lanes copy rows that lane 0 has acquired
           if (!go) { ok = false; break; }
           if (lane == 0) MSK_TRD(4, tri, 1 + phase);
           first_piece = must_wait || phase == 1;

@@ -465,3 +465,16 @@ def test_few_token_kernel_gives_up_a_warp_at_a_time():
     assert len(waits) >= 5 and set(waits) == {"warp_mbar_wait", "warp_mail_post"}
     assert "__all_sync" in _kernel_body("few.cuh", "bool warp_mbar_wait")
     assert "__shfl_sync" in _kernel_body("few.cuh", "bool warp_mail_post").split("return")[-1]
+
+
+def test_kernels_read_other_ctas_rows_behind_a_barrier():
+    """Rows that other CTAs wrote are read by all lanes after lane 0 acquired their counter: a shuffle orders no
+    memory, so the wait ends in __syncwarp() (the one of the norm sums, by a single thread, in __syncthreads())."""
+    body = _kernel_body("few.cuh", "moe_few_kernel")
+    waits = [m.end() for m in re.finditer(r"\bwarp_counter_wait\(", body)]
+    assert len(waits) == 2
+    assert re.findall(r"\bgrid_counter_spin\([^;]*;\s*\}\s*(\w+)", body) == ["__syncthreads"] * body.count("grid_counter_spin(")
+    tail = _kernel_body("few.cuh", "bool warp_counter_wait")
+    assert tail.index("__shfl_sync") < tail.index("__syncwarp")
+    gather = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "muse-spark-kernels_b200", "csrc", "gemm_gather.inl")).read())
+    assert re.findall(r"go = __shfl_sync\([^;]*;\s*(\w+)", gather) == ["__syncwarp"]
