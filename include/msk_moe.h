@@ -223,6 +223,12 @@ int msk_moe_static_status(int* host_status, void* stream);
  * token count the same way (muse_moe_w4a16/py/03_kernel_fn.py:33-40). */
 int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out);
 
+/* Whether a step of n_tokens runs in the few-token kernel (a form of path 0): *host_fits = 1 or 0. inputs: the bits
+ * below. No GPU needed. No counterpart in the reference. */
+#define MSK_FEW_GIVEN_IDS 1   /* topk_ids and topk_weights are given, no router logits */
+#define MSK_FEW_PRE_NORM 2    /* msk_moe_forward_prenorm */
+int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_fits);
+
 /* How the GEMM kernels deal their work (host-side twin of the device code, a test hook): the pieces
  * that CTA `cta` of `shares` gets from n_base base units of n_stages K stages each. flat == 0: whole
  * units, round-robin; flat != 0: equal shares of the flat (unit, stage) list. host_out receives six

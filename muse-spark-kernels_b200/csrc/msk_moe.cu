@@ -860,6 +860,7 @@ static int launch_gemm_fused(int N, const GemmParams& p, int grid, cudaStream_t 
 struct FewPlan {
   int n_slots, slot_kb, part_bytes, n_light, w_light, w_heavy;
   int xb_off, ys_off, part_off, ctl_off, smem;
+  uint32_t inv_oct1;
 };
 
 // Tokens up to which the few-token kernel is the faster one (H4096 I1536 E128 top-8, us inside the launch, against
@@ -868,10 +869,15 @@ struct FewPlan {
 // norm the alternative is three launches, and the line lies higher.
 constexpr int FEW_BEST_TOKENS = 3, FEW_BEST_TOKENS_PRENORM = 6;
 
-// False when the step does not fit: more than eight tokens, or token rows and owned output rows that leave
-// less than two K blocks per warp (74 KB in flight per SM).
+// False when the step does not fit: more than eight tokens, token rows and owned output rows that leave less than
+// two K blocks per warp (55 KB in flight per SM), or so many gate/up units that their tile number by the
+// reciprocal of I / 8 could be one too large: u * ceil(2^32 / n) / 2^32 has the integer part u / n as long as u times
+// the reciprocal's excess stays below 2^32 (nothing below I = 53,000 is refused by this).
 static bool few_plan(const MskMoeCfg* c, int T, bool given_ids, int grid, FewPlan* f) {
   if (T > FEW_TOKENS || T * c->top_k > FEW_ENTRIES) return false;
+  const uint64_t oct1 = static_cast<uint64_t>(c->inter) / 8, inv = ((1ull << 32) + oct1 - 1) / oct1;
+  if (static_cast<uint64_t>(T) * c->top_k * oct1 * (inv * oct1 - (1ull << 32)) >= (1ull << 32)) return false;
+  f->inv_oct1 = static_cast<uint32_t>(inv);
   const int groups = c->hidden / (2 * OCT_ROWS), own = (groups + grid - 1) / grid;
   const int x_bytes = T * (c->hidden * 2 + 64), ys_bytes = T * c->top_k * own * 64;
   // rows of a tile: one per token when the top-k is taken here; given ids may repeat an expert
@@ -910,6 +916,12 @@ static bool few_plan(const MskMoeCfg* c, int T, bool given_ids, int grid, FewPla
     }
   }
   return true;
+}
+
+// Whether a step of path 0 runs in the few-token kernel; inputs: MSK_FEW_* bits.
+static bool few_takes(const MskMoeCfg* c, int T, int inputs, int grid, FewPlan* f) {
+  return T <= ((inputs & MSK_FEW_PRE_NORM) != 0 ? FEW_BEST_TOKENS_PRENORM : FEW_BEST_TOKENS) &&
+         few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
 }
 
 static int launch_few(const FewParams& p, int grid, int smem, cudaStream_t st) {
@@ -1322,8 +1334,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   p.post_norm_w = static_cast<const __nv_bfloat16*>(post_norm_w);
   p.eps = cfg->post_norm_eps;
   FewPlan few;
-  if (plan.path == 0 && n_tokens <= (pre_norm_w != nullptr ? FEW_BEST_TOKENS_PRENORM : FEW_BEST_TOKENS) &&
-      few_plan(cfg, n_tokens, logits == nullptr, plan.grid, &few)) {
+  const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0);
+  if (plan.path == 0 && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
     f.gs13 = gs13; f.gs2 = gs2;
@@ -1340,7 +1352,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     f.lo = cfg->local_start; f.nloc = cfg->local_count; f.mode = cfg->routing_mode; f.route_scale = cfg->route_scale;
     f.route = logits != nullptr ? 1 : 2;
     f.share_x = cfg->host_inputs != 0 && pre_norm_w == nullptr ? 1 : 0;
-    f.inv_oct1 = static_cast<uint32_t>(((1ull << 32) + cfg->inter / 8 - 1) / (cfg->inter / 8));
+    f.inv_oct1 = few.inv_oct1;
     f.n_slots = few.n_slots; f.slot_kb = few.slot_kb; f.part_bytes = few.part_bytes; f.part_off = few.part_off;
     f.n_light = few.n_light; f.w_light = few.w_light; f.w_heavy = few.w_heavy;
     f.xb_off = few.xb_off; f.ys_off = few.ys_off; f.ctl_off = few.ctl_off;
@@ -1751,6 +1763,17 @@ int msk_l2_sweep(const void* buf, size_t bytes, uint32_t* sink, void* stream) {
 #define MSK_BUILD_ID "unknown"
 #endif
 const char* msk_build_id(void) { return MSK_BUILD_ID; }
+
+int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_fits) {
+  const int rc = check_cfg(cfg);
+  if (rc != MSK_OK) return rc;
+  if (!host_fits) return MSK_ERR_NULL;
+  if (n_tokens < 1) return MSK_ERR_SHAPE;
+  FewPlan f;
+  const Plan p = make_plan(cfg, n_tokens);
+  *host_fits = p.path == 0 && few_takes(cfg, n_tokens, inputs, p.grid, &f) ? 1 : 0;
+  return MSK_OK;
+}
 
 int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out) {
   const int rc = check_cfg(cfg);

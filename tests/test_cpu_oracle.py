@@ -307,6 +307,34 @@ def test_plan_is_a_function_of_the_configuration_only():
     assert lib.msk_moe_plan(ctypes.byref(cfg), 64, plan) == 0 and tuple(plan) == (16, 1, 0, 37)
 
 
+def _few_fits(T, inputs=0, **shape):
+    from muse_moe_w4a16 import _lib
+
+    cfg = _lib.MskMoeCfg(**dict(dict(local_start=0, max_tokens=64), **shape))
+    fits = ctypes.c_int(-1)
+    assert _lib.load().msk_moe_few_fits(ctypes.byref(cfg), T, inputs, ctypes.byref(fits)) == 0
+    return bool(fits.value)
+
+
+@pytest.mark.parametrize("T,k,inputs", [(1, 1, 0), (3, 8, 0), (1, 16, 1), (6, 16, 2), (6, 16, 3)])
+def test_few_token_kernel_numbers_its_tiles_exactly(T, k, inputs):
+    """moe_few_kernel finds the tile of gate/up unit u as the high half of u * ceil(2^32 / (I / 8)): where a step is
+    accepted that is u // (I / 8) for every unit it can have (at most one tile per routed row), and wider experts go to
+    another kernel. Sizes: the usual ones, around the line for 96 rows, and around those for 24, 16 and one."""
+    widths = [256, 1536, 4096, 8192, 14336, 28672] + [256 * i for i in range(200, 240)] + [256 * i for i in range(410, 440)] \
+        + [256 * i for i in range(500, 540)] + [256 * i for i in range(2040, 2060)]
+    seen = set()
+    for width in widths:
+        fits = _few_fits(T, inputs, hidden=256, inter=width, n_experts=64, local_count=64, top_k=k)
+        n = width // 8
+        inv = -(-2 ** 32 // n)
+        last = np.arange(1, T * k + 1, dtype=object) * n - 1          # the last unit of every tile goes wrong first
+        exact = all((int(u) * inv) >> 32 == int(u) // n for u in last)
+        assert fits == exact or (not fits and width > 53000), width
+        seen.add(fits)
+    assert True in seen and (k * T < 96 or False in seen)
+
+
 def test_workspace_init_covers_every_control_word():
     """msk_moe_workspace_init zeroes everything in front of `inter`: the status word, the sort tables,
     both ticket regions, the control words of the few-token paths (token tickets, grid and tile
