@@ -294,8 +294,8 @@ template <> struct YOct<true> {
 constexpr int COMBINE_COLS_WARPS = 4;
 template <bool YB, int G, int C>
 __global__ void __launch_bounds__(COMBINE_COLS_WARPS * 32)
-    combine_cols_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv, const float* __restrict__ tw,
-                        __nv_bfloat16* __restrict__ out, int T, int H, int k) {
+    combine_cols_kernel(const float* y, const int32_t* inv, const float* tw, __nv_bfloat16* __restrict__ out, int T, int H,
+                        int k) {   // (what earlier launches of the chain write is not __restrict__: coherent loads)
   const int lane = threadIdx.x & 31, chunks = (H + C * 256 - 1) / (C * 256);
   const long long item = static_cast<long long>(blockIdx.x) * COMBINE_COLS_WARPS + (threadIdx.x >> 5);
   const int t = static_cast<int>(item / chunks), col = static_cast<int>(item % chunks) * (C * 256) + lane * 8;

@@ -369,7 +369,9 @@ __device__ __forceinline__ void sort_count_range(SortSmem& sm, const int32_t* id
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const float* __restrict__ logits,
+// (The logits may come from a launch of this chain that still runs when this one starts, as ids and blk of the scatter
+// kernel do: ordinary coherent loads behind the wait, not the read-only path, so none of them is __restrict__.)
+__global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const float* logits,
                                                                         const float* __restrict__ bias, int32_t* ids,
                                                                         float* wts, int T, int E, int k, int mode,
                                                                         float scale, int lo, int nloc, int32_t* blk) {
@@ -394,9 +396,8 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_multi_count_kernel(const fl
   }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const int32_t* __restrict__ ids, int T, int k,
-                                                                          int lo, int nloc,
-                                                                          const int32_t* __restrict__ blk,
+__global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const int32_t* ids, int T, int k, int lo, int nloc,
+                                                                          const int32_t* blk,
                                                                           int32_t* __restrict__ cnt,
                                                                           int32_t* __restrict__ off,
                                                                           int32_t* __restrict__ perm,
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const 
   if (tid < nloc) {
 #pragma unroll 16
     for (int b = 0; b < static_cast<int>(gridDim.x); ++b) {
-      const int c = __ldg(blk + b * MAX_LOCAL_EXPERTS + tid);
+      const int c = __ldcg(blk + b * MAX_LOCAL_EXPERTS + tid);
       before += b < static_cast<int>(blockIdx.x) ? c : 0;
       total += c;
     }
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_multi_scatter_kernel(const 
 
 // Routing and sort in one launch for small token counts: every warp routes the tokens
 // t = warp, warp + 32, ...; after a block barrier the same CTA sorts the entries it just wrote.
-__global__ void __launch_bounds__(SORT_THREADS) route_sort_kernel(const float* __restrict__ logits,
+__global__ void __launch_bounds__(SORT_THREADS) route_sort_kernel(const float* logits,
                                                                   const float* __restrict__ bias,
                                                                   int32_t* __restrict__ ids, float* __restrict__ wts,
                                                                   int T, int E, int k, int mode, float scale, int lo,

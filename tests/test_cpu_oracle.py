@@ -506,3 +506,18 @@ def test_kernels_read_other_ctas_rows_behind_a_barrier():
     assert tail.index("__shfl_sync") < tail.index("__syncwarp")
     gather = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "muse-spark-kernels_b200", "csrc", "gemm_gather.inl")).read())
     assert re.findall(r"go = __shfl_sync\([^;]*;\s*(\w+)", gather) == ["__syncwarp"]
+
+
+@pytest.mark.parametrize("name,kernel,written", [("route_sort.cuh", "sort_multi_scatter_kernel", ("ids", "blk")),
+                                                 ("route_sort.cuh", "sort_multi_count_kernel", ("logits",)),
+                                                 ("route_sort.cuh", "route_sort_kernel", ("logits",)),
+                                                 ("msk_moe.cu", "combine_cols_kernel", ("y", "inv", "tw"))])
+def test_what_the_launch_before_writes_is_read_coherently(name, kernel, written):
+    """A kernel started by programmatic launch is there while its predecessor still writes: what that one writes must
+    not go through the read-only path, which __ldg asks for and const __restrict__ allows."""
+    src = open(os.path.join(ROOT, "muse-spark-kernels_b200", "csrc", name)).read()
+    at = re.search(kernel + r"\((const)", src).start()
+    args = src[at:src.index(")", at)]
+    for arg in written:
+        assert not re.search(r"__restrict__ " + arg + r"\b", args), arg
+        assert not re.search(r"__ldg\([^;]*\b" + arg + r"\b", _kernel_body(name, kernel)), arg
