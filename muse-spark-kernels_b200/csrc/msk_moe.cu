@@ -1162,6 +1162,12 @@ static int launch_sort_multi(const MskMoeCfg* cfg, const float* logits, const fl
 
 constexpr int FUSED_ROUTE_MAX_TOKENS = 32;  // up to here one CTA routes and sorts in a single launch
 
+static bool sort_on_several_ctas(const MskMoeCfg* cfg, int n_tokens) {
+  const long long entries = static_cast<long long>(n_tokens) * cfg->top_k;
+  return n_tokens > FUSED_ROUTE_MAX_TOKENS &&
+         (entries >= SORT_MULTI_MIN || entries * cfg->local_count >= static_cast<long long>(SORT_MULTI_MIN_LOCAL) * cfg->n_experts);
+}
+
 static int launch_route_sort(const MskMoeCfg* cfg, const float* logits, const float* bias, int32_t* ids, float* tw,
                              int n_tokens, int32_t* cnt, int32_t* off, int32_t* perm, int32_t* inv, cudaStream_t st,
                              const __nv_bfloat16* x, __half* xh, const void* pre_w = nullptr, float pre_eps = 0.f) {
@@ -1441,7 +1447,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (logits != nullptr && n_tokens <= FUSED_ROUTE_MAX_TOKENS) {
     e = launch_route_sort(cfg, logits, bias, ids_out, tw_out, n_tokens, cnt, off, perm, inv, st, xin, xh_in_sort,
                           pre_norm_w, pre_norm_eps);
-  } else if (n_tokens > FUSED_ROUTE_MAX_TOKENS && n_tokens * cfg->top_k >= SORT_MULTI_MIN) {
+  } else if (sort_on_several_ctas(cfg, n_tokens)) {
     e = launch_sort_multi(cfg, logits, bias, const_cast<int32_t*>(topk_ids), tw_out, n_tokens, cnt, off, perm, inv,
                           reinterpret_cast<int32_t*>(b + k.sort_blk), st);
   } else {

@@ -345,7 +345,12 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_kernel(const int32_t* __res
 // chain of dependent loads and stores, a launch of its own for the top-k, and one CTA sorting everything below 16384
 // entries, the tables of 256, 777 and 8192 tokens took 13, 19 and 19 us; now 12, 14 and 15. At 64 tokens, 512
 // entries, one CTA behind the top-k kernel is the faster form: 9 against 12 us.)
-constexpr int SORT_MULTI_MIN = 1024;     // entries from which several CTAs sort
+// From how many entries on: one CTA's time grows with the entries it walks, and more with those that have a local
+// expert. Tables of a whole step with small experts, one CTA / several: all experts local, 1600 entries 33.7 / 35.1 us with
+// ids given (36.7 / 37.6 with logits), 2048 35.5 / 34.6 (39.3 / 37.9), 4096 45.4 / 42.0 (51.0 / 46.7); one local expert in
+// eight, 1600 entries 19.7 / 23.7 (24.6 / 27.4), 8192 31.8 / 32.7 (38.7 / 37.8), 16376 28.6 / 24.9 (37.9 / 33.9).
+constexpr int SORT_MULTI_MIN_LOCAL = 1792;   // expected entries with a local expert
+constexpr int SORT_MULTI_MIN = 12288;        // or entries in all
 constexpr int SORT_MULTI_BLOCKS = 64;
 constexpr int SORT_MULTI_TOKENS = 8;     // tokens per CTA while that makes fewer CTAs
 

@@ -396,6 +396,29 @@ def test_top_k_and_sort_on_several_ctas(cuda_dev, T, E, k, lo, nloc):
     _check_forward(out, ref, parts, views)
 
 
+@pytest.mark.parametrize("T,E,k,lo,nloc,several", [(425, 300, 5, 20, 256, True),     # 54 CTAs, the last with one token
+                                                   (223, 128, 8, 0, 128, False), (224, 128, 8, 0, 128, True),   # 1784, 1792 local entries
+                                                   (384, 256, 8, 64, 32, False),     # one rank of eight
+                                                   (1535, 256, 8, 0, 8, False), (1536, 256, 8, 0, 8, True)])    # 12280, 12288 entries
+def test_sort_moves_to_several_ctas_where_they_are_faster(cuda_dev, T, E, k, lo, nloc, several):
+    """Few entries with a local expert are sorted by one CTA, many by several (whose counts are what the workspace
+    then holds): the same tables as the oracle's either way, for logits and for the ids they gave."""
+    m, inputs, _lib, orc = _mods()
+    for given in (False, True):
+        out, ref, parts, views, st, (x, ids, tw, w) = _run_forward(m, inputs, orc, cuda_dev, 256, 256, E, k, T, seed=83, lo=lo, nloc=nloc)
+        if given:
+            m.reinit_workspace(st)
+            out = m.kernel_fn({"hidden_states": x, "topk_ids": ids, "topk_weights": tw}, st)
+            torch.cuda.synchronize()
+            views = m.workspace_views(st, T)
+        _check_forward(out, ref, parts, views)
+        ptr = ctypes.c_void_p()
+        _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 9, ctypes.byref(ptr)),
+                   "view")
+        o = ptr.value - st["workspace"].data_ptr()
+        assert bool(st["workspace"][o:o + 64 * 256 * 4].any()) == several
+
+
 @pytest.mark.parametrize("tile,path,post,H,I", [(64, 0, False, 512, 256), (64, 1, True, 768, 512), (128, 0, True, 512, 256),
                                                 (128, 0, False, 768, 512)])
 def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
