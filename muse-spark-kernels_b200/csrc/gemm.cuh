@@ -327,13 +327,11 @@ __device__ __forceinline__ __half inter_value(float v) {
   return __float2half_rn(fminf(fmaxf(r, -65504.f), 65504.f));
 }
 
-// Two SwiGLU values as inter_value gives them, packed (first one in the low half). For the wide token tile, where
-// the dequant warps do this between two units of work: the quotient by reciprocal and the roundings two at a time,
-// 13 instructions a value instead of 30.
+// Two SwiGLU values, bit for bit as inter_value(silu_f(g) * u) gives them, packed (first one in the low half): the
+// roundings and the clamps two at a time. For the wide token tile, where the dequant warps do this between two units of work.
 __device__ __forceinline__ uint32_t inter_pair(uint32_t g0, uint32_t u0, uint32_t g1, uint32_t u1, float gs) {
-  const float a0 = __uint_as_float(g0) * gs, a1 = __uint_as_float(g1) * gs;
-  const float v0 = __fdividef(a0, 1.0f + __expf(-a0)) * (__uint_as_float(u0) * gs);
-  const float v1 = __fdividef(a1, 1.0f + __expf(-a1)) * (__uint_as_float(u1) * gs);
+  const float v0 = silu_f(__uint_as_float(g0) * gs) * (__uint_as_float(u0) * gs);
+  const float v1 = silu_f(__uint_as_float(g1) * gs) * (__uint_as_float(u1) * gs);
   const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
   const __half2 h = __floats2half2_rn(__low2float(b), __high2float(b));
   const __half2 c = __hmin2(__hmax2(h, __half2half2(__ushort_as_half(0xFBFF))), __half2half2(__ushort_as_half(0x7BFF)));   // +-65504

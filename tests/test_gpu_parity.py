@@ -442,6 +442,28 @@ def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
         _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
+@pytest.mark.parametrize("T,scale", [(131, 1.0), (700, 1.0), (300, 60.0)])
+def test_every_token_tile_gives_the_same_swiglu_values(cuda_dev, T, scale):
+    """inter of the 16-, 64- and 128-token tiles, bit for bit: the accumulators sum in the same order and the SwiGLU value
+    is one formula (exactly rounded quotient included), whatever the epilogue. The last case takes gates to where the
+    exponential over- and underflows."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 768, 512, 6, 3
+    w = inputs.make_weights(H, I, E, 91, cuda_dev)
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    x = (torch.randn((T, H), generator=g, device=cuda_dev) * scale).to(torch.bfloat16)
+    logits = torch.randn((T, E), generator=g, device=cuda_dev)
+    got = {}
+    for tile in (16, 64, 128):
+        st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+        m.kernel_fn({"hidden_states": x, "router_logits": logits}, st)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        got[tile] = m.workspace_views(st, T)["inter"]
+    assert torch.isfinite(got[16]).all() and float(got[16].abs().max()) > 0
+    assert torch.equal(got[64], got[16]) and torch.equal(got[128], got[16])
+
+
 def test_graphed_step_with_pinned_host_inputs(cuda_dev):
     """GraphedStep (static buffers + CUDA graph) returns what kernel_fn returns, bit for bit, for
     device inputs and for pinned host inputs, call after call."""
