@@ -74,8 +74,6 @@ typedef struct MskMoeCfg {
   int32_t stop_after;    /* measuring aid: 0 = whole step; 1/2/3 = return after sort / gate-up GEMM / down GEMM */
   int32_t flat_shares;   /* non-zero (with n_tokens * top_k <= 256 and paths 1, 2): the last rounds of the weight stream
                             are cut into equal shares per CTA instead of whole units (see msk_moe_share_pieces) */
-  int32_t host_inputs;   /* non-zero: x of the call lies in pinned host memory, so it is read once by all CTAs together
-                            and not once by each (results do not depend on it) */
 } MskMoeCfg;
 
 /* ---- prepare-time repack (lossless; replaces the four layouts built by
@@ -227,6 +225,7 @@ int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out);
  * below. No GPU needed. No counterpart in the reference. */
 #define MSK_FEW_GIVEN_IDS 1   /* topk_ids and topk_weights are given, no router logits */
 #define MSK_FEW_PRE_NORM 2    /* msk_moe_forward_prenorm */
+#define MSK_FEW_HOST_X 4      /* x lies in host memory */
 int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_fits);
 
 /* How the GEMM kernels deal their work (host-side twin of the device code, a test hook): the pieces

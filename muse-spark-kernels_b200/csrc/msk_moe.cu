@@ -919,9 +919,22 @@ static bool few_plan(const MskMoeCfg* c, int T, bool given_ids, int grid, FewPla
 }
 
 // Whether a step of path 0 runs in the few-token kernel; inputs: MSK_FEW_* bits.
+// Token rows in host memory: the CTAs read them over PCIe once, a slice each, and share an F16 copy. With the pre-expert
+// norm every CTA needs whole rows, and 148 times the bytes over PCIe cost far more than the kernel saves (H4096, 1 / 6
+// tokens 68 / 265 us against 44 / 122): another kernel norms them once.
 static bool few_takes(const MskMoeCfg* c, int T, int inputs, int grid, FewPlan* f) {
+  if ((inputs & MSK_FEW_PRE_NORM) != 0 && (inputs & MSK_FEW_HOST_X) != 0) return false;
   return T <= ((inputs & MSK_FEW_PRE_NORM) != 0 ? FEW_BEST_TOKENS_PRENORM : FEW_BEST_TOKENS) &&
          few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
+}
+
+static bool in_host_memory(const void* p) {   // page-locked, or pageable where the device can read that
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();   // not this call's error
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
 }
 
 static int launch_few(const FewParams& p, int grid, int smem, cudaStream_t st) {
@@ -1340,7 +1353,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   p.post_norm_w = static_cast<const __nv_bfloat16*>(post_norm_w);
   p.eps = cfg->post_norm_eps;
   FewPlan few;
-  const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0);
+  const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
+  const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
+                         (host_x ? MSK_FEW_HOST_X : 0);
   if (plan.path == 0 && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
@@ -1357,7 +1372,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     f.H = cfg->hidden; f.I = cfg->inter; f.T = n_tokens; f.E = cfg->n_experts; f.k = cfg->top_k;
     f.lo = cfg->local_start; f.nloc = cfg->local_count; f.mode = cfg->routing_mode; f.route_scale = cfg->route_scale;
     f.route = logits != nullptr ? 1 : 2;
-    f.share_x = cfg->host_inputs != 0 && pre_norm_w == nullptr ? 1 : 0;
+    f.share_x = host_x ? 1 : 0;
     f.inv_oct1 = few.inv_oct1;
     f.n_slots = few.n_slots; f.slot_kb = few.slot_kb; f.part_bytes = few.part_bytes; f.part_off = few.part_off;
     f.n_light = few.n_light; f.w_light = few.w_light; f.w_heavy = few.w_heavy;

@@ -13,7 +13,6 @@ py/03_kernel_fn.py:18-45). Extensions, all optional:
   pre_norm_w (bf16 [H]) may be present  -> the layer callers' pre-expert RMS norm is applied to x first
 There is no CPU path: tensors must be CUDA tensors and the native library must load.
 """
-import copy
 import ctypes
 
 import torch
@@ -147,7 +146,7 @@ def load_state_dict(sd, device=None):
     the packed weights are taken as they are (those saved in another order are put in order first), so kernel_fn
     gives the same bits as on the state they came from."""
     lib = _lib.load()
-    cfg = MskMoeCfg(**sd["config"])
+    cfg = MskMoeCfg(**{k: v for k, v in sd["config"].items() if k != "host_inputs"})   # a field that some saved states have
     t = {k: (sd[k] if device is None else sd[k].to(device)) for k in _SD_TENSORS if sd.get(k) is not None}
     if not t["packed13"].is_cuda:
         raise RuntimeError("muse_moe_w4a16.load_state_dict: tensors must be CUDA tensors (there is no CPU path)")
@@ -374,8 +373,7 @@ class HostMappedStep:
 
     def __init__(self, state, like):
         self.state = state
-        cfg = self.cfg = copy.deepcopy(state["cfg"])
-        cfg.host_inputs = 1
+        cfg = state["cfg"]
         dev = state["packed13"].device
         if state.get("pre_norm_w") is not None:
             raise RuntimeError("HostMappedStep: states with a pre-expert norm are not supported")
@@ -415,7 +413,7 @@ class HostMappedStep:
 
     def _launch(self, i):
         state, inp = self.state, self.inputs[i]
-        cfg, lib = self.cfg, state["lib"].lib
+        cfg, lib = state["cfg"], state["lib"].lib
         args = (ctypes.byref(cfg), _lib.ptr(state["packed13"]), _lib.ptr(state["packed2"]), _lib.ptr(state["gs13"]),
                 _lib.ptr(state["gs2"]), _lib.ptr(state["post_norm_w"]), _lib.ptr(inp["hidden_states"]))
         tail = (_lib.ptr(self.outs[i]), _lib.ptr(state["workspace"]), state["workspace_bytes"], self.T, _stream())

@@ -44,7 +44,6 @@ class MskMoeCfg(ctypes.Structure):
         ("trace", ctypes.c_int32),
         ("stop_after", ctypes.c_int32),
         ("flat_shares", ctypes.c_int32),
-        ("host_inputs", ctypes.c_int32),
     ]
 
     def __deepcopy__(self, memo):

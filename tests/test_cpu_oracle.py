@@ -335,6 +335,27 @@ def test_few_token_kernel_numbers_its_tiles_exactly(T, k, inputs):
     assert True in seen and (k * T < 96 or False in seen)
 
 
+def test_configuration_struct_is_the_documented_one():
+    """A host compiled against the documented struct must hand over every byte the library reads: the same fields in
+    the same order in the header, the Python binding and the integration guide."""
+    from muse_moe_w4a16 import _lib
+
+    header = open(os.path.join(ROOT, "include", "msk_moe.h")).read()
+    body = re.sub(r"/\*.*?\*/", "", header[header.index("typedef struct MskMoeCfg"):header.index("} MskMoeCfg;")], flags=re.S)
+    fields = re.findall(r"(?:int32_t|float)\s+(\w+);", body)
+    assert fields == [n for n, _ in _lib.MskMoeCfg._fields_]
+    guide = open(os.path.join(ROOT, "INTEGRATION.md")).read()
+    stub = guide[guide.index("class MskMoeCfg"):guide.index("lib = ctypes.CDLL")]
+    assert re.findall(r'"(\w+)"', stub) == fields
+
+
+def test_few_token_kernel_leaves_normed_rows_in_host_memory_to_another():
+    """With the pre-expert norm every CTA of moe_few_kernel reads whole token rows: not over PCIe."""
+    shape = dict(hidden=4096, inter=1536, n_experts=128, local_count=128, top_k=8)
+    assert _few_fits(1, 2, **shape) and _few_fits(1, 4, **shape) and _few_fits(1, 5, **shape)
+    assert not any(_few_fits(T, 2 | 4 | given, **shape) for T in (1, 2, 6) for given in (0, 1))
+
+
 def test_workspace_init_covers_every_control_word():
     """msk_moe_workspace_init zeroes everything in front of `inter`: the status word, the sort tables,
     both ticket regions, the control words of the few-token paths (token tickets, grid and tile

@@ -515,6 +515,36 @@ def test_host_mapped_step_reads_and_writes_pinned_host_memory(cuda_dev, T, route
     assert m.read_status(st) == 0
 
 
+@pytest.mark.parametrize("T,pre", [(1, False), (2, False), (1, True), (3, True)])
+def test_pinned_token_rows_through_the_c_interface(cuda_dev, T, pre):
+    """A host hands msk_moe_forward* pinned token rows and nothing else that says so: the CTAs share one F16 copy of them
+    (it stands in the workspace afterwards), normed ones are read by another kernel, and the output is the one on device tensors."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1024, 512, 16, 4
+    w = inputs.make_weights(H, I, E, 53, cuda_dev, post_norm=True)
+    g = torch.Generator(device=cuda_dev).manual_seed(20 + T)
+    if pre:
+        w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    tw, ids = torch.softmax(torch.randn((T, E), generator=g, device=cuda_dev), dim=-1).topk(k, dim=-1)
+    ids, tw = ids.to(torch.int32).contiguous(), tw.contiguous()
+    want = m.kernel_fn({"hidden_states": x, "topk_ids": ids, "topk_weights": tw}, st)
+    st["workspace"].zero_()
+    xh, out = x.cpu().pin_memory(), torch.empty((T, H), dtype=torch.bfloat16, device=cuda_dev)
+    m._forward(st, st["cfg"], st["lib"].lib, xh.data_ptr(), None, ids.data_ptr(), tw.data_ptr(), out.data_ptr(), T)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    if pre:
+        assert _rel(out, want.float()) <= 8e-3      # two kernels, sums in another order: one BF16 rounding
+    else:
+        assert torch.equal(out, want)
+        row = x[T - 1].to(torch.float16).view(torch.int64)
+        words = st["workspace"].view(torch.int64)
+        at = (words == row[0]).nonzero().flatten()
+        assert any(torch.equal(words[int(a):int(a) + row.numel()], row) for a in at)
+
+
 @pytest.mark.parametrize("T,tile", [(9, 0), (40, 0), (100, 16), (100, 32), (260, 32)])
 def test_both_gemms_in_one_launch_behind_the_sort_gives_the_chain_bits(cuda_dev, T, tile):
     """decode_path = 4 (sort launches, then the gate/up and the down GEMM in one cooperative launch that
@@ -883,6 +913,19 @@ def test_state_dict_round_trip_skips_the_repack(cuda_dev):
     assert torch.equal(m.kernel_fn({"hidden_states": x}, copy.deepcopy(st2)), want)
     back = m.export_weights(st2)
     assert torch.equal(back["w13"], w["w13"]) and torch.equal(back["w2_sf"], w["w2_sf"].view(torch.uint8))
+
+
+def test_state_saved_with_the_host_inputs_field_loads(cuda_dev):
+    """States saved while the configuration had a field host_inputs load like any other."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 512, 256, 8, 2, 3
+    st = m.prepare(inputs.make_weights(H, I, E, 21, cuda_dev), n_experts=E, top_k=k, max_tokens=T)
+    g = torch.Generator(device=cuda_dev).manual_seed(6)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    sd = m.state_dict(st)
+    sd["config"] = dict(sd["config"], host_inputs=0)
+    assert torch.equal(m.kernel_fn(data, m.load_state_dict(sd)), m.kernel_fn(data, st))
 
 
 def test_state_saved_in_128_row_tiles_loads(cuda_dev):
