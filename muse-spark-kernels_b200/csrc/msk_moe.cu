@@ -863,12 +863,6 @@ struct FewPlan {
   uint32_t inv_oct1;
 };
 
-// Tokens up to which the few-token kernel is the faster one (H4096 I1536 E128 top-8, us inside the launch, against
-// the tcgen05 kernel): 1 token 28 / 40, 2: 44 / 43 (but 7 us less outside it), 3: 53 / 52, 4: 71 / 65, 8: 121 / 108:
-// from four tokens on the decode work in its warps sets the pace, not the latencies it saves. With the pre-expert
-// norm the alternative is three launches, and the line lies higher.
-constexpr int FEW_BEST_TOKENS = 3, FEW_BEST_TOKENS_PRENORM = 6;
-
 // False when the step does not fit: more than eight tokens, token rows and owned output rows that leave less than
 // two K blocks per warp (55 KB in flight per SM), or so many gate/up units that their tile number by the
 // reciprocal of I / 8 could be one too large: u * ceil(2^32 / n) / 2^32 has the integer part u / n as long as u times
@@ -918,14 +912,23 @@ static bool few_plan(const MskMoeCfg* c, int T, bool given_ids, int grid, FewPla
   return true;
 }
 
-// Whether a step of path 0 runs in the few-token kernel; inputs: MSK_FEW_* bits.
-// Token rows in host memory: the CTAs read them over PCIe once, a slice each, and share an F16 copy. With the pre-expert
-// norm every CTA needs whole rows, and 148 times the bytes over PCIe cost far more than the kernel saves (H4096, 1 / 6
-// tokens 68 / 265 us against 44 / 122): another kernel norms them once.
+// Whether a step of path 0 runs in the few-token kernel; inputs: MSK_FEW_* bits. It saves latency (prologue, hand-overs,
+// launches) and loses where the decode work in its warps sets the pace: with the touched experts, which the host does not
+// know, so the lines lie where independent routes are no slower than in the tcgen05 kernel. rows: routed rows expected
+// for this rank's experts, T * k * nloc / E. Measured, whole steps in us, this kernel / the other: all of 128 experts
+// (H4096 I1536 top-8, eight rows a token) 3 tokens 62 / 63, with the post-expert norm 69 / 69 (Zipf routes 46 / 55); a
+// rank with one row a token (H4096 I4096) 3: 38 / 50, (H7168 I2048) 32 / 39; a small model (H2048 I1024, four rows) 24 / 38.
+//   Pre-expert norm (the other: three launches): eight rows 4: 89 / 90, 5: 99 / 92 (Zipf, 6: 78 / 96); one row, H4096
+// 5: 59 / 65, H7168 6: 62 / 56 (each CTA holds and norms six such rows); four rows 6: 34 / 41.
+//   Token rows in host memory: the CTAs read them over PCIe once, a slice each, and share an F16 copy, one exchange more,
+// and short runs of output columns go back: eight rows 2: 59 / 66, 3: 76 / 73, with given ids and the post-expert norm
+// 86 / 78; one row 3: 49 / 56; four rows 3: 35 / 43. With the pre-expert norm every CTA needs whole rows, and 148 times the
+// bytes over PCIe cost far more than the kernel saves (eight rows 1: 68 / 44, 6: 265 / 122): another kernel norms them once.
 static bool few_takes(const MskMoeCfg* c, int T, int inputs, int grid, FewPlan* f) {
-  if ((inputs & MSK_FEW_PRE_NORM) != 0 && (inputs & MSK_FEW_HOST_X) != 0) return false;
-  return T <= ((inputs & MSK_FEW_PRE_NORM) != 0 ? FEW_BEST_TOKENS_PRENORM : FEW_BEST_TOKENS) &&
-         few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
+  const bool pre = (inputs & MSK_FEW_PRE_NORM) != 0, host = (inputs & MSK_FEW_HOST_X) != 0;
+  const double rows = static_cast<double>(T) * c->top_k * c->local_count / c->n_experts;
+  const int most = pre ? (host ? 0 : c->hidden <= 4096 && rows <= 24 ? 6 : 4) : host && rows > 16 ? 2 : 3;
+  return T <= most && few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
 }
 
 static bool in_host_memory(const void* p) {   // page-locked, or pageable where the device can read that

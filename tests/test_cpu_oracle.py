@@ -316,12 +316,12 @@ def _few_fits(T, inputs=0, **shape):
     return bool(fits.value)
 
 
-@pytest.mark.parametrize("T,k,inputs", [(1, 1, 0), (3, 8, 0), (1, 16, 1), (6, 16, 2), (6, 16, 3)])
+@pytest.mark.parametrize("T,k,inputs", [(1, 1, 0), (3, 8, 0), (1, 16, 1), (4, 16, 2), (4, 16, 3)])
 def test_few_token_kernel_numbers_its_tiles_exactly(T, k, inputs):
     """moe_few_kernel finds the tile of gate/up unit u as the high half of u * ceil(2^32 / (I / 8)): where a step is
     accepted that is u // (I / 8) for every unit it can have (at most one tile per routed row), and wider experts go to
-    another kernel. Sizes: the usual ones, around the line for 96 rows, and around those for 24, 16 and one."""
-    widths = [256, 1536, 4096, 8192, 14336, 28672] + [256 * i for i in range(200, 240)] + [256 * i for i in range(410, 440)] \
+    another kernel. Sizes: the usual ones, around the line for 64 rows, and around those for 24, 16 and one."""
+    widths = [256, 1536, 4096, 8192, 14336, 28672] + [256 * i for i in range(200, 280)] + [256 * i for i in range(410, 440)] \
         + [256 * i for i in range(500, 540)] + [256 * i for i in range(2040, 2060)]
     seen = set()
     for width in widths:
@@ -332,7 +332,7 @@ def test_few_token_kernel_numbers_its_tiles_exactly(T, k, inputs):
         exact = all((int(u) * inv) >> 32 == int(u) // n for u in last)
         assert fits == exact or (not fits and width > 53000), width
         seen.add(fits)
-    assert True in seen and (k * T < 96 or False in seen)
+    assert True in seen and (k * T < 64 or False in seen)
 
 
 def test_configuration_struct_is_the_documented_one():
@@ -347,6 +347,17 @@ def test_configuration_struct_is_the_documented_one():
     guide = open(os.path.join(ROOT, "INTEGRATION.md")).read()
     stub = guide[guide.index("class MskMoeCfg"):guide.index("lib = ctypes.CDLL")]
     assert re.findall(r'"(\w+)"', stub) == fields
+
+
+@pytest.mark.parametrize("shape,takes", [      # tokens up to which the kernel is taken: plain, rows in host memory, pre-norm
+    (dict(hidden=4096, inter=1536, n_experts=128, local_count=128, top_k=8), (3, 2, 4)),     # eight local routes a token
+    (dict(hidden=4096, inter=4096, n_experts=256, local_count=32, top_k=8), (3, 3, 6)),      # one
+    (dict(hidden=7168, inter=2048, n_experts=256, local_count=32, top_k=8), (3, 3, 4)),      # one, longer rows
+    (dict(hidden=2048, inter=1024, n_experts=64, local_count=64, top_k=4), (3, 3, 6))])      # four
+def test_few_token_kernel_is_taken_where_it_was_measured_faster(shape, takes):
+    for inputs, most in zip((0, 4, 2), takes):
+        for given in (0, 1):
+            assert [T for T in range(1, 9) if _few_fits(T, inputs | given, **shape)] == list(range(1, most + 1)), (inputs, given)
 
 
 def test_few_token_kernel_leaves_normed_rows_in_host_memory_to_another():
