@@ -1082,7 +1082,9 @@ int msk_moe_router_logits(const MskMoeCfg* cfg, const void* x, const float* rout
   if (n_tokens < 0) return MSK_ERR_SHAPE;
   if (n_tokens == 0) return MSK_OK;
   auto* kern = aligned16(x) && aligned16(router_w) ? router_logits_kernel<true> : router_logits_kernel<false>;
-  kern<<<static_cast<unsigned>(cfg->n_experts), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  const dim3 grid(static_cast<unsigned>(cfg->n_experts),
+                  static_cast<unsigned>(std::min((n_tokens + ROUTER_TOKENS - 1) / ROUTER_TOKENS, 65535)));
+  kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), router_w, logits, n_tokens, cfg->hidden, cfg->n_experts);
   return static_cast<int>(cudaGetLastError());
 }

@@ -17,13 +17,15 @@ constexpr int MAX_EXPERTS = 512;
 constexpr int MAX_TOP_K = 16;
 
 // ------------------------------------------------------------------ router
-// One block per expert: the FP32 weight row is read once (four 16-byte loads per thread in flight) for all
-// tokens, each warp takes an eighth of H, and the partial sums of a token meet by a fixed shuffle tree and
+// One block per expert and ROUTER_TOKENS tokens: the FP32 weight row is read once (four 16-byte loads per thread in
+// flight) for all of them, each warp takes an eighth of H, and the partial sums of a token meet by a fixed shuffle tree and
 // then in warp order, so the sum order depends on H only (precedent: muse_decode_layer/cuda/router_fp32.cu:4-40).
-// Bound by the latency of the weight row (2 MB in all at E = 128, H = 4096). A warp per (token, expert) with
-// 4-byte loads, as this was before, took 13 us at two tokens; this form takes 3.
+// Few tokens: bound by the latency of the weight row (2 MB in all at E = 128, H = 4096). A warp per (token, expert) with
+// 4-byte loads, as this was before, took 13 us at two tokens; this form takes 3. Many tokens: bound by L2, which serves
+// 48 KB per block. (With one block per expert for all tokens one after the other 15 / 64 / 1024 tokens took 12.4 / 37.5 /
+// 555 us, now 8.5 / 10.3 / 95; a warp per (token, expert) 10.5 / 16.9 / 175.)
 // VEC = false: weight or token rows that are not 16-byte aligned, the same sums with element-wise loads.
-constexpr int ROUTER_TOKENS = 4;   // tokens whose sums a thread keeps at a time
+constexpr int ROUTER_TOKENS = 4;   // tokens of a block, whose sums each thread keeps at a time
 template <bool VEC>
 __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* __restrict__ x,
                                                             const float* __restrict__ w, float* __restrict__ logits,
@@ -31,7 +33,7 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
   __shared__ float part[8][ROUTER_TOKENS];
   const int e = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* wr = w + static_cast<size_t>(e) * H;
-  for (int t0 = 0; t0 < T; t0 += ROUTER_TOKENS) {
+  for (int t0 = blockIdx.y * ROUTER_TOKENS; t0 < T; t0 += gridDim.y * ROUTER_TOKENS) {
     float acc[ROUTER_TOKENS] = {0.f, 0.f, 0.f, 0.f};
     // a thread takes 4 consecutive h of every 1024 (H is a multiple of 256: the last round may be partial)
     for (int h0 = 0; h0 < H; h0 += 4096) {

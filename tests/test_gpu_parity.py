@@ -1060,6 +1060,32 @@ def test_router_logits_gemm_on_the_hi_lo_pair(cuda_dev, T, E, H):
     assert len(set(rows.tolist())) <= max(1, T // 50)
 
 
+@pytest.mark.parametrize("T,E,H,off", [(5, 130, 768, 0), (15, 8, 256, 1), (263, 16, 4352, 0)])
+def test_router_matvec_of_many_tokens_gives_the_bits_of_each_alone(cuda_dev, T, E, H, off):
+    """msk_moe_router_logits: tokens are spread over blocks of four, the last one ragged; a token's logits are those of a
+    call with that token alone, from aligned and (off = 1) element-aligned rows, and the FP64 product up to FP32 sums."""
+    m, inputs, _lib, orc = _mods()
+    lib = _lib.load()
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    w = torch.randn((E, H), generator=g, device=cuda_dev) * 0.02
+    x = torch.randn((T * H + off,), generator=g, device=cuda_dev).to(torch.bfloat16)[off:].view(T, H)
+    cfg = _lib.MskMoeCfg(hidden=H, inter=256, n_experts=E, local_start=0, local_count=E, top_k=1, max_tokens=T)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def logits(rows):
+        out = torch.full((rows.shape[0], E), float("nan"), device=cuda_dev)
+        _lib.check(lib.msk_moe_router_logits(ctypes.byref(cfg), _lib.ptr(rows), _lib.ptr(w), _lib.ptr(out), rows.shape[0], st),
+                   "router_logits")
+        return out
+
+    got = logits(x)
+    for t in sorted({0, 3, 4, T // 2, T - 1}):
+        assert torch.equal(got[t], logits(x[t:t + 1])[0])
+    want = x.double() @ w.double().T
+    # at most 32 products added up by a thread, five shuffle steps, eight warps: 45 roundings on the way of a product
+    assert bool(((got.double() - want).abs() <= 45 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
+
+
 @pytest.mark.parametrize("T,E,H", [(64, 130, 256),      # four K steps: four CTAs of one step; two tiles of experts
                                    (65, 8, 768),        # twelve steps over eight CTAs
                                    (2051, 128, 256)])   # 128-token tiles, the last with three tokens
