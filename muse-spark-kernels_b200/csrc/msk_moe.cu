@@ -974,7 +974,7 @@ static long long n_og_of(const MskMoeCfg* c, const RepackGeom& g) {   // octet-g
 
 template <int N>
 static int launch_router_hilo(const CUtensorMap& mw, const CUtensorMap& mx, float* logits, int32_t* status, int T, int E,
-                              int H, cudaStream_t st) {
+                              int H, int pdl, cudaStream_t st) {
   const int smem = RG_STAGES * (2 * RG_A_BYTES + N * RG_KSTEP * 2) + static_cast<int>(sizeof(RouterGemmCtrl));
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -995,7 +995,7 @@ static int launch_router_hilo(const CUtensorMap& mw, const CUtensorMap& mx, floa
   lc.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = pdl;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = static_cast<unsigned>(split);
   at[1].val.clusterDim.y = 1;
@@ -1107,11 +1107,12 @@ int msk_moe_router_logits_hilo(const MskMoeCfg* cfg, const void* x, const void* 
   e = encode_act_map(&mx, x, static_cast<size_t>(n_tokens), cfg->hidden, N, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
   if (e != 0) return e;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int pdl = cfg->no_pdl ? 0 : 1;
   switch (N) {
-    case 128: return launch_router_hilo<128>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, st);
-    case 64: return launch_router_hilo<64>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, st);
-    case 32: return launch_router_hilo<32>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, st);
-    default: return launch_router_hilo<16>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, st);
+    case 128: return launch_router_hilo<128>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, pdl, st);
+    case 64: return launch_router_hilo<64>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, pdl, st);
+    case 32: return launch_router_hilo<32>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, pdl, st);
+    default: return launch_router_hilo<16>(mw, mx, logits, status_word, n_tokens, cfg->n_experts, cfg->hidden, pdl, st);
   }
 }
 
@@ -1147,7 +1148,7 @@ static int launch_sort(const MskMoeCfg* cfg, const int32_t* ids, int n_tokens, i
   lc.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = cfg->no_pdl ? 0 : 1;
   lc.attrs = at;
   lc.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&lc, sort_kernel, ids, static_cast<int>(n_tokens * cfg->top_k),
@@ -1166,7 +1167,7 @@ static int launch_sort_multi(const MskMoeCfg* cfg, const float* logits, const fl
   lc.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = cfg->no_pdl ? 0 : 1;
   lc.attrs = at;
   lc.numAttrs = 1;
   const int k = static_cast<int>(cfg->top_k), lo = static_cast<int>(cfg->local_start), nloc = static_cast<int>(cfg->local_count);
@@ -1205,7 +1206,7 @@ static int launch_route_sort(const MskMoeCfg* cfg, const float* logits, const fl
   lc.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = cfg->no_pdl ? 0 : 1;
   lc.attrs = at;
   lc.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&lc, route_sort_kernel, logits, bias, ids, tw, n_tokens,

@@ -608,6 +608,47 @@ def test_okc_ext_runs_the_decode_layer_call_site(cuda_dev):
     assert torch.equal(out2, out)
 
 
+def _programmatic_edges(graph):
+    """Dependencies of a captured graph that are programmatic launches (driver API, CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC)."""
+    driver, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(0)
+    raw = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert driver.cuGraphGetEdges_v2(raw, None, None, None, ctypes.byref(n)) == 0
+    if n.value == 0:
+        return 0
+    src, dst, data = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (ctypes.c_ubyte * (8 * n.value))()
+    assert driver.cuGraphGetEdges_v2(raw, src, dst, data, ctypes.byref(n)) == 0
+    return sum(1 for i in range(n.value) if data[8 * i + 2] == 1)
+
+
+@pytest.mark.parametrize("T,tile", [(24, 16), (40, 16), (300, 64), (300, 128)])     # one CTA sorts, routes apart, several CTAs
+def test_no_step_is_chained_programmatically_when_that_is_switched_off(cuda_dev, T, tile):
+    """okc_set_pdl(0) / cfg.no_pdl: every launch of a step that computes its logits, routes and sorts waits for the
+    whole launch before it; with the switch on some of them do not. Same bits."""
+    from muse_moe_w4a16 import compat
+
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 512, 256, 16, 8
+    w = inputs.make_weights(H, I, E, 57, cuda_dev)
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    w["router"] = torch.randn((E, H), generator=g, device=cuda_dev) * 0.02
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+    outs = []
+    for on in (1, 0):
+        compat.OkcExt(st).okc_set_pdl(on)
+        m.kernel_fn(data, st)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            out = m.kernel_fn(data, st)
+        assert (_programmatic_edges(graph) > 0) == bool(on)
+        graph.instantiate()
+        graph.replay()
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert m.read_status(st) == 0 and torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("T,given_ids", [(3, False), (7, True), (40, True), (300, False), (600, True)])
 def test_forward_with_pre_expert_norm(cuda_dev, T, given_ids):
     """weights["pre_norm_w"]: the layer callers' pre-expert RMS norm (eps 1e-5, x (1 + g)) fused into
