@@ -13,6 +13,7 @@ py/03_kernel_fn.py:18-45). Extensions, all optional:
   pre_norm_w (bf16 [H]) may be present  -> the layer callers' pre-expert RMS norm is applied to x first
 There is no CPU path: tensors must be CUDA tensors and the native library must load.
 """
+import copy
 import ctypes
 
 import torch
@@ -271,13 +272,16 @@ class GraphedStep:
     they reach the device in a single asynchronous copy, and the graph is replayed. Device inputs of the
     types the kernels read are used where they lie: the step's launches are issued on them directly,
     because copying them into the static buffers first put two copies and their gaps (8 us) in front of a
-    one-token step of 30; others are copied tensor by tensor and the graph is replayed. Inputs:
-    hidden_states and either router_logits or topk_ids + topk_weights, whichever `like` holds."""
+    one-token step of 30 (host time of a call, direct / copies and replay: 8 / 13 us up to 8 tokens, 17 / 13 from
+    64 tokens on, where the step takes far longer than either); others are copied tensor by tensor and the
+    graph is replayed. Either way it is the step of the state and configuration at the time of the capture.
+    Inputs: hidden_states and either router_logits or topk_ids + topk_weights, whichever `like` holds."""
 
     STAGES = 4
 
     def __init__(self, state, like):
-        self.state = state
+        # what the graph holds is held here too: later changes of the caller's state reach neither
+        state = self.state = dict(state, cfg=copy.deepcopy(state["cfg"]))
         dev = state["packed13"].device
         self.keys = [k for k in ("hidden_states", "router_logits", "topk_ids", "topk_weights") if like.get(k) is not None]
         spans, total = {}, 0

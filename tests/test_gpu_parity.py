@@ -485,6 +485,70 @@ def test_graphed_step_with_pinned_host_inputs(cuda_dev):
     assert m.read_status(st) == 0
 
 
+def test_graphed_step_runs_one_plan_for_all_inputs(cuda_dev):
+    """A change of the state's configuration after the capture (okc_set_pdl, a forced tile) reaches neither the replays nor
+    the calls launched on device tensors: both give the bits of the captured plan."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 512, 256, 8, 2, 40
+    st = m.prepare(inputs.make_weights(H, I, E, 58, cuda_dev), n_experts=E, top_k=k, max_tokens=T, token_tile=16)
+    g = torch.Generator(device=cuda_dev).manual_seed(11)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    want = m.kernel_fn(data, st).clone()
+    step = m.GraphedStep(st, data)
+    st["cfg"].token_tile = 128                        # keeps y in BF16: other bits
+    assert not torch.equal(m.kernel_fn(data, st), want)
+    assert torch.equal(step({key: v.cpu() for key, v in data.items()}), want)
+    assert torch.equal(step(data), want)
+
+
+@pytest.mark.parametrize("T,routed", [(2, False), (5, True), (40, True)])
+def test_graphed_step_copies_device_tensors_the_kernels_cannot_read(cuda_dev, T, routed):
+    """Device inputs of another type, off their alignment, strided, or some of them on the host are copied into the
+    captured buffers and the graph is replayed: the bits of kernel_fn on the plain tensors, call after call."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 512, 256, 8, 2
+    st = m.prepare(inputs.make_weights(H, I, E, 59, cuda_dev, post_norm=True), n_experts=E, top_k=k, max_tokens=T)
+    g = torch.Generator(device=cuda_dev).manual_seed(13 + T)
+
+    def draw():
+        d = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+        logits = torch.randn((T, E), generator=g, device=cuda_dev).to(torch.bfloat16).float()
+        if routed:
+            tw, ids = torch.softmax(logits, dim=-1).topk(k, dim=-1)
+            d["topk_ids"], d["topk_weights"] = ids.to(torch.int32).contiguous(), tw.contiguous()
+        else:
+            d["router_logits"] = logits
+        return d
+
+    def misaligned(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:]
+        return flat.view(t.shape).copy_(t)
+
+    def strided(t):
+        return torch.stack([t, t], -1)[..., 0]
+
+    step = m.GraphedStep(st, draw())
+    second = "topk_weights" if routed else "router_logits"
+    for form in ("plain", "misaligned", "strided", "type", "host"):
+        d = draw()
+        want = m.kernel_fn(d, st).clone()
+        e = dict(d)
+        if form in ("misaligned", "strided"):
+            e = {key: (misaligned if form == "misaligned" else strided)(v) for key, v in d.items()}
+            assert not step._usable(e)
+        elif form == "type":
+            key = "topk_ids" if routed else "router_logits"
+            e[key] = d[key].long() if routed else d[key].to(torch.bfloat16)      # (values of both survive the change)
+            assert not step._usable(e)
+        elif form == "host":
+            e[second] = d[second].cpu()
+        got = step(e)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want), form
+    assert m.read_status(st) == 0
+
+
 @pytest.mark.parametrize("T,routed", [(1, False), (5, False), (8, True), (40, False)])
 def test_host_mapped_step_reads_and_writes_pinned_host_memory(cuda_dev, T, routed):
     """HostMappedStep (kernels read the inputs from, and write the output to, pinned host memory; no copy
