@@ -739,6 +739,73 @@ def test_forward_with_pre_expert_norm(cuda_dev, T, given_ids):
     assert _rel(out, orc.moe_forward(x, ids, tw, plain).float()) > 0.05   # the norm is not a no-op here
 
 
+@pytest.mark.parametrize("T,H,post,given,sigmoid", [
+    (1, 1280, True, False, False),     # four warps norm one row: sums of squares across warps, an odd number of 256-column steps
+    (1, 256, False, True, False),      # most lanes of those warps have nothing
+    (2, 1280, False, False, True),     # two warps a row; sigmoid weights and selection bias
+    (3, 768, True, False, True),       # a warp a row
+    (4, 2304, True, True, False),
+    (5, 1280, False, False, True),     # warps come round for a second row, the last round partly
+    (6, 4096, True, True, False)])
+def test_few_token_kernel_with_pre_expert_norm_and_sigmoid_routing(cuda_dev, T, H, post, given, sigmoid):
+    """moe_few_kernel norms the token rows in its prologue in a form that depends on the token count; its top-k must give
+    the ids and weights of the routing kernel, bit for bit, in both modes. Twice on one state."""
+    m, inputs, _lib, orc = _mods()
+    I, E, k = 512, 16, 4
+    w = inputs.make_weights(H, I, E, 73, cuda_dev, post_norm=post)
+    g = torch.Generator(device=cuda_dev).manual_seed(T + H)
+    w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    if sigmoid:
+        w["route_bias"] = torch.randn((E,), generator=g, device=cuda_dev) * 0.05
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8, routing_mode="sigmoid_bias" if sigmoid else "softmax_topk")
+    fits = ctypes.c_int(0)
+    assert st["lib"].lib.msk_moe_few_fits(ctypes.byref(st["cfg"]), T, 2 + int(given), ctypes.byref(fits)) == 0 and fits.value == 1
+    for _ in range(2):
+        x = (torch.randn((T, H), generator=g, device=cuda_dev) * 3.0).to(torch.bfloat16)
+        data = {"hidden_states": x, "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+        ids, tw = m._route(data, st, x, T)
+        if given:
+            out = m.kernel_fn({"hidden_states": x, "topk_ids": ids, "topk_weights": tw}, st)
+        else:
+            out, got_ids, got_tw = m.kernel_fn(data, st, return_routing=True)
+            assert torch.equal(got_ids, ids) and torch.equal(got_tw, tw)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        rid, rtw = orc.route_topk(data["router_logits"].cpu(), k, "sigmoid_bias" if sigmoid else "softmax_topk",
+                                  w["route_bias"].cpu() if sigmoid else None)
+        assert torch.equal(ids.cpu(), rid) and torch.allclose(tw.cpu(), rtw, rtol=1e-5)    # expf and a sum of four: some 1e-6
+        ref, parts = orc.moe_forward(x, ids, tw, w, return_parts=True)
+        _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
+@pytest.mark.parametrize("T,routed", [(2, False), (3, True)])
+def test_few_token_kernel_shares_pinned_rows_of_several_tokens(cuda_dev, T, routed):
+    """HostMappedStep at two and three tokens: several CTAs' slices make up a row, two warps or one copy it."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1280, 512, 16, 2
+    st = m.prepare(inputs.make_weights(H, I, E, 74, cuda_dev, post_norm=routed), n_experts=E, top_k=k, max_tokens=8)
+    fits = ctypes.c_int(0)
+    assert st["lib"].lib.msk_moe_few_fits(ctypes.byref(st["cfg"]), T, 4 + int(routed), ctypes.byref(fits)) == 0 and fits.value == 1
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    datas = []
+    for _ in range(6):
+        d = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+        logits = torch.randn((T, E), generator=g, device=cuda_dev)
+        if routed:
+            tw, ids = torch.softmax(logits, dim=-1).topk(k, dim=-1)
+            d["topk_ids"], d["topk_weights"] = ids.to(torch.int32), tw.contiguous()
+        else:
+            d["router_logits"] = logits
+        datas.append(d)
+    step = m.HostMappedStep(st, {key: v.cpu() for key, v in datas[0].items()})
+    for d in datas:
+        want = m.kernel_fn(d, st)
+        got = step({key: v.cpu() for key, v in d.items()})
+        step.done.synchronize()
+        assert torch.equal(got, want.cpu())
+    assert m.read_status(st) == 0
+
+
 @pytest.mark.parametrize("T", [64, 8192])
 def test_full_size_properties(cuda_dev, T):
     """Benchmark-size shapes (H4096 I1536 E128 top-8; T = 64 decode sweep point, T = 8192 prefill),
