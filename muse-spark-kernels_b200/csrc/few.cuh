@@ -1,6 +1,7 @@
-// The whole routed-expert step of up to eight tokens in one cooperative launch.
+// The whole routed-expert step of a few tokens in one cooperative launch: two or three, up to six with the pre-expert
+// norm (the rule is few_takes() in msk_moe.cu; the tables below hold eight).
 //
-// At one to eight tokens the step streams 85 to 600 MB of weights and every microsecond in which nothing
+// There the step streams 85 to 300 MB of weights and every microsecond in which nothing
 // streams counts: the kernel is built around a short prologue and as few hand-overs as possible, not around the
 // tensor pipe. Weights go from shared memory to registers, are decoded there and multiplied with mma.sync
 // (m16n8k16: 8 + 8 weight rows by up to 8 tokens), so there is no TMEM to allocate and no descriptor.
@@ -43,7 +44,7 @@ constexpr int FEW_TEAM = 2;                                // warps of a gate/up
 constexpr int FEW_TEAMS = FEW_WARPS / FEW_TEAM;
 constexpr int FEW_ROUTE_WARPS = 8;                         // route and sort; the others fetch the token rows
 constexpr int FEW_THREADS = (FEW_WARPS + 1) * 32;         // the last warp signals finished units
-constexpr int FEW_TOKENS = 8;                              // tokens of a step, and rows of a tile
+constexpr int FEW_TOKENS = 8;                              // rows of a tile, and most tokens the tables hold
 constexpr int FEW_ENTRIES = FEW_TOKENS * MAX_TOP_K;        // (token, slot) entries, and tiles
 constexpr int FEW_KB_BYTES = 2 * OCT_BYTES;                // one K block of 8 + 8 rows
 // Ring of a warp. More than some fifty bulk copies outstanding per SM slow the stream down, and 50 to 70 KB in flight
@@ -162,7 +163,7 @@ struct FewDeal {
 };
 
 // The units of one warp in order: of the CTA's gate/up units every n_teams-th from its team's number on, then
-// its down units (tile-major, own groups within a tile) number j, j + 16, ...
+// its down units (tile-major, own groups within a tile) number j, j + FEW_WARPS, ...
 struct FewIter {
   int left;                 // gate/up units of this CTA from the current one on
   int base, pass;           // the current one's place in the deal
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
         if (++slot == p.n_slots) { slot = 0; par ^= 1u; }
       }
       if (!ok) break;
-      // the team meets: the warps take turns in adding the four partials (in K order) and finishing the unit
+      // the team meets: its warps take turns in adding the two partials (in K order) and finishing the unit
       const uint32_t pb = n_unit & 1u, pp = (n_unit >> 1) & 1u;
       if (!warp_mbar_wait(&ctl.part_empty[team][pb], pp ^ 1u, abortw)) { ok = false; break; }
       uint8_t* pbuf = parts + pb * FEW_TEAM * p.part_bytes + (q * 8 + r) * 16;

@@ -685,8 +685,9 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   // few tokens: the kernels route, sort and combine themselves
   const bool few = rows <= SMALL_SORT_MAX_ENTRIES && T <= FOLD_MAX_TOKENS && p.N <= 32 && c->stop_after == 0;
   if (few) {
-    // measured (H4096 I1536 E128 top-8, cold L2): one launch 47 / 64 / 89 / 136 us at 1 / 2 / 4 / 8 tokens
-    // against 57 / 72 / 94 / 135 for the chain; at 16 and 32 tokens 195 / 268 against 197 / 249
+    // measured (H4096 I1536 E128 top-8, cold L2): the one-launch form of the tcgen05 kernel 89 / 136 us at 4 / 8 tokens
+    // against 94 / 135 for the chain; at 16 and 32 tokens 195 / 268 against 197 / 249. (Fewer tokens mostly take the
+    // few-token kernel, few_takes(); by the tcgen05 kernel 1 / 2 tokens take 47 / 64 against 57 / 72.)
     switch (c->decode_path) {
       case 1: p.path = 1; break;
       case 4: p.path = 1; break;   // becomes 4 below

@@ -387,8 +387,8 @@ def test_forward_many_entries_sorted_on_several_ctas(cuda_dev, T, E, k, lo, nloc
                                            (520, 16, 16, 0, 16),      # 64 CTAs of nine tokens, the last ones without any
                                            (1024, 8, 1, 5, 2)])       # most routes elsewhere
 def test_top_k_and_sort_on_several_ctas(cuda_dev, T, E, k, lo, nloc):
-    """From 1024 entries on the top-k and the stable sort run on several CTAs: tables equal to the oracle's. (The
-    combine of the last case runs with few routes local.)"""
+    """The top-k and the stable sort around the sizes from which they run on several CTAs (the second case does):
+    tables equal to the oracle's. (The combine of the last case runs with few routes local.)"""
     m, inputs, _lib, orc = _mods()
     out, ref, parts, views, st, (x, ids, tw, w) = _run_forward(m, inputs, orc, cuda_dev, 256, 256, E, k, T, seed=79, lo=lo, nloc=nloc)
     rid, _ = orc.route_topk(inputs.make_logits(T, E, "normal", 79, cuda_dev).cpu(), k)
