@@ -24,6 +24,7 @@ with the step; the reference sweeps by reading for that reason), and the steps c
 pool of different routings.
 """
 import argparse
+import ctypes
 import json
 import math
 import os
@@ -42,7 +43,9 @@ DTYPE = "bf16 x nvfp4 -> fp32 acc"
 POOL = 8  # distinct seeded inputs cycled through
 SWEEP = ("sweepT8", "sweepT32", "sweepT64", "sweepT128", "sweepT256", "prefill")
 HOST_MAPPED_MAX_TOKENS = 64   # up to here the end-to-end leg also tries the copy-free transport
-NCU_TRAFFIC_RATIO = 1.015   # ncu: DRAM bytes read + written / algorithmic bytes of the weight-streaming GEMM kernel
+# ncu, 32 experts resident: DRAM bytes read + written / algorithmic bytes, of each kernel's own capture
+NCU_TRAFFIC_RATIO = {"moe_few_kernel": 1.03, "moe_gemm_kernel<N,2> T8": 1.01, "moe_gemm_kernel<16,2>": 1.00,
+                     "moe_gemm_kernel<64,2>": 0.99, "moe_gemm_kernel<N,0>": 1.11}
 
 
 def workload_spec(name, n_gpus):
@@ -353,19 +356,23 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     if one_launch:
         alg = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(n_prof)) / n_prof
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
+        few = ctypes.c_int(0)
+        state["lib"].lib.msk_moe_few_fits(ctypes.byref(state["cfg"]), T, 1, ctypes.byref(few))   # (timed with given ids)
+        ratio = NCU_TRAFFIC_RATIO["moe_few_kernel" if few.value else "moe_gemm_kernel<N,2> T8"]
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / peaks["hbm_gbs"], "traffic": alg * NCU_TRAFFIC_RATIO,
-                "traffic_source": "ncu dram bytes of a weight-streaming GEMM capture / its algorithmic bytes (1.015), scaled",
-                "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if T <= 3 else "moe_gemm_kernel<N,2>"),
+                "frac": achieved / peaks["hbm_gbs"], "traffic": alg * ratio,
+                "traffic_source": "ncu dram bytes of the kernel's 32-expert capture / its algorithmic bytes (%.2f), scaled" % ratio,
+                "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if few.value else "moe_gemm_kernel<N,2>"),
                 "peak_source": peaks["source"] + " (burst copy)"}
     elif both_gemms:
         # both GEMMs in one launch: the touched experts' tiles of both, x read and converted (64-token tile: the sorted
         # rows read), inter written and read back, y written
         alg = mean_touched * (3 * I * H * 0.5625 + 8) + (2.0 * R * H if plan[0] == 64 else 4.0 * T * H) + 4.0 * R * I + 4.0 * R * H
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
+        ratio = NCU_TRAFFIC_RATIO["moe_gemm_kernel<%d,2>" % (64 if plan[0] == 64 else 16)]
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / peaks["hbm_gbs"], "traffic": alg * NCU_TRAFFIC_RATIO,
-                "traffic_source": "ncu dram bytes of a weight-streaming GEMM capture / its algorithmic bytes (1.015), scaled",
+                "frac": achieved / peaks["hbm_gbs"], "traffic": alg * ratio,
+                "traffic_source": "ncu dram bytes of the kernel's 32-expert capture / its algorithmic bytes (%.2f), scaled" % ratio,
                 "kernel": "moe_gemm_kernel<N,2> (gate/up and down GEMM in one launch)",
                 "peak_source": peaks["source"] + " (burst copy)"}
     elif T <= 1024:
@@ -373,8 +380,8 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
         alg13 = mean_touched * (2 * I * H * 0.5625 + 4) + 2.0 * T * H + 2.0 * R * I
         achieved = alg13 / (k_ms[2] * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / peaks["hbm_gbs"], "traffic": alg13 * NCU_TRAFFIC_RATIO,
-                "traffic_source": "ncu dram bytes of the 32-expert T=64 capture / its algorithmic bytes (1.015), scaled",
+                "frac": achieved / peaks["hbm_gbs"], "traffic": alg13 * NCU_TRAFFIC_RATIO["moe_gemm_kernel<N,0>"],
+                "traffic_source": "ncu dram bytes of a 32-expert T=64 capture / its algorithmic bytes (1.11), scaled",
                 "kernel": "moe_gemm_kernel<N,0> (gate/up)", "peak_source": peaks["source"] + " (burst copy)"}
     else:
         fl13 = 2.0 * R * 2 * I * H
