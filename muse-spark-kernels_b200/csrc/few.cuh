@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
           }
         }
       }
-      if (p.pre_w != nullptr) {   // x * rsqrt(mean(x^2) + eps) * (1 + pre_w), one BF16 rounding (gather_rows_kernel)
+      if (p.pre_w != nullptr) {   // x * rsqrt(mean(x^2) + eps) * (1 + pre_w), one BF16 rounding (copy_rows_kernel)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         float tot = ss;

@@ -114,121 +114,97 @@ __global__ void __launch_bounds__(128) dequant_packed_kernel(const uint8_t* pack
   }
 }
 
-// ------------------------------------------------------------- row gather
-// xs[q, :] = x[perm[q] / top_k, :] for the routed rows q < off[nloc]: token rows in sorted
-// (expert-major) order, so that wide token tiles can be fetched as plain 2-D TMA boxes. The
-// reference's prefill path gathers rows into per-expert tiles the same way
-// (muse_prefill_layer/cuda/prefill.cu:1446-1608), there fused with its pre-expert norm.
-// The copy also converts BF16 -> F16, the operand type of the MMA (layout.cuh).
-// gather != 0: xs[q] = f16(x[perm[q] / top_k]) for q < off[nloc] (grid = T * top_k blocks);
-// gather == 0: xs[t] = f16(x[t]) (grid = T blocks), for the narrow token tiles that gather rows
-// through the permutation themselves.
+// --------------------------------------------------------------- row copy
+// F16 copy of the token rows, a block per token. With `inv` a row goes to each of its routes' places in sorted
+// (expert-major) order, xs[inv[t, s]] = f16(x[t]), so that wide token tiles can be fetched as plain 2-D TMA boxes (the
+// reference's prefill path gathers rows into per-expert tiles, muse_prefill_layer/cuda/prefill.cu:1446-1608, fused with
+// its pre-expert norm); without it xs[t] = f16(x[t]), for the narrow token tiles that gather rows through the permutation.
+// F16 is the operand type of the MMA (layout.cuh).
 // With pre_w the pre-expert RMS norm of the layer callers is applied on the way:
 // x' = bf16( x * rsqrt(mean(x^2) + eps) * (1 + pre_w) ), FP32 arithmetic on the row the block holds in
 // registers (muse_decode_layer/py/04_triton_kernels.py:556-568: the reference's routing kernel does the
 // same before it stores the expert input). The sum of squares is a fixed shuffle tree followed by a
 // fixed-order sum of the eight warp partials.
-__global__ void __launch_bounds__(256) gather_rows_kernel(const __nv_bfloat16* __restrict__ x,
-                                                          const int32_t* __restrict__ perm,
-                                                          const int32_t* __restrict__ off, int nloc, int top_k, int H,
-                                                          int gather, __half* __restrict__ xs,
-                                                          const __nv_bfloat16* __restrict__ pre_w, float pre_eps) {
-  __shared__ float wsum[8];
+// Bound by memory: a row is read and normalised once however many routes it has, and the row and its routes are loaded
+// side by side. Going by sorted row instead (its entry first, then the row, each as often as it has routes) took 154 us for
+// 8192 tokens of 8 routes at H = 4096 where this takes 102 (600 MB, 5.9 TB/s), and 18.3 for 777 tokens with the norm (14.3).
+// look_first: a rank that holds a part of the experts has no route of many a token, whose row is then not read.
+constexpr int COPY_THREADS = 256;
+__global__ void __launch_bounds__(COPY_THREADS) copy_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* inv, int top_k,
+                                                                 int look_first, int H, __half* __restrict__ xs,
+                                                                 const __nv_bfloat16* __restrict__ pre_w, float pre_eps) {
+  __shared__ float wsum[COPY_THREADS / 32];
+  constexpr int MAXV = 4;   // 8 values per uint4, 256 threads: H <= 8192
   pdl_wait();
   pdl_launch_dependents();
-  const int q = blockIdx.x;
-  if (gather && q >= off[nloc]) return;
-  const size_t row = gather ? static_cast<size_t>(perm[q] / top_k) : static_cast<size_t>(q);
-  const uint4* src = reinterpret_cast<const uint4*>(x + row * H);
-  uint4* dst = reinterpret_cast<uint4*>(xs + static_cast<size_t>(q) * H);
-  if (pre_w == nullptr) {
-    for (int i = threadIdx.x; i < H / 8; i += 256) {
-      const uint4 v = src[i];
-      dst[i] = make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
-    }
-    return;
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  int dst_row = -1;         // lane s: the place of route s
+  if (inv == nullptr) {
+    if (lane == 0) dst_row = t;
+  } else if (lane < top_k) {
+    dst_row = __ldcg(inv + static_cast<size_t>(t) * top_k + lane);   // by an earlier launch of the chain: a coherent load
   }
-  constexpr int MAXV = 4;   // 8 values per uint4, 256 threads: H <= 8192
+  if (look_first && __ballot_sync(0xffffffffu, dst_row >= 0) == 0u) return;   // the same in every warp of the block
+  const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t) * H);
   uint4 v[MAXV];
-  float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
-    const int i = j * 256 + threadIdx.x;
+    const int i = j * COPY_THREADS + threadIdx.x;
     v[j] = make_uint4(0u, 0u, 0u, 0u);
     if (i < H / 8) v[j] = src[i];
-    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+  }
+  unsigned routes = __ballot_sync(0xffffffffu, dst_row >= 0);
+  if (routes == 0u) return;
+  if (pre_w == nullptr) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float lo = __uint_as_float(w[c] << 16), hi = __uint_as_float(w[c] & 0xFFFF0000u);
-      ss += lo * lo + hi * hi;
+    for (int j = 0; j < MAXV; ++j)
+      v[j] = make_uint4(bf16x2_to_f16x2(v[j].x), bf16x2_to_f16x2(v[j].y), bf16x2_to_f16x2(v[j].z), bf16x2_to_f16x2(v[j].w));
+  } else {
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {
+      const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float lo = __uint_as_float(w[c] << 16), hi = __uint_as_float(w[c] & 0xFFFF0000u);
+        ss += lo * lo + hi * hi;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) wsum[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int w8 = 0; w8 < COPY_THREADS / 32; ++w8) tot += wsum[w8];
+    const float rs = rsqrtf(tot / static_cast<float>(H) + pre_eps);
+    const uint4* gsrc = reinterpret_cast<const uint4*>(pre_w);
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {
+      const int i = j * COPY_THREADS + threadIdx.x;
+      if (i >= H / 8) continue;
+      const uint4 gv = gsrc[i];
+      const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+      const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+      uint32_t o4[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float lo = __uint_as_float(w[c] << 16) * rs * (1.0f + __uint_as_float(gw[c] << 16));
+        const float hi = __uint_as_float(w[c] & 0xFFFF0000u) * rs * (1.0f + __uint_as_float(gw[c] & 0xFFFF0000u));
+        const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);   // the expert input is BF16
+        o4[c] = bf16x2_to_f16x2(*reinterpret_cast<const uint32_t*>(&b));
+      }
+      v[j] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int w8 = 0; w8 < 8; ++w8) tot += wsum[w8];
-  const float rs = rsqrtf(tot / static_cast<float>(H) + pre_eps);
-  const uint4* gsrc = reinterpret_cast<const uint4*>(pre_w);
-#pragma unroll
-  for (int j = 0; j < MAXV; ++j) {
-    const int i = j * 256 + threadIdx.x;
-    if (i >= H / 8) continue;
-    const uint4 gv = gsrc[i];
-    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-    uint32_t o4[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float lo = __uint_as_float(w[c] << 16) * rs * (1.0f + __uint_as_float(gw[c] << 16));
-      const float hi = __uint_as_float(w[c] & 0xFFFF0000u) * rs * (1.0f + __uint_as_float(gw[c] & 0xFFFF0000u));
-      const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);   // the expert input is BF16
-      o4[c] = bf16x2_to_f16x2(*reinterpret_cast<const uint32_t*>(&b));
-    }
-    dst[i] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-  }
-}
-
-// The sorted copy without the pre-expert norm, as a persistent kernel: a warp per routed row, eight
-// 16-byte loads in flight per lane, the next row's permutation entry fetched while the current row
-// moves. (One block per row, as gather_rows_kernel works, spends most of its time on the two dependent
-// loads every block starts with: 65,536 rows took 0.22 ms against 0.1 ms of memory time.)
-__global__ void __launch_bounds__(256) gather_rows_sorted_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                 const int32_t* __restrict__ perm,
-                                                                 const int32_t* __restrict__ off, int nloc, int top_k,
-                                                                 int H, __half* __restrict__ xs) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  const int n_rows = off[nloc];
-  const int n16 = H / 8;   // 16-byte chunks per row
-  int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int entry = q < n_rows ? perm[q] : 0;
-  while (q < n_rows) {
-    const int qn = q + warps;
-    const int entry_next = qn < n_rows ? perm[qn] : 0;
-    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(entry / top_k) * H);
+  for (; routes != 0u; routes &= routes - 1u) {
+    const int q = __shfl_sync(0xffffffffu, dst_row, __ffs(routes) - 1);
     uint4* dst = reinterpret_cast<uint4*>(xs + static_cast<size_t>(q) * H);
-    for (int i0 = 0; i0 < n16; i0 += 256) {
-      uint4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int i = i0 + j * 32 + lane;
-        if (i < n16) v[j] = __ldg(src + i);
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int i = i0 + j * 32 + lane;
-        if (i < n16)
-          __stcs(dst + i, make_uint4(bf16x2_to_f16x2(v[j].x), bf16x2_to_f16x2(v[j].y), bf16x2_to_f16x2(v[j].z),
-                                     bf16x2_to_f16x2(v[j].w)));
-      }
+    for (int j = 0; j < MAXV; ++j) {
+      const int i = j * COPY_THREADS + threadIdx.x;
+      if (i < H / 8) dst[i] = v[j];
     }
-    q = qn;
-    entry = entry_next;
   }
 }
 
@@ -1434,10 +1410,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
       if (pre) {
         lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
         lc.blockDim = dim3(256);
-        e = static_cast<int>(cudaLaunchKernelEx(&lc, gather_rows_kernel, static_cast<const __nv_bfloat16*>(x),
-                                                static_cast<const int32_t*>(perm), static_cast<const int32_t*>(off),
-                                                static_cast<int>(cfg->local_count), static_cast<int>(cfg->top_k),
-                                                static_cast<int>(cfg->hidden), 0, xs,
+        e = static_cast<int>(cudaLaunchKernelEx(&lc, copy_rows_kernel, static_cast<const __nv_bfloat16*>(x),
+                                                static_cast<const int32_t*>(nullptr), static_cast<int>(cfg->top_k), 0,
+                                                static_cast<int>(cfg->hidden), xs,
                                                 static_cast<const __nv_bfloat16*>(pre_norm_w), pre_norm_eps));
       } else {
         const int n8 = n_tokens * (cfg->hidden / 8);
@@ -1488,28 +1463,19 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (!convert_in_sort && (tma_b || !both_gemms)) {
     // F16 copy of the token rows: sorted (expert-major) for the TMA tiles, plain [T, H] otherwise
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(static_cast<unsigned>(tma_b ? n_tokens * cfg->top_k : n_tokens));
-    lc.blockDim = dim3(256);
+    lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
+    lc.blockDim = dim3(COPY_THREADS);
     lc.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = pdl;
     lc.attrs = at;
     lc.numAttrs = 1;
-    if (tma_b && pre_norm_w == nullptr) {
-      lc.gridDim = dim3(static_cast<unsigned>(std::min<long long>((static_cast<long long>(n_tokens) * cfg->top_k + 7) / 8,
-                                                                  8LL * sm_count())));
-      e = static_cast<int>(cudaLaunchKernelEx(&lc, gather_rows_sorted_kernel, static_cast<const __nv_bfloat16*>(x),
-                                              static_cast<const int32_t*>(perm), static_cast<const int32_t*>(off),
-                                              static_cast<int>(cfg->local_count), static_cast<int>(cfg->top_k),
-                                              static_cast<int>(cfg->hidden), xs));
-    } else {
-      e = static_cast<int>(cudaLaunchKernelEx(&lc, gather_rows_kernel, static_cast<const __nv_bfloat16*>(x),
-                                              static_cast<const int32_t*>(perm), static_cast<const int32_t*>(off),
-                                              static_cast<int>(cfg->local_count), static_cast<int>(cfg->top_k),
-                                              static_cast<int>(cfg->hidden), tma_b ? 1 : 0, xs,
-                                              static_cast<const __nv_bfloat16*>(pre_norm_w), pre_norm_eps));
-    }
+    e = static_cast<int>(cudaLaunchKernelEx(&lc, copy_rows_kernel, static_cast<const __nv_bfloat16*>(x),
+                                            static_cast<const int32_t*>(tma_b ? inv : nullptr), static_cast<int>(cfg->top_k),
+                                            cfg->local_count < cfg->n_experts ? 1 : 0,
+                                            static_cast<int>(cfg->hidden), xs,
+                                            static_cast<const __nv_bfloat16*>(pre_norm_w), pre_norm_eps));
     if (e != 0) return e;
     if (tma_b) {
       for (int i = 0; (16 << i) <= plan.N; ++i) {
@@ -1718,8 +1684,8 @@ int msk_moe_forward_static(const MskMoeCfg* cfg, const void* packed13, const voi
 
   int e = launch_sort(cfg, topk_ids, n_tokens, cnt, off, perm, inv, st);
   if (e != 0) return e;
-  gather_rows_kernel<<<static_cast<unsigned>(n_tokens), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(x), perm, off, cfg->local_count, cfg->top_k, cfg->hidden, 0, xh, nullptr, 0.f);
+  copy_rows_kernel<<<static_cast<unsigned>(n_tokens), COPY_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(x), nullptr, cfg->top_k, 0,
+                                                                            cfg->hidden, xh, nullptr, 0.f);
   e = static_cast<int>(cudaGetLastError());
   if (e != 0) return e;
   GemmParams p{};
