@@ -68,7 +68,8 @@ typedef struct MskMoeCfg {
   int32_t no_pdl;        /* non-zero: launches are not chained with programmatic dependent launch (the reference's
                             okc_set_pdl(0), muse_moe_w4a16/cuda/moe.cu:2348,2565) */
   int32_t token_tile;    /* MMA N (tokens per tile): 16/32/64/128; 0 = chosen from the mean rows per expert
-                            (up to 12: 16, up to 32: 64, beyond: 128) */
+                            (up to 12: 16, up to 40: 64, beyond: 128). 128 stands for the kernel on pairs of SMs,
+                            whose tiles hold up to 256 rows; it rounds num_ctas up to an even number */
   int32_t max_tokens;    /* token capacity the workspace is sized for (msk_moe_forward rejects more) */
   int32_t trace;         /* non-zero: the GEMM kernels stamp %globaltimer per CTA into the workspace (view 6) */
   int32_t stop_after;    /* measuring aid: 0 = whole step; 1/2/3 = return after sort / gate-up GEMM / down GEMM */
@@ -254,7 +255,7 @@ int msk_moe_read_status(const void* workspace, int* host_status, void* stream);
 
 /* Registers / static + dynamic shared memory / local memory per kernel, as the reference's
  * okc_attrs() reports (muse_moe_w4a16/cuda/moe.cu:2789-2794). which: 0 sort, 1 route,
- * 2 gate/up GEMM, 3 down GEMM, 4 combine. host_out: int[4] = regs, static smem, max dyn smem, local. */
+ * 2 gate/up GEMM, 3 down GEMM (token_tile 128: one kernel for both), 4 combine. host_out: int[4] = regs, static smem, max dyn smem, local. */
 int msk_moe_attrs(int which, int token_tile, int* host_out);
 
 /* Expert-parallel combine at a token's home rank: out[t] = bf16(sum over ranks d, in rank order, of

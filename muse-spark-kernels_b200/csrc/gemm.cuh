@@ -9,8 +9,7 @@
 //   warp 2       activations: cp.async gather of the token rows of the tile (through the permutation for
 //                the gate/up GEMM) into the K-major core-matrix layout, or TMA boxes of sorted rows;
 //   warps 4-7    epilogue (gemm_epilogue.inl): TMEM accumulators -> SwiGLU / scale -> global,
-//                or split-K partials (token tiles up to 64; for 128 the accumulators are single-
-//                buffered and the sixteen dequant warps, idle by then, share the epilogue);
+//                or split-K partials;
 //   warps 8-23   dequant (gemm_dequant.inl): 2 tiles x 4 lane quarters x 2 K halves. A thread
 //                owns one weight row of its tile: shared-memory codes -> BF16 (layout.cuh) ->
 //                tcgen05.st into a ring of TMEM A slots (128 K each) the MMA warp consumes.
@@ -21,7 +20,7 @@
 // TMEM lane, and (row tile 2j, row tile 2j+1) for the down GEMM (phase 1). Both tiles of a pair
 // share the B operand.
 //
-// One kernel template, three modes: MODE 0 runs phase 0, MODE 1 phase 1 (two launches chained by
+// Token tiles of 16, 32 and 64; wider ones are pair.cuh's. One kernel template, three modes: MODE 0 runs phase 0, MODE 1 phase 1 (two launches chained by
 // programmatic dependent launch, any token count), MODE 2 both phases in one launch for a few tokens:
 // the weight stream, the dequant ring and the MMA pipeline run on from the last gate/up stage into
 // the first down stage without draining; only the activation gather of phase 1 waits, per token tile,
@@ -43,7 +42,7 @@
 //          ascending K order (the order never depends on arrival) and runs the epilogue. Cut points
 //          depend on the shapes, the number of token tiles and the grid size given by the host, not
 //          on the device.
-// Accumulators are double-buffered in TMEM (N <= 64) so the epilogue of a piece overlaps the main
+// Accumulators are double-buffered in TMEM so the epilogue of a piece overlaps the main
 // loop of the next.
 //
 // Numerics: operands are e2m1*e4m3 (exact in F16) and the BF16 activations held as F16 (exact
@@ -76,10 +75,11 @@ template <int N>
 struct GemmCfg {
   static constexpr int B_STAGE_BYTES = N * KS * 2;
   static constexpr int STAGE_BYTES = 2 * TILE_BYTES + B_STAGE_BYTES;
-  static constexpr int NST = N <= 16 ? 5 : (N <= 32 ? 4 : (N <= 64 ? 3 : 2));
+  static_assert(N <= 64, "wider token tiles: pair.cuh");
+  static constexpr int NST = N <= 16 ? 5 : (N <= 32 ? 4 : 3);
   // TMEM: NDBUF accumulator buffers of 2N columns (tile 0 | tile 1) from column 0; above them
   // the A ring: two groups (tiles) of NSLOT slots, 64 columns (128 K = half a stage) each.
-  static constexpr int NDBUF = N <= 64 ? 2 : 1;
+  static constexpr int NDBUF = 2;
   static constexpr int A_BASE = N <= 32 ? 128 : 256;
   static constexpr int NSLOT = N <= 32 ? 3 : 2;
   static constexpr int SLOT_COLS = 64;
@@ -338,75 +338,6 @@ __device__ __forceinline__ uint32_t inter_pair(uint32_t g0, uint32_t u0, uint32_
   return *reinterpret_cast<const uint32_t*>(&c);
 }
 
-// Epilogue of a unit of the 128-token tile for the thread that owns TMEM lane `row`: four warps share a lane quarter.
-// Phase 0: quarter `part` of the columns, gate (tile 0) and up (tile 1) -> bf16(silu(g) * u) into inter; phase 1: half
-// `part >> 1` of the columns of tile `part & 1` -> rows scaled by gs (and 1 + post_norm_w) into y as BF16, as the
-// reference's wide-tile build keeps them. The tensor core stands still from the last MMA of a unit until
-// release() hands the accumulators back: before that, the first half of this thread's values is only brought
-// down to packed results and the second half into registers; the rest of the arithmetic and all stores run
-// beside the next unit's MMAs. (Both halves as raw values would need 64 registers beside the main loop's: 80 are there.)
-template <typename Release>
-__device__ __forceinline__ void epilogue_wide(const GemmParams& p, const PhaseParams& pp, int phase, const UnitInfo& ui,
-                                              uint32_t d_tmem, int row, int part, Release release) {
-  constexpr int N = 128;
-  const float gsc = pp.gs[ui.expert];
-  size_t ld = static_cast<size_t>(pp.out_ld);
-  asm volatile("" : "+l"(ld));   // or its multiples are kept in registers through the main loop
-  const int c_beg = phase == 0 ? part * (N / 4) : (part >> 1) * (N / 2);
-  const int n = ui.rows - c_beg;   // rows of this thread's columns
-  if (n <= 0) {
-    release();
-    return;
-  }
-  if (phase == 0) {
-    uint32_t a[16], b[16], first[8];
-    tmem_ld16(d_tmem + c_beg, a);
-    tmem_ld16(d_tmem + N + c_beg, b);
-    tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) first[j] = inter_pair(a[2 * j], b[2 * j], a[2 * j + 1], b[2 * j + 1], gsc);
-    tmem_ld16(d_tmem + c_beg + 16, a);
-    tmem_ld16(d_tmem + N + c_beg + 16, b);
-    tmem_wait_ld();
-    release();
-    __half* outp = static_cast<__half*>(pp.outp) + static_cast<size_t>(ui.row0 + c_beg) * ld + ui.pair * 128 + row;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const uint32_t h = j < 8 ? first[j & 7] : inter_pair(a[2 * (j & 7)], b[2 * (j & 7)], a[2 * (j & 7) + 1], b[2 * (j & 7) + 1], gsc);
-      if (2 * j < n) *outp = __ushort_as_half(static_cast<unsigned short>(h));
-      outp += ld;
-      if (2 * j + 1 < n) *outp = __ushort_as_half(static_cast<unsigned short>(h >> 16));
-      outp += ld;
-    }
-  } else {
-    const int col = (2 * ui.pair + (part & 1)) * 128 + row;
-    float osc = gsc;
-    if (p.post_norm_w != nullptr) osc *= 1.0f + __bfloat162float(p.post_norm_w[col]);
-    const uint32_t src = d_tmem + (part & 1) * N + c_beg;
-    uint32_t a[32], first[16];
-    auto pack = [osc](uint32_t lo, uint32_t hi) -> uint32_t {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(lo) * osc, __uint_as_float(hi) * osc);
-      return *reinterpret_cast<const uint32_t*>(&h);
-    };
-    tmem_ld32(src, a);
-    tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) first[j] = pack(a[2 * j], a[2 * j + 1]);
-    tmem_ld32(src + 32, a);
-    tmem_wait_ld();
-    release();
-    unsigned short* outp = static_cast<unsigned short*>(pp.outp) + static_cast<size_t>(ui.row0 + c_beg) * ld + col;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const uint32_t h = j < 16 ? first[j & 15] : pack(a[2 * (j & 15)], a[2 * (j & 15) + 1]);
-      if (2 * j < n) *outp = static_cast<unsigned short>(h);
-      outp += ld;
-      if (2 * j + 1 < n) *outp = static_cast<unsigned short>(h >> 16);
-      outp += ld;
-    }
-  }
-}
-
 // Folded combine (phase 1, fold): out[t] = bf16( sum over the token's local slots, in slot order, of
 // w[t,s] * norm_s * y[inv[t,s]] ), norm_s = rsqrt(mean(y^2) + eps) with the post-expert norm, else 1
 // (muse_moe_w4a16/cuda/moe.cu:2604-2766). Run by all threads of the CTA that retired the token's
@@ -527,7 +458,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
   constexpr int PH_FIRST = MODE == 1 ? 1 : 0, PH_LAST = MODE == 0 ? 0 : 1;
   constexpr bool FUSED = MODE == 2;
   constexpr bool TMA_B = C::TMA_B;
-  static_assert(!(FUSED && NDBUF == 1), "the one-launch mode is built for token tiles up to 64");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* ring = smem;                                        // NST x [tile g0 | tile g1 | B]
   GemmCtrl& ctl = *reinterpret_cast<GemmCtrl*>(smem + NST * C::STAGE_BYTES + C::LUT_BYTES);
@@ -557,7 +487,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&ctl.d_full[i], 2);  // one commit per MMA issuer
-      mbar_init(&ctl.d_empty[i], C::NDBUF == 1 ? 16 : 4);  // single buffer: the dequant warps run the epilogue
+      mbar_init(&ctl.d_empty[i], 4);
     }
     mbar_init(&ctl.epi_bar, 128);
     ctl.abort_word = 0;
@@ -685,7 +615,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
 
   const uint32_t tmem = ctl.tmem_base;
   if (tid == 0) MSK_TR(TR_SETUP);
-  const int iter_mode = (N < 128 && p.flat) ? 1 : 0;
+  const int iter_mode = p.flat ? 1 : 0;
   // Down launch behind a gate/up launch with the per-tile hand-over: its CTAs start as the gate/up CTAs
   // leave, in block order, so the last blocks start on the SMs whose gate/up CTA held one unit more than
   // the others. They are dealt fewer down units, the way the one-launch kernel deals its second phase

@@ -2,7 +2,7 @@
 // Warp = (K half kh, tile g, lane quarter). Thread `row` of a quarter owns one weight row of
 // tile g. Per K stage the warps of half kh fill one A slot (128 K): four 16-byte code chunks
 // and eight scale bytes -> 4 x 16 F16x2 registers -> four tcgen05.st, each issued right after
-// its chunk is decoded (the 128-token tile: the first two once both are). With three slots per tile a slot is handed to the MMA warp (`retire`) after
+// its chunk is decoded. With three slots per tile a slot is handed to the MMA warp (`retire`) after
 // the first chunk of the following slot has been decoded, so the store latency hides behind it; with
 // two slots right behind its stores (see below). Slots of half the size (64 K, twice as many
 // hand-overs) were measured too: 10 - 20 % slower at every size, the hand-over itself is what costs.
@@ -26,33 +26,9 @@
       if (lane == 0) mbar_arrive(&ctl.a_full[g][pending_slot]);
       pending = false;
     };
-    uint32_t unit_i = 0;
-    // Single accumulator buffer (the 128-token tile): the main loop cannot go on until the accumulators
-    // are drained, and the sixteen dequant warps drain them together (the four warps of a lane quarter
-    // split the columns). The drain of a unit is put off until this warp has decoded the first stage
-    // of the next unit into the A slots, which are free by then: when the drain ends, the MMA warps find
-    // their operands ready, and the bubble between two units is the drain alone, not the drain plus
-    // a refill of the decode pipeline.
-    bool owe_drain = false;
-    int owed_base = 0;
-    uint32_t owed_unit_i = 0;
     MSK_PHASES {
       MSK_PHASE_SETUP;
-      auto drain = [&]() -> bool {
-        const UnitInfo owed_ui = decode_unit(owed_base, tile_start, pp.n_pairs, p.nloc, N);
-        if (!MSK_WAIT(&ctl.d_full[0], owed_unit_i & 1u, abortw)) return false;
-        tc_fence_after();
-        if (tid == 256) { if (owed_unit_i == 0) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); }
-        epilogue_wide(p, pp, phase, owed_ui, tmem + lane_base, row, kh * 2 + g, [&]() {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl.d_empty[0]);
-        });
-        if (tid == 256 && owed_unit_i == 0) MSK_TR(TR_FIRST_EPI_DONE);
-        owe_drain = false;
-        return true;
-      };
-      for (; ok && pieces.next(base, ks0, ks1); ++unit_i) {
+      while (ok && pieces.next(base, ks0, ks1)) {
         for (int ks = ks0; ks < ks1 && ok; ++ks, ++it) {
           const uint32_t slot = it % NST, par = (it / NST) & 1u;
 #ifdef MSK_TRACE_DETAIL
@@ -70,97 +46,52 @@
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(sfa[0]), "=r"(sfa[1]), "=r"(sfa[2]), "=r"(sfa[3])
                        : "r"(tile_row + OCT_CODE_BYTES));
-          if constexpr (N == 128) {
-            // The 128-token tile has two slots per tile, a K stage in all, and between the MMAs that free a slot and those
-            // that use it again lie the decode that is left, the stores and the hand-over: two of the four
-            // chunks are decoded before the wait (one: 777 tokens 467 us, two: 444, three: 467; 3012 tokens at
-            // the layer shape 600, 533, 600 in a long run). With the accumulators of the 64-token tile the A ring is
-            // not what the MMAs wait for (256 tokens 279, 281, 288 us), so it keeps the form below.
-            uint32_t o[2][16];
-            auto decode = [&](int c, uint32_t (&d)[16]) {
-              uint32_t q[4];
-              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
-                           : "r"(tile_row + (kh * 4 + c) * 128));
-              const uint32_t sfw = kh ? (c < 2 ? sfa[2] : sfa[3]) : (c < 2 ? sfa[0] : sfa[1]);
-              decode_chunk(q, (c & 1) ? (sfw >> 16) : sfw, d);
-            };
+          // this warp's slot of the stage: K half kh = chunks 4*kh .. 4*kh+3
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              decode(c, o[c]);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(o[c][j]));   // here, not behind the wait
-            }
-            if (!MSK_WAIT(&ctl.a_empty[g][as], apar ^ 1u, abortw)) { ok = false; break; }
-            tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (c >= 2) decode(c, o[c & 1]);
-              tmem_st16(a_tmem + as * C::SLOT_COLS + c * 16, o[c & 1]);
-            }
-            pending_slot = as;
-            retire();   // right behind the stores: the MMAs of this half can start
-            if (it == 0 && tid == 256) MSK_TR(TR_FIRST_AFULL);
-            as += 2;
-            if (as >= NSLOT) { as -= NSLOT; apar ^= 1u; }
-          } else {
-            // this warp's slot of the stage: K half kh = chunks 4*kh .. 4*kh+3
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int chunk = kh * 4 + c;
-              uint32_t q[4];
-              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
-                           : "r"(tile_row + chunk * 128));
-              const uint32_t sfw = kh ? (c < 2 ? sfa[2] : sfa[3]) : (c < 2 ? sfa[0] : sfa[1]);
-              uint32_t o[16];
-              decode_chunk(q, (c & 1) ? (sfw >> 16) : sfw, o);
-              if (c == 0) {
-                // hand over the previous slot (its stores had the decode above to land), claim this one
-                if (pending) retire();
+          for (int c = 0; c < 4; ++c) {
+            const int chunk = kh * 4 + c;
+            uint32_t q[4];
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
+                         : "r"(tile_row + chunk * 128));
+            const uint32_t sfw = kh ? (c < 2 ? sfa[2] : sfa[3]) : (c < 2 ? sfa[0] : sfa[1]);
+            uint32_t o[16];
+            decode_chunk(q, (c & 1) ? (sfw >> 16) : sfw, o);
+            if (c == 0) {
+              // hand over the previous slot (its stores had the decode above to land), claim this one
+              if (pending) retire();
 #ifdef MSK_TRACE_DETAIL
-                if (lane == 0 && (didx == 0 || didx == 15) && !mbar_test(&ctl.a_empty[g][as], apar ^ 1u))
-                  MSK_TRD(didx ? 5 : 0, tri, 9);   // the A slot was not free yet
+              if (lane == 0 && (didx == 0 || didx == 15) && !mbar_test(&ctl.a_empty[g][as], apar ^ 1u))
+                MSK_TRD(didx ? 5 : 0, tri, 9);   // the A slot was not free yet
 #endif
-                if (!MSK_WAIT(&ctl.a_empty[g][as], apar ^ 1u, abortw)) { ok = false; break; }
-                if (lane == 0 && (didx == 0 || didx == 15)) MSK_TRD(didx ? 5 : 0, tri, 6);
-                tc_fence_after();
-              }
-              tmem_st16(a_tmem + as * C::SLOT_COLS + c * 16, o);
+              if (!MSK_WAIT(&ctl.a_empty[g][as], apar ^ 1u, abortw)) { ok = false; break; }
+              if (lane == 0 && (didx == 0 || didx == 15)) MSK_TRD(didx ? 5 : 0, tri, 6);
+              tc_fence_after();
             }
-            if (!ok) break;
-            pending = true;
-            pending_slot = as;
-            // Two-slot rings (the 64-token tile; the branch above does the same): this K half's slot is refilled every stage, and the refill
-            // has to wait until the MMAs of the stage before have drained it. Handing the slot over right
-            // here, instead of behind the first decode of the next stage, lets those MMAs start a decode
-            // earlier (8192 tokens: gate/up GEMM 1.47 -> 1.34 ms; 256 tokens 309 -> 300 us a step). With three
-            // slots (the narrow tiles) it changes nothing, and the deferred hand-over hides the store latency.
-            // (Letting both warp groups of a tile decode the same slot, so that a slot fills in half the time,
-            // was measured on top of this: no change.)
-            if (NSLOT == 2) retire();
-            if (it == 0 && tid == 256) MSK_TR(TR_FIRST_AFULL);
-            // the other K half takes the next ring slot; this warp's next one is two further
-            as += 2;
-            if (as >= NSLOT) { as -= NSLOT; apar ^= 1u; }
+            tmem_st16(a_tmem + as * C::SLOT_COLS + c * 16, o);
           }
+          if (!ok) break;
+          pending = true;
+          pending_slot = as;
+          // Two-slot rings (the 64-token tile): this K half's slot is refilled every stage, and the refill
+          // has to wait until the MMAs of the stage before have drained it. Handing the slot over right
+          // here, instead of behind the first decode of the next stage, lets those MMAs start a decode
+          // earlier (8192 tokens: gate/up GEMM 1.47 -> 1.34 ms; 256 tokens 309 -> 300 us a step). With three
+          // slots (the narrow tiles) it changes nothing, and the deferred hand-over hides the store latency.
+          // (Letting both warp groups of a tile decode the same slot, so that a slot fills in half the time,
+          // was measured on top of this: no change.)
+          if (NSLOT == 2) retire();
+          if (it == 0 && tid == 256) MSK_TR(TR_FIRST_AFULL);
+          // the other K half takes the next ring slot; this warp's next one is two further
+          as += 2;
+          if (as >= NSLOT) { as -= NSLOT; apar ^= 1u; }
           if (!ok) break;
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.raw_empty[slot]);
           if (lane == 0 && (didx == 0 || didx == 15)) MSK_TRD(didx ? 5 : 0, tri, 7);
-          if (NDBUF == 1 && owe_drain) {
-            if (pending) retire();   // the first stage of this unit is ready for the MMA warps
-            if (!drain()) { ok = false; break; }
-          }
         }
         if (!ok) break;
         if (pending) retire();  // the accumulators need every slot of the piece
-        if (NDBUF == 1) {
-          owe_drain = true;
-          owed_base = base;
-          owed_unit_i = unit_i;
-        }
       }
-      if (ok && NDBUF == 1 && owe_drain && !drain()) ok = false;   // the last unit of the phase
       if (!ok) break;
     }

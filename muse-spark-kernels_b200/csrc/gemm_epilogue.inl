@@ -4,7 +4,6 @@
 // shares) stores its raw accumulators to this CTA's slot of the partial buffer and takes the
 // unit's ticket; the CTA that draws the last ticket sums the pieces in ascending K order and
 // finishes the unit.
-    if (NDBUF > 1) {
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     uint32_t unit_i = 0, epi_par = 0;
@@ -215,5 +214,4 @@
         if (tid == 128 && unit_i == 0) MSK_TR(TR_FIRST_EPI_DONE);
       }
       if (!ok) break;
-    }
     }

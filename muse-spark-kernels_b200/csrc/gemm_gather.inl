@@ -121,9 +121,9 @@
     drain();
     } else if (lane == 0) {
       // Wide token tiles: four boxes per K stage, rows row0.. of the sorted matrix, no higher than the tile's
-      // rows need (16, 32, 64 or 128: a tensor map each). The copies of a stage stay four; only their bytes
+      // rows need (16, 32 or 64: a tensor map each). The copies of a stage stay four; only their bytes
       // shrink. (Whole 32-row boxes put side by side, more copies per stage, were slower than full height.) A full
-      // box of 128 rows is 64 KB a stage beside 36 KB of weights; an expert with 48 tokens needs half of it.
+      // box of 64 rows is 32 KB a stage beside 36 KB of weights.
       const uint64_t keep = policy_evict_last();  // token rows are re-read by every pair of the expert
       uint32_t it = 0;
       bool ok = true;
@@ -134,7 +134,7 @@
         (void)last_tile;
         while (ok && pieces.next(base, ks0, ks1)) {
           const UnitInfo ui = decode_unit(base, tile_start, pp.n_pairs, p.nloc, N);
-          const int h = ui.rows <= 16 ? 0 : ui.rows <= 32 ? 1 : ui.rows <= 64 ? 2 : 3;
+          const int h = ui.rows <= 16 ? 0 : ui.rows <= 32 ? 1 : 2;
           const CUtensorMap* map = &p.tmap_act[phase][h];
           if (FUSED && phase == 1) {   // the gate/up units of this token tile, as above
             if (ui.tile != last_tile) {

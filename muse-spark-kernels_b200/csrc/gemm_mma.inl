@@ -20,8 +20,7 @@
         tc_fence_after();
         if (mg == 0 && lane == 0) MSK_TRD(1, tri, 3);
         const uint32_t d_tmem = tmem + db * (2 * N) + mg * N;
-        // a ragged last token tile of an expert only pays for the columns it has (MMA N in steps of 16):
-        // at N = 128 an MMA costs 64 cycles, at N = 16 nine
+        // a ragged last token tile of an expert only pays for the columns it has (MMA N in steps of 16)
         const uint32_t idesc_u = N >= 64 ? idesc_f16(FMT_F16, FMT_F16, 128, static_cast<uint32_t>((ui.rows + 15) & ~15)) : idesc;
         const uint32_t a_base = tmem + C::A_BASE + mg * C::A_GROUP_COLS;
         for (int ks = ks0; ks < ks1 && ok; ++ks, ++it) {

@@ -14,6 +14,7 @@
 #include "route_sort.cuh"
 #include "gemm.cuh"
 #include "few.cuh"
+#include "pair.cuh"
 #include "router_gemm.cuh"
 
 namespace msk {
@@ -639,13 +640,12 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     p.N = c->token_tile;
   } else {
     const double rpe = static_cast<double>(T) * c->top_k / c->n_experts;  // mean tokens per expert
-    // measured at H4096 I1536 E128 (us a step with 16 / 64 / 128-token tiles, near-even routing): T = 160 (rpe 10):
-    // 268 / 281 / 370; T = 192 (rpe 12): 313 / 302 / 390; T = 512 (rpe 32): - / 352 / 428; T = 640 (rpe 40): - / 374 /
-    // 440; T = 900 (rpe 56): - / 450 / 466; T = 1024 (rpe 64): - / 594 / 504. The 16-token tile is the fastest per K stage
-    // and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The host does not
-    // know the counts, and the less even they are the lower that line lies: with a few experts taking most tokens
-    // T = 512 takes 322 / 330 and T = 640 428 / 424, with a random router T = 777 (rpe 49) 536 / 524 in all. The
-    // 32-token tile never wins at these shapes (it stays selectable with cfg.token_tile)
+    // measured at H4096 I1536 E128 (us a step with 16 / 64-token tiles, near-even routing): T = 160 (rpe 10): 268 / 281;
+    // T = 192 (rpe 12): 313 / 302. 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
+    // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. The 16-token tile is the
+    // fastest per K stage and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The
+    // host does not know the counts, and the less even they are the lower that line lies. The 32-token tile never wins at
+    // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh)
     p.N = rpe <= 12 ? 16 : rpe <= 40 ? 64 : 128;
   }
   const long long rows = static_cast<long long>(T) * c->top_k;
@@ -684,9 +684,7 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
       (c->decode_path == 4 || (c->decode_path == 0 && T >= BOTH_GEMMS_MIN_TOKENS)))
     p.path = 4;
   // The 64-token tile keeps the row copy in front of the GEMMs and shares one launch between them as well, unless the
-  // chain is asked for: 256 tokens 279 us against 287. For the 128-token tile the same was built and
-  // slower (777 tokens 556 against 524 us, 8192 tokens 2890 against 2764): its units are long, few CTAs stand idle
-  // between the two launches, and the decode warps, which drain the accumulators there, lose more to the hand-over.
+  // chain is asked for: 256 tokens 279 us against 287.
   p.both = p.path == 4 || (p.path == 1 && p.N == 64 && resident && c->decode_path != 1);
   return p;
 }
@@ -819,7 +817,6 @@ static int launch_gemm_n(int N, const GemmParams& p, int grid, cudaStream_t st, 
     case 16: return launch_gemm<16, MODE>(p, grid, st, pdl);
     case 32: return launch_gemm<32, MODE>(p, grid, st, pdl);
     case 64: return launch_gemm<64, MODE>(p, grid, st, pdl);
-    case 128: return launch_gemm<128, MODE>(p, grid, st, pdl);
     default: return MSK_ERR_SHAPE;
   }
 }
@@ -831,6 +828,34 @@ static int launch_gemm_fused(int N, const GemmParams& p, int grid, cudaStream_t 
     case 64: return launch_gemm<64, 2>(p, grid, st, 0);
     default: return MSK_ERR_SHAPE;
   }
+}
+
+// The kernel on pairs of SMs (pair.cuh). An odd grid is rounded up to whole pairs.
+static int launch_pair(PairParams& p, const __half* xs, size_t rows, int grid, cudaStream_t st, int pdl) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(moe_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    attr_set[dev] = true;
+  }
+  for (int i = 0; i < PAIR_MAPS; ++i) {
+    int e = encode_act_map(&p.tmap[0][i], xs, rows, p.K[0], 16 * (i + 1));
+    if (e == 0) e = encode_act_map(&p.tmap[1][i], p.inter, rows, p.K[1], 16 * (i + 1));
+    if (e != 0) return e;
+  }
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(static_cast<unsigned>((grid + 1) / 2 * 2));
+  lc.blockDim = dim3(PAIR_THREADS);
+  lc.dynamicSmemBytes = PairCfg::SMEM_BYTES;
+  lc.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&lc, moe_pair_kernel, p));
 }
 
 // ---- the few-token kernel (few.cuh): shapes it takes, its shared memory and its dealing of work
@@ -1477,7 +1502,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
                                             static_cast<int>(cfg->hidden), xs,
                                             static_cast<const __nv_bfloat16*>(pre_norm_w), pre_norm_eps));
     if (e != 0) return e;
-    if (tma_b) {
+    if (tma_b && plan.N != 128) {
       for (int i = 0; (16 << i) <= plan.N; ++i) {
         e = encode_act_map(&p.tmap_act[0][i], xs, r_max, cfg->hidden, 16 << i);
         if (e == 0) e = encode_act_map(&p.tmap_act[1][i], inter, r_max, cfg->inter, 16 << i);
@@ -1486,7 +1511,33 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     }
   }
   if (ev) cudaEventRecord(ev[5], st);
-  if (both_gemms) {
+  if (plan.N == 128) {
+    // tiles of up to 256 rows on pairs of SMs, both GEMMs in one launch unless two are asked for
+    PairParams q{};
+    q.w[0] = g13.w; q.w[1] = g2.w; q.gs[0] = gs13; q.gs[1] = gs2;
+    q.inter = inter; q.y = y; q.post_norm_w = p.post_norm_w;
+    q.cnt = cnt; q.off = off; q.status = status; q.trace = trace;
+    q.ctr = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
+    q.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);
+    q.tile_seen = q.tile_done + max_tiles(cfg, cfg->max_tokens);
+    q.K[0] = g13.K; q.K[1] = g2.K; q.n_pairs[0] = g13.n_pairs; q.n_pairs[1] = g2.n_pairs;
+    q.nloc = cfg->local_count; q.H = cfg->hidden; q.I = cfg->inter;
+    q.y_bf16 = 1;
+    const bool split = cfg->decode_path == 1 || cfg->stop_after == 2;
+    q.first = 0; q.last = split ? 0 : 1;
+    e = launch_pair(q, xs, r_max, plan.grid, st, pdl);
+    if (e != 0) return e;
+    if (ev) cudaEventRecord(ev[2], st);
+    if (cfg->stop_after == 2) return MSK_OK;
+    if (split) {
+      q.first = q.last = 1;
+      if (trace) q.trace = trace + TRACE_WORDS;
+      e = launch_pair(q, xs, r_max, plan.grid, st, pdl);
+      if (e != 0) return e;
+    }
+    if (ev) cudaEventRecord(ev[3], st);
+    if (cfg->stop_after == 3) return MSK_OK;
+  } else if (both_gemms) {
     p.route = 0; p.fold = 0; p.flat = 0;
     p.x_bf16 = static_cast<const __nv_bfloat16*>(x);
     p.T = n_tokens;
@@ -1505,8 +1556,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   // keep a producing one off the machine), whole units (a cut unit would be counted once per piece) and
   // both launches of the step. Narrow token tiles only, where the gather warp does the waiting: measured at
   // H4096 I1536 E128, 16 / 32 / 64 / 128 tokens take 187 / 242 / 257 / 270 us with it against 190 / 248 /
-  // 266 / 274 without. With the 128-token tile the same hand-over was slower (8192 tokens 2.62 against 2.58 ms) and is
-  // not built; the 64-token tile shares one launch between its GEMMs.
+  // 266 / 274 without. The 64-token tile shares one launch between its GEMMs.
   p.handover = (pdl != 0 && !tma_b && plan.flat == 0 && plan.grid <= sm_count() && cfg->stop_after == 0) ? 1 : 0;
   if (handover_env_off()) p.handover = 0;
   p.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);
@@ -1801,7 +1851,7 @@ int msk_moe_attrs(int which, int token_tile, int* host_out) {
         case 16: e = ph1 ? cudaFuncGetAttributes(&a, moe_gemm_kernel<16, 1>) : cudaFuncGetAttributes(&a, moe_gemm_kernel<16, 0>); break;
         case 32: e = ph1 ? cudaFuncGetAttributes(&a, moe_gemm_kernel<32, 1>) : cudaFuncGetAttributes(&a, moe_gemm_kernel<32, 0>); break;
         case 64: e = ph1 ? cudaFuncGetAttributes(&a, moe_gemm_kernel<64, 1>) : cudaFuncGetAttributes(&a, moe_gemm_kernel<64, 0>); break;
-        case 128: e = ph1 ? cudaFuncGetAttributes(&a, moe_gemm_kernel<128, 1>) : cudaFuncGetAttributes(&a, moe_gemm_kernel<128, 0>); break;
+        case 128: e = cudaFuncGetAttributes(&a, moe_pair_kernel); break;   // both GEMMs
         default: return MSK_ERR_SHAPE;
       }
       break;

@@ -243,6 +243,41 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// This CTA's shared address `addr` as a cluster address of CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+// 16 bytes into the shared memory of any CTA of the cluster, counted on a barrier of that CTA (both cluster addresses).
+__device__ __forceinline__ void st_async_v4(uint32_t addr, int4 v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(v.x),
+               "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+               : "memory");
+}
+// Arrive on a barrier of any CTA of the cluster (a cluster address). What the CTAs of a pair hand over lies in TMEM (ordered by
+// the tcgen05 fences) or was read from the arriving CTA's own shared memory, so no memory is released: with .release.cluster every arrive waits
+// for all of the thread's stores to global memory (the pair kernel took a third longer).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// 2-D tiled TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair (a cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, int c0, int c1, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(bar), "l"(policy)
+      : "memory");
+}
+
 // ------------------------------------------------------------ cp.async 16 B
 __device__ __forceinline__ void cp_async16_hint(void* smem_dst, const void* gmem_src, bool valid, uint64_t policy) {
   // src-size 0 zero-fills the 16 destination bytes (used for padding rows).
@@ -279,6 +314,79 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+// The same for a pair of CTAs (cta_group::2): allocation and release are made by one warp of either CTA, MMAs and commits by
+// one thread of CTA 0; a commit arrives on the barrier at this offset in both CTAs.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+// D[256 rows over both CTAs' TMEM, N] (+)= A[256 rows, 256] (128 rows in either TMEM) * B[N, 256] (N / 2 rows in either CTA): the
+// sixteen MMAs of a K stage (two slots) by one elected lane, and the commits that hand its slots back in both CTAs (empty_bar and
+// the barrier behind it). The answer of a probe of `next_full` (true: complete) is asked for before the MMAs and read behind them, so
+// that its latency hides behind the issue. b_desc: the first of four sub-tiles of 64 K, SUB_BYTES apart.
+template <int SUB_BYTES>
+__device__ __forceinline__ bool mma_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                               uint32_t empty_bar, uint32_t next_full, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred q, e, acc, t;\n\t.reg .b64 b, d;\n\t.reg .b32 a;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%7], %8;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 acc, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [%2], %3, %4, acc;\n\t"
+      "mov.b64 b, %3;\n\tadd.s64 d, b, 2;\n\tadd.u32 a, %2, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], %10;\n\t"
+      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
+      "add.u32 a, %6, 8;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [a], %10;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_full), "r"(parity),
+        "n"(SUB_BYTES >> 4), "h"(static_cast<uint16_t>(3))
+      : "memory");
+  return ok != 0;
 }
 
 // Shared-memory matrix descriptor, K-major, no swizzle ("interleave"): the tile is

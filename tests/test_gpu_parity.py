@@ -442,6 +442,40 @@ def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
         _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
+@pytest.mark.parametrize("H,I,ctas,post,inf", [(256, 256, 0, False, False), (512, 768, 2, True, False), (768, 256, 37, False, True),
+                                               (1024, 512, 296, True, False), (512, 256, 1, False, False)])
+def test_pair_kernel_at_tile_edges(cuda_dev, H, I, ctas, post, inf):
+    """The kernel on pairs of SMs around its tile heights (up to 256 rows an expert a tile, even shares of 32 beyond, one or both
+    accumulator buffers), at its shortest reductions, with an odd grid, one pair and more CTAs than SMs; both GEMMs in one launch
+    and in two give the same bits, twice on one state. A token whose values overflow leaves the rows of the others alone."""
+    m, inputs, _lib, orc = _mods()
+    counts = [1, 31, 32, 33, 64, 127, 128, 129, 160, 255, 256, 257, 300, 511, 513, 600]
+    T, E = 600, len(counts)
+    w = inputs.make_weights(H, I, E, 71, cuda_dev, post_norm=post)
+    kw = dict(n_experts=E, top_k=E, max_tokens=T, token_tile=128, num_ctas=ctas)
+    st, two = m.prepare(w, **kw), m.prepare(w, decode_path=1, **kw)
+    g = torch.Generator(device=cuda_dev).manual_seed(73)
+    ids = torch.stack([torch.where(torch.randperm(T, generator=g, device=cuda_dev) < c, e, -1) for e, c in enumerate(counts)], 1)
+    ids = ids.to(torch.int32).contiguous()
+    tw = torch.rand((T, E), generator=g, device=cuda_dev)
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    data = {"hidden_states": x, "topk_ids": ids, "topk_weights": tw}
+    ref, parts = orc.moe_forward(x, ids, tw, w, return_parts=True)
+    for _ in range(2):
+        out = m.kernel_fn(data, st)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        _check_forward(out, ref, parts, m.workspace_views(st, T))
+        assert torch.equal(m.kernel_fn(data, two), out)
+        assert m.read_status(two) == 0
+    if inf:
+        bad = dict(data, hidden_states=x.clone())
+        bad["hidden_states"][5] = float("nan")
+        got = m.kernel_fn(bad, st)
+        keep = torch.arange(T, device=cuda_dev) != 5
+        assert torch.equal(got[keep], out[keep])
+
+
 @pytest.mark.parametrize("T,scale", [(131, 1.0), (700, 1.0), (300, 60.0)])
 def test_every_token_tile_gives_the_same_swiglu_values(cuda_dev, T, scale):
     """inter of the 16-, 64- and 128-token tiles, bit for bit: the accumulators sum in the same order and the SwiGLU value
