@@ -32,7 +32,7 @@
         if (tid == 128) { if (unit_i == 0) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); MSK_TRD(3, tri, 1); }
         const uint32_t d_tmem = tmem + lane_base + db * (2 * N);
         const float gsc = pp.gs[ui.expert];
-        const bool whole = ks0 == 0 && ks1 == nst_total;
+        const bool whole = (FUSED && TMA_B) || (ks0 == 0 && ks1 == nst_total);   // (one launch: units are never cut; said here where it frees registers)
         bool finish = true;
         int c_first = 0, c_last = 0;
         if (!whole) {
