@@ -26,9 +26,12 @@
       if (lane == 0) mbar_arrive(&ctl.a_full[g][pending_slot]);
       pending = false;
     };
+    // Counts units and is read by nobody: without it the compiler lays this loop out in a form that is 2 % slower with the
+    // 16-token tile (8 / 64 tokens 115.7 / 238.6 us a step, with it 112.6 / 234.2).
+    uint32_t unit_i = 0;
     MSK_PHASES {
       MSK_PHASE_SETUP;
-      while (ok && pieces.next(base, ks0, ks1)) {
+      for (; ok && pieces.next(base, ks0, ks1); ++unit_i) {
         for (int ks = ks0; ks < ks1 && ok; ++ks, ++it) {
           const uint32_t slot = it % NST, par = (it / NST) & 1u;
 #ifdef MSK_TRACE_DETAIL
