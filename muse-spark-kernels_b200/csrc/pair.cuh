@@ -24,9 +24,10 @@
 // Work is dealt one unit at a time from one list, gate/up units (phase 0) before down units (phase 1), ordered (token tile,
 // pair). Units differ in cost by the rows of their tile (an expert's rows are split evenly over its tiles), so a fixed
 // deal leaves SMs idle at the end of each GEMM; drawn from a counter, the down units fill the end of the gate/up
-// phase. A down unit waits for the gate/up units of its token tile: those are drawn before any down unit, by CTAs
-// that are running and wait for nothing themselves, so the wait ends whatever part of the grid is resident. Which cluster
-// computes a unit does not change its bits.
+// phase. A down unit waits for the gate/up units of its token tile: those are drawn before any down unit, by clusters
+// that are running, and a cluster stores its last gate/up unit whether or not the MMAs of its first down unit can start
+// (pair_slots_before_drain), so the wait ends whatever part of the grid is resident. Which cluster computes a unit does not
+// change its bits.
 //
 // Numerics as in gemm.cuh: the same products, FP32 accumulation along K, the same roundings (the same bits as its tiles).
 //
@@ -45,6 +46,7 @@
 
 #include "gemm.cuh"
 #include "layout.cuh"
+#include "pair_sched.h"
 #include "ptx.cuh"
 
 namespace msk {
@@ -52,21 +54,18 @@ namespace msk {
 constexpr int PAIR_THREADS = 640;
 constexpr int PAIR_DQ_WARP = 4;          // first decode warp
 constexpr int PAIR_DQ_WARPS = 16;
-constexpr int PAIR_SLOT_K = 128;         // K of an A / B slot
-constexpr int PAIR_GROUPS = 4;           // of decode warps
 constexpr int PAIR_SLOT_COLS = PAIR_SLOT_K / 2;
-constexpr int PAIR_UNITS = 4;            // units handed out ahead of their use
 constexpr int PAIR_MAPS = 8;             // tensor maps per phase: boxes of 16, 32 .. 128 rows
 
 struct PairCfg {
-  static constexpr int BH = 128;                         // most token rows a CTA holds of a tile
+  static constexpr int BH = PAIR_BH;
   static constexpr int MAX_ROWS = 2 * BH;
   // TMEM: accumulators in the low columns (two buffers of BH columns, or both for a tile of more rows than that), the A ring above
-  static constexpr int NSLOT = 4;
+  static constexpr int NSLOT = PAIR_NSLOT;
   static constexpr int A_BASE = TMEM_COLS - NSLOT * PAIR_SLOT_COLS;
   static constexpr int B_SUB_BYTES = BH * 128;           // 64 K of BH rows
   static constexpr int B_SLOT_BYTES = 2 * B_SUB_BYTES;
-  static constexpr int NST = 5;                          // weight stages
+  static constexpr int NST = PAIR_NST;
   static constexpr int CTRL_BYTES = 1024;
   static constexpr int TABLE_INTS = MAX_LOCAL_EXPERTS + 4;
   static constexpr int SMEM_BYTES = NSLOT * B_SLOT_BYTES + NST * TILE_BYTES + CTRL_BYTES + 3 * TABLE_INTS * 4 + 1024;
@@ -118,10 +117,6 @@ struct PairCtrl {
   int abort_word;
 };
 static_assert(sizeof(PairCtrl) <= 1024 && offsetof(PairCtrl, unit) % 16 == 0, "control block");
-
-// Rows of each tile of an expert with c rows in n tiles: even shares, in steps of 32 (the last tile has the rest, which
-// is never empty: a share is below its limit only while the limit exceeds c / n by more than the rounding).
-__host__ __device__ inline int pair_tile_rows(int c, int n) { return ((c + n - 1) / n + 31) & ~31; }
 
 // The accumulator buffer of each unit in turn: a tile of up to BH rows takes one of two buffers of BH columns, a wider
 // one takes both. MMA issuer and decode warps walk the same sequence.
@@ -523,7 +518,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     PairBuffers db;
     bool ok = true, owe = false;
     uint32_t di = 0;                               // next unit to drain; its record stays in the list until then
-    int owed_cols = 0;
+    int owed_cols = 0, owed_phase = 0;
     auto drain = [&]() -> bool {
       const uint32_t at = di % PAIR_UNITS;
       ++di;
@@ -558,9 +553,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       const int phase = ctl.unit[us].phase, cols = ctl.unit[us].nmma;
       more = phase >= 0;
       const int nsl = more ? p.K[phase] / PAIR_SLOT_K : 0;
-      // The unit before is drained once this warp has decoded ahead for this one: its first slot when this unit's MMAs
-      // need the accumulators back, its second one when they have the other buffer; at the latest when its slots are done.
-      int ahead = (cols > BH || owed_cols > BH) ? 1 : 2;
+      // the unit before is drained once this warp has decoded ahead for this one, at the latest when its slots are done
+      int ahead = pair_slots_before_drain(owed_phase, owed_cols, phase, cols);
       int s = static_cast<int>((static_cast<uint32_t>(g) - sc) & 3u);
       sc += static_cast<uint32_t>(nsl);
       while (true) {
@@ -611,6 +605,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         if (!slot) break;
       }
       owed_cols = cols;
+      owed_phase = phase;
       owe = true;
     }
   }

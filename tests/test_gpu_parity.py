@@ -476,6 +476,50 @@ def test_pair_kernel_at_tile_edges(cuda_dev, H, I, ctas, post, inf):
         assert torch.equal(got[keep], out[keep])
 
 
+@pytest.mark.parametrize("H,I,ctas,counts", [(512, 768, 0, [64] * 8), (512, 768, 2, [100]), (1024, 1536, 0, [41, 128, 97, 64]),
+                                             (1024, 1536, 2, [0, 90, 0]), (512, 4096, 0, [64, 65]), (512, 4096, 2, [128, 41, 77]),
+                                             (2048, 1024, 0, [64] * 8), (2048, 1024, 37, [128] * 5 + [33]), (4096, 1536, 0, [64] * 6)])
+def test_pair_kernel_hands_few_narrow_tiles_from_gate_up_to_down(cuda_dev, H, I, ctas, counts):
+    """Few token tiles of one accumulator buffer and reductions of more A slots than the ring has: a cluster goes from its last gate/up
+    unit straight to a down unit that may wait for it. Both GEMMs in one launch against two launches, bit for bit, and the oracle."""
+    m, inputs, _lib, orc = _mods()
+    E, T = len(counts), 128
+    w = inputs.make_weights(H, I, E, 83, cuda_dev)
+    kw = dict(n_experts=E, top_k=E, max_tokens=T, token_tile=128, num_ctas=ctas)
+    st, two = m.prepare(w, **kw), m.prepare(w, decode_path=1, **kw)
+    g = torch.Generator(device=cuda_dev).manual_seed(89)
+    ids = torch.stack([torch.where(torch.randperm(T, generator=g, device=cuda_dev) < c, e, -1) for e, c in enumerate(counts)], 1)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "topk_ids": ids.to(torch.int32).contiguous(), "topk_weights": torch.rand((T, E), generator=g, device=cuda_dev)}
+    ref, parts = orc.moe_forward(data["hidden_states"], data["topk_ids"], data["topk_weights"], w, return_parts=True)
+    want = m.kernel_fn(data, two)
+    assert m.read_status(two) == 0
+    for _ in range(3):
+        out = m.kernel_fn(data, st)
+        assert m.read_status(st) == 0
+        assert torch.equal(out, want)
+    _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
+@pytest.mark.parametrize("E,k,nloc,T", [(8, 2, 8, 256), (128, 8, 4, 700)])
+def test_pair_kernel_by_default_on_a_handful_of_experts(cuda_dev, E, k, nloc, T):
+    """The default plan takes the pair kernel by the mean rows per expert, also where only a handful of experts is there."""
+    m, inputs, _lib, orc = _mods()
+    H, I = 1024, 1536
+    w = inputs.make_weights(H, I, nloc, 97, cuda_dev)
+    st = m.prepare(w, n_experts=E, top_k=k, local_start=E // 2 - nloc // 2 if nloc < E else 0, max_tokens=T)
+    assert m.plan(st, T)[0] == 128
+    data = dict(hidden_states=torch.randn((T, H), device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(5)).to(torch.bfloat16))
+    ids = torch.stack([(torch.arange(T, device=cuda_dev) * k + j) % E for j in range(k)], 1).to(torch.int32)   # even rows
+    tw = torch.full((T, k), 1.0 / k, device=cuda_dev)
+    data.update(topk_ids=ids.contiguous(), topk_weights=tw)
+    for _ in range(2):
+        out = m.kernel_fn(data, st)
+        assert m.read_status(st) == 0
+    ref, parts = orc.moe_forward(data["hidden_states"], ids, tw, w, local_start=E // 2 - nloc // 2 if nloc < E else 0, return_parts=True)
+    _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
 @pytest.mark.parametrize("T,scale", [(131, 1.0), (700, 1.0), (300, 60.0)])
 def test_every_token_tile_gives_the_same_swiglu_values(cuda_dev, T, scale):
     """inter of the 16-, 64- and 128-token tiles, bit for bit: the accumulators sum in the same order and the SwiGLU value
