@@ -293,11 +293,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
   if (tid == 0) MSK_TR(TR_SETUP);
   auto lead_bar = [&](const uint64_t* bar) -> uint32_t { return lead + (smem_u32(bar) - smem_u32(&ctl)); };
 
-  // Units, as the single-lane roles walk them: wait_unit() waits for the next one and copies it, done_unit() hands its place back.
+  // Units, as the roles beside the decode warps walk them: wait_unit() waits for the next one and copies it (for a single
+  // lane, or for a whole warp with one outcome), done_unit() hands its place back. Every wait of a whole warp is mbar_wait_warp:
+  // what follows are full-warp instructions (elect, tcgen05.ld / st, __syncwarp).
   uint32_t ui = 0;
-  auto wait_unit = [&](PairUnit& u) -> bool {
+  auto wait_unit = [&](PairUnit& u, auto wait) -> bool {
     const uint32_t s = ui % PAIR_UNITS;
-    if (!mbar_wait_inline(&ctl.u_full[s], (ui / PAIR_UNITS) & 1u, abortw)) return false;
+    if (!wait(&ctl.u_full[s], (ui / PAIR_UNITS) & 1u, abortw)) return false;
     const int4 x = *reinterpret_cast<const int4*>(&ctl.unit[s]), y = *(reinterpret_cast<const int4*>(&ctl.unit[s]) + 1);
     u.phase = x.x; u.expert = x.y; u.row0 = x.z; u.rows = x.w;
     u.pair = y.x; u.tile = y.y; u.nmma = y.z;
@@ -313,7 +315,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       uint32_t ws = 0, wpar = 0;
       bool ok = true;
       PairUnit u;
-      while (ok && wait_unit(u)) {
+      while (ok && wait_unit(u, mbar_wait_inline)) {
         done_unit();
         if (u.phase < 0) break;
         const int nst = p.K[u.phase] / KS;
@@ -336,18 +338,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       bool ready = false;                          // the stage at sl was seen full while the one before was issued
       bool ok = true;
       PairUnit u;
-      while (ok && wait_unit(u)) {
+      while (ok && wait_unit(u, mbar_wait_warp)) {
         __syncwarp();
         if (lane == 0) done_unit();
         if (u.phase < 0) break;
         const uint32_t idesc = idesc_f16(FMT_F16, FMT_F16, 256, static_cast<uint32_t>(u.nmma));
         db.take(u.nmma);
-        if (db.uses(0) && !mbar_wait_inline(&ctl.d_empty[0], db.p0 ^ 1u, abortw)) { ok = false; break; }
-        if (db.uses(1) && !mbar_wait_inline(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) { ok = false; break; }
+        if (db.uses(0) && !mbar_wait_warp(&ctl.d_empty[0], db.p0 ^ 1u, abortw)) { ok = false; break; }
+        if (db.uses(1) && !mbar_wait_warp(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) { ok = false; break; }
         const uint32_t d_tmem = tmem + db.buf * static_cast<uint32_t>(BH);
         tc_fence_after();
         for (int k = 0; k < p.K[u.phase]; k += KS) {
-          if (!ready && !mbar_wait_inline(&ctl.full[sl >> 1], spar, abortw)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.full[sl >> 1], spar, abortw)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sn = sl + 2 == NSLOT ? 0u : sl + 2, pn = sn == 0u ? spar ^ 1u : spar;
           ready = mma_stage_pair<C::B_SUB_BYTES>(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + sl * (C::B_SLOT_BYTES >> 4), idesc,
@@ -370,7 +372,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     bool ok = true;
     int last_tile = -1;
     PairUnit u;
-    while (ok && wait_unit(u)) {
+    while (ok && wait_unit(u, mbar_wait_warp)) {
       __syncwarp();
       if (lane == 0) done_unit();
       if (u.phase < 0) break;
@@ -380,7 +382,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       const uint32_t bytes = static_cast<uint32_t>(half) * 256u * 2u * 2u;   // 256 K of both CTAs' rows
       if (u.phase == 1 && p.first == 0) {
         if (u.tile != last_tile) {
-          if (!grid_counter_wait(p.tile_done + u.tile, 2u * static_cast<unsigned>(p.n_pairs[0]), abortw)) { ok = false; break; }
+          const bool seen = grid_counter_wait(p.tile_done + u.tile, 2u * static_cast<unsigned>(p.n_pairs[0]), abortw);
+          if (!__all_sync(0xffffffffu, seen)) { ok = false; break; }
           fence_proxy_async_all();                 // ordinary stores of other SMs, about to be read by bulk copies
           last_tile = u.tile;
           __syncwarp();
@@ -399,7 +402,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         const uint32_t bar = lead_bar(&ctl.full[sl >> 1]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if (!mbar_wait_inline(&ctl.empty[sl + h], spar ^ 1u, abortw)) { ok = false; break; }
+          if (!mbar_wait_warp(&ctl.empty[sl + h], spar ^ 1u, abortw)) { ok = false; break; }
           if (elect_one()) {
             if (h == 0 && rank == 0) mbar_arrive_expect_tx(&ctl.full[sl >> 1], bytes);
             uint8_t* dst = b_ring + (sl + h) * C::B_SLOT_BYTES;
@@ -414,7 +417,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     }
     // the commits of the last slots arrive in this CTA's shared memory: it stays until they have
     for (int i = 0; ok && i < NSLOT; ++i) {
-      if (!mbar_wait_inline(&ctl.empty[sl], spar ^ 1u, abortw)) break;
+      if (!mbar_wait_warp(&ctl.empty[sl], spar ^ 1u, abortw)) break;
       if (++sl == NSLOT) { sl = 0; spar ^= 1u; }
     }
   } else if (warp == 3) {
@@ -429,7 +432,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     };
     if (rank != 0) {
       PairUnit u;
-      while (lane == 0 && wait_unit(u)) {
+      while (lane == 0 && wait_unit(u, mbar_wait_inline)) {
         const uint32_t i = ui - 1u;
         const bool ok = u.phase != 0 || p.last == 0 || announce(i % PAIR_UNITS, (i / PAIR_UNITS) & 1u, u.tile);
         done_unit();
@@ -526,8 +529,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       PairUnit u;
       u.phase = r.phase; u.expert = r.expert; u.row0 = r.row0; u.rows = r.rows; u.pair = r.pair; u.tile = r.tile; u.nmma = r.nmma;
       db.take(u.nmma);
-      if (db.uses(0) && !mbar_wait_inline(&ctl.d_full[0], db.p0, abortw)) return false;
-      if (db.uses(1) && !mbar_wait_inline(&ctl.d_full[1], db.p1, abortw)) return false;
+      if (db.uses(0) && !mbar_wait_warp(&ctl.d_full[0], db.p0, abortw)) return false;
+      if (db.uses(1) && !mbar_wait_warp(&ctl.d_full[1], db.p1, abortw)) return false;
       tc_fence_after();
       pair_epilogue(p, u, tmem + lane_base + db.buf * static_cast<uint32_t>(BH), static_cast<int>(rank), q, g, lane, [&]() {
         tc_fence_before();
@@ -548,7 +551,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     bool more = true;
     while (ok && more) {
       const uint32_t us = ui % PAIR_UNITS;
-      if (!mbar_wait_inline(&ctl.u_full[us], (ui / PAIR_UNITS) & 1u, abortw)) break;
+      if (!mbar_wait_warp(&ctl.u_full[us], (ui / PAIR_UNITS) & 1u, abortw)) break;
       ++ui;
       const int phase = ctl.unit[us].phase, cols = ctl.unit[us].nmma;
       more = phase >= 0;
@@ -560,7 +563,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       while (true) {
         const bool slot = s < nsl;
         if (slot) {
-          if (!mbar_wait_inline(&ctl.raw_full[ws], wpar, abortw)) { ok = false; break; }
+          if (!mbar_wait_warp(&ctl.raw_full[ws], wpar, abortw)) { ok = false; break; }
           const uint32_t tile_row = smem_u32(w_ring + ws * TILE_BYTES) + row_off;
           uint32_t sf[2];
           asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(sf[0]), "=r"(sf[1]) : "r"(tile_row + OCT_CODE_BYTES + kh * 8));
@@ -579,7 +582,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
 #pragma unroll
             for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(o[c][j]));   // here, not behind the wait
           }
-          if (!mbar_wait_inline(&ctl.empty[as], spar ^ 1u, abortw)) { ok = false; break; }
+          if (!mbar_wait_warp(&ctl.empty[as], spar ^ 1u, abortw)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_tmem = a_ring + as * PAIR_SLOT_COLS;
 #pragma unroll

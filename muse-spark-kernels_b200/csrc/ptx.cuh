@@ -131,6 +131,22 @@ __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same wait for a whole warp, with one outcome: every lane polls for itself (and so acquires what the barrier publishes),
+// and the warp goes on once all lanes have seen the phase complete, or gives up together. Lanes that gave up one by one
+// would leave the others behind in full-warp instructions. All 32 lanes call it.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t polls = 0;
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait_parked(bar, parity, 4000u))) return true;
+    if ((++polls & 15u) == 0u && __any_sync(0xffffffffu, *abort_word != 0 || globaltimer_ns() - t0 > MSK_WAIT_LIMIT_NS)) {
+      *abort_word = 1;
+      return false;
+    }
+  }
+}
+
 // The same wait for hand-offs that complete within a few hundred cycles (the 128 epilogue threads
 // meeting at their barrier): poll without parking first, so that the wake-up latency of a parked
 // thread is not paid on every meeting; then fall back to the parked wait.

@@ -1139,6 +1139,33 @@ def test_few_token_kernel_gives_up_cleanly_and_recovers(cuda_dev, T, post):
     assert m.read_status(st) == 0
 
 
+@pytest.mark.parametrize("ctas,rows", [(2, 64), (2, 200), (6, 64)])
+def test_pair_kernel_gives_up_cleanly_and_recovers(cuda_dev, ctas, rows):
+    """The same for the pair kernel: the first token tile's counter one short. Each cluster has announced gate/up units of that
+    tile before it asks for the count (a place of its unit list is used again behind the announcement), so the wait of
+    the tile's down units cannot be met and runs out; whole warps give up together and the status says so."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E = 512, 1024 * (ctas // 2), 2
+    w = inputs.make_weights(H, I, E, 8, cuda_dev)
+    st = m.prepare(w, n_experts=E, top_k=1, max_tokens=2 * rows, token_tile=128, num_ctas=ctas)
+    g = torch.Generator(device=cuda_dev).manual_seed(4)
+    data = {"hidden_states": torch.randn((2 * rows, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "topk_ids": torch.arange(2 * rows, device=cuda_dev, dtype=torch.int32).remainder(2).reshape(-1, 1).contiguous(),
+            "topk_weights": torch.ones((2 * rows, 1), device=cuda_dev)}
+    clean = m.kernel_fn(data, st).clone()
+    assert m.read_status(st) == 0
+    ptr = ctypes.c_void_p()
+    _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 10, ctypes.byref(ptr)), "view")
+    tile0 = ptr.value - st["workspace"].data_ptr()
+    st["workspace"][tile0:tile0 + 4].fill_(255)
+    m.kernel_fn(data, st)
+    assert m.read_status(st) == 1
+    m.reinit_workspace(st)
+    for _ in range(2):
+        assert torch.equal(m.kernel_fn(data, st), clean)
+    assert m.read_status(st) == 0
+
+
 def test_state_dict_round_trip_skips_the_repack(cuda_dev):
     """state_dict() / load_state_dict(): the packed tiles, scales and configuration are enough to
     rebuild a state; kernel_fn on the rebuilt state gives the same bits."""
