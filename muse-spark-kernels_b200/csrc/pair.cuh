@@ -15,7 +15,8 @@
 //   warp 1        CTA 0: MMA issuer; both: TMEM allocation;
 //   warp 2        activations: four TMA boxes (64 K x half the tile's rows, 128-byte swizzle) per K stage; the copies of
 //                 both CTAs complete on CTA 0's barrier;
-//   warp 3        CTA 0: scheduler: draws units from a counter in global memory and hands them to both CTAs;
+//   warp 3        CTA 0: scheduler: draws units from a counter in global memory and hands them to both CTAs; both: counts
+//                 drained gate/up units for their token tile;
 //   warps 4-19    decode: group g = 0..3 of four warps fills every fourth A slot (128 K) of the ring; the same warps drain the
 //                 accumulators.
 // TMEM lanes 32q .. 32q+15 hold rows of the first tile of the pair (gate, or the even row tile), lanes 32q+16 .. 32q+31 the
@@ -109,8 +110,8 @@ struct PairCtrl {
   uint64_t d_full[2];                    // committed into both CTAs
   uint64_t d_empty[2];                   // CTA 0: drained by both CTAs
   uint64_t u_full[PAIR_UNITS];           // local
-  uint64_t u_empty[PAIR_UNITS];          // CTA 0
-  uint64_t stored[PAIR_UNITS];           // local: the decode warps have stored their values of a gate/up unit
+  uint64_t u_empty[PAIR_UNITS];          // CTA 0: CTA 1 is done with the unit
+  uint64_t u_done[PAIR_UNITS];           // local: the decode warps have stored their values of a unit, and every role has read its record
   PairUnit unit[PAIR_UNITS];
   int owed_tile[PAIR_UNITS];             // scheduler: tile to announce when a place's gate/up unit is stored, else -1
   uint32_t tmem_base;
@@ -269,8 +270,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     }
     for (int i = 0; i < PAIR_UNITS; ++i) {
       mbar_init(&ctl.u_full[i], 1);
-      mbar_init(&ctl.u_empty[i], 2 * (PAIR_DQ_WARPS + 2) + 2);   // decode warps, producer and activations of either CTA, MMA issuer, CTA 1's warp 3
-      mbar_init(&ctl.stored[i], PAIR_DQ_WARPS);
+      mbar_init(&ctl.u_empty[i], 1);
+      mbar_init(&ctl.u_done[i], PAIR_DQ_WARPS + 3 - rank);   // producer, activations and, in CTA 0, the MMA issuer
     }
     ctl.abort_word = 0;
     fence_mbar_init();
@@ -306,7 +307,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     ++ui;
     return true;
   };
-  auto done_unit = [&]() { mbar_arrive_cluster(lead_bar(&ctl.u_empty[(ui - 1u) % PAIR_UNITS])); };
+  auto done_unit = [&]() { mbar_arrive(&ctl.u_done[(ui - 1u) % PAIR_UNITS]); };
 
   if (warp == 0) {
     // ------------------------------------------------------- weight producer
@@ -422,21 +423,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     }
   } else if (warp == 3) {
     // ------------------------------------------- scheduler; announces stored gate/up units
-    // The decode warps' stores are released to the other SMs here: a fence in the decode warps costs them a round trip to
-    // memory per unit. A place of the unit list is handed back behind the stores, so a barrier is not met twice in a phase.
-    auto announce = [&](uint32_t s, uint32_t par, int tile) -> bool {
-      if (!mbar_wait_inline(&ctl.stored[s], par, abortw)) return false;
+    // What the other roles do with a unit they release to this CTA only (u_done). From here the decode warps' stores are released to
+    // the other SMs, and CTA 1's reads of the unit's record to CTA 0, which writes the next one there: a fence of that scope costs
+    // a round trip to memory per unit, in the decode warps or the MMA issuer 1 to 5 % of the kernel. A place of the unit list is
+    // handed back behind the drain of its unit, so a barrier is not met twice in a phase.
+    auto announce = [&](int tile) {
       fence_proxy_async_all();                     // the rows' readers are bulk copies
       red_release_add(p.tile_done + tile, 1u);
-      return true;
     };
     if (rank != 0) {
       PairUnit u;
-      while (lane == 0 && wait_unit(u, mbar_wait_inline)) {
+      while (lane == 0 && wait_unit(u, mbar_wait_inline) && u.phase >= 0) {
         const uint32_t i = ui - 1u;
-        const bool ok = u.phase != 0 || p.last == 0 || announce(i % PAIR_UNITS, (i / PAIR_UNITS) & 1u, u.tile);
-        done_unit();
-        if (!ok || u.phase < 0) break;
+        if (!mbar_wait_inline(&ctl.u_done[i % PAIR_UNITS], (i / PAIR_UNITS) & 1u, abortw)) break;
+        if (u.phase == 0 && p.last == 1) announce(u.tile);
+        mbar_arrive_release_cluster(lead_bar(&ctl.u_empty[i % PAIR_UNITS]));
       }
     } else {
       int carry = 0;
@@ -486,8 +487,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             b = make_int4(pair, tile, (rows + 31) & ~31, 0);
           }
           const uint32_t s = i % PAIR_UNITS;
-          if (i >= PAIR_UNITS && ctl.owed_tile[s] >= 0 && !announce(s, ((i / PAIR_UNITS) & 1u) ^ 1u, ctl.owed_tile[s])) { ok = false; break; }
-          if (!mbar_wait_inline(&ctl.u_empty[s], ((i / PAIR_UNITS) & 1u) ^ 1u, abortw)) { ok = false; break; }
+          const uint32_t par = ((i / PAIR_UNITS) & 1u) ^ 1u;   // of the unit whose place this one takes
+          if (i >= PAIR_UNITS) {
+            if (!mbar_wait_inline(&ctl.u_done[s], par, abortw)) { ok = false; break; }
+            if (ctl.owed_tile[s] >= 0) announce(ctl.owed_tile[s]);
+          }
+          if (!mbar_wait_cluster(&ctl.u_empty[s], par, abortw)) { ok = false; break; }
           const uint32_t at = smem_u32(&ctl.unit[s]) - smem_u32(&ctl), bar = smem_u32(&ctl.u_full[s]) - smem_u32(&ctl);
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
@@ -501,7 +506,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         }
         for (uint32_t j = i >= PAIR_UNITS ? i - PAIR_UNITS : 0u; ok && j < i; ++j) {   // the units still in the list
           const uint32_t s = j % PAIR_UNITS;
-          if (ctl.owed_tile[s] >= 0) ok = announce(s, (j / PAIR_UNITS) & 1u, ctl.owed_tile[s]);
+          if (ctl.owed_tile[s] < 0) continue;
+          ok = mbar_wait_inline(&ctl.u_done[s], (j / PAIR_UNITS) & 1u, abortw);
+          if (ok) announce(ctl.owed_tile[s]);
         }
       }
     }
@@ -541,10 +548,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         }
       });
       __syncwarp();
-      if (lane == 0) {
-        if (u.phase == 0 && p.last == 1) mbar_arrive(&ctl.stored[at]);
-        mbar_arrive_cluster(lead_bar(&ctl.u_empty[at]));
-      }
+      if (lane == 0) mbar_arrive(&ctl.u_done[at]);   // (releases to this CTA only, which waits for no store)
       owe = false;
       return true;
     };

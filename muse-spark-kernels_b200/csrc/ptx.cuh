@@ -131,6 +131,30 @@ __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same wait, acquiring what threads of the other CTAs of the cluster have released by their arrives.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t polls = 0;
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(4000u)
+        : "memory");
+    if (ok) return true;
+    if ((++polls & 15u) == 0u) {
+      if (*abort_word != 0) return false;
+      if (globaltimer_ns() - t0 > MSK_WAIT_LIMIT_NS) {
+        *abort_word = 1;
+        return false;
+      }
+    }
+  }
+}
+
 // The same wait for a whole warp, with one outcome: every lane polls for itself (and so acquires what the barrier publishes),
 // and the warp goes on once all lanes have seen the phase complete, or gives up together. Lanes that gave up one by one
 // would leave the others behind in full-warp instructions. All 32 lanes call it.
@@ -276,11 +300,14 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, int4 v, uint32_t bar)
                "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
                : "memory");
 }
-// Arrive on a barrier of any CTA of the cluster (a cluster address). What the CTAs of a pair hand over lies in TMEM (ordered by
-// the tcgen05 fences) or was read from the arriving CTA's own shared memory, so no memory is released: with .release.cluster every arrive waits
-// for all of the thread's stores to global memory (the pair kernel took a third longer).
+// Arrive on a barrier of any CTA of the cluster (a cluster address). The relaxed form is for what lies in TMEM, ordered by the
+// tcgen05 fences; the other one releases this thread's reads and writes of memory as well, and so waits for all of its stores to
+// global memory (in place of the relaxed one everywhere the pair kernel took a third longer).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
