@@ -118,7 +118,7 @@ struct PhaseParams {
 };
 
 struct GemmParams {
-  CUtensorMap tmap_act[2][4];   // TMA_B only, per phase: [rows, K] f16, boxes 64 x (16 << i) up to 64 x N, 128-byte swizzle
+  CUtensorMap tmap_act[2][3];   // TMA_B only, per phase: [rows, K] f16, boxes 64 x (16 << i) up to 64 x N, 128-byte swizzle
                                 // (64-byte aligned: first member)
   PhaseParams ph[2];         // [0] gate/up, [1] down; a single-phase launch uses its own entry only
   const __nv_bfloat16* post_norm_w;  // phase 1, nullable
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) moe_gemm_kernel(const __grid_
     ctl.fin_n = 0;
     fence_mbar_init();
   }
-  if (TMA_B && warp == 2 && lane < 4 && (16 << lane) <= N) prefetch_tensormap(&p.tmap_act[PH_FIRST][lane]);
+  if (TMA_B && warp == 2 && lane < 3 && (16 << lane) <= N) prefetch_tensormap(&p.tmap_act[PH_FIRST][lane]);
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, TMEM_COLS);
     tmem_relinquish();

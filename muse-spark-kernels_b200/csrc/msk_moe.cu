@@ -235,7 +235,7 @@ constexpr int COMBINE_THREADS = 512;
 constexpr int COMBINE_MAX_F4 = 4;   // float4 per thread per row: H <= 8192
 constexpr int COMBINE_WIDE_TOKENS = 512;  // from here on two blocks per SM, two slots per group
 
-// Eight consecutive y values of a row, FP32 or BF16 (the 128-token tile), in registers while in flight.
+// Eight consecutive y values of a row, FP32 or BF16 (the pair kernel's), in registers while in flight.
 template <bool YB> struct YOct;
 template <> struct YOct<false> {
   float4 a, b;
@@ -1273,7 +1273,7 @@ int msk_moe_workspace_view(const MskMoeCfg* cfg, void* workspace, int which, voi
   return MSK_OK;
 }
 
-// y_bf16: the 128-token tile keeps y in BF16 (half the bytes written and read back).
+// y_bf16: the pair kernel keeps y in BF16 (half the bytes written and read back).
 static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, const int32_t* inv, const float* tw, void* out,
                           int n_tokens, bool post_norm, int pdl, cudaStream_t st) {
   cudaLaunchConfig_t lc{};
@@ -1515,14 +1515,13 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     // tiles of up to 256 rows on pairs of SMs, both GEMMs in one launch unless two are asked for
     PairParams q{};
     q.w[0] = g13.w; q.w[1] = g2.w; q.gs[0] = gs13; q.gs[1] = gs2;
-    q.inter = inter; q.y = y; q.post_norm_w = p.post_norm_w;
+    q.inter = inter; q.y = reinterpret_cast<__nv_bfloat16*>(y); q.post_norm_w = p.post_norm_w;
     q.cnt = cnt; q.off = off; q.status = status; q.trace = trace;
     q.ctr = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
     q.tile_done = reinterpret_cast<unsigned int*>(b + k.tile_ctr);
     q.tile_seen = q.tile_done + max_tiles(cfg, cfg->max_tokens);
     q.K[0] = g13.K; q.K[1] = g2.K; q.n_pairs[0] = g13.n_pairs; q.n_pairs[1] = g2.n_pairs;
     q.nloc = cfg->local_count; q.H = cfg->hidden; q.I = cfg->inter;
-    q.y_bf16 = 1;
     const bool split = cfg->decode_path == 1 || cfg->stop_after == 2;
     q.first = 0; q.last = split ? 0 : 1;
     e = launch_pair(q, xs, r_max, plan.grid, st, pdl);

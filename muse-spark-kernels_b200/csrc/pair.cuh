@@ -79,7 +79,7 @@ struct PairParams {
   const uint8_t* w[2];                   // packed tiles
   const float* gs[2];
   __half* inter;                         // [R, I]
-  void* y;                               // [R, H]
+  __nv_bfloat16* y;                      // [R, H]
   const __nv_bfloat16* post_norm_w;      // nullable
   const int32_t* cnt;
   const int32_t* off;
@@ -92,7 +92,6 @@ struct PairParams {
   int n_pairs[2];
   int nloc;
   int H, I;
-  int y_bf16;                            // y in BF16, else FP32
   int first, last;                       // phases of this launch
 };
 
@@ -209,21 +208,13 @@ __device__ __forceinline__ void pair_epilogue(const PairParams& p, const PairUni
     const int col = (2 * u.pair + t) * 128 + r;
     float osc = gsc;
     if (p.post_norm_w != nullptr) osc *= 1.0f + __bfloat162float(p.post_norm_w[col]);
-    const size_t at = static_cast<size_t>(u.row0 + c0) * ld + col;
-    __nv_bfloat16* yb = static_cast<__nv_bfloat16*>(p.y) + at;
-    float* yf = static_cast<float*>(p.y) + at;
+    __nv_bfloat16* outp = p.y + static_cast<size_t>(u.row0 + c0) * ld + col;
     int left = lim;
     auto store = [&](const uint32_t (&v)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const float f = __uint_as_float(v[j]) * osc;
-        if (p.y_bf16) {
-          if (left > j) *yb = __float2bfloat16_rn(f);
-        } else {
-          if (left > j) *yf = f;
-        }
-        yb += ld;
-        yf += ld;
+        if (left > j) *outp = __float2bfloat16_rn(__uint_as_float(v[j]) * osc);
+        outp += ld;
       }
       left -= 16;
     };
@@ -530,11 +521,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     uint32_t di = 0;                               // next unit to drain; its record stays in the list until then
     int owed_cols = 0, owed_phase = 0;
     auto drain = [&]() -> bool {
-      const uint32_t at = di % PAIR_UNITS;
-      ++di;
-      const PairUnit& r = ctl.unit[at];
+      const PairUnit& r = ctl.unit[di % PAIR_UNITS];
       PairUnit u;
-      u.phase = r.phase; u.expert = r.expert; u.row0 = r.row0; u.rows = r.rows; u.pair = r.pair; u.tile = r.tile; u.nmma = r.nmma;
+      u.phase = r.phase; u.expert = r.expert; u.row0 = r.row0; u.rows = r.rows; u.pair = r.pair; u.nmma = r.nmma;
       db.take(u.nmma);
       if (db.uses(0) && !mbar_wait_warp(&ctl.d_full[0], db.p0, abortw)) return false;
       if (db.uses(1) && !mbar_wait_warp(&ctl.d_full[1], db.p1, abortw)) return false;
@@ -548,7 +537,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         }
       });
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl.u_done[at]);   // (releases to this CTA only, which waits for no store)
+      if (lane == 0) mbar_arrive(&ctl.u_done[di % PAIR_UNITS]);   // (releases to this CTA only, which waits for no store)
+      ++di;
       owe = false;
       return true;
     };
