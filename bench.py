@@ -351,6 +351,7 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     one_launch = plan[1] == 0 and T <= 32 and R <= 256
     # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine
     both_gemms = plan[1] == 4 or (plan[0] == 64 and not plan[2] and state["cfg"].decode_path != 1)
+    pair = plan[0] == 128 and state["cfg"].decode_path != 1     # both GEMMs in one launch on pairs of SMs
     step_bytes = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(steps)) / steps
     step_flops = inputs.algorithmic_flops(H, I, R)
     if one_launch:
@@ -375,6 +376,13 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
                 "traffic_source": "ncu dram bytes of the kernel's 32-expert capture / its algorithmic bytes (%.2f), scaled" % ratio,
                 "kernel": "moe_gemm_kernel<N,2> (gate/up and down GEMM in one launch)",
                 "peak_source": peaks["source"] + " (burst copy)"}
+    elif pair and T <= 1024:
+        # the touched experts' tiles of both GEMMs, the sorted rows read, inter written and read back, y written (BF16)
+        alg = mean_touched * (3 * I * H * 0.5625 + 8) + 2.0 * R * H + 4.0 * R * I + 2.0 * R * H
+        achieved = alg / (k_ms[2] * 1e-3) / 1e9
+        roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                "frac": achieved / peaks["hbm_gbs"], "traffic": None,
+                "kernel": "moe_pair_kernel (gate/up and down GEMM in one launch)", "peak_source": peaks["source"] + " (burst copy)"}
     elif T <= 1024:
         # gate/up GEMM: touched experts' W13 tiles + the x rows it gathers + the inter rows it writes
         alg13 = mean_touched * (2 * I * H * 0.5625 + 4) + 2.0 * T * H + 2.0 * R * I
@@ -385,7 +393,6 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
                 "kernel": "moe_gemm_kernel<N,0> (gate/up)", "peak_source": peaks["source"] + " (burst copy)"}
     else:
         # 128-token plans run both GEMMs in one launch; the narrower ones are timed for the gate/up GEMM
-        pair = plan[0] == 128 and state["cfg"].decode_path != 1
         fl = 2.0 * R * (3 if pair else 2) * I * H
         achieved = fl / (k_ms[2] * 1e-3) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
@@ -401,7 +408,7 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     elif both_gemms:      # top-k and sort (one launch up to 32 tokens, two beyond), [row copy,] both GEMMs, combine
         launches = (3 if T <= 32 else 4) + (1 if plan[0] == 64 else 0)
     else:                 # top-k and sort, row copy (in the sort launch up to 32 tokens), GEMMs (two, 128-token plans one), combine
-        launches = 4 if T <= 32 else 5 if plan[0] == 128 and state["cfg"].decode_path != 1 else 6
+        launches = 4 if T <= 32 else 5 if pair else 6
     return {
         "workload": spec["name"], "tokens": T, "steps": steps, "ms_per_step": total_ms / steps,
         "value": T / sec, "unit": UNIT,
