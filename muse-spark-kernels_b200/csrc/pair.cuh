@@ -316,6 +316,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
           if (!mbar_wait_inline(&ctl.raw_empty[ws], wpar ^ 1u, abortw)) { ok = false; break; }
           mbar_arrive_expect_tx(&ctl.raw_full[ws], TILE_BYTES);
           bulk_g2s(w_ring + ws * TILE_BYTES, src, TILE_BYTES, &ctl.raw_full[ws], pol);
+          if (ui == 1u && ks == 0) MSK_TR(TR_FIRST_BULK);
           src += STAGE_W_BYTES;
           if (++ws == NST) { ws = 0; wpar ^= 1u; }
         }
@@ -528,6 +529,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       if (db.uses(0) && !mbar_wait_warp(&ctl.d_full[0], db.p0, abortw)) return false;
       if (db.uses(1) && !mbar_wait_warp(&ctl.d_full[1], db.p1, abortw)) return false;
       tc_fence_after();
+      if (tid == PAIR_DQ_WARP * 32) { if (di == 0u) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); }
       pair_epilogue(p, u, tmem + lane_base + db.buf * static_cast<uint32_t>(BH), static_cast<int>(rank), q, g, lane, [&]() {
         tc_fence_before();
         __syncwarp();
@@ -537,6 +539,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         }
       });
       __syncwarp();
+      if (tid == PAIR_DQ_WARP * 32 && di == 0u) MSK_TR(TR_FIRST_EPI_DONE);
       if (lane == 0) mbar_arrive(&ctl.u_done[di % PAIR_UNITS]);   // (releases to this CTA only, which waits for no store)
       ++di;
       owe = false;
