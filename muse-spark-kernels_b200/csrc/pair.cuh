@@ -34,10 +34,13 @@
 //
 // Measured (both GEMMs, us, against one CTA to a tile of up to 128 tokens, which this replaces): 8192 tokens of Zipf routes at
 // H4096 I1536 E128 1997 -> 1928; 8192 tokens at one rank of eight, H7168 I2048, 605 -> 540; 3012 skewed tokens at a rank, H4096 I4096,
-// 462 -> 444; 777 tokens, 49 rows an expert, 397 -> 369. Bound by the hand-over of the two K stages of the ring (activation rows and A
+// 462 -> 444; 777 tokens, 49 rows an expert, 397 -> 369. Bound by the hand-over of the K stages of the rings (activation rows and A
 // slots come back, are refilled over L2 and by the decode warps, 1100 cycles a stage at the least) and, with full tiles, by the MMAs
-// and the power limit; the tensor core also stands still while an accumulator of more than 128 columns is drained. Between 64
-// and 96 rows an expert, evenly spread (1100 tokens: 440 -> 449), it is up to 2 % behind, on uneven loads of that size ahead (463 -> 453).
+// and the power limit; the tensor core also stands still while an accumulator of more than 128 columns is drained.
+// Two K stages of token rows are in flight with tiles of more than 128 rows; narrower ones, which fill half of a place, have four
+// (pair_b_waits_for). With two for all, the loads of 64 to 96 rows an expert, evenly spread, were up to 4 % behind the kernel replaced:
+// whole steps at H4096 I1536 E128 with that kernel / two stages / four, 64 rows 468 / 476 / 458 us, 80 rows 552 / 560 / 541, 96
+// rows 565 / 586 / 570; 32 of 256 experts at H7168 I2048, 80 rows 305 / 313 / 300, 128 rows 387 / 374 / 364.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -104,8 +107,8 @@ struct alignas(16) PairUnit {              // written and read 16 bytes at a tim
 
 struct PairCtrl {
   uint64_t raw_full[PairCfg::NST], raw_empty[PairCfg::NST];  // weight stages (local)
-  uint64_t full[PairCfg::NSLOT / 2];     // CTA 0: A and B of two slots (a K stage), from both CTAs
-  uint64_t empty[PairCfg::NSLOT];        // committed into both CTAs
+  uint64_t full[PAIR_MARKS / 2];         // CTA 0: A and B of two slots (a K stage), from both CTAs
+  uint64_t empty[PAIR_MARKS];            // the MMAs of a slot are done, committed into both CTAs
   uint64_t d_full[2];                    // committed into both CTAs
   uint64_t d_empty[2];                   // CTA 0: drained by both CTAs
   uint64_t u_full[PAIR_UNITS];           // local
@@ -251,9 +254,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       mbar_init(&ctl.raw_full[i], 1);
       mbar_init(&ctl.raw_empty[i], 8);             // two decode groups read a stage
     }
-    for (int i = 0; i < NSLOT; ++i) {
+    for (int i = 0; i < PAIR_MARKS; ++i) {
       mbar_init(&ctl.empty[i], 1);
-      if (i < NSLOT / 2) mbar_init(&ctl.full[i], 1 + 16);   // CTA 0's activation warp (with the bytes of both), eight decode warps of either CTA
+      if (i < PAIR_MARKS / 2) mbar_init(&ctl.full[i], 1 + 16);   // CTA 0's activation warp (with the bytes of both), eight decode warps of either CTA
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&ctl.d_full[i], 1);
@@ -327,8 +330,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     if (rank == 0) {
       const uint64_t b_desc0 = smem_desc_kmajor_sw128(smem_u32(b_ring));   // slots and K steps advance its address field
       PairBuffers db;
-      uint32_t sl = 0, spar = 0;
-      bool ready = false;                          // the stage at sl was seen full while the one before was issued
+      uint32_t st = 0;                             // K stage, through all units
+      bool ready = false;                          // stage st was seen full while the one before was issued
       bool ok = true;
       PairUnit u;
       while (ok && wait_unit(u, mbar_wait_warp)) {
@@ -341,14 +344,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         if (db.uses(1) && !mbar_wait_warp(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) { ok = false; break; }
         const uint32_t d_tmem = tmem + db.buf * static_cast<uint32_t>(BH);
         tc_fence_after();
+        const uint64_t sub = static_cast<uint64_t>(db.wide ? C::B_SUB_BYTES : C::B_SUB_BYTES / 2) >> 4;
         for (int k = 0; k < p.K[u.phase]; k += KS) {
-          if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.full[sl >> 1], spar, abortw)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.full[st & 3u], (st >> 2) & 1u, abortw)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sn = sl + 2 == NSLOT ? 0u : sl + 2, pn = sn == 0u ? spar ^ 1u : spar;
-          ready = mma_stage_pair<C::B_SUB_BYTES>(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + sl * (C::B_SLOT_BYTES >> 4), idesc,
-                                                 k > 0 ? 1u : 0u, smem_u32(&ctl.empty[sl]), smem_u32(&ctl.full[sn >> 1]), pn);
-          sl = sn;
-          spar = pn;
+          const uint32_t sn = st + 1u, sl = (st & 1u) * 2u;
+          const uint32_t place = sl * C::B_SLOT_BYTES + (db.wide ? 0u : ((st >> 1) & 1u) * (C::B_SLOT_BYTES / 2));
+          ready = mma_stage_pair(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + (place >> 4), idesc, k > 0 ? 1u : 0u,
+                                 smem_u32(&ctl.empty[(st & 3u) * 2u]), smem_u32(&ctl.full[sn & 3u]), (sn >> 2) & 1u, sub,
+                                 (C::B_SLOT_BYTES >> 4) - sub);
+          st = sn;
         }
         if (ok && elect_one()) {
           if (db.uses(0)) tc_commit_pair(&ctl.d_full[0]);
@@ -361,7 +366,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     // ---------------------------------------------------------- activations
     // (the whole warp walks the loop, one elected lane issues: addresses and coordinates stay in uniform registers)
     const uint64_t keep = policy_evict_last();     // token rows are re-read by every pair of the expert
-    uint32_t sl = 0, spar = 0;
+    uint32_t n = 0, wide_end = 0;                  // slot, through all units; the one behind the last wide tile's
     bool ok = true;
     int last_tile = -1;
     PairUnit u;
@@ -392,26 +397,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
       }
       for (int k = 0; k < K; k += KS) {
         // half a stage at a time, as its slots come back: the MMAs wait for these rows more than for the weights
-        const uint32_t bar = lead_bar(&ctl.full[sl >> 1]);
+        const uint32_t bar = lead_bar(&ctl.full[(n >> 1) & 3u]);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (!mbar_wait_warp(&ctl.empty[sl + h], spar ^ 1u, abortw)) { ok = false; break; }
+        for (int h = 0; h < 2; ++h, ++n) {
+          const uint32_t before = pair_b_waits_for(n, u.nmma, wide_end);   // (of the first slots: a barrier that nothing has completed, parity 1)
+          if (!mbar_wait_warp(&ctl.empty[before & 7u], (before >> 3) & 1u, abortw)) { ok = false; break; }
           if (elect_one()) {
-            if (h == 0 && rank == 0) mbar_arrive_expect_tx(&ctl.full[sl >> 1], bytes);
-            uint8_t* dst = b_ring + (sl + h) * C::B_SLOT_BYTES;
+            if (h == 0 && rank == 0) mbar_arrive_expect_tx(&ctl.full[(n >> 1) & 3u], bytes);
+            uint8_t* dst = b_ring + (n & 3u) * C::B_SLOT_BYTES + (half > BH / 2 ? 0u : ((n >> 2) & 1u) * (C::B_SLOT_BYTES / 2));
             tma_load_2d_pair(dst, map, k + h * 128, row, bar, keep);
-            tma_load_2d_pair(dst + C::B_SUB_BYTES, map, k + h * 128 + 64, row, bar, keep);
+            tma_load_2d_pair(dst + (half > BH / 2 ? C::B_SUB_BYTES : C::B_SUB_BYTES / 2), map, k + h * 128 + 64, row, bar, keep);
           }
           __syncwarp();
         }
         if (!ok) break;
-        if ((sl += 2) == NSLOT) { sl = 0; spar ^= 1u; }
       }
+      if (half > BH / 2) wide_end = n;
     }
     // the commits of the last slots arrive in this CTA's shared memory: it stays until they have
-    for (int i = 0; ok && i < NSLOT; ++i) {
-      if (!mbar_wait_warp(&ctl.empty[sl], spar ^ 1u, abortw)) break;
-      if (++sl == NSLOT) { sl = 0; spar ^= 1u; }
+    for (int i = 0; ok && i < PAIR_MARKS; ++i) {
+      --n;
+      if (!mbar_wait_warp(&ctl.empty[n & 7u], (n >> 3) & 1u, abortw)) break;
     }
   } else if (warp == 3) {
     // ------------------------------------------- scheduler; announces stored gate/up units
@@ -511,11 +517,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     // lane -> row of the stage: octet 2q + (lane >> 3 & 1) of this CTA's eight, tile lane >> 4 of the pair
     const uint32_t row_off = static_cast<uint32_t>((2 * (2 * q + ((lane >> 3) & 1)) + (lane >> 4)) * OCT_BYTES + (lane & 7) * 16);
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t a_ring = tmem + lane_base + C::A_BASE;
+    const uint32_t a_tmem = tmem + lane_base + C::A_BASE + static_cast<uint32_t>(g * PAIR_SLOT_COLS);
     const uint32_t full_bar = lead_bar(&ctl.full[0]);
-    uint32_t as = static_cast<uint32_t>(g);        // A slot of this group's next turn
+    uint32_t turn = 0;                             // slots this group has filled: always A slot g
     uint32_t ws = static_cast<uint32_t>(g >> 1), wpar = 0;   // stage of this group's next slot
-    uint32_t spar = 0;
     uint32_t sc = 0;                               // slots of the units before
     PairBuffers db;
     bool ok = true, owe = false;
@@ -579,9 +584,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
 #pragma unroll
             for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(o[c][j]));   // here, not behind the wait
           }
-          if (!mbar_wait_warp(&ctl.empty[as], spar ^ 1u, abortw)) { ok = false; break; }
+          // the slot this group filled last, NSLOT before this one
+          if (!mbar_wait_warp(&ctl.empty[g + ((turn & 1u) ? 0 : NSLOT)], ((turn - 1u) >> 1) & 1u, abortw)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_tmem = a_ring + as * PAIR_SLOT_COLS;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             if (c >= 2) decode(c, o[c & 1]);
@@ -591,11 +596,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
-            mbar_arrive_cluster(full_bar + (as >> 1) * 8u);
+            mbar_arrive_cluster(full_bar + (static_cast<uint32_t>(g >> 1) + (turn & 1u) * 2u) * 8u);
             mbar_arrive(&ctl.raw_empty[ws]);
           }
-          as += PAIR_GROUPS;
-          if (as >= NSLOT) { as -= NSLOT; spar ^= 1u; }
+          ++turn;
           ws += 2;
           if (ws >= NST) { ws -= NST; wpar ^= 1u; }
           s += PAIR_GROUPS;

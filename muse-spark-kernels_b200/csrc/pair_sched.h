@@ -13,7 +13,8 @@ namespace msk {
 
 constexpr int PAIR_BH = 128;             // most token rows a CTA holds of a tile; columns of an accumulator buffer
 constexpr int PAIR_SLOT_K = 128;         // K of an A / B slot
-constexpr int PAIR_NSLOT = 4;            // A / B slots
+constexpr int PAIR_NSLOT = 4;            // A slots; B slots of PAIR_BH rows
+constexpr int PAIR_MARKS = 2 * PAIR_NSLOT;   // slots whose MMAs have their own barrier; B slots of PAIR_BH / 2 rows
 constexpr int PAIR_GROUPS = 4;           // of decode warps: group g fills the slots g, g + PAIR_GROUPS, ... of the list of all slots
 constexpr int PAIR_NST = 5;              // weight stages
 constexpr int PAIR_UNITS = 4;            // units handed out ahead of their use
@@ -21,6 +22,13 @@ constexpr int PAIR_UNITS = 4;            // units handed out ahead of their use
 // Rows of each tile of an expert with c rows in n tiles: even shares, in steps of 32 (the last tile has the rest, which
 // is never empty: a share is below its limit only while the limit exceeds c / n by more than the rounding).
 MSK_HOST_DEVICE inline int pair_tile_rows(int c, int n) { return ((c + n - 1) / n + 31) & ~31; }
+
+// The slot whose MMAs have to be done before token rows are copied into slot n: the last one that used any of its bytes. A
+// tile of up to PAIR_BH rows (half of them in either CTA) fills half a place of the ring and alternates between the halves, so that its
+// rows are fetched twice as many slots ahead; `wide_end`: the number behind the last slot of a wider tile.
+MSK_HOST_DEVICE inline unsigned pair_b_waits_for(unsigned n, int cols, unsigned wide_end) {
+  return cols <= PAIR_BH && n >= wide_end + PAIR_NSLOT ? n - PAIR_MARKS : n - PAIR_NSLOT;
+}
 
 // Slots of its next unit that a decode warp fills before it drains the unit it owes (phase 0 gate/up, 1 down; cols: columns
 // of the accumulators). A group's next slot is free once the MMAs have read the slot it filled before, so the first slot of a

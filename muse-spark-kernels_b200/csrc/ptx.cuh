@@ -380,10 +380,10 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
 // D[256 rows over both CTAs' TMEM, N] (+)= A[256 rows, 256] (128 rows in either TMEM) * B[N, 256] (N / 2 rows in either CTA): the
 // sixteen MMAs of a K stage (two slots) by one elected lane, and the commits that hand its slots back in both CTAs (empty_bar and
 // the barrier behind it). The answer of a probe of `next_full` (true: complete) is asked for before the MMAs and read behind them, so
-// that its latency hides behind the issue. b_desc: the first of four sub-tiles of 64 K, SUB_BYTES apart.
-template <int SUB_BYTES>
+// that its latency hides behind the issue. b_desc: the first of four sub-tiles of 64 K; the second one of a slot lies `sub` behind the
+// first, the next slot's first `gap` behind that (in units of 16 bytes).
 __device__ __forceinline__ bool mma_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
-                                               uint32_t empty_bar, uint32_t next_full, uint32_t parity) {
+                                               uint32_t empty_bar, uint32_t next_full, uint32_t parity, uint64_t sub, uint64_t gap) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred q, e, acc, t;\n\t.reg .b64 b, d;\n\t.reg .b32 a;\n\t"
@@ -406,7 +406,7 @@ __device__ __forceinline__ bool mma_stage_pair(uint32_t d_tmem, uint32_t a_tmem,
       "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
       "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
       "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], %10;\n\t"
-      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
+      "add.s64 b, b, %11;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
       "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
       "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
       "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
@@ -427,7 +427,7 @@ __device__ __forceinline__ bool mma_stage_pair(uint32_t d_tmem, uint32_t a_tmem,
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(ok)
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_full), "r"(parity),
-        "n"(SUB_BYTES >> 4), "h"(static_cast<uint16_t>(3))
+        "l"(sub), "h"(static_cast<uint16_t>(3)), "l"(gap)
       : "memory");
   return ok != 0;
 }

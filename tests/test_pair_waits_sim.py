@@ -16,7 +16,7 @@ import subprocess
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "muse-spark-kernels_b200", "csrc")
-NAMES = ("PAIR_BH", "PAIR_SLOT_K", "PAIR_NSLOT", "PAIR_GROUPS", "PAIR_NST", "PAIR_UNITS")
+NAMES = ("PAIR_BH", "PAIR_SLOT_K", "PAIR_NSLOT", "PAIR_GROUPS", "PAIR_NST", "PAIR_UNITS", "PAIR_MARKS")
 
 
 @pytest.fixture(scope="module")
@@ -25,6 +25,7 @@ def sched(tmp_path_factory):
     src, so = d / "shim.cpp", d / "shim.so"
     src.write_text('#include "pair_sched.h"\nextern "C" {\n'
                    "int tile_rows(int c, int n) { return msk::pair_tile_rows(c, n); }\n"
+                   "int b_waits_for(int n, int c, int w) { return (int)msk::pair_b_waits_for(n, c, w); }\n"
                    "int before_drain(int a, int b, int c, int d) { return msk::pair_slots_before_drain(a, b, c, d); }\n"
                    + "".join(f"int c_{n}() {{ return msk::{n}; }}\n" for n in NAMES) + "}\n")
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", str(so), str(src)], check=True)
@@ -34,14 +35,15 @@ def sched(tmp_path_factory):
 class Cluster:
     """One cluster; unit: (phase, tile, columns, slots). Slots are numbered through all units."""
 
-    def __init__(self, c, deal, before_drain):
-        self.c, self.deal, self.before_drain = c, deal, before_drain
+    def __init__(self, c, deal, before_drain, b_waits_for):
+        self.c, self.deal, self.before_drain, self.b_waits_for = c, deal, before_drain, b_waits_for
         self.units = []                 # as handed out, the end marker last
         self.first = []                 # number of each unit's first slot
         self.slots = 0                  # slots of the units handed out
         self.announced = 0              # units whose stores were announced (or need not be)
         self.done = False
-        self.act_unit = self.act_slots = 0              # activations: unit walked, slots filled
+        self.act_unit = self.act_slots = 0              # activations: unit walked, slots filled,
+        self.wide_end = 0                               # number behind the last slot of a wide tile
         self.raw_unit = self.raw_stages = 0             # weights: unit walked, stages issued
         self.mma_unit = self.mma_slots = 0              # MMAs: unit walked, slots read and handed back
         G = c["PAIR_GROUPS"]
@@ -99,14 +101,16 @@ class Cluster:
     def activate(self):
         if self.act_unit >= len(self.units) or self.units[self.act_unit] is None:
             return False
-        phase, tile, _, nsl = self.units[self.act_unit]
+        phase, tile, cols, nsl = self.units[self.act_unit]
         if phase == 1 and self.act_slots == self.first[self.act_unit] and not self.deal.complete(tile):
             return False
-        if self.act_slots - self.c["PAIR_NSLOT"] >= self.mma_slots:
+        if self.b_waits_for(self.act_slots, cols, self.wide_end) >= self.mma_slots:
             return False
         self.act_slots += 1
         if self.act_slots == self.first[self.act_unit] + nsl:
             self.act_unit += 1
+            if cols > self.c["PAIR_BH"]:
+                self.wide_end = self.act_slots
         return True
 
     def mma(self):
@@ -197,12 +201,12 @@ class Deal:
         return self.stored[tile] == self.n_pairs[0]
 
 
-def ends(c, before_drain, tiles, H, inter, clusters, seed):
+def ends(c, before_drain, b_waits_for, tiles, H, inter, clusters, seed):
     """True when every cluster reaches the end of the list. seed 0: all clusters at one speed, drawing in turn; others: each
     at a speed of its own, some starting late."""
     rng = random.Random(seed)
     deal = Deal(c, tiles, H, inter)
-    cl = [Cluster(c, deal, before_drain) for _ in range(clusters)]
+    cl = [Cluster(c, deal, before_drain, b_waits_for) for _ in range(clusters)]
     speed = [2 if seed == 0 else rng.choice((1, 2, 4, 8)) for _ in cl]
     draws = [1 if seed == 0 else rng.choice((1, 1, 2, 4)) for _ in cl]
     late = [0 if seed == 0 else rng.choice((0, 0, 1, 5, 40)) for _ in cl]
@@ -243,7 +247,7 @@ def test_every_cluster_reaches_the_end(sched, H, inter, clusters):
     for n in counts:
         for kind in ("narrow", "wide", "mixed"):
             for seed in range(1 if n > 8 else 3):
-                assert ends(c, sched.before_drain, _tiles(kind, n, n + seed), H, inter, clusters, seed), (n, kind, seed)
+                assert ends(c, sched.before_drain, sched.b_waits_for, _tiles(kind, n, n + seed), H, inter, clusters, seed), (n, kind, seed)
 
 
 @pytest.mark.parametrize("H,inter,clusters,tiles,seeds", [(4096, 1536, 74, 4, 1), (4096, 1536, 74, 5, 1), (4096, 1536, 74, 6, 1),
@@ -252,7 +256,31 @@ def test_every_cluster_reaches_the_end(sched, H, inter, clusters):
 def test_the_model_sees_a_drain_behind_the_down_units_mmas(sched, H, inter, clusters, tiles, seeds):
     """Not vacuous: with the drain always behind the second slot of narrow tiles the same loads stand still."""
     c = _constants(sched)
-    assert not all(ends(c, old_rule(c), [64] * tiles, H, inter, clusters, seed) for seed in range(seeds))
+    assert not all(ends(c, old_rule(c), sched.b_waits_for, [64] * tiles, H, inter, clusters, seed) for seed in range(seeds))
+
+
+def test_token_rows_overwrite_only_what_the_mmas_have_read(sched):
+    """The ring of token rows, byte by byte: a slot of a wide tile takes a whole place, one of a narrow tile the half that the place's
+    slot before did not take (the addresses of the activation warp). Every slot that last used a byte is, by number, at or before
+    the one the copy waits for; MMAs are done in order."""
+    c = _constants(sched)
+    N = c["PAIR_NSLOT"]
+    for seed in range(40):
+        rng = random.Random(seed)
+        user = [[-1, -1] for _ in range(N)]
+        n = wide_end = 0
+        for _ in range(60):
+            wide = rng.random() < (0.5, 0.1, 0.9)[seed % 3]
+            for _ in range(2 * rng.choice((1, 1, 2, 3, 5, 8))):
+                halves = (0, 1) if wide else ((n // N) % 2,)
+                waits = sched.b_waits_for(n, 2 * c["PAIR_BH"] if wide else c["PAIR_BH"], wide_end)
+                assert max(user[n % N][h] for h in halves) <= max(waits, -1) and waits < n
+                assert waits >= n - c["PAIR_MARKS"]      # the barrier of that slot has not come round again
+                for h in halves:
+                    user[n % N][h] = n
+                n += 1
+            if wide:
+                wide_end = n
 
 
 def test_tile_rows_share_an_expert_evenly(sched):
