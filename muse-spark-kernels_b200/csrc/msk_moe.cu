@@ -642,7 +642,10 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     const double rpe = static_cast<double>(T) * c->top_k / c->n_experts;  // mean tokens per expert
     // measured at H4096 I1536 E128 (us a step with 16 / 64-token tiles, near-even routing): T = 160 (rpe 10): 268 / 281;
     // T = 192 (rpe 12): 313 / 302. 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
-    // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. The 16-token tile is the
+    // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. Beyond: rpe 48 near-even
+    // 406 / 464, 32 of 256 experts at H4096 I4096 255 / 289, a few experts taking most 456 / 420, the same at H2048 I1024 E64
+    // 107 / 88; rpe 56 445 / 477, 279 / 295, 508 / 452, 114 / 95; rpe 64 near-even 566 / 505. At rpe 40 the 64-token tile loses 13 %
+    // at worst and the pair kernel 18, at 48 it is 21 and 20. The 16-token tile is the
     // fastest per K stage and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The
     // host does not know the counts, and the less even they are the lower that line lies. The 32-token tile never wins at
     // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh)
