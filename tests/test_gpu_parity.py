@@ -442,12 +442,13 @@ def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
         _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
-@pytest.mark.parametrize("H,I,ctas,post,inf", [(256, 256, 0, False, False), (512, 768, 2, True, False), (768, 256, 37, False, True),
-                                               (1024, 512, 296, True, False), (512, 256, 1, False, False)])
-def test_pair_kernel_at_tile_edges(cuda_dev, H, I, ctas, post, inf):
+@pytest.mark.parametrize("H,I,ctas,post,nan", [(256, 256, 0, False, False), (512, 768, 2, True, False), (768, 256, 37, False, True),
+                                               (1024, 512, 296, True, False), (512, 256, 1, False, False),
+                                               (1536, 1280, 4, False, False)])
+def test_pair_kernel_at_tile_edges(cuda_dev, H, I, ctas, post, nan):
     """The kernel on pairs of SMs around its tile heights (up to 256 rows an expert a tile, even shares of 32 beyond, one or both
     accumulator buffers), at its shortest reductions, with an odd grid, one pair and more CTAs than SMs; both GEMMs in one launch
-    and in two give the same bits, twice on one state. A token whose values overflow leaves the rows of the others alone."""
+    and in two give the same bits, twice on one state. A token of NaN leaves the rows of the others alone."""
     m, inputs, _lib, orc = _mods()
     counts = [1, 31, 32, 33, 64, 127, 128, 129, 160, 255, 256, 257, 300, 511, 513, 600]
     T, E = 600, len(counts)
@@ -468,7 +469,7 @@ def test_pair_kernel_at_tile_edges(cuda_dev, H, I, ctas, post, inf):
         _check_forward(out, ref, parts, m.workspace_views(st, T))
         assert torch.equal(m.kernel_fn(data, two), out)
         assert m.read_status(two) == 0
-    if inf:
+    if nan:
         bad = dict(data, hidden_states=x.clone())
         bad["hidden_states"][5] = float("nan")
         got = m.kernel_fn(bad, st)
