@@ -39,8 +39,8 @@
 // and the power limit; the tensor core also stands still while an accumulator of more than 128 columns is drained.
 // Two K stages of token rows are in flight with tiles of more than 128 rows; narrower ones, which fill half of a place, have four
 // (pair_b_waits_for). With two for all, the loads of 64 to 96 rows an expert, evenly spread, were up to 4 % behind the kernel replaced:
-// whole steps at H4096 I1536 E128 with that kernel / two stages / four, 64 rows 468 / 476 / 458 us, 80 rows 552 / 560 / 541, 96
-// rows 565 / 586 / 570; 32 of 256 experts at H7168 I2048, 80 rows 305 / 313 / 300, 128 rows 387 / 374 / 364.
+// whole steps at H4096 I1536 E128 with that kernel / two stages / four, 64 rows 468 / 471 / 458 us, 80 rows 552 / 560 / 541, 96
+// rows 565 / 586 / 572; 32 of 256 experts at H7168 I2048, 80 rows 305 / 313 / 300, 128 rows 387 / 374 / 364.
 #pragma once
 #include <cstddef>
 #include <cstdint>
