@@ -348,7 +348,11 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     mean_touched = sum(touched[i % POOL] for i in range(n_prof)) / n_prof
     R = T * k
     plan = moe.plan(state, T)
-    one_launch = plan[1] == 0 and T <= 32 and R <= 256
+    few, nvf4 = ctypes.c_int(0), ctypes.c_int(0)
+    state["lib"].lib.msk_moe_few_fits(ctypes.byref(state["cfg"]), T, 1, ctypes.byref(few))   # (timed with given ids)
+    state["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(state["cfg"]), T, ctypes.byref(nvf4))
+    nvf4 = bool(nvf4.value) and not few.value
+    one_launch = plan[1] == 0 and T <= 32 and R <= 256 and not nvf4
     # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine
     both_gemms = plan[1] == 4 or (plan[0] == 64 and not plan[2] and state["cfg"].decode_path != 1)
     pair = plan[0] == 128 and state["cfg"].decode_path != 1     # both GEMMs in one launch on pairs of SMs
@@ -357,14 +361,20 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     if one_launch:
         alg = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(n_prof)) / n_prof
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
-        few = ctypes.c_int(0)
-        state["lib"].lib.msk_moe_few_fits(ctypes.byref(state["cfg"]), T, 1, ctypes.byref(few))   # (timed with given ids)
         ratio = NCU_TRAFFIC_RATIO["moe_few_kernel" if few.value else "moe_gemm_kernel<N,2> T8"]
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": alg * ratio,
                 "traffic_source": "ncu dram bytes of the kernel's 32-expert capture / its algorithmic bytes (%.2f), scaled" % ratio,
                 "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if few.value else "moe_gemm_kernel<N,2>"),
                 "peak_source": peaks["source"] + " (burst copy)"}
+    elif nvf4:
+        # both GEMMs in one launch: the touched experts' tiles, x read, its digits written and read (25/8 bytes a value), inter written, read
+        # and its digits written and read, y written
+        alg = mean_touched * (3 * I * H * 0.5625 + 8) + 2.0 * T * H + 6.25 * R * (H + I) + 4.0 * R * I + 4.0 * R * H
+        achieved = alg / (k_ms[2] * 1e-3) / 1e9
+        roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                "frac": achieved / peaks["hbm_gbs"], "traffic": None,
+                "kernel": "moe_nvf4_kernel (gate/up and down GEMM in one launch)", "peak_source": peaks["source"] + " (burst copy)"}
     elif both_gemms:
         # both GEMMs in one launch: the touched experts' tiles of both, x read and converted (64-token tile: the sorted
         # rows read), inter written and read back, y written
@@ -405,6 +415,8 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
         launches = 1
     elif plan[1] == 2 and T <= 32 and R <= 256:
         launches = 3      # row copy, gate/up kernel (routes, sorts), down kernel (combines)
+    elif nvf4:            # top-k and sort (one launch up to 32 tokens, two beyond), both GEMMs, combine
+        launches = 3 if T <= 32 else 4
     elif both_gemms:      # top-k and sort (one launch up to 32 tokens, two beyond), [row copy,] both GEMMs, combine
         launches = (3 if T <= 32 else 4) + (1 if plan[0] == 64 else 0)
     else:                 # top-k and sort, row copy (in the sort launch up to 32 tokens), GEMMs (two, 128-token plans one), combine

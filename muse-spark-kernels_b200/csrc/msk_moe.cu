@@ -15,6 +15,7 @@
 #include "gemm.cuh"
 #include "few.cuh"
 #include "pair.cuh"
+#include "nvf4.cuh"
 #include "router_gemm.cuh"
 
 namespace msk {
@@ -692,9 +693,33 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   return p;
 }
 
+// The kernel on the FP4 tensor cores (nvf4.cuh). Its lines, whole steps in us by this kernel / the other one, in turn on one box. It takes the
+// sort and combine launches that the few-token paths fold into theirs: at H4096 I1536 E128 top-8 4 tokens 65 / 65, 5: 76 / 76, 6: 82 /
+// 86, 8: 97 / 102; a rank with one row a token (32 of 256, H4096 I4096, two experts taking most) 4: 50 / 51. Beyond, near-even
+// routes: 24: 172 / 199, 64: 222 / 263, 160: 258 / 296, 192 (12 rows an expert) 275 / 318; a few experts taking most 24: 80 / 83, 64:
+// 108 / 133, 192: 207 / 278; the rank 24: 79 / 79, 160: 161 / 199, 384: 234 / 315; H7168 I2048, even, 64: 117 / 125, 384: 156 / 192. From
+// there on the other one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one
+// for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238. A small model (H2048
+// I1024 E64 top-4), whose down units are four K stages long and wait for their epilogues: 8: 46 / 41, 24: 52 / 52 (Zipf routes
+// 41 / 36), 64: 60 / 61 (50 / 44).
+constexpr int NV_MIN_TOKENS = 6;
+constexpr int NV_MAX_MEAN_ROWS = 12;
+constexpr int NV_MIN_INTER = 1536;
+
+static int nv_max_tokens(const MskMoeCfg* c, int T) {   // of the steps of up to T tokens that may take it
+  if (c->inter < NV_MIN_INTER || c->hidden > NV_MAX_BLOCKS * 16) return 0;
+  return static_cast<int>(std::min(static_cast<long long>(T), static_cast<long long>(NV_MAX_MEAN_ROWS) * c->n_experts / c->top_k));
+}
+
+// Whether a step runs in it. A form that the configuration asks for is always the asked one.
+static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p) {
+  return c->token_tile == 0 && c->decode_path == 0 && c->flat_shares == 0 && c->stop_after == 0 && p.grid <= sm_count() &&
+         T >= NV_MIN_TOKENS && T <= nv_max_tokens(c, T);
+}
+
 // Workspace carving. Everything is sized for max_tokens with the worst plan.
 struct Carve {
-  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, total;
+  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, nv_tiles, nv_img[2], nv_rs[2], nv_max, total;
 };
 constexpr size_t TRACE_CTAS = 256;
 constexpr size_t TRACE_WORDS = TRACE_CTAS * 16 + 3 * 256;
@@ -733,11 +758,22 @@ static Carve carve(const MskMoeCfg* c, int T) {
   // tile hand-over between the gate/up and the down launch: per token tile the finished gate/up units and
   // the down units that have seen them all (two counters per tile, zero between steps)
   k.tile_ctr = o; o += round_up(2 * max_tiles(c, T) * 4, 256);
+  // the FP4 kernel, for the most tokens it takes: counters of its tiles (no more than it has groups of eight rows); its rows further down
+  const size_t nv_rows = static_cast<size_t>(nv_max_tokens(c, T)) * c->top_k;
+  const size_t nv_groups = nv_groups_bound(nv_rows, static_cast<size_t>(c->local_count));
+  k.nv_tiles = o; o += round_up(nv_groups * NV_TILE_WORDS * 4, 256);
   // everything above is control state: msk_moe_workspace_init zeroes [0, inter)
   k.inter = o; o += round_up(R * c->inter * 2, 256);
   k.y = o; o += round_up(R * c->hidden * 4, 256);
   k.partial = o; o += 2 * round_up(partial_floats(c) * 4, 256);  // one region per GEMM
   k.xs = o; o += round_up(R * c->hidden * 2, 256);  // F16 copy of the token rows ([T, H], or sorted [R, H] for wide token tiles)
+  // the FP4 kernel's split rows
+  const int nv_k[2] = {c->hidden, c->inter};
+  for (int i = 0; i < 2; ++i) {
+    k.nv_img[i] = o; o += round_up(nv_groups * (nv_k[i] / KS) * NV_GROUP_BYTES, 256);
+    k.nv_rs[i] = o; o += round_up(nv_rows * 4, 256);
+  }
+  k.nv_max = o; o += round_up(nv_rows * (c->inter / 32) * 2, 256);
   k.total = o;
   return k;
 }
@@ -859,6 +895,30 @@ static int launch_pair(PairParams& p, const __half* xs, size_t rows, int grid, c
   lc.attrs = at;
   lc.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&lc, moe_pair_kernel, p));
+}
+
+static int launch_nvf4(const NvParams& p, int grid, cudaStream_t st, int pdl) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(moe_nvf4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NvCfg::SMEM_BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    attr_set[dev] = true;
+  }
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(static_cast<unsigned>(grid));
+  lc.blockDim = dim3(NV_THREADS);
+  lc.dynamicSmemBytes = NvCfg::SMEM_BYTES;
+  lc.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeCooperative;   // its CTAs wait for one another: all resident, or the launch fails
+  at[0].val.cooperative = fused_plain_launch() ? 0 : 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = pdl;
+  lc.attrs = at;
+  lc.numAttrs = 2;
+  return static_cast<int>(cudaLaunchKernelEx(&lc, moe_nvf4_kernel, p));
 }
 
 // ---- the few-token kernel (few.cuh): shapes it takes, its shared memory and its dealing of work
@@ -1403,7 +1463,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
 
-  if (plan.path != 1 && plan.path != 4) {
+  const bool nv = nv_takes(cfg, n_tokens, plan);
+  if (!nv && plan.path != 1 && plan.path != 4) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
     p.route = logits != nullptr ? 1 : 2;
     p.logits = logits; p.bias = bias; p.ids_in = topk_ids; p.ids_out = ids_out; p.tw_out = tw_out;
@@ -1464,9 +1525,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (ev) cudaEventRecord(ev[0], st);
   int e = 0;
   // narrow token tiles read an F16 copy of x; for few tokens the sorting CTA makes it
-  const bool tma_b = plan.N >= 64;  // GemmCfg<N>::TMA_B
-  const bool both_gemms = plan.both && (tma_b || pre_norm_w == nullptr);   // narrow tiles: the pre-expert norm needs the row-copy kernel
-  const bool convert_in_sort = !tma_b && !both_gemms && n_tokens <= FUSED_ROUTE_MAX_TOKENS;
+  const bool tma_b = !nv && plan.N >= 64;  // GemmCfg<N>::TMA_B
+  const bool both_gemms = !nv && plan.both && (tma_b || pre_norm_w == nullptr);   // narrow tiles: the pre-expert norm needs the row-copy kernel
+  const bool convert_in_sort = !nv && !tma_b && !both_gemms && n_tokens <= FUSED_ROUTE_MAX_TOKENS;
   const __nv_bfloat16* xin = convert_in_sort ? static_cast<const __nv_bfloat16*>(x) : nullptr;
   __half* xh_in_sort = convert_in_sort ? xs : nullptr;
   if (logits != nullptr && n_tokens <= FUSED_ROUTE_MAX_TOKENS) {
@@ -1488,7 +1549,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (ev) cudaEventRecord(ev[1], st);
   if (cfg->stop_after == 1) return MSK_OK;
 
-  if (!convert_in_sort && (tma_b || !both_gemms)) {
+  if (!nv && !convert_in_sort && (tma_b || !both_gemms)) {
     // F16 copy of the token rows: sorted (expert-major) for the TMA tiles, plain [T, H] otherwise
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
@@ -1514,7 +1575,26 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     }
   }
   if (ev) cudaEventRecord(ev[5], st);
-  if (plan.N == 128) {
+  if (nv) {
+    NvParams q{};
+    q.w[0] = g13.w; q.w[1] = g2.w; q.gs[0] = gs13; q.gs[1] = gs2;
+    q.x = static_cast<const __nv_bfloat16*>(x);
+    q.pre_w = static_cast<const __nv_bfloat16*>(pre_norm_w); q.pre_eps = pre_norm_eps;
+    q.ids = topk_ids; q.inv = inv; q.cnt = cnt; q.off = off; q.post_norm_w = p.post_norm_w;
+    q.inter = inter; q.y = y; q.status = status; q.trace = trace;
+    for (int i = 0; i < 2; ++i) {
+      q.img[i] = b + k.nv_img[i];
+      q.rs[i] = reinterpret_cast<float*>(b + k.nv_rs[i]);
+      q.K[i] = p.ph[i].K; q.n_pairs[i] = p.ph[i].n_pairs;
+    }
+    q.part_max = reinterpret_cast<__half*>(b + k.nv_max);
+    q.ctr = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
+    q.tiles = reinterpret_cast<unsigned int*>(b + k.nv_tiles);
+    q.nloc = cfg->local_count; q.lo = cfg->local_start; q.H = cfg->hidden; q.I = cfg->inter; q.T = n_tokens; q.k = cfg->top_k;
+    e = launch_nvf4(q, plan.grid, st, pdl);
+    if (e != 0) return e;
+    if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); }
+  } else if (plan.N == 128) {
     // tiles of up to 256 rows on pairs of SMs, both GEMMs in one launch unless two are asked for
     PairParams q{};
     q.w[0] = g13.w; q.w[1] = g2.w; q.gs[0] = gs13; q.gs[1] = gs2;
@@ -1575,7 +1655,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   if (cfg->stop_after == 3) return MSK_OK;
   }
 
-  e = launch_combine(cfg, plan.N == 128, y, inv, topk_weights, out, n_tokens, post_norm_w != nullptr, pdl, st);
+  e = launch_combine(cfg, !nv && plan.N == 128, y, inv, topk_weights, out, n_tokens, post_norm_w != nullptr, pdl, st);
   if (ev) cudaEventRecord(ev[4], st);
   return e;
 }
@@ -1818,6 +1898,15 @@ int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_f
   FewPlan f;
   const Plan p = make_plan(cfg, n_tokens);
   *host_fits = p.path == 0 && few_takes(cfg, n_tokens, inputs, p.grid, &f) ? 1 : 0;
+  return MSK_OK;
+}
+
+int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int* host_takes) {
+  const int rc = check_cfg(cfg);
+  if (rc != MSK_OK) return rc;
+  if (!host_takes) return MSK_ERR_NULL;
+  if (n_tokens < 1) return MSK_ERR_SHAPE;
+  *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens)) ? 1 : 0;
   return MSK_OK;
 }
 

@@ -1267,6 +1267,122 @@ def test_prefill_moe_runs_the_prefill_layer_call_site(cuda_dev):
     assert np.array_equal(ex["rrow"].tensor().cpu().numpy().reshape(-1), parts["inv"])
 
 
+def _nvf4_takes(st, T):
+    takes = ctypes.c_int(0)
+    assert st["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(st["cfg"]), T, ctypes.byref(takes)) == 0
+    return takes.value == 1
+
+
+def _ids_of_counts(counts, lo, k, dev):
+    """Global ids [T, k] that give local expert e counts[e] rows (one local route a token, at any slot) and others dropped."""
+    ids = torch.full((sum(counts), k), -1, dtype=torch.int32)
+    rows = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts)).to(torch.int32) + lo
+    g = torch.Generator().manual_seed(sum(counts))
+    ids[torch.arange(len(rows)), torch.randint(0, k, (len(rows),), generator=g)] = rows[torch.randperm(len(rows), generator=g)]
+    return ids.to(dev)
+
+
+@pytest.mark.parametrize("H,I,counts,ctas,pre,post", [
+    (256, 1536, [1, 8, 9, 16, 17, 24], 0, False, False),       # tiles of every width, one K stage: a unit shorter than any ring
+    (768, 1536, [25, 0, 49, 5, 48, 1], 0, True, True),         # two and three tiles an expert, the last ones narrower
+    (2304, 1792, [31, 24, 2, 0, 0, 7], 37, False, True),       # odd numbers of stages, fewer CTAs than rows
+    (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
+    (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
+    (512, 4096, [12], 1, False, True),                         # one CTA waits for nobody but itself
+    (2048, 1536, [130, 0, 160], 0, True, True),                # two rows a CTA: the second one is fetched while the first is split
+])
+def test_nvf4_kernel_at_tile_edges(cuda_dev, H, I, counts, ctas, pre, post):
+    """moe_nvf4_kernel against the oracle where its tiles, rings and dealing can go wrong, twice on one state (bit for bit)."""
+    m, inputs, _lib, orc = _mods()
+    E, k, lo, n = 64, 2, 7, len(counts)
+    w = inputs.make_weights(H, I, n, 61, cuda_dev, post_norm=post)
+    g = torch.Generator(device=cuda_dev).manual_seed(H + I)
+    if pre:
+        w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    T = sum(counts)
+    st = m.prepare(w, local_start=lo, n_experts=E, top_k=k, max_tokens=T, num_ctas=ctas)
+    assert _nvf4_takes(st, T)
+    x = (torch.randn((T, H), generator=g, device=cuda_dev) * 2.0).to(torch.bfloat16)
+    d = {"hidden_states": x, "topk_ids": _ids_of_counts(counts, lo, k, cuda_dev),
+         "topk_weights": torch.rand((T, k), generator=g, device=cuda_dev) + 0.1}
+    out = m.kernel_fn(d, st).clone()
+    views = m.workspace_views(st, T)
+    again = m.kernel_fn(d, st)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0 and torch.equal(again, out)
+    ref, parts = orc.moe_forward(x, d["topk_ids"], d["topk_weights"], w, local_start=lo, return_parts=True)
+    assert parts["cnt"].tolist() == counts
+    _check_forward(out, ref, parts, views)
+
+
+@pytest.mark.parametrize("scale", [1.0, 3.0e-3])
+def test_nvf4_kernel_is_no_further_from_64_bits_than_the_f16_kernel(cuda_dev, scale):
+    """Both GEMMs on their own: inter against 64 bits from the same token rows (its rounding to BF16, 1.6e-3 and 2.8e-3, hides all
+    else), y against 64 bits from each kernel's own inter: seven digits hold an element to 2^-21 of the largest of sixteen, FP32 sums
+    lose what they lose in the F16 kernel."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 4096, 1536, 8, 2, 48
+    w = inputs.make_weights(H, I, E, 17, cuda_dev)
+    g = torch.Generator(device=cuda_dev).manual_seed(5)
+    x = (torch.randn((T, H), generator=g, device=cuda_dev) * scale).to(torch.bfloat16)
+    d = {"hidden_states": x, "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    err = {}
+    for tile in (0, 16):
+        st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+        assert _nvf4_takes(st, T) == (tile == 0)
+        m.kernel_fn(d, st)
+        torch.cuda.synchronize()
+        v = m.workspace_views(st, T)
+        dq13, dq2 = m.dequant_packed(st)
+        off, perm = v["off"].tolist(), v["perm"].long() // k
+        i64, y64 = torch.empty((T * k, I), dtype=torch.float64, device=cuda_dev), torch.empty((T * k, H), dtype=torch.float64, device=cuda_dev)
+        for e in range(E):
+            r = slice(off[e], off[e + 1])
+            gu = x[perm[r]].double() @ dq13[e].double().T * w["w13_gs"][e].double()
+            i64[r] = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+            y64[r] = v["inter"][r].double() @ dq2[e].double().T * w["w2_gs"][e].double()
+        err[tile] = [float((a.double() - b).norm() / b.norm()) for a, b in ((v["inter"], i64), (v["y"], y64))]
+    assert err[0][0] <= err[16][0] * 1.001 and err[0][0] <= 4.0e-3, err
+    assert err[0][1] <= err[16][1] and err[0][1] <= 2.0e-6, err
+    print(err)
+
+
+def test_nvf4_kernel_with_negative_and_nan_scales_and_tokens_out_of_range(cuda_dev):
+    """What the FP4 operands cannot hold as such: scale bytes with the sign bit (the codes take the sign), NaN scales, and tokens
+    with NaN, infinite and huge elements, a zero row and values far below the row's largest. The F16 kernel is the reference: the
+    same NaN places, close elsewhere."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 768, 1536, 8, 2, 40
+    w = inputs.make_weights(H, I, E, 23, cuda_dev)
+    g = torch.Generator(device=cuda_dev).manual_seed(9)
+    for key in ("w13_sf", "w2_sf"):
+        b = w[key].view(torch.uint8)
+        b |= (torch.rand(b.shape, generator=g, device=cuda_dev) < 0.3).to(torch.uint8) << 7
+    w["w2_sf"].view(torch.uint8)[3, 5, 7] = 0x7F
+    w["w2_sf"].view(torch.uint8)[6, 700, 0] = 0xFF
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    x[1] = 0.0
+    x[2, 3] = float("nan")
+    x[3, 100] = float("inf")
+    x[4, 50:60] = -3.0e38
+    x[5, 1:] *= 1.0e-6
+    d = {"hidden_states": x, "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    got = {}
+    for tile in (0, 16):
+        st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+        assert _nvf4_takes(st, T) == (tile == 0)
+        out = m.kernel_fn(d, st).float()
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        got[tile] = (out, m.workspace_views(st, T)["y"])
+    for a, b in zip(got[0], got[16]):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and bool(torch.isnan(a).any())
+    (a, ya), (b, yb) = got[0], got[16]
+    row = lambda v: v.nan_to_num(0.0).norm(dim=1)  # noqa: E731
+    assert bool((row(a - b) <= TOL * row(b)).all())
+    assert float(a[1].nan_to_num(0.0).abs().max()) == 0.0
+
+
 def test_activations_outside_the_f16_range_saturate_as_documented(cuda_dev):
     """The MMA operands are F16: a BF16 activation beyond +-65504 enters the GEMM as +-65504 (and one
     below 2^-24 as zero), and so does a SwiGLU value that large. The result must equal the oracle
