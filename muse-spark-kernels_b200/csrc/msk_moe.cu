@@ -693,16 +693,19 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   return p;
 }
 
-// The kernel on the FP4 tensor cores (nvf4.cuh). Its lines, whole steps in us by this kernel / the other one, in turn on one box. It takes the
-// sort and combine launches that the few-token paths fold into theirs: at H4096 I1536 E128 top-8 4 tokens 65 / 65, 5: 76 / 76, 6: 82 /
-// 86, 8: 97 / 102; a rank with one row a token (32 of 256, H4096 I4096, two experts taking most) 4: 50 / 51. Beyond, near-even
-// routes: 24: 172 / 199, 64: 222 / 263, 160: 258 / 296, 192 (12 rows an expert) 275 / 318; a few experts taking most 24: 80 / 83, 64:
-// 108 / 133, 192: 207 / 278; the rank 24: 79 / 79, 160: 161 / 199, 384: 234 / 315; H7168 I2048, even, 64: 117 / 125, 384: 156 / 192. From
-// there on the other one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one
-// for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238. A small model (H2048
-// I1024 E64 top-4), whose down units are four K stages long and wait for their epilogues: 8: 46 / 41, 24: 52 / 52 (Zipf routes
-// 41 / 36), 64: 60 / 61 (50 / 44).
+// The kernel on the FP4 tensor cores (nvf4.cuh). Its lines, whole steps in us by this kernel / the other one, in turn on one box.
+// All of 128 experts (H4096 I1536 top-8), near-even routes: 4 tokens 65 / 65, 5: 76 / 76, 6: 83 / 86, 8: 96 / 103, 12: 123 / 138, 24:
+// 173 / 208, 64: 221 / 262, 160: 258 / 291, 192 (12 rows an expert) 275 / 318; a few experts taking most tokens 8: 63 / 65, 12: 68 / 65,
+// 16: 74 / 71, 24: 81 / 84, 48: 95 / 114, 192: 207 / 278.
+// A rank with one row a token (32 of 256, H4096 I4096, two experts taking most) 6: 54 / 58, 8: 59 / 66; 12: 63 / 62, 16: 68 / 66
+// (from nine tokens on the other one has its cheaper form as well, and there is little to stream); 24: 78 / 79, 32: 85 / 95, 160: 159 /
+// 198, 384: 234 / 315; H7168 I2048, even, 16: 75 / 75, 64: 115 / 123, 256: 138 / 158, 384: 156 / 192.
+// Beyond 12 rows an expert the other one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of
+// them, this one for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238.
+// A small model (H2048 I1024 E64 top-4), whose down units are four K stages long and wait for their epilogues: 8: 46 / 41, 24: 52 / 52
+// (a few experts taking most 41 / 36), 64: 60 / 61 (50 / 44).
 constexpr int NV_MIN_TOKENS = 6;
+constexpr int NV_MIN_RANK_TOKENS = 24;       // of a rank that holds a part of the experts, beyond the one-launch form's tokens
 constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
 
@@ -714,7 +717,8 @@ static int nv_max_tokens(const MskMoeCfg* c, int T) {   // of the steps of up to
 // Whether a step runs in it. A form that the configuration asks for is always the asked one.
 static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p) {
   return c->token_tile == 0 && c->decode_path == 0 && c->flat_shares == 0 && c->stop_after == 0 && p.grid <= sm_count() &&
-         T >= NV_MIN_TOKENS && T <= nv_max_tokens(c, T);
+         T >= NV_MIN_TOKENS && T <= nv_max_tokens(c, T) &&
+         (c->local_count == c->n_experts || T <= ONE_LAUNCH_MAX_TOKENS || T >= NV_MIN_RANK_TOKENS);
 }
 
 // Workspace carving. Everything is sized for max_tokens with the worst plan.

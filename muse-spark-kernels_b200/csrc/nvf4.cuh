@@ -577,11 +577,17 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         x = n_ctas + static_cast<int>(atomicAdd(p.ctr, 1u));   // the next one: its number is back long before this one's last stage
         const int nst = p.K[u.phase] / KS;
         const uint8_t* src = p.w[u.phase] + static_cast<size_t>(u.expert * p.n_pairs[u.phase] + u.pair) * nst * STAGE_W_BYTES;
-        // while the token rows are split memory would stand still once the ring is full: the next stages go to L2
-        if (i == 0u && nst > NV_W_STAGES) bulk_prefetch_l2(src + NV_W_STAGES * STAGE_W_BYTES, static_cast<uint32_t>(min(nst - NV_W_STAGES, NV_AHEAD) * STAGE_W_BYTES));
         for (int ks = 0; ks < nst; ++ks, ++st) {
           const uint32_t ws = st % NV_W_STAGES;
           const uint32_t before = st - NV_W_STAGES;   // the stage whose place this one takes
+          if (st == NV_W_STAGES && i == 0u) {
+            // While the token rows are split memory would stand still once the ring is full: the next stages go to L2, at the pace of memory
+            // (all at once they held up the reading of the rows, 3 us) and until the first MMAs are done.
+            for (int a = 0; a < min(nst - ks, NV_AHEAD) && !mbar_test(&ctl.done[0], 0u); ++a) {
+              bulk_prefetch_l2(src + a * STAGE_W_BYTES, STAGE_W_BYTES);
+              __nanosleep(700);
+            }
+          }
           if (st >= NV_W_STAGES && !mbar_wait_inline(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
           mbar_arrive_expect_tx(&ctl.w_full[ws], STAGE_W_BYTES);
           bulk_g2s(w_ring + ws * STAGE_W_BYTES, src, STAGE_W_BYTES, &ctl.w_full[ws], pol);

@@ -171,31 +171,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   }
 }
 
-// As mbar_wait_warp, acquiring what threads of the other CTAs of the cluster have released by their arrives.
-__device__ __forceinline__ bool mbar_wait_warp_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
-  auto test = [&]() -> bool {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(4000u)
-        : "memory");
-    return __all_sync(0xffffffffu, ok != 0u);
-  };
-  if (test()) return true;
-  const uint64_t t0 = globaltimer_ns();
-  uint32_t polls = 0;
-  while (true) {
-    if (test()) return true;
-    if ((++polls & 15u) == 0u && __any_sync(0xffffffffu, *abort_word != 0 || globaltimer_ns() - t0 > MSK_WAIT_LIMIT_NS)) {
-      *abort_word = 1;
-      return false;
-    }
-  }
-}
-
 // The same wait for hand-offs that complete within a few hundred cycles (the 128 epilogue threads
 // meeting at their barrier): poll without parking first, so that the wake-up latency of a parked
 // thread is not paid on every meeting; then fall back to the parked wait.
@@ -534,12 +509,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
 }
 
 // ---------------------------------------------------- register-operand MMA
