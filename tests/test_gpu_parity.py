@@ -1288,7 +1288,7 @@ def _ids_of_counts(counts, lo, k, dev):
     (2304, 1792, [31, 24, 2, 0, 0, 7], 37, False, True),       # odd numbers of stages, fewer CTAs than rows
     (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
     (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
-    (512, 4096, [12], 1, False, True),                         # one CTA waits for nobody but itself
+    (512, 4096, [24], 1, False, True),                         # one CTA waits for nobody but itself
     (2048, 1536, [130, 0, 160], 0, True, True),                # two rows a CTA: the second one is fetched while the first is split
 ])
 def test_nvf4_kernel_at_tile_edges(cuda_dev, H, I, counts, ctas, pre, post):
@@ -1381,6 +1381,35 @@ def test_nvf4_kernel_with_negative_and_nan_scales_and_tokens_out_of_range(cuda_d
     row = lambda v: v.nan_to_num(0.0).norm(dim=1)  # noqa: E731
     assert bool((row(a - b) <= TOL * row(b)).all())
     assert float(a[1].nan_to_num(0.0).abs().max()) == 0.0
+
+
+def test_nvf4_kernel_gives_up_cleanly_and_recovers(cuda_dev):
+    """A unit counter that starts far behind the last unit: every CTA computes its first unit and finds no more, the warps that
+    wait for whole tiles run into their limit of a second, the kernel reports it and returns, and after
+    reinit_workspace the state gives the clean bits again."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 512, 1536, 16, 4, 24
+    w = inputs.make_weights(H, I, E, 29, cuda_dev)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T)
+    assert _nvf4_takes(st, T)
+    g = torch.Generator(device=cuda_dev).manual_seed(3)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    clean = m.kernel_fn(data, st).clone()
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    ptr = ctypes.c_void_p()
+    _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 8, ctypes.byref(ptr)), "view")
+    at = ptr.value - st["workspace"].data_ptr() + 4096        # units drawn
+    st["workspace"][at:at + 4].copy_(torch.tensor([0, 0, 16, 0], dtype=torch.uint8))
+    m.kernel_fn(data, st)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 1
+    m.reinit_workspace(st)
+    for _ in range(2):
+        assert torch.equal(m.kernel_fn(data, st), clean)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
 
 
 def test_activations_outside_the_f16_range_saturate_as_documented(cuda_dev):
