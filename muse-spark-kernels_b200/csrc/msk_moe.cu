@@ -1185,6 +1185,20 @@ int msk_moe_router_logits_hilo(const MskMoeCfg* cfg, const void* x, const void* 
   }
 }
 
+static int launch_topk(const MskMoeCfg* cfg, const float* logits, const float* bias, int32_t* ids, float* tw, int n_tokens, cudaStream_t st) {
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(static_cast<unsigned>((n_tokens + 7) / 8));
+  lc.blockDim = dim3(256);
+  lc.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = cfg->no_pdl ? 0 : 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&lc, route_topk_kernel, logits, bias, ids, tw, n_tokens, static_cast<int>(cfg->n_experts),
+                                             static_cast<int>(cfg->top_k), static_cast<int>(cfg->routing_mode), cfg->route_scale));
+}
+
 int msk_moe_route(const MskMoeCfg* cfg, const float* logits, const float* bias, int32_t* topk_ids,
                   float* topk_weights, int n_tokens, void* stream) {
   const int rc = check_cfg(cfg);
@@ -1192,10 +1206,7 @@ int msk_moe_route(const MskMoeCfg* cfg, const float* logits, const float* bias, 
   if (!logits || !topk_ids || !topk_weights) return MSK_ERR_NULL;
   if (n_tokens < 0 || cfg->top_k > cfg->n_experts) return MSK_ERR_SHAPE;
   if (n_tokens == 0) return MSK_OK;
-  route_topk_kernel<<<static_cast<unsigned>((n_tokens + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      logits, bias, topk_ids, topk_weights, n_tokens, cfg->n_experts, cfg->top_k, cfg->routing_mode,
-      cfg->route_scale);
-  return static_cast<int>(cudaGetLastError());
+  return launch_topk(cfg, logits, bias, topk_ids, topk_weights, n_tokens, static_cast<cudaStream_t>(stream));
 }
 
 static int launch_sort(const MskMoeCfg* cfg, const int32_t* ids, int n_tokens, int32_t* cnt, int32_t* off,
@@ -1542,9 +1553,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
                           reinterpret_cast<int32_t*>(b + k.sort_blk), st);
   } else {
     if (logits != nullptr) {
-      route_topk_kernel<<<static_cast<unsigned>((n_tokens + 7) / 8), 256, 0, st>>>(
-          logits, bias, ids_out, tw_out, n_tokens, cfg->n_experts, cfg->top_k, cfg->routing_mode, cfg->route_scale);
-      e = static_cast<int>(cudaGetLastError());
+      e = launch_topk(cfg, logits, bias, ids_out, tw_out, n_tokens, st);
       if (e != 0) return e;
     }
     e = launch_sort(cfg, topk_ids, n_tokens, cnt, off, perm, inv, st, xin, xh_in_sort, pre_norm_w, pre_norm_eps);

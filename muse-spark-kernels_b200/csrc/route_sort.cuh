@@ -174,10 +174,12 @@ __device__ __forceinline__ void route_token_dispatch(const float* row, const flo
   else route_one_token<MAX_EXPERTS / 32>(row, bias, ids_row, wts_row, E, k, mode, scale, lane);
 }
 
-__global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict__ logits,
-                                                         const float* __restrict__ bias, int32_t* __restrict__ ids,
+// (Chained by programmatic dependent launch like the sort behind it: started behind a drained GPU it began 2 us later.)
+__global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, const float* __restrict__ bias, int32_t* __restrict__ ids,
                                                          float* __restrict__ wts, int T, int E, int k, int mode,
                                                          float scale) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");               // the logits may come from the kernel before
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
