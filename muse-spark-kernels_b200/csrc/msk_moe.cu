@@ -1604,6 +1604,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     q.ctr = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
     q.tiles = reinterpret_cast<unsigned int*>(b + k.nv_tiles);
     q.nloc = cfg->local_count; q.lo = cfg->local_start; q.H = cfg->hidden; q.I = cfg->inter; q.T = n_tokens; q.k = cfg->top_k;
+    q.share_rows = in_host_memory(x) ? 0 : 1;
     e = launch_nvf4(q, plan.grid, st, pdl);
     if (e != 0) return e;
     if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); }

@@ -105,6 +105,7 @@ struct NvParams {
   float pre_eps;
   int K[2], n_pairs[2];
   int nloc, lo, H, I, T, k;
+  int share_rows;                        // a token row may be read by several CTAs
 };
 
 struct alignas(16) NvUnit {
@@ -334,8 +335,9 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
   // has completed (the sort lets this launch begin only behind its own wait).
   constexpr int NT = NV_SPLIT_THREADS, NW = NT / 32, PER = (NV_MAX_BLOCKS + NT - 1) / NT;
   const int th = tid - NV_SPLIT_WARP * 32, nb = p.H / 16;
-  // up to 74 tokens several CTAs share a row: each reads all of it for its largest value and splits some of the K stages
-  const int parts = max(1, min(n_ctas / p.T, p.H / KS)), items = p.T * parts;
+  // up to 74 tokens several CTAs share a row: each reads all of it for its largest value and splits some of the K stages (not over
+  // PCIe, where every reader costs the bytes again: 8 rows in host memory, a whole step 121 us shared, 103 not, 119 by the other kernel)
+  const int parts = p.share_rows ? max(1, min(n_ctas / p.T, p.H / KS)) : 1, items = p.T * parts;
   uint32_t h[PER][8];
   float bm[PER];
   int U = 0;
