@@ -229,10 +229,11 @@ int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out);
 #define MSK_FEW_HOST_X 4      /* x lies in host memory */
 int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_fits);
 
-/* Whether a step of n_tokens that does not run in the few-token kernel runs in the kernel on the FP4 tensor cores (sort launches, both
- * GEMMs, combine), whatever path and tile msk_moe_plan names for it: *host_takes = 1 or 0. No GPU needed. No counterpart in
- * the reference. */
-int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int* host_takes);
+/* Whether a step of n_tokens runs in the kernel on the FP4 tensor cores (sort launches, both GEMMs, combine), whatever path and tile
+ * msk_moe_plan names for it: *host_takes = 1 or 0. norms: non-zero with a pre- or post-expert norm. Where msk_moe_few_fits says
+ * 1 as well, a state that holds all experts runs here and a rank's in the few-token kernel. No GPU needed. No
+ * counterpart in the reference. */
+int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_takes);
 
 /* How the GEMM kernels deal their work (host-side twin of the device code, a test hook): the pieces
  * that CTA `cta` of `shares` gets from n_base base units of n_stages K stages each. flat == 0: whole

@@ -704,7 +704,12 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
 // them, this one for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238.
 // A small model (H2048 I1024 E64 top-4), whose down units are four K stages long and wait for their epilogues: 8: 46 / 41, 24: 52 / 52
 // (a few experts taking most 41 / 36), 64: 60 / 61 (50 / 44).
+// With an expert norm the others take an exchange or a launch more, and this one, whose combine is a launch anyway, does not: all of 128
+// experts with both norms and routing, near-even (a few experts taking most) 3: 67 / 73 (61 / 60), 4: 75 / 91 (62 / 66), 5: 82 / 98
+// (64 / 91), with the post-expert norm 3: 67 / 71 (60 / 57), 4: 74 / 78 (62 / 77), 5: 81 / 92; the rank with it 3: 45 / 40, 4: 49 / 51, 5: 49 / 53.
+// Where the few-token kernel takes four tokens and more (pre-expert norm), it keeps a rank's: 4: 48 / 45, 6: 55 / 52.
 constexpr int NV_MIN_TOKENS = 6;
+constexpr int NV_MIN_NORM_TOKENS = 4;
 constexpr int NV_MIN_RANK_TOKENS = 24;       // of a rank that holds a part of the experts, beyond the one-launch form's tokens
 constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
@@ -715,9 +720,9 @@ static int nv_max_tokens(const MskMoeCfg* c, int T) {   // of the steps of up to
 }
 
 // Whether a step runs in it. A form that the configuration asks for is always the asked one.
-static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p) {
+static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, bool norm) {
   return c->token_tile == 0 && c->decode_path == 0 && c->flat_shares == 0 && c->stop_after == 0 && p.grid <= sm_count() &&
-         T >= NV_MIN_TOKENS && T <= nv_max_tokens(c, T) &&
+         T >= (norm ? NV_MIN_NORM_TOKENS : NV_MIN_TOKENS) && T <= nv_max_tokens(c, T) &&
          (c->local_count == c->n_experts || T <= ONE_LAUNCH_MAX_TOKENS || T >= NV_MIN_RANK_TOKENS);
 }
 
@@ -1442,7 +1447,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
   const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
                          (host_x ? MSK_FEW_HOST_X : 0);
-  if (plan.path == 0 && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
+  const bool nv = nv_takes(cfg, n_tokens, plan, pre_norm_w != nullptr || post_norm_w != nullptr);
+  if (plan.path == 0 && !(nv && cfg->local_count == cfg->n_experts) && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
     f.gs13 = gs13; f.gs2 = gs2;
@@ -1478,7 +1484,6 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
 
-  const bool nv = nv_takes(cfg, n_tokens, plan);
   if (!nv && plan.path != 1 && plan.path != 4) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
     p.route = logits != nullptr ? 1 : 2;
@@ -1915,12 +1920,12 @@ int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_f
   return MSK_OK;
 }
 
-int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int* host_takes) {
+int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_takes) {
   const int rc = check_cfg(cfg);
   if (rc != MSK_OK) return rc;
   if (!host_takes) return MSK_ERR_NULL;
   if (n_tokens < 1) return MSK_ERR_SHAPE;
-  *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens)) ? 1 : 0;
+  *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens), norms != 0) ? 1 : 0;
   return MSK_OK;
 }
 

@@ -1269,7 +1269,7 @@ def test_prefill_moe_runs_the_prefill_layer_call_site(cuda_dev):
 
 def _nvf4_takes(st, T):
     takes = ctypes.c_int(0)
-    assert st["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(st["cfg"]), T, ctypes.byref(takes)) == 0
+    assert st["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(st["cfg"]), T, int(st["post_norm_w"] is not None or st["pre_norm_w"] is not None), ctypes.byref(takes)) == 0
     return takes.value == 1
 
 
@@ -1289,6 +1289,7 @@ def _ids_of_counts(counts, lo, k, dev):
     (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
     (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
     (512, 4096, [24], 1, False, True),                         # one CTA waits for nobody but itself
+    (768, 1536, [2, 0, 2], 0, False, True),                    # the fewest tokens it takes
     (2048, 1536, [130, 0, 160], 0, True, True),                # two rows a CTA: the second one is fetched while the first is split
 ])
 def test_nvf4_kernel_at_tile_edges(cuda_dev, H, I, counts, ctas, pre, post):
