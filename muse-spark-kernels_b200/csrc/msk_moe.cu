@@ -698,7 +698,7 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
 // 173 / 208, 64: 221 / 262, 160: 258 / 291, 192 (12 rows an expert) 275 / 318; a few experts taking most tokens 8: 63 / 65, 12: 68 / 65,
 // 16: 74 / 71, 24: 81 / 84, 48: 95 / 114, 192: 207 / 278.
 // A rank with one row a token (32 of 256, H4096 I4096, two experts taking most) 6: 54 / 58, 8: 59 / 66; 12: 63 / 62, 16: 68 / 66
-// (from nine tokens on the other one has its cheaper form as well, and there is little to stream); 24: 78 / 79, 32: 85 / 95, 160: 159 /
+// (from nine tokens on the other one has its cheaper form as well, and there is little to stream); 24: 75 / 74 to 81 / 85, 32: 85 / 95, 160: 159 /
 // 198, 384: 234 / 315; H7168 I2048, even, 16: 75 / 75, 64: 115 / 123, 256: 138 / 158, 384: 156 / 192.
 // Beyond 12 rows an expert the other one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of
 // them, this one for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238.
@@ -710,7 +710,7 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
 // Where the few-token kernel takes four tokens and more (pre-expert norm), it keeps a rank's: 4: 48 / 45, 6: 55 / 52.
 constexpr int NV_MIN_TOKENS = 6;
 constexpr int NV_MIN_NORM_TOKENS = 4;
-constexpr int NV_MIN_RANK_TOKENS = 24;       // of a rank that holds a part of the experts, beyond the one-launch form's tokens
+constexpr int NV_MIN_RANK_TOKENS = 28;       // of a rank that holds a part of the experts, beyond the one-launch form's tokens
 constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
 

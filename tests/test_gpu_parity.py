@@ -1288,7 +1288,7 @@ def _ids_of_counts(counts, lo, k, dev):
     (2304, 1792, [31, 24, 2, 0, 0, 7], 37, False, True),       # odd numbers of stages, fewer CTAs than rows
     (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
     (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
-    (512, 4096, [24], 1, False, True),                         # one CTA waits for nobody but itself
+    (512, 4096, [28], 1, False, True),                         # one CTA waits for nobody but itself
     (768, 1536, [2, 0, 2], 0, False, True),                    # the fewest tokens it takes
     (2048, 1536, [130, 0, 160], 0, True, True),                # two rows a CTA: the second one is fetched while the first is split
 ])
