@@ -354,8 +354,8 @@ template <> struct YQuad<true> {
 // the registers per row in flight, which is what lets all eight rows of a token be loaded at once).
 template <int G, bool YB, int MINB, int NF4 = COMBINE_MAX_F4>
 __global__ void __launch_bounds__(COMBINE_THREADS, MINB)
-    combine_norm_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv, const float* __restrict__ tw,
-                   __nv_bfloat16* __restrict__ out, int H, int k, float eps) {
+    combine_norm_kernel(const float* y, const int32_t* inv, const float* tw, __nv_bfloat16* __restrict__ out, int H, int k,
+                        float eps) {   // (y, inv and tw: as above)
   constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
   static_assert(G == 1 << LG, "two, four or eight rows together");
   __shared__ __align__(16) float wsum[G][COMBINE_THREADS / 32];

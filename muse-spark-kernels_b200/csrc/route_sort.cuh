@@ -323,7 +323,8 @@ __device__ __forceinline__ void convert_rows_block(const __nv_bfloat16* __restri
   }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) sort_kernel(const int32_t* __restrict__ ids, int n, int lo, int nloc,
+// (The ids may come from a top-k launch that still runs when this one starts: not __restrict__, as in the kernels below.)
+__global__ void __launch_bounds__(SORT_THREADS) sort_kernel(const int32_t* ids, int n, int lo, int nloc,
                                                             int32_t* __restrict__ cnt, int32_t* __restrict__ off,
                                                             int32_t* __restrict__ perm, int32_t* __restrict__ inv,
                                                             const __nv_bfloat16* __restrict__ x,

@@ -543,6 +543,9 @@ def test_kernels_read_other_ctas_rows_behind_a_barrier():
 @pytest.mark.parametrize("name,kernel,written", [("route_sort.cuh", "sort_multi_scatter_kernel", ("ids", "blk")),
                                                  ("route_sort.cuh", "sort_multi_count_kernel", ("logits",)),
                                                  ("route_sort.cuh", "route_sort_kernel", ("logits",)),
+                                                 ("route_sort.cuh", "route_topk_kernel", ("logits",)),
+                                                 ("route_sort.cuh", " sort_kernel", ("ids",)),
+                                                 ("msk_moe.cu", "combine_norm_kernel", ("y", "inv", "tw")),
                                                  ("msk_moe.cu", "combine_cols_kernel", ("y", "inv", "tw"))])
 def test_what_the_launch_before_writes_is_read_coherently(name, kernel, written):
     """A kernel started by programmatic launch is there while its predecessor still writes: what that one writes must

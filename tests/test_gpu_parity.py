@@ -419,6 +419,40 @@ def test_sort_moves_to_several_ctas_where_they_are_faster(cuda_dev, T, E, k, lo,
         assert bool(st["workspace"][o:o + 64 * 256 * 4].any()) == several
 
 
+@pytest.mark.parametrize("T", [33, 64, 200])
+def test_sort_reads_the_ids_of_the_top_k_in_front_of_it(cuda_dev, T):
+    """Top-k and a sort on one CTA are two launches, the second there before the first has stored its ids: tables of back-to-back replays
+    with other logits each time, each against its own ids."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 256, 256, 128, 8
+    st = m.prepare(inputs.make_weights(H, I, E, 12, cuda_dev), n_experts=E, top_k=k, max_tokens=T)
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    many = torch.randn((12, T, E), generator=g, device=cuda_dev)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16), "router_logits": many[0].clone()}
+    m.kernel_fn(data, st)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out, ids, tw = m.kernel_fn(data, st, return_routing=True)
+    tables, ptr = [], ctypes.c_void_p()
+    for which, n in ((0, E), (1, E + 1), (2, T * k), (3, T * k)):
+        _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), which, ctypes.byref(ptr)), "view")
+        at = ptr.value - st["workspace"].data_ptr()
+        tables.append(st["workspace"][at:at + 4 * n].view(torch.int32))
+    got = []
+    for logits in many:
+        data["router_logits"].copy_(logits)
+        graph.replay()
+        got.append([ids.clone()] + [t.clone() for t in tables])
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    for logits, (ids, *mine) in zip(many, got):
+        rid, _ = orc.route_topk(logits.cpu(), k, "softmax_topk", None)
+        assert torch.equal(ids.cpu(), rid)
+        for a, b in zip(mine, orc.sort_routes(rid.numpy(), 0, E)):
+            assert np.array_equal(a.cpu().numpy(), np.asarray(b).reshape(-1))
+
+
 @pytest.mark.parametrize("tile,path,post,H,I", [(64, 0, False, 512, 256), (64, 1, True, 768, 512), (128, 0, True, 512, 256),
                                                 (128, 0, False, 768, 512)])
 def test_wide_tiles_at_ragged_row_counts(cuda_dev, tile, path, post, H, I):
