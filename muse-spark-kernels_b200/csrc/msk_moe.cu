@@ -715,7 +715,7 @@ constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
 
 static int nv_max_tokens(const MskMoeCfg* c, int T) {   // of the steps of up to T tokens that may take it
-  if (c->inter < NV_MIN_INTER || c->hidden > NV_MAX_BLOCKS * 16) return 0;
+  if (c->inter < NV_MIN_INTER || c->inter > NV_MAX_INTER || c->hidden > NV_MAX_BLOCKS * 16) return 0;
   return static_cast<int>(std::min(static_cast<long long>(T), static_cast<long long>(NV_MAX_MEAN_ROWS) * c->n_experts / c->top_k));
 }
 
@@ -728,7 +728,7 @@ static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, bool norm) {
 
 // Workspace carving. Everything is sized for max_tokens with the worst plan.
 struct Carve {
-  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, nv_tiles, nv_img[2], nv_rs[2], nv_max, total;
+  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, nv_tiles, nv_img[2], total;
 };
 constexpr size_t TRACE_CTAS = 256;
 constexpr size_t TRACE_WORDS = TRACE_CTAS * 16 + 3 * 256;
@@ -780,9 +780,7 @@ static Carve carve(const MskMoeCfg* c, int T) {
   const int nv_k[2] = {c->hidden, c->inter};
   for (int i = 0; i < 2; ++i) {
     k.nv_img[i] = o; o += round_up(nv_groups * (nv_k[i] / KS) * NV_GROUP_BYTES, 256);
-    k.nv_rs[i] = o; o += round_up(nv_rows * 4, 256);
   }
-  k.nv_max = o; o += round_up(nv_rows * (c->inter / 32) * 2, 256);
   k.total = o;
   return k;
 }
@@ -1602,10 +1600,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     q.inter = inter; q.y = y; q.status = status; q.trace = trace;
     for (int i = 0; i < 2; ++i) {
       q.img[i] = b + k.nv_img[i];
-      q.rs[i] = reinterpret_cast<float*>(b + k.nv_rs[i]);
       q.K[i] = p.ph[i].K; q.n_pairs[i] = p.ph[i].n_pairs;
     }
-    q.part_max = reinterpret_cast<__half*>(b + k.nv_max);
     q.ctr = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4096);
     q.tiles = reinterpret_cast<unsigned int*>(b + k.nv_tiles);
     q.nloc = cfg->local_count; q.lo = cfg->local_start; q.H = cfg->hidden; q.I = cfg->inter; q.T = n_tokens; q.k = cfg->top_k;

@@ -1,4 +1,4 @@
-// Grouped GEMMs of the routed experts on the FP4 tensor cores, for token tiles of up to 24 rows: both GEMMs in one
+// Grouped GEMMs of the routed experts on the FP4 tensor cores, for token tiles of up to 16 rows: both GEMMs in one
 // cooperative launch behind the sort.
 //
 // D[128 weight rows, N columns] = W[128, K] * B[N, K]^T with tcgen05.mma.kind::mxf4nvf4 (E2M1 operands, one E4M3 scale per 16
@@ -10,32 +10,35 @@
 // row of whole steps 288 and 240 (both sides of the other sizes: nv_takes() in msk_moe.cu). Bound by memory, some 6.8 TB/s between the
 // first MMA and the last, and by the 10 us before it (tables, split of the token rows) and 6 after.
 //
-// Activations. A token row (F16 values, as in gemm.cuh) enters as seven E2M1 rows of its own, the digits of a fixed-point
-// number: in a block of 16 K an element is x = 2^u * (d0 + d1 / 8 + ... + d6 / 8^6), digits -4 .. 3, which E2M1 holds exactly (as
-// d / 2). The block's exponent u, relative to the row's, is its E4M3 scale, one byte for all seven rows; 8^-p and the row's
-// power of two are applied to the FP32 accumulators, which each digit has to itself, in the epilogue. An element is exact to
-// 2^-20 of the largest of its block of 16 (BF16 values are held exactly down to 2^-12 of it), blocks keep that down to 2^-17
-// of the row's largest value. Products are exact and accumulate in FP32. Measured against 64 bits (relative 2-norm of the raw
-// sums, this / the F16 form): gate/up sums of normal rows, K = 4096, 1e-7 / 1.5e-6; down sums of SwiGLU values, K = 1536,
-// 1.6e-7 / 9.0e-7; the rounding of the values to BF16 behind them is 1.7e-3. (Six digits: 5e-7 and 2.8e-6; the seventh costs some 4
-// cycles of 56 an MMA.)
+// Activations enter exactly as in the F16 kernels: every F16 value, whatever lies beside it (tested bit for bit). A token row becomes nine E2M1
+// rows of its own, the digits of a fixed-point number: in a block of 16 K an element is x = 2^u * (d0 + d1 / 8 + ... + d8 / 8^8), digits
+// -4 .. 3 (the first to 4), which E2M1 holds exactly (as d / 2). The block's 2^u is its E4M3 scale, one byte for all nine rows; 8^-p is applied to
+// the FP32 accumulators, which each digit has to itself, in the epilogue. These 27 bits hold all F16 values of blocks with magnitudes below 4, and
+// BF16 values down to 2^-17 of the block's largest. What is left over of others, whole steps of 2^-24, is split in the same way with the
+// scale 2^-9: its last two digits as a second level, four more as a third one that only blocks with magnitudes from 128 on can need.
+// Levels add up in the accumulators of their digits, so a K stage with such an element has another pass of MMAs on the same weights. Which
+// stages have one is kept in words per tile. Products are exact and accumulate in FP32. Measured against 64 bits (relative 2-norm of the raw
+// down sums, K = 1536, this / the F16 form): SwiGLU values 3.7e-8 / 9.0e-7; beside channels 100 times as large that the weights ignore
+// 4.1e-8 / 8.3e-7. (Seven digits and no levels lost bits beside large channels: 1.0e-4 there. Eight digits, with tiles of up to 24 rows:
+// a third of the K stages of SwiGLU values have a second level, whole steps of 64 tokens 234 us for 229 now; a few experts taking most tokens,
+// 8 tokens 67 for 64, 32 tokens 96 for 92.)
 // NaN elements make the block's scale NaN; weight scales with a sign bit (no quantiser writes them) turn the signs of their
 // 16 codes in shared memory, because the hardware's scales are unsigned.
 //
 // Per CTA (512 threads, one CTA per SM):
 //   warp 0       draws units from a counter and streams their weights: one bulk copy per K stage (two tiles of 128 rows) into a ring;
-//   warp 1       MMA issuer (and TMEM allocation): per stage 2 tiles x 4 MMAs of 64 K, one commit;
-//   warp 2       token rows of the unit's tile, split and laid out beforehand: one bulk copy per K stage;
+//   warp 1       MMA issuer (and TMEM allocation): per pass 2 tiles x 4 MMAs of 64 K, one commit;
+//   warp 2       token rows of the unit's tile, split and laid out beforehand: one bulk copy per K stage and level;
 //   warps 4-7    scales: shared memory -> TMEM, each warp for its lane quarter (the hardware wants four copies);
 //   warps 8-11   epilogue: digits summed, SwiGLU / scale, rows to global memory;
 //   warp 3       counts stored gate/up units for their tiles;
 //   warps 12-15  split `inter`: pieces of eight rows x 256 columns of a token tile, dealt over the CTAs in the order of the tiles, as each tile's
-//                gate/up units are all stored (a row's power of two needs its largest value). Whole tiles, split by the CTA that
-//                stored their last unit, kept a rank's 24-token step waiting for some 20 us.
+//                gate/up units are all stored. Whole tiles, split by the CTA that stored their last unit, kept a rank's 24-token step waiting
+//                for some 20 us.
 // Warps 4-15 first split the token rows, a row or a part of one per CTA at a time, while the first weights are on their way.
 //
-// Work is dealt one unit at a time, gate/up units before down units, as in pair.cuh (but a unit is drawn when its weights are next to
-// be fetched, not further ahead); a down unit waits for its tile's rows. Units of an expert with several tiles are ordered pair
+// Work is dealt one unit at a time, gate/up units before down units, as in pair.cuh (but a unit is drawn while the weights of the one before it are
+// fetched, not further ahead); a down unit waits for its tile's rows. Units of an expert with several tiles are ordered pair
 // first, so that the second tile finds the weights in L2.
 #pragma once
 #include <cstddef>
@@ -51,9 +54,16 @@
 namespace msk {
 
 constexpr int NV_THREADS = 512;
-constexpr int NV_ROWS = 24;                                // most token rows of a tile
-constexpr int NV_PARTS = 7;                                // digits of an activation
-constexpr int NV_GROUP_BYTES = NV_PARTS * 1024 + 128;      // eight token rows x 256 K: digits, scales
+constexpr int NV_ROWS = 16;                                // most token rows of a tile
+constexpr int NV_PARTS = 9;                                // digits of an activation
+// Levels of a K stage of eight token rows (1 KB a digit, 128 bytes of scales each): their digits, the accumulators of the first
+// one, their place in the stage.
+constexpr int NV_LEVELS = 3;
+__host__ __device__ constexpr int nv_digits(int level) { return level == 0 ? NV_PARTS : level == 1 ? 2 : 4; }
+__host__ __device__ constexpr int nv_first(int level) { return level == 0 ? 0 : level == 1 ? 6 : 2; }
+__host__ __device__ constexpr int nv_level_at(int level) { return level == 0 ? 0 : level == 1 ? nv_digits(0) * 1024 + 128 : (nv_digits(0) + nv_digits(1)) * 1024 + 256; }
+constexpr int NV_LEVEL_BYTES = nv_level_at(1);             // of the first level, the widest
+constexpr int NV_GROUP_BYTES = nv_level_at(2) + nv_digits(2) * 1024 + 128;   // eight token rows x 256 K
 constexpr int NV_W_STAGES = 4, NV_S_STAGES = 2;            // rings: weights, scales in TMEM
 constexpr int NV_MARKS = 8;                                // stages whose MMAs have a barrier of their own
 constexpr int NV_UNITS = 4;
@@ -66,22 +76,25 @@ constexpr int NV_AHEAD = 8;                                // stages of the firs
 __host__ __device__ inline int nv_tiles(int c) { return (c + NV_ROWS - 1) / NV_ROWS; }
 __host__ __device__ inline int nv_tile_rows(int c, int n) { return n <= 1 ? c : ((c + n - 1) / n + 7) & ~7; }
 __host__ __device__ inline int nv_width(int rows) { return (rows + 7) >> 3; }
-// Groups that the image of an expert's rows takes (every tile but a lone one has room for three).
+// Groups that the image of an expert's rows takes: all tiles but the last have whole ones.
 constexpr int NV_GROUPS = NV_ROWS / 8;
-__host__ __device__ inline int nv_groups(int c) { return c <= NV_ROWS ? nv_width(c) : NV_GROUPS * nv_tiles(c); }
-// A bound on their sum over experts with `rows` rows in all: nv_groups(c) <= 1 + (c - 1) * 7 / 32.
+__host__ __device__ inline int nv_groups(int c) { return nv_width(c); }
+// A bound on their sum over experts with `rows` rows in all: nv_groups(c) <= 1 + (c - 1) / 8.
 inline size_t nv_groups_bound(size_t rows, size_t experts) {
   const size_t e = rows < experts ? rows : experts;
-  return e + ((rows - e) * 7 + 31) / 32;
+  return e + (rows - e) / 8;
 }
 
 // Counters of a tile, a cache line for each: CTAs that wait for a tile poll another line than those that count for its neighbours.
-constexpr int NV_TILE_WORDS = 32;
+constexpr int NV_TILE_WORDS = 64;
 enum : int {
   NV_DONE = 0,     // stored gate/up units
   NV_READY = 8,    // pieces of inter that are split
-  NV_SEEN = 16,    // down units that have seen all of them
+  NV_SEEN = 16,    // down units that have fetched them all
+  NV_MORE = 32,    // bit per K stage, a word for 32 of them: stages with a second level, a third level; token rows, then inter
+  NV_MORE_INTER = NV_MORE + 2 * (NV_MAX_BLOCKS * 16 / KS / 32),
 };
+constexpr int NV_MAX_INTER = (NV_TILE_WORDS - NV_MORE_INTER) / 2 * 32 * KS;   // 122880
 
 struct NvParams {
   const uint8_t* w[2];
@@ -96,12 +109,10 @@ struct NvParams {
   __half* inter;                         // [R, I]
   float* y;                              // [R, H]
   uint8_t* img[2];                       // split rows (see the split below): token rows, rows of inter
-  float* rs[2];                          // [R] the rows' powers of two: token rows, rows of inter
-  __half* part_max;                      // [R, I / 32] largest magnitude in 32 columns of a row of inter
   int32_t* status;
   unsigned long long* trace;
   unsigned int* ctr;                     // [0] units drawn, [1] CTAs that have left, [2] CTAs that have split their token rows
-  unsigned int* tiles;                   // NV_TILE_WORDS a tile: counters NV_DONE, NV_READY, NV_SEEN, all zero between launches
+  unsigned int* tiles;                   // NV_TILE_WORDS a tile: NV_DONE and so on, all zero between launches
   float pre_eps;
   int K[2], n_pairs[2];
   int nloc, lo, H, I, T, k;
@@ -116,34 +127,38 @@ struct alignas(16) NvUnit {
 
 struct NvCtrl {
   uint64_t w_full[NV_W_STAGES], b_full[NV_MARKS], s_full[NV_S_STAGES];
-  uint64_t done[NV_MARKS];               // the MMAs of stage n (n % 8): its places in all three rings are free
+  uint64_t done[NV_MARKS];               // the MMAs of pass n (n % 8): its places for scales and token rows are free
+  uint64_t w_done[NV_W_STAGES];          // those of a stage's last pass: its weights' place is
   uint64_t d_full[2], d_empty[2];
   uint64_t u_full[NV_UNITS], u_empty[NV_UNITS];
   uint64_t stored[NV_UNITS];             // the epilogue has stored its values of a unit
   NvUnit unit[NV_UNITS];
-  uint4 route[MAX_TOP_K];                // of the token row that is split: place of its digits in the image, width, row in its group, row
-  float red[2][NV_SPLIT_THREADS / 32];
+  uint4 route[MAX_TOP_K];                // of the token row that is split: place of its digits in the image, tile's width, tile, row in it
+  float red[NV_SPLIT_THREADS / 32];
   int n_routes;
   uint32_t tmem_base;
   int abort_word;
   int b_stages, b_bytes;                 // ring of token rows: places, bytes of one
+  int b_pass[NV_MARKS];                  // what a place holds: its level, and NV_LAST in the last pass of a K stage
 };
 static_assert(sizeof(NvCtrl) <= 1024 && offsetof(NvCtrl, unit) % 16 == 0, "control block");
 
-__host__ __device__ constexpr int nv_place_bytes(int width) { return (width * NV_GROUP_BYTES + 1023) / 1024 * 1024; }
+constexpr int NV_LAST = 4;
+__host__ __device__ constexpr int nv_place_bytes(int width) { return (width * NV_LEVEL_BYTES + 1023) / 1024 * 1024; }
 
 struct NvCfg {
   static constexpr int TABLE_INTS = MAX_LOCAL_EXPERTS + 4;
-  // The ring of token rows has places for the widest tile of the launch (whole swizzle atoms of 1 KB): 3, 5 or 8 of them.
-  static constexpr int B_RING = 75 * 1024;
+  // The ring of token rows has places for the widest tile of the launch (whole swizzle atoms of 1 KB): 4 or 7 of them. (Places of each pass's
+  // own size, more of them: 1 % slower; three of them, and three stages of weights ahead: 2 %.)
+  static constexpr int B_RING = 76 * 1024;
   static constexpr int W_OFF = 0, B_OFF = NV_W_STAGES * STAGE_W_BYTES, CTL_OFF = B_OFF + B_RING, TABLE_OFF = CTL_OFF + 1024;
   static constexpr int SMEM_BYTES = TABLE_OFF + 4 * TABLE_INTS * 4;
-  static_assert(SMEM_BYTES <= 232448 && 3 * nv_place_bytes(NV_GROUPS) <= B_RING, "shared memory of a CTA");
+  static_assert(SMEM_BYTES <= 232448 && 4 * nv_place_bytes(NV_GROUPS) <= B_RING, "shared memory of a CTA");
   // TMEM: accumulators of two tiles (digits x rows columns each; those of a tile of eight rows twice), two stages of scales
   static constexpr int D_WIDE = NV_PARTS * NV_ROWS, D_NARROW = NV_PARTS * 8;
-  static constexpr int S_BASE = 2 * D_WIDE, S_COLS = 64, S_B = 32;   // 4 x 4 columns per weight tile, 4 x 8 for the token rows
+  static constexpr int S_BASE = 2 * D_WIDE, S_COLS = 32, S_B = S_BASE + NV_S_STAGES * S_COLS;   // 4 x 4 columns per weight tile, 4 x 8 for the token rows
   static_assert(4 * D_NARROW <= S_BASE && (D_WIDE + 31) / 32 <= 8, "TMEM layout");
-  static_assert(S_BASE + NV_S_STAGES * S_COLS <= TMEM_COLS, "TMEM budget");
+  static_assert(S_B + NV_S_STAGES * S_COLS <= TMEM_COLS, "TMEM budget");
 };
 
 __host__ __device__ constexpr uint32_t idesc_nvf4(uint32_t N) {   // E2M1 x E2M1, E4M3 scales, M = 128
@@ -151,20 +166,20 @@ __host__ __device__ constexpr uint32_t idesc_nvf4(uint32_t N) {   // E2M1 x E2M1
 }
 // D[tmem] (+)= A[smem, 128 x 256] * B[smem, N x 256]^T for the two tiles of a stage, four MMAs of 64 K each: a scale per row and 16 K in
 // TMEM, lane r % 32 (in every lane quarter), column r / 32, the four bytes of 64 K. `sf`: 4 x 4 columns of tile 0, of tile 1, 4 x 8 of the
-// token rows. By one elected lane, with the commit that hands the stage back (done_bar); the answer of a probe of `next_full` (true:
-// complete) is asked for before the MMAs and read behind them. In one block of assembly: as separate calls in a branch of that lane
+// token rows. By one elected lane, with the commit that hands the pass's places back (done_bar) and, with `last`, the one for the weights
+// (w_done_bar); the answer of a probe of `next_full` (true: complete) is asked for before the MMAs and read behind them. In one block of assembly: as separate calls in a branch of that lane
 // the operands went to the issue unit one by one, some 150 cycles an MMA.
 #define NV_MMA "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X"
-__device__ __forceinline__ bool mma_nvf4_stage(uint32_t d0, uint32_t d1, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sf, uint32_t accumulate,
-                                               uint32_t done_bar, uint32_t next_full, uint32_t parity) {
+__device__ __forceinline__ bool mma_nvf4_stage(uint32_t d0, uint32_t d1, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate,
+                                               uint32_t done_bar, uint32_t w_done_bar, uint32_t last, uint32_t next_full, uint32_t parity) {
   static_assert(OCT_BYTES / 16 == 72, "the second tile's octet blocks");
   uint32_t ok;
   asm volatile(
-      "{\n\t.reg .pred q, e, acc, t;\n\t.reg .b64 a, b, c;\n\t.reg .b32 f, g, h;\n\t"
+      "{\n\t.reg .pred q, e, acc, t, l;\n\t.reg .b64 a, b, c;\n\t.reg .b32 f, g, h;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 q, [%9], %10;\n\t"
       "elect.sync _|e, 0xffffffff;\n\t"
       "setp.ne.b32 acc, %8, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
-      "mov.b64 a, %3;\n\tmov.b64 b, %4;\n\tmov.b32 f, %6;\n\tadd.u32 g, %6, 32;\n\t"
+      "mov.b64 a, %3;\n\tmov.b64 b, %4;\n\tmov.b32 f, %6;\n\tmov.b32 g, %13;\n\t"
       "@e " NV_MMA " [%1], a, b, %5, [f], [g], acc;\n\t"
       "add.s64 c, a, 72;\n\tadd.u32 h, f, 16;\n\t"
       "@e " NV_MMA " [%2], c, b, %5, [h], [g], acc;\n\t"
@@ -181,28 +196,23 @@ __device__ __forceinline__ bool mma_nvf4_stage(uint32_t d0, uint32_t d1, uint64_
       "add.s64 c, a, 72;\n\tadd.u32 h, f, 16;\n\t"
       "@e " NV_MMA " [%2], c, b, %5, [h], [g], t;\n\t"
       "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
+      "setp.ne.and.b32 l, %12, 0, e;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(ok)
-      : "r"(d0), "r"(d1), "l"(a), "l"(b), "r"(idesc), "r"(sf), "r"(done_bar), "r"(accumulate), "r"(next_full), "r"(parity)
+      : "r"(d0), "r"(d1), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(done_bar), "r"(accumulate), "r"(next_full), "r"(parity), "r"(w_done_bar), "r"(last), "r"(sfb)
       : "memory");
   return ok != 0u;
 }
 #undef NV_MMA
 
-// ---- the split. Image of a tile (width W groups, K): per K stage of 256, digits [7][W][8 rows][128 bytes], the eight 16-byte
-// chunks of a row in the order of the 128-byte swizzle (chunk c of row r at c ^ r: a row's digit is one line to write), then
-// scales [8 W rows][16]; NV_GROUP_BYTES * W bytes a stage, one contiguous copy.
-
-// Exponent of a block's unit: its largest magnitude m is at most 3.4 units (digits reach 24 / 7 upwards).
-__device__ __forceinline__ int nv_unit_exp(float m) {
-  const int b = __float_as_int(m);
-  return m > 0.f ? (b >> 23) - 127 - ((b & 0x7fffff) > 0x599999 ? 0 : 1) : -200;
-}
+// ---- the split. Image of a tile (width W groups, K): per K stage of 256 and level, digits [9, 2 or 4][W][8 rows][128 bytes], the eight
+// 16-byte chunks of a row in the order of the 128-byte swizzle (chunk c of row r at c ^ r: a row's digit is one line to write), then
+// scales [8 W rows][16]; one contiguous copy a level, NV_GROUP_BYTES * W bytes a stage.
 __device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
-// The row's, from its largest magnitude (zero and NaN: that of the smallest F16 value).
-__device__ __forceinline__ int nv_row_exp(float m) { return max(nv_unit_exp(m), -25); }
-// The power of two that a row's sums are multiplied by, from its unit exponent: the largest block has scale 2^8 (and its codes are d / 2).
-__device__ __forceinline__ float nv_row_scale(int U) { return exp2_int(U - 7); }
+constexpr int NV_MAX_EXP = 14;   // of a block's unit: 65504 is below four of 2^14
+constexpr int NV_MIN_EXP = 0;    // its ninth digit is a step of 2^-24, the smallest there is
+constexpr float NV_SUM_SCALE = 128.f;   // what sums are multiplied by: units of 2^14 have scale 2^8, and codes are d / 2
 
 // Largest magnitude of sixteen values; NaN if one of them is.
 __device__ __forceinline__ float nv_block_max(const uint32_t (&h)[8]) {
@@ -212,48 +222,98 @@ __device__ __forceinline__ float nv_block_max(const uint32_t (&h)[8]) {
   return __half2float(__hmax_nan(__low2half(m), __high2half(m)));
 }
 
-// Sixteen values -> for each the number x * 8^6 / unit as 21 bits that hold digit + 4 in each three; returns the scale byte. bm: the
-// block's largest magnitude, U: the row's unit exponent.
-__device__ __forceinline__ uint32_t nv_fixed16(const uint32_t (&h)[8], float bm, int U, uint32_t (&f)[16]) {
-  const int u = max(nv_unit_exp(bm), U - 17), e = u - U + 8;
-  const float scale = exp2_int(3 * (NV_PARTS - 1) - u);
-  constexpr float BIAS = 12582912.f + 4.f * ((1 << (3 * NV_PARTS)) - 1) / 7.f;   // rounds by the addition; 4 in every digit
+// d digits of -4 .. 3 that are all 4 in the bits of a number: what is added so that they come out as 0 .. 7.
+__host__ __device__ constexpr uint32_t nv_bias(int d) { return ((1u << (3 * d)) - 1u) / 7u * 4u; }
+
+struct NvBlock {
+  int u;              // its unit is 2^u, the smallest with its largest magnitude below four units (as far as NV_MIN_EXP)
+  uint32_t scale;     // as E4M3
+  uint32_t levels;    // bit per level that it needs
+};
+// Sixteen values -> for each the number of steps of 2^-24 units nearest to it, biased: digits + 4 in three bits each, the first of 0 .. 8.
+// What is left is at most half a step, 2^13 steps of 2^-24: the lowest two digits of that number are the second level, the four above
+// them the third.
+__device__ __forceinline__ NvBlock nv_fixed16(const uint32_t (&h)[8], uint32_t (&f)[16]) {
+  NvBlock k;
+  const float bm = nv_block_max(h);
+  k.u = min(max((__float_as_int(bm) >> 23) - 128, NV_MIN_EXP), NV_MAX_EXP);
+  const float scale = exp2_int(3 * (NV_PARTS - 1) - k.u);
+  float hi = 0.f, lo = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h[i]));
-    f[2 * i] = __float_as_uint(fmaf(v.x, scale, BIAS));
-    f[2 * i + 1] = __float_as_uint(fmaf(v.y, scale, BIAS));
+    const float x0 = v.x * scale, x1 = v.y * scale;
+    const int q0 = __float2int_rn(x0), q1 = __float2int_rn(x1);
+    f[2 * i] = static_cast<uint32_t>(q0) + nv_bias(NV_PARTS);
+    f[2 * i + 1] = static_cast<uint32_t>(q1) + nv_bias(NV_PARTS);
+    const float r0 = x0 - static_cast<float>(q0), r1 = x1 - static_cast<float>(q1);
+    hi = fmaxf(hi, fmaxf(r0, r1));
+    lo = fminf(lo, fminf(r0, r1));
   }
-  return bm != bm ? 0x7Fu : e >= -6 ? static_cast<uint32_t>(e + 7) << 3 : 1u << (e + 9);
+  const float steps = exp2_int(k.u - NV_MIN_EXP);
+  k.levels = bm != bm || (hi == 0.f && lo == 0.f) ? 1u : hi * steps <= 27.f && lo * steps >= -36.f ? 3u : 7u;
+  const int e = k.u - (NV_MAX_EXP - 8);
+  k.scale = bm != bm ? 0x7Fu : e >= -6 ? static_cast<uint32_t>(e + 7) << 3 : 1u << (e + 9);
+  return k;
 }
-// The last digits of the sixteen as E2M1 codes, a nibble each; the numbers lose them. (The loops over the digits are not unrolled: this
-// code runs from a cold instruction cache while the weights stream, where a line takes a microsecond; all digits in line made
-// the steps 5 to 20 us longer.)
-__device__ __forceinline__ uint2 nv_next_digit(uint32_t (&f)[16]) {
+// The number of steps of 2^-24 that is left of each, biased by six digits.
+__device__ __forceinline__ void nv_rest16(const uint32_t (&h)[8], int u, uint32_t (&f)[16]) {
+  const float scale = exp2_int(3 * (NV_PARTS - 1) - u), steps = exp2_int(u - NV_MIN_EXP);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h[i]));
+    const float x0 = v.x * scale, x1 = v.y * scale;
+    f[2 * i] = static_cast<uint32_t>(__float2int_rn((x0 - rintf(x0)) * steps)) + nv_bias(6);
+    f[2 * i + 1] = static_cast<uint32_t>(__float2int_rn((x1 - rintf(x1)) * steps)) + nv_bias(6);
+  }
+}
+// The last digits of the sixteen (bits `mask` of the numbers) as E2M1 codes, a nibble each; the numbers lose three bits.
+__device__ __forceinline__ uint2 nv_next_digit(uint32_t (&f)[16], uint32_t mask) {
   uint32_t q[2];
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
     uint32_t t = 0u;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      t += (f[8 * c + i] & 7u) * (1u << (4 * i));
+      t += (f[8 * c + i] & mask) * (1u << (4 * i));
       f[8 * c + i] >>= 3;
     }
-    const uint32_t pos = ((t >> 2) & 0x11111111u) * 15u;   // nibbles of digits >= 0: the digit; of the others: sign and magnitude 4 - t
-    q[c] = (t & 0x33333333u & pos) | ((0xCCCCCCCCu - t) & ~pos);
+    const uint32_t pos = (((t >> 2) | (t >> 3)) & 0x11111111u) * 15u;   // nibbles of digits >= 0: the digit; of the others: sign and magnitude 4 - t
+    q[c] = (((t & 0x33333333u) | ((t >> 1) & 0x44444444u)) & pos) | ((0xCCCCCCCCu - t) & ~pos);
   }
   return make_uint2(q[0], q[1]);
 }
+// A lane's block (where `mine`; called by whole warps): put_scales(bytes of the three levels, 0 for one that it does not need), put(level, digit,
+// codes) for the digits of the others. more1, more2: the lanes whose blocks have a second, a third level. (The loops over the digits are not
+// unrolled: this code runs from a cold instruction cache while the weights stream, where a line takes a microsecond; all digits in line made
+// the steps 5 to 20 us longer.)
+template <class PutScales, class Put>
+__device__ __forceinline__ void nv_split_block(const uint32_t (&h)[8], bool mine, unsigned& more1, unsigned& more2, PutScales put_scales, Put put) {
+  uint32_t f[16];
+  const NvBlock k = nv_fixed16(h, f);
+  more1 = __ballot_sync(0xffffffffu, mine && (k.levels & 2u) != 0u);
+  more2 = __ballot_sync(0xffffffffu, mine && (k.levels & 4u) != 0u);
+  if (mine) put_scales(k.scale, (k.levels >> 1) & 1u, k.levels >> 2);
+  const int n = more2 != 0u ? 3 : more1 != 0u ? 2 : 1;   // (a third level has a second one in front)
+#pragma unroll 1
+  for (int level = 0; level < n; ++level) {
+    if (level == 1) nv_rest16(h, k.u, f);
+    const bool has = mine && ((k.levels >> level) & 1u) != 0u;
+#pragma unroll 1
+    for (int d = nv_digits(level) - 1; d >= 0; --d) {
+      const uint2 w = nv_next_digit(f, level == 0 && d == 0 ? 15u : 7u);
+      if (has) put(level, d, w);
+    }
+  }
+}
 
-// Where block `blk`'s stage begins in the image of a tile; in it the block's digit 0 and its scale for row `slot`.
-__device__ __forceinline__ uint8_t* nv_stage(uint8_t* img, int group, int width, int K, int blk) {
-  return img + (static_cast<size_t>(group) * (K / KS) + static_cast<size_t>(blk >> 4) * width) * NV_GROUP_BYTES;
-}
+// Where a row of a tile lies in a digit, a block's codes in its row, its scale in a level.
 __device__ __forceinline__ int nv_row_at(int slot) { return (slot >> 3) * 1024 + (slot & 7) * 128; }
-__device__ __forceinline__ int nv_digit_at(int slot, int blk) {
-  return nv_row_at(slot) + ((((blk & 15) >> 1) ^ (slot & 7)) * 16) + (blk & 1) * 8;
+__device__ __forceinline__ int nv_code_at(int slot, int blk) { return ((((blk & 15) >> 1) ^ (slot & 7)) * 16) + (blk & 1) * 8; }
+__device__ __forceinline__ int nv_digit_at(int width, int level, int d) { return width * (nv_level_at(level) + d * 1024); }
+__device__ __forceinline__ int nv_scale_at(int width, int level, int slot, int blk) {
+  return nv_digit_at(width, level, nv_digits(level)) + slot * 16 + (blk & 15);
 }
-__device__ __forceinline__ int nv_scale_at(int width, int slot, int blk) { return NV_PARTS * width * 1024 + slot * 16 + (blk & 15); }
 
 // Which accumulators the units take in turn: tiles of up to eight rows one or the other, wider ones both (as PairBuffers).
 struct NvBuffers {
@@ -309,10 +369,13 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
   // ---------------------------------------------------------------- set-up
   if (tid == 0) {
     MSK_TR(TR_START);
-    for (int i = 0; i < NV_W_STAGES; ++i) mbar_init(&ctl.w_full[i], 1);
+    for (int i = 0; i < NV_W_STAGES; ++i) {
+      mbar_init(&ctl.w_full[i], 1);
+      mbar_init(&ctl.w_done[i], 1);
+    }
     for (int i = 0; i < NV_S_STAGES; ++i) mbar_init(&ctl.s_full[i], 4);
     for (int i = 0; i < NV_MARKS; ++i) {
-      mbar_init(&ctl.b_full[i], 1);
+      mbar_init(&ctl.b_full[i], 2);
       mbar_init(&ctl.done[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -331,16 +394,14 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     tmem_alloc(&ctl.tmem_base, TMEM_COLS);
     tmem_relinquish();
   }
-  // The first token row (or its part) of this CTA, up to its largest value: it does not depend on the sort, and the launch before the sort
+  // The first token row (or its part) of this CTA, as F16 values: it does not depend on the sort, and the launch before the sort
   // has completed (the sort lets this launch begin only behind its own wait).
   constexpr int NT = NV_SPLIT_THREADS, NW = NT / 32, PER = (NV_MAX_BLOCKS + NT - 1) / NT;
   const int th = tid - NV_SPLIT_WARP * 32, nb = p.H / 16;
-  // up to 74 tokens several CTAs share a row: each reads all of it for its largest value and splits some of the K stages (not over
+  // up to 74 tokens several CTAs share a row: each reads all of it, as the norm needs, and splits some of the K stages (not over
   // PCIe, where every reader costs the bytes again: 8 rows in host memory, a whole step 121 us shared, 103 not, 119 by the other kernel)
   const int parts = p.share_rows ? max(1, min(n_ctas / p.T, p.H / KS)) : 1, items = p.T * parts;
   uint32_t h[PER][8];
-  float bm[PER];
-  int U = 0;
   auto fetch_row = [&](int t) {
     const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(t) * p.H);
 #pragma unroll
@@ -351,8 +412,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       h[i][4] = v1.x; h[i][5] = v1.y; h[i][6] = v1.z; h[i][7] = v1.w;
     }
   };
-  auto finish_row = [&]() {   // norm, F16 values, the row's exponent
-    const int sw = warp - NV_SPLIT_WARP;
+  auto finish_row = [&]() {   // norm, F16 values
     if (p.pre_w != nullptr) {   // x * rsqrt(mean(x^2) + eps) * (1 + pre_w), one BF16 rounding (copy_rows_kernel)
       float ss = 0.f;
 #pragma unroll
@@ -365,11 +425,11 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if (lane == 0) ctl.red[1][sw] = ss;
+      if (lane == 0) ctl.red[warp - NV_SPLIT_WARP] = ss;
       named_bar_sync(1, NT);
       float tot = 0.f;
 #pragma unroll
-      for (int i = 0; i < NW; ++i) tot += ctl.red[1][i];
+      for (int i = 0; i < NW; ++i) tot += ctl.red[i];
       const float rs = rsqrtf(tot / static_cast<float>(p.H) + p.pre_eps);
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
@@ -386,20 +446,11 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         }
       }
     }
-    float rm = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) h[i][j] = bf16x2_to_f16x2(h[i][j]);
-      bm[i] = nv_block_max(h[i]);
-      rm = fmaxf(rm, bm[i]);
     }
-    rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
-    if (lane == 0) ctl.red[0][sw] = rm;
-    named_bar_sync(1, NT);
-#pragma unroll
-    for (int i = 0; i < NW; ++i) rm = fmaxf(rm, ctl.red[0][i]);
-    U = nv_row_exp(rm);
   };
   if (warp >= NV_SPLIT_WARP && static_cast<int>(blockIdx.x) < items) {
     fetch_row(static_cast<int>(blockIdx.x) / parts);
@@ -481,7 +532,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     u.row0 = off_s[e] + ti * per;
     u.rows = min(per, c - ti * per);
     u.width = nv_width(u.rows);
-    u.group = group_start[e] + ti * NV_GROUPS;
+    u.group = group_start[e] + ti * (per >> 3);
   };
 
   if (warp >= NV_SPLIT_WARP) {
@@ -501,21 +552,18 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         const unsigned have = __ballot_sync(0xffffffffu, q >= 0);
         if (q >= 0) {
           const int e = id - p.lo, c = cnt_s[e], per = nv_tile_rows(c, nv_tiles(c)), r = q - off_s[e], ti = r / per, slot = r - ti * per;
-          const int group = group_start[e] + ti * NV_GROUPS, width = nv_width(min(per, c - ti * per));
+          const int group = group_start[e] + ti * (per >> 3), width = nv_width(min(per, c - ti * per));
           ctl.route[__popc(have & ((1u << th) - 1u))] =
-              make_uint4(static_cast<uint32_t>(group * (p.H / KS) * NV_GROUP_BYTES + nv_row_at(slot)), static_cast<uint32_t>(width),
-                         static_cast<uint32_t>(slot & 7), static_cast<uint32_t>(slot));
-          if (part == 0) p.rs[0][q] = nv_row_scale(U);
+              make_uint4(static_cast<uint32_t>(group * (p.H / KS) * NV_GROUP_BYTES), static_cast<uint32_t>(width),
+                         static_cast<uint32_t>(tile_start[e] + ti), static_cast<uint32_t>(slot));
         }
         if (th == 0) ctl.n_routes = __popc(have);
       }
       named_bar_sync(1, NT);
-      const int n_routes = ctl.n_routes, row_exp = U;
+      const int n_routes = ctl.n_routes;
       uint32_t g[PER][8];
-      float gm[PER];
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        gm[i] = bm[i];
 #pragma unroll
         for (int j = 0; j < 8; ++j) g[i][j] = h[i][j];
       }
@@ -526,24 +574,44 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       }
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        const int b = th + i * NT;
-        if (b >= nb || n_routes == 0 || (parts > 1 && (b >> 4) % parts != part)) continue;
-        uint32_t f[16];
-        const uint32_t sf = nv_fixed16(g[i], gm[i], row_exp, f), chunk = (b & 15) >> 1;
+        const int b = th + i * NT, stage = b >> 4;
+        const bool mine = b < nb && n_routes != 0 && (parts == 1 || stage % parts == part);
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        unsigned more[2];
+        auto at = [&](const uint4& to) { return p.img[0] + (to.x + to.y * static_cast<uint32_t>(stage * NV_GROUP_BYTES)); };
+        nv_split_block(g[i], mine, more[0], more[1],
+            [&](uint32_t s0, uint32_t s1, uint32_t s2) {
 #pragma unroll 1
-        for (int d = NV_PARTS - 1; d >= -1; --d) {   // digits, then the scale
-          const uint2 w = nv_next_digit(f);
+              for (int s = 0; s < n_routes; ++s) {
+                const uint4 to = ctl.route[s];
+                const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
+                uint8_t* img = at(to);
+                img[nv_scale_at(width, 0, slot, b)] = static_cast<uint8_t>(s0);
+                img[nv_scale_at(width, 1, slot, b)] = static_cast<uint8_t>(s1);
+                img[nv_scale_at(width, 2, slot, b)] = static_cast<uint8_t>(s2);
+              }
+            },
+            [&](int level, int d, uint2 w) {
 #pragma unroll 1
-          for (int s = 0; s < n_routes; ++s) {
-            const uint4 to = ctl.route[s];
-            uint8_t* row = p.img[0] + to.x + to.y * ((b >> 4) * NV_GROUP_BYTES);
-            if (d >= 0) *reinterpret_cast<uint2*>(row + to.y * (d * 1024) + (chunk ^ to.z) * 16 + (b & 1) * 8) = w;
-            else row[nv_scale_at(to.y, to.w, b) - nv_row_at(to.w)] = static_cast<uint8_t>(sf);
-          }
+              for (int s = 0; s < n_routes; ++s) {
+                const uint4 to = ctl.route[s];
+                const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
+                *reinterpret_cast<uint2*>(at(to) + nv_digit_at(width, level, d) + nv_row_at(slot) + nv_code_at(slot, b)) = w;
+              }
+            });
+        if (more[0] != 0u && lane < n_routes) {     // the warp's blocks are those of two stages
+          unsigned int* flags = p.tiles + ctl.route[lane].z * NV_TILE_WORDS + NV_MORE;
+          const int first = (th - lane + i * NT) >> 4;
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            if (more[m] != 0u) atomicOr(flags + m, ((more[m] & 0xFFFFu) != 0u ? 1u << first : 0u) | (more[m] >> 16 != 0u ? 2u << first : 0u));
         }
       }
       item = next;
-      if (item < items) finish_row();              // (with a barrier, behind which the routes' places may be written again)
+      if (item < items) {
+        finish_row();
+        named_bar_sync(1, NT);                     // the routes' places may be written again
+      }
     }
     named_bar_sync(1, NT);
     if (th == 0) {
@@ -557,11 +625,8 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     if (lane == 0) {
       const uint64_t pol = policy_evict_first();
       const int tiles = tile_start[p.nloc], n0 = tiles * p.n_pairs[0], n = n0 + tiles * p.n_pairs[1];
-      int x = static_cast<int>(blockIdx.x);         // the first unit, then what the counter gives
-      uint32_t st = 0;
-      bool ok = true;
-      for (uint32_t i = 0; ok; ++i) {
-        NvUnit u;
+      uint32_t st = 0;                              // K stages
+      auto publish = [&](NvUnit& u, uint32_t i, int x) -> bool {   // unit x becomes the i-th of this CTA
         u.phase = -1;
         if (x < n) {
           u.phase = x >= n0 ? 1 : 0;
@@ -571,17 +636,21 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
           set_tile(u, e, idx - u.pair * nt);
         }
         const uint32_t s = i % NV_UNITS;
-        if (!mbar_wait_inline(&ctl.u_empty[s], ((i / NV_UNITS) & 1u) ^ 1u, abortw)) break;
+        if (!mbar_wait_inline(&ctl.u_empty[s], ((i / NV_UNITS) & 1u) ^ 1u, abortw)) return false;
         *reinterpret_cast<int4*>(&ctl.unit[s]) = make_int4(u.phase, u.expert, u.row0, u.rows);
         *(reinterpret_cast<int4*>(&ctl.unit[s]) + 1) = make_int4(u.pair, u.tile, u.group, u.width);
         mbar_arrive(&ctl.u_full[s]);
-        if (u.phase < 0) break;
-        x = n_ctas + static_cast<int>(atomicAdd(p.ctr, 1u));   // the next one: its number is back long before this one's last stage
+        return true;
+      };
+      NvUnit u;
+      bool ok = publish(u, 0u, static_cast<int>(blockIdx.x));   // the first unit, then what the counter gives
+      for (uint32_t i = 0; ok && u.phase >= 0; ++i) {
+        const int x = n_ctas + static_cast<int>(atomicAdd(p.ctr, 1u));   // the next one: its number is back before the third stage
+        NvUnit next;
         const int nst = p.K[u.phase] / KS;
         const uint8_t* src = p.w[u.phase] + static_cast<size_t>(u.expert * p.n_pairs[u.phase] + u.pair) * nst * STAGE_W_BYTES;
         for (int ks = 0; ks < nst; ++ks, ++st) {
           const uint32_t ws = st % NV_W_STAGES;
-          const uint32_t before = st - NV_W_STAGES;   // the stage whose place this one takes
           if (st == NV_W_STAGES && i == 0u) {
             // While the token rows are split memory would stand still once the ring is full: the next stages go to L2, at the pace of memory
             // (all at once they held up the reading of the rows, 3 us) and until the first MMAs are done.
@@ -590,12 +659,16 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
               __nanosleep(700);
             }
           }
-          if (st >= NV_W_STAGES && !mbar_wait_inline(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
+          if (!mbar_wait_inline(&ctl.w_done[ws], ((st / NV_W_STAGES) & 1u) ^ 1u, abortw)) { ok = false; break; }
           mbar_arrive_expect_tx(&ctl.w_full[ws], STAGE_W_BYTES);
           bulk_g2s(w_ring + ws * STAGE_W_BYTES, src, STAGE_W_BYTES, &ctl.w_full[ws], pol);
           if (st == 0u) MSK_TR(TR_FIRST_BULK);
           src += STAGE_W_BYTES;
+          // The next unit is published early in this one: the word of its tile's levels and its first token rows are fetched meanwhile (published
+          // with its first weights it cost 8 tokens 1.5 us).
+          if (ks == min(2, nst - 1) && !publish(next, i + 1u, x)) { ok = false; break; }
         }
+        u = next;
       }
     }
   } else if (warp == 1) {
@@ -603,8 +676,8 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     const uint64_t a0 = smem_desc_kmajor_noswz(smem_u32(w_ring), 128, 2 * OCT_BYTES);
     const uint64_t b0 = smem_desc_kmajor_sw128(smem_u32(b_ring));
     NvBuffers db;
-    uint32_t st = 0, bs = 0;
-    bool ok = true, ready = false;               // ready: the next stage was seen complete
+    uint32_t st = 0, wst = 0, bs = 0;            // passes, K stages
+    bool ok = true, ready = false;               // ready: the next pass was seen complete
     NvUnit u;
     while (ok && wait_unit(u, mbar_wait_warp)) {
       __syncwarp();
@@ -613,20 +686,28 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       db.take(u.width);
       if (db.uses(0) && !mbar_wait_warp(&ctl.d_empty[0], db.p0 ^ 1u, abortw)) break;
       if (db.uses(1) && !mbar_wait_warp(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) break;
-      const uint32_t idesc = idesc_nvf4(static_cast<uint32_t>(NV_PARTS * 8 * u.width));
       const uint32_t d0 = tmem + db.col(), d1 = d0 + db.tile_cols();
       const int nst = p.K[u.phase] / KS;
-      for (int ks = 0; ks < nst; ++ks) {
-        const uint32_t ws = st % NV_W_STAGES, ss = st % NV_S_STAGES;
-        // the scales; the warps that write them have seen the stage's weights and token rows land
-        if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.s_full[ss], (st / NV_S_STAGES) & 1u, abortw)) { ok = false; break; }
-        tc_fence_after();
-        if (st == 0u && lane == 0) MSK_TR(TR_FIRST_MMA);
-        const uint32_t mark = st % NV_MARKS;
-        ++st;
-        ready = mma_nvf4_stage(d0, d1, a0 + ((ws * STAGE_W_BYTES) >> 4), b0 + ((bs * b_bytes) >> 4), idesc, tmem + C::S_BASE + ss * C::S_COLS,
-                               ks > 0 ? 1u : 0u, smem_u32(&ctl.done[mark]), smem_u32(&ctl.s_full[st % NV_S_STAGES]), (st / NV_S_STAGES) & 1u);
-        if (++bs == b_stages) bs = 0;
+      uint32_t accumulate = 0u;
+      for (int ks = 0; ok && ks < nst; ++ks, ++wst) {
+        const uint32_t ws = wst % NV_W_STAGES;
+        for (uint32_t last = 0u; last == 0u;) {     // the stage's levels
+          const uint32_t ss = st % NV_S_STAGES;
+          // the scales; the warps that write them have seen the stage's weights and token rows land
+          if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.s_full[ss], (st / NV_S_STAGES) & 1u, abortw)) { ok = false; break; }
+          tc_fence_after();
+          if (st == 0u && lane == 0) MSK_TR(TR_FIRST_MMA);
+          const int pass = ctl.b_pass[bs], level = pass & 3;
+          last = static_cast<uint32_t>(pass & NV_LAST);
+          const uint32_t mark = st % NV_MARKS, rows = static_cast<uint32_t>(8 * u.width), first = static_cast<uint32_t>(nv_first(level)) * rows;
+          ++st;
+          ready = mma_nvf4_stage(d0 + first, d1 + first, a0 + ((ws * STAGE_W_BYTES) >> 4), b0 + ((bs * b_bytes) >> 4),
+                                 idesc_nvf4(static_cast<uint32_t>(nv_digits(level)) * rows), tmem + C::S_BASE + (wst % NV_S_STAGES) * C::S_COLS,
+                                 tmem + C::S_B + ss * C::S_COLS, accumulate,
+                                 smem_u32(&ctl.done[mark]), smem_u32(&ctl.w_done[ws]), last, smem_u32(&ctl.s_full[st % NV_S_STAGES]), (st / NV_S_STAGES) & 1u);
+          accumulate = 1u;
+          if (++bs == b_stages) bs = 0;
+        }
       }
       if (ok && elect_one()) {
         if (db.uses(0)) tc_commit(&ctl.d_full[0]);
@@ -650,31 +731,46 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
           fence_proxy_async_all();                 // ordinary stores of other SMs, about to be read by bulk copies
           split = true;
         }
+        unsigned int* tile = p.tiles + u.tile * NV_TILE_WORDS;
         if (u.phase == 1) {
-          unsigned int* tile = p.tiles + u.tile * NV_TILE_WORDS;
           if (u.tile != last_tile) {
             if (!grid_counter_wait(tile + NV_READY, static_cast<unsigned>(u.width * (p.I / KS)), abortw)) break;
             fence_proxy_async_all();
             last_tile = u.tile;
           }
-          // the last down unit of the tile to have seen it complete puts its counters back for the next launch
+        }
+        const int nst = p.K[u.phase] / KS;
+        const uint8_t* src = p.img[u.phase] + static_cast<size_t>(u.group) * nst * NV_GROUP_BYTES;
+        const unsigned int* flags = tile + (u.phase == 0 ? NV_MORE : NV_MORE_INTER);
+        unsigned int more1 = 0u, more2 = 0u;
+        for (int ks = 0; ok && ks < nst; ++ks, more1 >>= 1, more2 >>= 1, src += u.width * NV_GROUP_BYTES) {
+          if ((ks & 31) == 0) {
+            more1 = __ldcg(flags + ks / 16);
+            more2 = __ldcg(flags + ks / 16 + 1);
+          }
+          for (int level = 0; level < NV_LEVELS; ++level) {
+            if ((level == 1 && (more1 & 1u) == 0u) || (level == 2 && (more2 & 1u) == 0u)) continue;
+            const uint32_t before = st - b_stages;
+            if (st >= b_stages && !mbar_wait_inline(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
+            const uint32_t bytes = static_cast<uint32_t>(u.width * (nv_digits(level) * 1024 + 128));
+            mbar_arrive_expect_tx(&ctl.b_full[bs], bytes);
+            bulk_g2s(b_ring + bs * b_bytes, src + u.width * nv_level_at(level), bytes, &ctl.b_full[bs], keep);
+            const bool last = level == 2 || ((level == 1 || (more1 & 1u) == 0u) && (more2 & 1u) == 0u);
+            ctl.b_pass[bs] = level | (last ? NV_LAST : 0);
+            mbar_arrive(&ctl.b_full[bs]);
+            ++st;
+            if (++bs == b_stages) bs = 0;
+          }
+        }
+        if (ok && u.phase == 1) {
+          // the last down unit of the tile to have fetched its rows puts its counters back for the next launch
           const unsigned seen = atomicAdd(tile + NV_SEEN, 1u);
           if (seen == static_cast<unsigned>(p.n_pairs[1]) - 1u) {
             atomicExch(tile + NV_DONE, 0u);
             atomicExch(tile + NV_READY, 0u);
             atomicExch(tile + NV_SEEN, 0u);
+            for (int i = NV_MORE; i < NV_MORE_INTER + 2 * ((nst + 31) / 32); ++i) atomicExch(tile + i, 0u);
           }
-        }
-        const int nst = p.K[u.phase] / KS;
-        const uint32_t bytes = static_cast<uint32_t>(u.width * NV_GROUP_BYTES);
-        const uint8_t* src = p.img[u.phase] + static_cast<size_t>(u.group) * nst * NV_GROUP_BYTES;
-        for (int ks = 0; ks < nst; ++ks, ++st) {
-          const uint32_t before = st - b_stages;
-          if (st >= b_stages && !mbar_wait_inline(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
-          mbar_arrive_expect_tx(&ctl.b_full[bs], bytes);
-          bulk_g2s(b_ring + bs * b_bytes, src, bytes, &ctl.b_full[bs], keep);
-          src += bytes;
-          if (++bs == b_stages) bs = 0;
         }
       }
     }
@@ -695,7 +791,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
   } else if (warp >= 4 && warp < 8) {
     // ------------------------------------------------------------------ scales
     const uint32_t quarter = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    uint32_t st = 0, bs = 0, bpar = 0;
+    uint32_t st = 0, wst = 0, bs = 0, bpar = 0;   // passes, K stages
     bool ok = true;
     NvUnit u;
     while (ok && wait_unit(u, mbar_wait_warp)) {
@@ -703,14 +799,12 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       if (lane == 0) done_unit();
       if (u.phase < 0) break;
       const int nst = p.K[u.phase] / KS;
-      // This lane's token rows: column c of a stage's scales is that of the MMA's columns 32 c + lane, digit after digit of the tile's
-      // rows. With one or two groups of eight all columns are alike, with three they repeat after three.
-      const uint32_t b_off = static_cast<uint32_t>(NV_PARTS * 1024 * u.width), n_row = static_cast<uint32_t>(8 * u.width);
-      const uint32_t row0 = (lane % n_row) * 16u, row1 = ((lane + 32u) % n_row) * 16u, row2 = ((lane + 64u) % n_row) * 16u;
-      const bool three = u.width == 3;
-      for (int ks = 0; ks < nst; ++ks, ++st) {
-        const uint32_t ws = st % NV_W_STAGES, ss = st % NV_S_STAGES;
-        if (!mbar_wait_warp(&ctl.w_full[ws], (st / NV_W_STAGES) & 1u, abortw)) { ok = false; break; }
+      // This lane's token row: column c of a stage's scales is that of the MMA's columns 32 c + lane, digit after digit of the tile's
+      // rows: with one or two groups of eight all columns are alike.
+      const uint32_t row_at = (lane % static_cast<uint32_t>(8 * u.width)) * 16u;
+      for (int ks = 0; ok && ks < nst; ++ks, ++wst) {
+        const uint32_t ws = wst % NV_W_STAGES;
+        if (!mbar_wait_warp(&ctl.w_full[ws], (wst / NV_W_STAGES) & 1u, abortw)) { ok = false; break; }
         uint8_t* stage = w_ring + ws * STAGE_W_BYTES;
         uint32_t r[2][16], neg = 0u;   // [tile][64 K x row quarter]: the scales of row 32 c + lane
 #pragma unroll
@@ -742,29 +836,32 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
           }
           fence_proxy_async_smem();
         }
-        if (!mbar_wait_warp(&ctl.b_full[bs], bpar, abortw)) { ok = false; break; }
-        const uint8_t* sc = b_ring + bs * b_bytes + b_off;
-        const uint4 v = *reinterpret_cast<const uint4*>(sc + row0);
-        uint4 v1 = v, v2 = v;
-        if (three) {
-          v1 = *reinterpret_cast<const uint4*>(sc + row1);
-          v2 = *reinterpret_cast<const uint4*>(sc + row2);
+        for (bool last = false; !last; ++st) {     // the stage's levels, each beside the same weights
+          const uint32_t ss = st % NV_S_STAGES;
+          if (!mbar_wait_warp(&ctl.b_full[bs], bpar, abortw)) { ok = false; break; }
+          const int pass = ctl.b_pass[bs];
+          last = (pass & NV_LAST) != 0;
+          const uint8_t* sc = b_ring + bs * b_bytes + nv_digits(pass & 3) * 1024 * u.width;
+          const uint4 v = *reinterpret_cast<const uint4*>(sc + row_at);
+          const uint32_t before = st - NV_S_STAGES;
+          if (st >= NV_S_STAGES && !mbar_wait_warp(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
+          tc_fence_after();
+          if ((pass & 3) == 0) {                   // (the passes of the stage before last are done too: the weights' place is free)
+            const uint32_t at = tmem + quarter + C::S_BASE + (wst % NV_S_STAGES) * C::S_COLS;
+            tmem_st16(at, r[0]);
+            tmem_st16(at + 16, r[1]);
+          }
+          const uint32_t lo[16] = {v.x, v.x, v.x, v.x, v.x, v.x, v.x, v.x, v.y, v.y, v.y, v.y, v.y, v.y, v.y, v.y};
+          const uint32_t hi[16] = {v.z, v.z, v.z, v.z, v.z, v.z, v.z, v.z, v.w, v.w, v.w, v.w, v.w, v.w, v.w, v.w};
+          const uint32_t at_b = tmem + quarter + C::S_B + ss * C::S_COLS;
+          tmem_st16(at_b, lo);
+          tmem_st16(at_b + 16, hi);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.s_full[ss]);
+          if (++bs == b_stages) { bs = 0; bpar ^= 1u; }
         }
-        const uint32_t before = st - NV_S_STAGES;
-        if (st >= NV_S_STAGES && !mbar_wait_warp(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t at = tmem + quarter + C::S_BASE + ss * C::S_COLS;
-        tmem_st16(at, r[0]);
-        tmem_st16(at + 16, r[1]);
-        const uint32_t lo[16] = {v.x, v1.x, v2.x, v.x, v1.x, v2.x, v.x, v1.x, v.y, v1.y, v2.y, v.y, v1.y, v2.y, v.y, v1.y};
-        const uint32_t hi[16] = {v.z, v1.z, v2.z, v.z, v1.z, v2.z, v.z, v1.z, v.w, v1.w, v2.w, v.w, v1.w, v2.w, v.w, v1.w};
-        tmem_st16(at + C::S_B, lo);
-        tmem_st16(at + C::S_B + 16, hi);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.s_full[ss]);
-        if (++bs == b_stages) { bs = 0; bpar ^= 1u; }
       }
     }
   } else if (warp >= 8 && warp < 12) {
@@ -781,7 +878,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       if (lane == 0) done_unit();
       if (u.phase < 0) break;
       db.take(u.width);
-      const float gsc = p.gs[u.phase][u.expert];
+      const float gsc = p.gs[u.phase][u.expert] * NV_SUM_SCALE;
       const int col = u.phase == 0 ? u.pair * 128 + row : 2 * u.pair * 128 + row;
       float o0 = gsc, o1 = gsc;
       if (u.phase == 1 && p.post_norm_w != nullptr) {
@@ -793,11 +890,10 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       tc_fence_after();
       if (leader) { if (n_unit == 0u) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); }
       const uint32_t d0 = tmem + quarter + db.col(), d1 = d0 + db.tile_cols();
-      const float my_rs = lane < u.rows ? __ldcg(p.rs[u.phase] + u.row0 + lane) : 0.f;   // lane r: row r's power of two
 #pragma unroll 1
       for (int c0 = 0; c0 < u.rows; c0 += 8) {
         const int left = u.rows - c0;
-        float rs[8], a0[8], a1[8];
+        float a0[8], a1[8];
         {
           uint32_t v[NV_PARTS][8];
 #pragma unroll
@@ -827,34 +923,18 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
             for (int q = NV_PARTS - 2; q >= 0; --q) a1[j] = fmaf(a1[j], 0.125f, __uint_as_float(v[q][j]));
           }
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) rs[j] = __shfl_sync(0xffffffffu, my_rs, c0 + j);
         if (u.phase == 0) {
           __half* out = p.inter + static_cast<size_t>(u.row0 + c0) * p.I + col;
-          __half2 most[4];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float f = gsc * rs[j];
-            const __half v = inter_value(silu_f(a0[j] * f) * (a1[j] * f));
-            if (j < left) out[static_cast<size_t>(j) * p.I] = v;
-            if (j & 1) most[j >> 1].y = __habs(v); else most[j >> 1].x = __habs(v);
-          }
-          // (a place for every warp's 32 columns: atomic maxima of the rows, from all CTAs in a few cache lines, took 10 us a round of units)
-#pragma unroll
-          for (int b = 16; b > 0; b >>= 1) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) most[j] = __hmax2(most[j], __shfl_xor_sync(0xffffffffu, most[j], b));
-          }
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (lane == j && j < left) p.part_max[static_cast<size_t>(u.row0 + c0 + j) * (p.I / 32) + 4 * u.pair + (warp & 3)] = j & 1 ? most[j >> 1].y : most[j >> 1].x;
+            if (j < left) out[static_cast<size_t>(j) * p.I] = inter_value(silu_f(a0[j] * gsc) * (a1[j] * gsc));
         } else {
           float* out = p.y + static_cast<size_t>(u.row0 + c0) * p.H + col;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             if (j < left) {
-              out[static_cast<size_t>(j) * p.H] = a0[j] * (o0 * rs[j]);
-              out[static_cast<size_t>(j) * p.H + 128] = a1[j] * (o1 * rs[j]);
+              out[static_cast<size_t>(j) * p.H] = a0[j] * o0;
+              out[static_cast<size_t>(j) * p.H + 128] = a1[j] * o1;
             }
           }
         }
@@ -877,52 +957,41 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         if (group_start[mid] <= group) lo = mid; else hi = mid;
       }
       NvUnit u;
-      set_tile(u, lo, (group - group_start[lo]) / NV_GROUPS);   // (an expert with one tile has at most three groups, others three a tile)
+      const int at_row = (group - group_start[lo]) * 8;
+      set_tile(u, lo, at_row / nv_tile_rows(cnt_s[lo], nv_tiles(cnt_s[lo])));
       const int first = (group - u.group) * 8;     // row of the tile
-      if (first >= u.width * 8) continue;          // room behind an expert's last tile
       const bool go = lane != 0 || nv_tile_wait(p.tiles + u.tile * NV_TILE_WORDS + NV_DONE, static_cast<unsigned>(p.n_pairs[0]), abortw);
       if (!__all_sync(0xffffffffu, go)) break;
       __syncwarp();   // the vote orders no memory: the other lanes read rows that lane 0 has acquired
-      if (first < u.rows) {
-        uint4 v0, v1, m;
-        auto load = [&](int slot) {   // stored by other SMs: from L2
-          const int r = u.row0 + min(slot, u.rows - 1);
-          const uint4* src = reinterpret_cast<const uint4*>(p.inter + static_cast<size_t>(r) * p.I + blk * 16);
-          v0 = __ldcg(src);
-          v1 = __ldcg(src + 1);
-          const uint4* mp = reinterpret_cast<const uint4*>(p.part_max + static_cast<size_t>(r) * (p.I / 32));
-          m = make_uint4(0u, 0u, 0u, 0u);
-          if ((lane & 15) < p.I / 256) m = __ldcg(mp + (lane & 15));
+      uint4 v0, v1;
+      auto load = [&](int slot) {   // stored by other SMs: from L2
+        const uint4* src = reinterpret_cast<const uint4*>(p.inter + static_cast<size_t>(u.row0 + min(slot, u.rows - 1)) * p.I + blk * 16);
+        v0 = __ldcg(src);
+        v1 = __ldcg(src + 1);
+      };
+      const int last = min(first + 8, u.rows);
+      unsigned any1 = 0u, any2 = 0u;
+      uint8_t* stage = p.img[1] + (static_cast<size_t>(u.group) * pieces + static_cast<size_t>(blk >> 4) * u.width) * NV_GROUP_BYTES;
+      load(first + (lane >> 4));
 #pragma unroll 1
-          for (int c = (lane & 15) + 16; c < p.I / 256; c += 16) {
-            const uint4 x = __ldcg(mp + c);
-            m = make_uint4(__vmaxu2(m.x, x.x), __vmaxu2(m.y, x.y), __vmaxu2(m.z, x.z), __vmaxu2(m.w, x.w));   // magnitudes compare as their bits
-          }
-        };
-        const int last = min(first + 8, u.rows);
-        load(first + (lane >> 4));
-#pragma unroll 1
-        for (int r0 = first; r0 < last; r0 += 2) {
-          const int slot = r0 + (lane >> 4);
-          const uint32_t h8[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-          uint32_t mm = __vmaxu2(__vmaxu2(m.x, m.y), __vmaxu2(m.z, m.w));
-          mm = max(mm & 0xFFFFu, mm >> 16);
-          load(slot + 2);                            // the next two rows, while these are split
-#pragma unroll
-          for (int o = 8; o > 0; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-          const int U = nv_row_exp(__half2float(__ushort_as_half(static_cast<unsigned short>(mm))));
-          uint32_t f[16];
-          const uint32_t sf = nv_fixed16(h8, nv_block_max(h8), U, f);
-          if (slot < last) {
-            if (blk == 0) p.rs[1][u.row0 + slot] = nv_row_scale(U);
-            uint8_t* stage = nv_stage(p.img[1], u.group, u.width, p.I, blk);
-            uint8_t* at = stage + nv_digit_at(slot, blk);
-#pragma unroll 1
-            for (int d = NV_PARTS - 1; d >= 0; --d) *reinterpret_cast<uint2*>(at + d * u.width * 1024) = nv_next_digit(f);
-            stage[nv_scale_at(u.width, slot, blk)] = static_cast<uint8_t>(sf);
-          }
-        }
+      for (int r0 = first; r0 < last; r0 += 2) {
+        const int slot = r0 + (lane >> 4);
+        const uint32_t h8[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        load(slot + 2);                            // the next two rows, while these are split
+        unsigned more1, more2;
+        uint8_t* at = stage + nv_row_at(slot) + nv_code_at(slot, blk);
+        nv_split_block(h8, slot < last, more1, more2,
+            [&](uint32_t s0, uint32_t s1, uint32_t s2) {
+              stage[nv_scale_at(u.width, 0, slot, blk)] = static_cast<uint8_t>(s0);
+              stage[nv_scale_at(u.width, 1, slot, blk)] = static_cast<uint8_t>(s1);
+              stage[nv_scale_at(u.width, 2, slot, blk)] = static_cast<uint8_t>(s2);
+            },
+            [&](int level, int d, uint2 w) { *reinterpret_cast<uint2*>(at + nv_digit_at(u.width, level, d)) = w; });
+        any1 |= more1;
+        any2 |= more2;
       }
+      if (any1 != 0u && lane < 2 && (lane == 0 || any2 != 0u))
+        atomicOr(p.tiles + u.tile * NV_TILE_WORDS + NV_MORE_INTER + (blk >> 9) * 2 + lane, 1u << ((blk >> 4) & 31));
       __syncwarp();
       if (lane == 0) red_release_add(p.tiles + u.tile * NV_TILE_WORDS + NV_READY, 1u);   // (its readers put the fence between their acquire and their bulk copies)
     }

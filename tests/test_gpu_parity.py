@@ -1319,6 +1319,7 @@ def _ids_of_counts(counts, lo, k, dev):
 @pytest.mark.parametrize("H,I,counts,ctas,pre,post", [
     (256, 1536, [1, 8, 9, 16, 17, 24], 0, False, False),       # tiles of every width, one K stage: a unit shorter than any ring
     (768, 1536, [25, 0, 49, 5, 48, 1], 0, True, True),         # two and three tiles an expert, the last ones narrower
+    (1024, 1536, [32, 33, 15, 48, 49, 64], 0, False, False),   # whole tiles, tiles with one row behind them
     (2304, 1792, [31, 24, 2, 0, 0, 7], 37, False, True),       # odd numbers of stages, fewer CTAs than rows
     (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
     (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
@@ -1353,8 +1354,8 @@ def test_nvf4_kernel_at_tile_edges(cuda_dev, H, I, counts, ctas, pre, post):
 @pytest.mark.parametrize("scale", [1.0, 3.0e-3])
 def test_nvf4_kernel_is_no_further_from_64_bits_than_the_f16_kernel(cuda_dev, scale):
     """Both GEMMs on their own: inter against 64 bits from the same token rows (its rounding to BF16, 1.6e-3 and 2.8e-3, hides all
-    else), y against 64 bits from each kernel's own inter: seven digits hold an element to 2^-21 of the largest of sixteen, FP32 sums
-    lose what they lose in the F16 kernel."""
+    else), y against 64 bits from each kernel's own inter: the digits hold every element, FP32 sums of a digit each lose less than those of the
+    F16 kernel."""
     m, inputs, _lib, orc = _mods()
     H, I, E, k, T = 4096, 1536, 8, 2, 48
     w = inputs.make_weights(H, I, E, 17, cuda_dev)
@@ -1380,6 +1381,93 @@ def test_nvf4_kernel_is_no_further_from_64_bits_than_the_f16_kernel(cuda_dev, sc
     assert err[0][0] <= err[16][0] * 1.001 and err[0][0] <= 4.0e-3, err
     assert err[0][1] <= err[16][1] and err[0][1] <= 2.0e-6, err
     print(err)
+
+
+def _wide_rows(T, H, g, dev):
+    """Token rows with BF16 values from 2^-24 to the end of the F16 range side by side, three kinds in turn: any magnitudes, one
+    magnitude in every block of sixteen far above the others (the largest on either side of a power of two), normal values."""
+    mant = 1.0 + torch.randint(0, 128, (T, H), generator=g, device=dev) / 128.0
+    x = mant * torch.exp2(torch.randint(-24, 16, (T, H), generator=g, device=dev).float())
+    top = torch.tensor([1.0, 1.6953125, 1.703125, 1.7109375, 1.9921875], device=dev)[torch.randint(0, 5, (T, H // 16), generator=g, device=dev)]
+    top = top * torch.exp2(torch.randint(-6, 16, (T, H // 16), generator=g, device=dev).float())
+    low = top[:, :, None] * torch.exp2(-torch.randint(9, 26, (T, H // 16, 16), generator=g, device=dev).float()) * mant.view(T, H // 16, 16)
+    low[:, :, 5] = top
+    x[1::3] = low.view(T, H)[1::3]
+    x[2::3] = torch.randn((T, H), generator=g, device=dev)[2::3].abs()
+    return (x * (torch.randint(0, 2, (T, H), generator=g, device=dev) * 2 - 1)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("tile", [0, 16])
+def test_activations_enter_the_gemms_exactly(cuda_dev, tile):
+    """Experts that hand their row through: gate x[0] = 32, up x[i] / 32, so inter = x, and y = inter. Whatever lies beside an element
+    in its row, what comes out is its F16 value, bit for bit, by the FP4 kernel as by the F16 one."""
+    m, inputs, _lib, orc = _mods()
+    H, E, k, T = 1536, 8, 1, 90
+    eye = torch.zeros((H, H), dtype=torch.uint8, device=cuda_dev)
+    eye.fill_diagonal_(2)                                         # E2M1 code of 1
+    gate = torch.zeros_like(eye)
+    gate[:, 0] = 2
+    pack = lambda c: (c[:, 0::2] | (c[:, 1::2] << 4)).expand(E, -1, -1).contiguous()  # noqa: E731
+    sf13 = torch.full((E, 2 * H, H // 16), 0x38, dtype=torch.uint8, device=cuda_dev)      # 1
+    sf13[:, H:] = 0x10                                            # 2^-5
+    one = torch.ones(E, device=cuda_dev)
+    w = {"w13": pack(torch.cat([gate, eye])), "w13_sf": sf13, "w13_gs": one, "w2": pack(eye),
+         "w2_sf": torch.full((E, H, H // 16), 0x38, dtype=torch.uint8, device=cuda_dev), "w2_gs": one}
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+    assert _nvf4_takes(st, T) == (tile == 0)
+    g = torch.Generator(device=cuda_dev).manual_seed(31)
+    x = _wide_rows(T, H, g, cuda_dev)
+    x[:, 0] = 32.0
+    d = {"hidden_states": x, "topk_ids": _ids_of_counts([24, 1, 0, 33, 8, 17, 0, 7], 0, k, cuda_dev),
+         "topk_weights": torch.ones((T, k), device=cuda_dev)}
+    for _ in range(2):
+        m.kernel_fn(d, st)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    v = m.workspace_views(st, T)
+    want = x.half()[v["perm"].long()]
+    assert torch.equal(v["inter"], want)
+    assert torch.equal(v["y"], want.float())
+
+
+@pytest.mark.parametrize("large", [1000.0, 20000.0])
+def test_nvf4_kernel_beside_large_channels_that_the_weights_ignore(cuda_dev, large):
+    """Every sixteenth channel large, in the token rows and in inter, the others orders below, and weights of zero
+    for the large ones: sums against 64 bits, no further off than the F16 kernel's."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, T = 4096, 1536, 8, 2, 48
+    w = inputs.make_weights(H, I, E, 17, cuda_dev)
+    w["w13"].view(torch.uint8)[:, :, 2::8] &= 0xF0                # codes of channels 4, 20, 36 ...
+    w["w2"].view(torch.uint8)[:, :, 2::8] &= 0xF0
+    sf = w["w13_sf"].view(torch.uint8)
+    small = torch.arange(I, device=cuda_dev) % 16 != 4            # gate and up rows of the other channels: 2^-4
+    sf[:, small.repeat(2)] = (sf[:, small.repeat(2)].int() - 0x20).clamp(min=1).to(torch.uint8)
+    w["w13_gs"] *= 16.0
+    g = torch.Generator(device=cuda_dev).manual_seed(5)
+    x = torch.randn((T, H), generator=g, device=cuda_dev)
+    x[:, 4::16] *= large
+    d = {"hidden_states": x.to(torch.bfloat16), "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
+    x = d["hidden_states"].float().clamp(-65504.0, 65504.0).half().double()
+    err, spread = {}, 0.0
+    for tile in (0, 16):
+        st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, token_tile=tile)
+        assert _nvf4_takes(st, T) == (tile == 0)
+        m.kernel_fn(d, st)
+        torch.cuda.synchronize()
+        v = m.workspace_views(st, T)
+        dq13, dq2 = m.dequant_packed(st)
+        off, perm = v["off"].tolist(), v["perm"].long() // k
+        i64, y64 = torch.empty((T * k, I), dtype=torch.float64, device=cuda_dev), torch.empty((T * k, H), dtype=torch.float64, device=cuda_dev)
+        for e in range(E):
+            r = slice(off[e], off[e + 1])
+            gu = x[perm[r]] @ dq13[e].double().T * w["w13_gs"][e].double()
+            i64[r] = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+            y64[r] = v["inter"][r].double() @ dq2[e].double().T * w["w2_gs"][e].double()
+        spread = float(v["inter"][:, ~small].double().norm() / v["inter"][:, small].double().norm())
+        err[tile] = [float((a.double() - b).norm() / b.norm()) for a, b in ((v["inter"][:, small], i64[:, small]), (v["y"], y64))]
+    assert spread > 50.0, (spread, err)
+    assert err[0][0] <= err[16][0] * 1.001 and err[0][0] <= 4.0e-3, err
+    assert err[0][1] <= err[16][1] and err[0][1] <= 2.0e-6, err
 
 
 def test_nvf4_kernel_with_negative_and_nan_scales_and_tokens_out_of_range(cuda_dev):
