@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     if (lane == 0) {
       tile_start[p.nloc] = tiles;
       group_start[p.nloc] = groups;
-      ctl.b_bytes = nv_place_bytes(nv_width(min(most, NV_ROWS)));
+      ctl.b_bytes = nv_place_bytes(nv_width(max(1, min(most, NV_ROWS))));   // (no tile at all: places that nobody uses)
       ctl.b_stages = min(NV_MARKS, C::B_RING / ctl.b_bytes);
     }
   }

@@ -1383,6 +1383,25 @@ def test_nvf4_kernel_is_no_further_from_64_bits_than_the_f16_kernel(cuda_dev, sc
     print(err)
 
 
+def test_nvf4_kernel_without_a_local_route(cuda_dev):
+    """A rank's step none of whose tokens go to its experts: zeros, a clean status and a state whose next step gives the clean bits."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, lo, n, T = 768, 1536, 64, 2, 7, 3, 40
+    w = inputs.make_weights(H, I, n, 33, cuda_dev)
+    st = m.prepare(w, local_start=lo, n_experts=E, top_k=k, max_tokens=T)
+    assert _nvf4_takes(st, T)
+    g = torch.Generator(device=cuda_dev).manual_seed(2)
+    d = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+         "topk_ids": _ids_of_counts([20, 0, 20], lo, k, cuda_dev), "topk_weights": torch.rand((T, k), generator=g, device=cuda_dev)}
+    clean = m.kernel_fn(d, st).clone()
+    away = torch.full((T, k), -1, dtype=torch.int32, device=cuda_dev)
+    away[::2] = lo + n
+    none = m.kernel_fn(dict(d, topk_ids=away), st)
+    assert not bool(none.any()) and torch.equal(m.kernel_fn(d, st), clean)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+
+
 def _wide_rows(T, H, g, dev):
     """Token rows with BF16 values from 2^-24 to the end of the F16 range side by side, three kinds in turn: any magnitudes, one
     magnitude in every block of sixteen far above the others (the largest on either side of a power of two), normal values."""
