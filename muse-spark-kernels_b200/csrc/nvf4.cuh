@@ -283,26 +283,33 @@ __device__ __forceinline__ uint2 nv_next_digit(uint32_t (&f)[16], uint32_t mask)
   }
   return make_uint2(q[0], q[1]);
 }
-// A lane's block (where `mine`; called by whole warps): put_scales(bytes of the three levels, 0 for one that it does not need), put(level, digit,
-// codes) for the digits of the others. more1, more2: the lanes whose blocks have a second, a third level. (The loops over the digits are not
-// unrolled: this code runs from a cold instruction cache while the weights stream, where a line takes a microsecond; all digits in line made
-// the steps 5 to 20 us longer.)
+// A lane's block (where `mine`; called by whole warps): put(0, digit, codes) for `n` digits of the first level, the last of them `to` - 1, and where
+// `rest` put_scales(bytes of the three levels, 0 for one that it does not need) and put(level, digit, codes) for the others. more1, more2: the
+// lanes whose blocks have a second, a third level. (The loops over the digits are not unrolled: this code runs from a cold instruction cache
+// while the weights stream, where a line takes a microsecond; all digits in line made the steps 5 to 20 us longer.)
 template <class PutScales, class Put>
-__device__ __forceinline__ void nv_split_block(const uint32_t (&h)[8], bool mine, unsigned& more1, unsigned& more2, PutScales put_scales, Put put) {
+__device__ __forceinline__ void nv_split_block(const uint32_t (&h)[8], bool mine, int n, int to, bool rest, unsigned& more1, unsigned& more2,
+                                               PutScales put_scales, Put put) {
   uint32_t f[16];
   const NvBlock k = nv_fixed16(h, f);
-  more1 = __ballot_sync(0xffffffffu, mine && (k.levels & 2u) != 0u);
-  more2 = __ballot_sync(0xffffffffu, mine && (k.levels & 4u) != 0u);
-  if (mine) put_scales(k.scale, (k.levels >> 1) & 1u, k.levels >> 2);
-  const int n = more2 != 0u ? 3 : more1 != 0u ? 2 : 1;   // (a third level has a second one in front)
+#pragma unroll
+  for (int i = 0; i < 16; ++i) f[i] >>= 3 * (NV_PARTS - to);
+  more1 = __ballot_sync(0xffffffffu, mine && rest && (k.levels & 2u) != 0u);
+  more2 = __ballot_sync(0xffffffffu, mine && rest && (k.levels & 4u) != 0u);
+  if (mine && rest) put_scales(k.scale, (k.levels >> 1) & 1u, k.levels >> 2);
+  const int levels = more2 != 0u ? 3 : more1 != 0u ? 2 : 1;   // (a third level has a second one in front)
 #pragma unroll 1
-  for (int level = 0; level < n; ++level) {
-    if (level == 1) nv_rest16(h, k.u, f);
+  for (int level = 0; level < levels; ++level) {
+    if (level > 0) {
+      n = to = nv_digits(level);
+      mine = mine && rest;
+      if (level == 1) nv_rest16(h, k.u, f);
+    }
     const bool has = mine && ((k.levels >> level) & 1u) != 0u;
 #pragma unroll 1
-    for (int d = nv_digits(level) - 1; d >= 0; --d) {
-      const uint2 w = nv_next_digit(f, level == 0 && d == 0 ? 15u : 7u);
-      if (has) put(level, d, w);
+    for (int i = 1; i <= n; ++i) {
+      const uint2 w = nv_next_digit(f, level == 0 && i == to ? 15u : 7u);
+      if (has) put(level, to - i, w);
     }
   }
 }
@@ -396,12 +403,13 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
   }
   // The first token row (or its part) of this CTA, as F16 values: it does not depend on the sort, and the launch before the sort
   // has completed (the sort lets this launch begin only behind its own wait).
-  constexpr int NT = NV_SPLIT_THREADS, NW = NT / 32, PER = (NV_MAX_BLOCKS + NT - 1) / NT;
+  constexpr int NT = NV_SPLIT_THREADS, NW = NT / 32, HALVES = NT / 16, PER = (NV_MAX_BLOCKS + NT - 1) / NT;
   const int th = tid - NV_SPLIT_WARP * 32, nb = p.H / 16;
   // up to 74 tokens several CTAs share a row: each reads all of it, as the norm needs, and splits some of the K stages (not over
   // PCIe, where every reader costs the bytes again: 8 rows in host memory, a whole step 121 us shared, 103 not, 119 by the other kernel)
   const int parts = p.share_rows ? max(1, min(n_ctas / p.T, p.H / KS)) : 1, items = p.T * parts;
   uint32_t h[PER][8];
+  uint4* row_s = reinterpret_cast<uint4*>(b_ring);   // the row's F16 values, while no token row is fetched yet
   auto fetch_row = [&](int t) {
     const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(t) * p.H);
 #pragma unroll
@@ -448,8 +456,13 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     }
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
+      const int b = th + i * NT;
 #pragma unroll
       for (int j = 0; j < 8; ++j) h[i][j] = bf16x2_to_f16x2(h[i][j]);
+      if (b < nb) {
+        row_s[2 * b] = make_uint4(h[i][0], h[i][1], h[i][2], h[i][3]);
+        row_s[2 * b + 1] = make_uint4(h[i][4], h[i][5], h[i][6], h[i][7]);
+      }
     }
   };
   if (warp >= NV_SPLIT_WARP && static_cast<int>(blockIdx.x) < items) {
@@ -458,6 +471,14 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
   }
   pdl_wait();
   pdl_launch_dependents();
+  int q = -1, id = 0;                              // lane s of the first of these warps: route s of the row
+  auto fetch_route = [&](int t) {
+    if (th >= 0 && th < p.k) {
+      q = __ldcg(p.inv + static_cast<size_t>(t) * p.k + th);
+      id = __ldcg(p.ids + static_cast<size_t>(t) * p.k + th);
+    }
+  };
+  if (static_cast<int>(blockIdx.x) < items) fetch_route(static_cast<int>(blockIdx.x) / parts);
   if (warp == 2) {   // exclusive prefixes of the experts' tiles and image groups
     constexpr int PE = (MAX_LOCAL_EXPERTS + 31) / 32;
     int cn[PE], of[PE], tiles = 0, groups = 0, most = 0;
@@ -537,15 +558,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
 
   if (warp >= NV_SPLIT_WARP) {
     // ------------------------------------------------- split of the token rows
-    int q = -1, id = 0;                            // lane s of the first of these warps: route s of the row
-    auto fetch_route = [&](int t) {
-      if (th < p.k) {
-        q = __ldcg(p.inv + static_cast<size_t>(t) * p.k + th);
-        id = __ldcg(p.ids + static_cast<size_t>(t) * p.k + th);
-      }
-    };
     int item = static_cast<int>(blockIdx.x);
-    if (item < items) fetch_route(item / parts);
     while (item < items) {
       const int part = item % parts, next = item + n_ctas;
       if (th < 32) {   // where its local routes' rows go
@@ -561,28 +574,28 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       }
       named_bar_sync(1, NT);
       const int n_routes = ctl.n_routes;
-      uint32_t g[PER][8];
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) g[i][j] = h[i][j];
-      }
       if (next < items) {                          // on its way while this one is split
         fetch_row(next / parts);
         q = -1;
         fetch_route(next / parts);
       }
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int b = th + i * NT, stage = b >> 4;
-        const bool mine = b < nb && n_routes != 0 && (parts == 1 || stage % parts == part);
-        if (!__any_sync(0xffffffffu, mine)) continue;
-        unsigned more[2];
+      // Half a warp to a K stage, a part of its routes and, with few tokens, a third of the digits: as many shares as there are half warps. (With the
+      // thread that holds a block writing all its digits to all routes, 16 threads did 8 tokens' work: first MMA after 11.8 us, now 10.8; 64
+      // tokens 14.5 and 13.2.)
+      const int stages = (p.H / KS - part + parts - 1) / parts, by_route = max(1, min(HALVES / stages, n_routes));
+      const int by_digit = HALVES / (stages * by_route) >= 3 ? 3 : 1, shares = n_routes != 0 ? stages * by_route * by_digit : 0;
+#pragma unroll 1
+      for (int first = (warp - NV_SPLIT_WARP) * 2; first < shares; first += HALVES) {
+        const int share = min(first + (lane >> 4), shares - 1), j = share / stages, stage = part + (share - j * stages) * parts;
+        const int third = j / by_route, r0 = j - third * by_route, b = stage * 16 + (lane & 15);
+        const uint4 v0 = row_s[2 * b], v1 = row_s[2 * b + 1];
+        const uint32_t g[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         auto at = [&](const uint4& to) { return p.img[0] + (to.x + to.y * static_cast<uint32_t>(stage * NV_GROUP_BYTES)); };
-        nv_split_block(g[i], mine, more[0], more[1],
+        unsigned more[2];
+        nv_split_block(g, first + (lane >> 4) < shares, NV_PARTS / by_digit, NV_PARTS / by_digit * (third + 1), third == 0, more[0], more[1],
             [&](uint32_t s0, uint32_t s1, uint32_t s2) {
 #pragma unroll 1
-              for (int s = 0; s < n_routes; ++s) {
+              for (int s = r0; s < n_routes; s += by_route) {
                 const uint4 to = ctl.route[s];
                 const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
                 uint8_t* img = at(to);
@@ -593,24 +606,23 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
             },
             [&](int level, int d, uint2 w) {
 #pragma unroll 1
-              for (int s = 0; s < n_routes; ++s) {
+              for (int s = r0; s < n_routes; s += by_route) {
                 const uint4 to = ctl.route[s];
                 const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
                 *reinterpret_cast<uint2*>(at(to) + nv_digit_at(width, level, d) + nv_row_at(slot) + nv_code_at(slot, b)) = w;
               }
             });
-        if (more[0] != 0u && lane < n_routes) {     // the warp's blocks are those of two stages
-          unsigned int* flags = p.tiles + ctl.route[lane].z * NV_TILE_WORDS + NV_MORE;
-          const int first = (th - lane + i * NT) >> 4;
 #pragma unroll
-          for (int m = 0; m < 2; ++m)
-            if (more[m] != 0u) atomicOr(flags + m, ((more[m] & 0xFFFFu) != 0u ? 1u << first : 0u) | (more[m] >> 16 != 0u ? 2u << first : 0u));
+        for (int m = 0; m < 2; ++m) {              // (lane i of a half: its share's i-th route)
+          const int s = r0 + (lane & 15) * by_route;
+          if (((more[m] >> (lane & 16)) & 0xFFFFu) != 0u && s < n_routes)
+            atomicOr(p.tiles + ctl.route[s].z * NV_TILE_WORDS + NV_MORE + m, 1u << stage);
         }
       }
       item = next;
       if (item < items) {
+        named_bar_sync(1, NT);                     // the row's and the routes' places may be written again
         finish_row();
-        named_bar_sync(1, NT);                     // the routes' places may be written again
       }
     }
     named_bar_sync(1, NT);
@@ -980,7 +992,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         load(slot + 2);                            // the next two rows, while these are split
         unsigned more1, more2;
         uint8_t* at = stage + nv_row_at(slot) + nv_code_at(slot, blk);
-        nv_split_block(h8, slot < last, more1, more2,
+        nv_split_block(h8, slot < last, NV_PARTS, NV_PARTS, true, more1, more2,
             [&](uint32_t s0, uint32_t s1, uint32_t s2) {
               stage[nv_scale_at(u.width, 0, slot, blk)] = static_cast<uint8_t>(s0);
               stage[nv_scale_at(u.width, 1, slot, blk)] = static_cast<uint8_t>(s1);
