@@ -350,7 +350,7 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     plan = moe.plan(state, T)
     few, nvf4 = ctypes.c_int(0), ctypes.c_int(0)
     state["lib"].lib.msk_moe_few_fits(ctypes.byref(state["cfg"]), T, 1, ctypes.byref(few))   # (timed with given ids)
-    state["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(state["cfg"]), T, int(state["post_norm_w"] is not None), ctypes.byref(nvf4))
+    state["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(state["cfg"]), T, int(state["post_norm_w"] is not None) + 2 * int(state["pre_norm_w"] is not None), ctypes.byref(nvf4))
     nvf4 = bool(nvf4.value) and not few.value
     one_launch = plan[1] == 0 and T <= 32 and R <= 256 and not nvf4
     # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine

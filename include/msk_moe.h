@@ -230,9 +230,11 @@ int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out);
 int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_fits);
 
 /* Whether a step of n_tokens runs in the kernel on the FP4 tensor cores (sort launches, both GEMMs, combine), whatever path and tile
- * msk_moe_plan names for it: *host_takes = 1 or 0. norms: non-zero with a pre- or post-expert norm. Where msk_moe_few_fits says
- * 1 as well, a state that holds all experts runs here and a rank's in the few-token kernel. No GPU needed. No
+ * msk_moe_plan names for it: *host_takes = 1 or 0. norms: MSK_NVF4_* bits of the step's expert norms. Where msk_moe_few_fits
+ * says 1 as well, a state that holds all experts runs here and a rank's in the few-token kernel. No GPU needed. No
  * counterpart in the reference. */
+#define MSK_NVF4_POST_NORM 1
+#define MSK_NVF4_PRE_NORM 2
 int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_takes);
 
 /* How the GEMM kernels deal their work (host-side twin of the device code, a test hook): the pieces

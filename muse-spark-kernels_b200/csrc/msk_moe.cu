@@ -693,37 +693,58 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   return p;
 }
 
-// The kernel on the FP4 tensor cores (nvf4.cuh). Its lines, whole steps in us by this kernel / the other one, in turn on one box.
-// All of 128 experts (H4096 I1536 top-8), near-even routes: 4 tokens 65 / 65, 5: 76 / 76, 6: 83 / 86, 8: 96 / 103, 12: 123 / 138, 24:
-// 173 / 208, 64: 221 / 262, 160: 258 / 291, 192 (12 rows an expert) 275 / 318; a few experts taking most tokens 8: 63 / 65, 12: 68 / 65,
-// 16: 74 / 71, 24: 81 / 84, 48: 95 / 114, 192: 207 / 278.
-// A rank with one row a token (32 of 256, H4096 I4096, two experts taking most) 6: 54 / 58, 8: 59 / 66; 12: 63 / 62, 16: 68 / 66
-// (from nine tokens on the other one has its cheaper form as well, and there is little to stream); 24: 75 / 74 to 81 / 85, 32: 85 / 95, 160: 159 /
-// 198, 384: 234 / 315; H7168 I2048, even, 16: 75 / 75, 64: 115 / 123, 256: 138 / 158, 384: 156 / 192.
-// Beyond 12 rows an expert the other one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of
-// them, this one for 24: near-even routes 256: 298 / 327, but with a few experts taking most 259 / 199, the rank (512) 273 / 238.
-// A small model (H2048 I1024 E64 top-4), whose down units are four K stages long and wait for their epilogues: 8: 46 / 41, 24: 52 / 52
-// (a few experts taking most 41 / 36), 64: 60 / 61 (50 / 44).
-// With an expert norm the others take an exchange or a launch more, and this one, whose combine is a launch anyway, does not: all of 128
-// experts with both norms and routing, near-even (a few experts taking most) 3: 67 / 73 (61 / 60), 4: 75 / 91 (62 / 66), 5: 82 / 98
-// (64 / 91), with the post-expert norm 3: 67 / 71 (60 / 57), 4: 74 / 78 (62 / 77), 5: 81 / 92; the rank with it 3: 45 / 40, 4: 49 / 51, 5: 49 / 53.
-// Where the few-token kernel takes four tokens and more (pre-expert norm), it keeps a rank's: 4: 48 / 45, 6: 55 / 52.
+// The kernel on the FP4 tensor cores (nvf4.cuh). It streams weights at the pace of memory and pays some 5 us more in front of the first MMA, so it
+// gains with the bytes that a step streams: those of the experts that get a token, which the host does not know. Whole steps in us, the other
+// kernel / this one, in turn on one box; "uneven": a few experts taking most tokens (Zipf routes).
+// All of 128 experts (H4096 I1536 top-8, 10.6 MB each), near-even (uneven): 4 tokens 66 / 68 (54 / 56), 5: 76 / 74 (57 / 59), 6: 86 / 82 (61 / 61), 8:
+// 106 / 96 (64 / 64), 9: 117 / 102 (61 / 66), 12: 145 / 127 (65 / 69), 16: 179 / 151 (71 / 75), 20: 206 / 176 (77 / 79), 24: 222 / 187 (84 / 84), 64: 276 / 227
+// (137 / 115), 192 (12 rows an expert) 339 / 317 (283 / 252); 224: 310 / 332 (208 / 279), 256: 271 / 322 (220 / 310): beyond 12 rows an expert the other
+// one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one for 16. So uneven steps of 9
+// to 20 tokens lose 1 to 8 %, near-even ones, which stream twice the bytes, gain 12 to 18: the line stays at 6.
+// A rank (32 of 256, one row a token): H4096 I4096, two experts taking most, 4: 46 / 46, 6: 50 / 52, 8: 59 / 59, 12: 61 / 64, 16: 66 / 70, 24: 78 / 78, 26: 81 /
+// 81, 28: 86 / 82, 32: 94 / 88, 64: 136 / 115, 384: 317 / 267 (512: 225 / 290); H7168 I2048, even, 6: 51 / 53, 8: 56 / 58, 16: 74 / 74, 26: 88 / 85, 28: 92 / 88,
+// 64: 131 / 117, 384: 203 / 193.
+// Layers of less: experts of 4.4 MB and less (a small model, H2048 I1024 E64 top-4, down units of four K stages) 8: 39 / 40 (38 / 37), 24: 50 / 53 (36 / 42), 64: 58
+// / 65 (43 / 51); H2048 I1536 E64 (340 MB in all) 8: 43 / 46 (39 / 40), 24: 64 / 63 (43 / 49), 160: 83 / 92 (78 / 89); H2048 I2048 E64 (453 MB) 24: 77 / 72 (50 / 55),
+// 64: 94 / 87 (62 / 66), 160: 103 / 106 (98 / 103); 32 experts of H4096 I1536 (340 MB) 6: 53 / 57, 32: 73 / 74 (59 / 64). H4096 I1280 E128 would gain 7 to 18 %
+// near-even, and lose 4 uneven (24 tokens 80 / 83). (Fewer than 32 experts: 8 of H4096 I14336 16 tokens 164 / 144.)
+// With an expert norm the others take an exchange or a launch more up to eight tokens, and this one, whose combine is a launch anyway, does not.
+// Post-expert norm, the 128 experts 3: 70 / 63 (56 / 57), 4: 73 / 71 (77 / 59), 8: 120 / 98 (99 / 66); the small model 4: 35 / 36 (41 / 34), 8: 44 / 42; a rank
+// 3: 40 / 45, 4: 51 / 46, 8: 65 / 59, H7168 3: 42 / 51, 4: 56 / 53, 8: 61 / 59. Pre-expert norm, the 128 experts 4: 77 / 69 (51 / 57), 5: 82 / 75 (61 / 59),
+// 8: 117 / 96 (67 / 63); H2048 I1536 E64 4: 35 / 41 (27 / 38), 6: 44 / 43 (32 / 40); 32 experts of H4096 I1536 6: 57 / 57 (42 / 47); a rank 4: 42 / 48, 8: 59 / 59, H7168 5: 50 / 54, 8: 58 / 59; from nine
+// tokens on the other one has a row copy in front as well: H2048 I1536 E64 9: 52 / 49 (38 / 41), 32: 79 / 67 (49 / 51).
+// Where the few-token kernel takes four tokens and more of a rank (both norms), it keeps them: 4: 46 / 48, 6: 53 / 55.
 constexpr int NV_MIN_TOKENS = 6;
-constexpr int NV_MIN_NORM_TOKENS = 4;
-constexpr int NV_MIN_RANK_TOKENS = 28;       // of a rank that holds a part of the experts, beyond the one-launch form's tokens
+constexpr int NV_MIN_NORM_TOKENS = 4;        // with an expert norm
+constexpr int NV_MIN_RANK_TOKENS = 28;       // of a rank that holds a part of the experts (with the post-expert norm: beyond the one-launch form's)
 constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
+// Bytes of near-even routes, where all of NV_MANY_EXPERTS experts or more are here: beyond the one-launch form's tokens, up to them, with the
+// pre-expert norm alone
+constexpr double NV_MIN_BYTES = 460e6, NV_MIN_BYTES_ONE_LAUNCH = 400e6, NV_MIN_BYTES_PRE = 300e6;
+constexpr int NV_MANY_EXPERTS = 32;
 
 static int nv_max_tokens(const MskMoeCfg* c, int T) {   // of the steps of up to T tokens that may take it
   if (c->inter < NV_MIN_INTER || c->inter > NV_MAX_INTER || c->hidden > NV_MAX_BLOCKS * 16) return 0;
   return static_cast<int>(std::min(static_cast<long long>(T), static_cast<long long>(NV_MAX_MEAN_ROWS) * c->n_experts / c->top_k));
 }
 
-// Whether a step runs in it. A form that the configuration asks for is always the asked one.
-static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, bool norm) {
-  return c->token_tile == 0 && c->decode_path == 0 && c->flat_shares == 0 && c->stop_after == 0 && p.grid <= sm_count() &&
-         T >= (norm ? NV_MIN_NORM_TOKENS : NV_MIN_TOKENS) && T <= nv_max_tokens(c, T) &&
-         (c->local_count == c->n_experts || T <= ONE_LAUNCH_MAX_TOKENS || T >= NV_MIN_RANK_TOKENS);
+// Weights that near-even routes of T tokens touch, where all experts are here.
+static double nv_even_bytes(const MskMoeCfg* c, int T) {
+  const double touched = c->n_experts * (1.0 - std::pow(1.0 - static_cast<double>(c->top_k) / c->n_experts, T));
+  return touched * 3.0 * c->hidden * c->inter * 0.5625;
+}
+
+// Whether a step runs in it; norms: MSK_NVF4_* bits. A form that the configuration asks for is always the asked one.
+static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, int norms) {
+  if (c->token_tile != 0 || c->decode_path != 0 || c->flat_shares != 0 || c->stop_after != 0 || p.grid > sm_count() || T > nv_max_tokens(c, T)) return false;
+  const bool all = c->local_count == c->n_experts, pre = (norms & MSK_NVF4_PRE_NORM) != 0, post = (norms & MSK_NVF4_POST_NORM) != 0;
+  const bool many = c->n_experts >= NV_MANY_EXPERTS;
+  if (T <= ONE_LAUNCH_MAX_TOKENS) {
+    if (post) return T >= NV_MIN_NORM_TOKENS;
+    return all && T >= (pre ? NV_MIN_NORM_TOKENS : NV_MIN_TOKENS) && (!many || nv_even_bytes(c, T) >= (pre ? NV_MIN_BYTES_PRE : NV_MIN_BYTES_ONE_LAUNCH));
+  }
+  return all ? pre || !many || nv_even_bytes(c, T) >= NV_MIN_BYTES : T >= NV_MIN_RANK_TOKENS;
 }
 
 // Workspace carving. Everything is sized for max_tokens with the worst plan.
@@ -1445,7 +1466,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
   const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
                          (host_x ? MSK_FEW_HOST_X : 0);
-  const bool nv = nv_takes(cfg, n_tokens, plan, pre_norm_w != nullptr || post_norm_w != nullptr);
+  const bool nv = nv_takes(cfg, n_tokens, plan, (pre_norm_w != nullptr ? MSK_NVF4_PRE_NORM : 0) | (post_norm_w != nullptr ? MSK_NVF4_POST_NORM : 0));
   if (plan.path == 0 && !(nv && cfg->local_count == cfg->n_experts) && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
@@ -1921,7 +1942,7 @@ int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_
   if (rc != MSK_OK) return rc;
   if (!host_takes) return MSK_ERR_NULL;
   if (n_tokens < 1) return MSK_ERR_SHAPE;
-  *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens), norms != 0) ? 1 : 0;
+  *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens), norms) ? 1 : 0;
   return MSK_OK;
 }
 

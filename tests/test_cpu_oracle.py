@@ -367,6 +367,36 @@ def test_few_token_kernel_leaves_normed_rows_in_host_memory_to_another():
     assert not any(_few_fits(T, 2 | 4 | given, **shape) for T in (1, 2, 6) for given in (0, 1))
 
 
+_ONE = dict(hidden=4096, inter=1536, n_experts=128, local_count=128, top_k=8)
+_RANK = dict(hidden=4096, inter=4096, n_experts=256, local_count=32, top_k=8)
+
+
+@pytest.mark.parametrize("shape,norms,taken", [      # ranges of token counts: with no norm 0, the post-expert one 1, the pre-expert one 2, both 3
+    (_ONE, 0, [(6, 192)]), (_ONE, 1, [(4, 192)]), (_ONE, 2, [(4, 192)]), (_ONE, 3, [(4, 192)]),
+    (_RANK, 0, [(28, 384)]), (_RANK, 1, [(4, 8), (28, 384)]), (_RANK, 2, [(28, 384)]), (_RANK, 3, [(4, 8), (28, 384)]),
+    (dict(_ONE, inter=1280), 0, []), (dict(_ONE, inter=1280), 1, []),
+    (dict(_ONE, hidden=2048, n_experts=64, local_count=64, top_k=4), 0, []),                   # 340 MB in all
+    (dict(_ONE, hidden=2048, n_experts=64, local_count=64, top_k=4), 1, [(4, 8)]),
+    (dict(_ONE, hidden=2048, n_experts=64, local_count=64, top_k=4), 2, [(9, 192)]),
+    (dict(_ONE, hidden=2048, inter=2048, n_experts=64, local_count=64, top_k=4), 0, []),       # 453 MB
+    (dict(_ONE, hidden=2048, inter=2304, n_experts=64, local_count=64, top_k=4), 0, [(37, 192)]),   # 510 MB
+    (dict(_ONE, n_experts=8, local_count=8, top_k=2), 0, [(6, 48)]),
+    (dict(_ONE, num_ctas=256), 0, []), (dict(_ONE, token_tile=16), 0, []), (dict(_ONE, decode_path=1), 0, []), (dict(_ONE, decode_path=4), 0, []),
+    (dict(_ONE, flat_shares=1), 0, []), (dict(_ONE, stop_after=1), 0, []), (dict(_ONE, hidden=8192), 0, [(6, 192)])])
+def test_fp4_kernel_is_taken_where_it_was_measured_faster(shape, norms, taken):
+    """Both sides of every line of the rule, and never where a tile, a path or a part of the step was asked for."""
+    from muse_moe_w4a16 import _lib
+
+    cfg = _lib.MskMoeCfg(**dict(dict(local_start=0, max_tokens=512), **shape))
+    got = []
+    for T in range(1, 513):
+        takes = ctypes.c_int(-1)
+        assert _lib.load().msk_moe_nvf4_takes(ctypes.byref(cfg), T, norms, ctypes.byref(takes)) == 0
+        if takes.value:
+            got.append(T)
+    assert got == [T for a, b in taken for T in range(a, b + 1)]
+
+
 def test_workspace_init_covers_every_control_word():
     """msk_moe_workspace_init zeroes everything in front of `inter`: the status word, the sort tables,
     both ticket regions, the control words of the few-token paths (token tickets, grid and tile

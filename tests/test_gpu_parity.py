@@ -1303,7 +1303,7 @@ def test_prefill_moe_runs_the_prefill_layer_call_site(cuda_dev):
 
 def _nvf4_takes(st, T):
     takes = ctypes.c_int(0)
-    assert st["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(st["cfg"]), T, int(st["post_norm_w"] is not None or st["pre_norm_w"] is not None), ctypes.byref(takes)) == 0
+    assert st["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(st["cfg"]), T, int(st["post_norm_w"] is not None) + 2 * int(st["pre_norm_w"] is not None), ctypes.byref(takes)) == 0
     return takes.value == 1
 
 
@@ -1321,7 +1321,7 @@ def _ids_of_counts(counts, lo, k, dev):
     (768, 1536, [25, 0, 49, 5, 48, 1], 0, True, True),         # two and three tiles an expert, the last ones narrower
     (1024, 1536, [32, 33, 15, 48, 49, 64], 0, False, False),   # whole tiles, tiles with one row behind them
     (2304, 1792, [31, 24, 2, 0, 0, 7], 37, False, True),       # odd numbers of stages, fewer CTAs than rows
-    (8192, 1536, [4, 0, 1, 0, 2, 0], 0, True, False),          # the longest rows, shared by several CTAs
+    (8192, 1536, [4, 0, 11, 0, 15, 0], 0, True, False),        # the longest rows, shared by several CTAs
     (6400, 2048, [40, 100, 9], 5, False, False),               # rows of more blocks than a CTA has threads; every ring wraps often
     (512, 4096, [28], 1, False, True),                         # one CTA waits for nobody but itself
     (768, 1536, [2, 0, 2], 0, False, True),                    # the fewest tokens it takes
