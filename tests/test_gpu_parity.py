@@ -662,15 +662,17 @@ def test_graphed_step_copies_device_tensors_the_kernels_cannot_read(cuda_dev, T,
     assert m.read_status(st) == 0
 
 
-@pytest.mark.parametrize("T,routed", [(1, False), (5, False), (8, True), (40, False)])
-def test_host_mapped_step_reads_and_writes_pinned_host_memory(cuda_dev, T, routed):
+@pytest.mark.parametrize("T,routed,I", [(1, False, 512), (5, False, 512), (8, True, 512), (40, False, 512),
+                                        (4, False, 1536), (6, True, 1536), (8, False, 1536), (40, True, 1536)])     # the FP4 kernel
+def test_host_mapped_step_reads_and_writes_pinned_host_memory(cuda_dev, T, routed, I):
     """HostMappedStep (kernels read the inputs from, and write the output to, pinned host memory; no copy
     launches) returns what kernel_fn returns on device tensors, bit for bit, call after call and across
-    its ring of blocks: one-launch path (1, 5, 8 tokens), chain (40 tokens), given ids and logits."""
+    its ring of blocks: one-launch path (1, 5, 8 tokens), chain (40 tokens), given ids and logits; the FP4 kernel."""
     m, inputs, _lib, orc = _mods()
-    H, I, E, k = 1024, 512, 16, 4
+    H, E, k = 1024, 16, 4
     w = inputs.make_weights(H, I, E, 52, cuda_dev, post_norm=True)
     st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T)
+    assert _nvf4_takes(st, T) == (I == 1536)
     g = torch.Generator(device=cuda_dev).manual_seed(10 + T)
     datas = []
     for _ in range(6):
@@ -1066,21 +1068,23 @@ def _guarded(t):
     return view, guard, buf[nbytes:pad]
 
 
-def test_state_hygiene_token_sequence_and_guard_words(cuda_dev):
+@pytest.mark.parametrize("I,cap,sequence", [(512, 256, (32, 16, 256, 8, 16, 128, 16)),
+                                            (1536, 700, (8, 700, 40, 2, 256, 48, 8, 130, 4, 40))])   # FP4, pair and few-token kernel, 64-token tile in turn
+def test_state_hygiene_token_sequence_and_guard_words(cuda_dev, I, cap, sequence):
     """One state driven through the reference's token-count sequence 32, 16, 256, 8, 16, 128, 16
     (muse_decode_layer/py/17_moev.py:882-908): every output must equal, bit for bit, the output of a
     freshly prepared state on the same input (nothing a call leaves in the workspace may leak into the
     next), and 64 Ki sentinel words behind the output, the workspace and both packed weight buffers
     must survive every call."""
     m, inputs, _lib, orc = _mods()
-    H, I, E, k, cap = 1024, 512, 16, 4, 256
+    H, E, k = 1024, 16, 4
     w = inputs.make_weights(H, I, E, 123, cuda_dev, post_norm=True)
     st = m.prepare(w, n_experts=E, top_k=k, max_tokens=cap)
     guards = []
     for key in ("workspace", "packed13", "packed2"):
         st[key], g, pad = _guarded(st[key])
         guards.append((key, g, pad))
-    for step, T in enumerate((32, 16, 256, 8, 16, 128, 16)):
+    for step, T in enumerate(sequence):
         g = torch.Generator(device=cuda_dev).manual_seed(500 + step)
         data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
                 "router_logits": torch.randn((T, E), generator=g, device=cuda_dev)}
@@ -1399,6 +1403,44 @@ def test_nvf4_kernel_without_a_local_route(cuda_dev):
     none = m.kernel_fn(dict(d, topk_ids=away), st)
     assert not bool(none.any()) and torch.equal(m.kernel_fn(d, st), clean)
     torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+
+
+@pytest.mark.parametrize("T,pre", [(8, False), (8, True), (40, False)])
+def test_nvf4_kernel_replayed_behind_the_kernel_that_writes_its_rows(cuda_dev, T, pre):
+    """Its CTAs read their first token row in front of their wait for the sort: rows that the launch before the step writes, other ones with
+    every replay and replay behind replay, against steps on their own; and the same rows in pinned host memory."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1024, 1536, 16, 4
+    w = inputs.make_weights(H, I, E, 71, cuda_dev, post_norm=True)
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    if pre:
+        w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T)
+    assert _nvf4_takes(st, T)
+    rows = torch.randn((8, T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    logits = torch.randn((8, T, E), generator=g, device=cuda_dev)
+    a, b, x, l = rows[0].clone(), logits[0].clone(), torch.empty_like(rows[0]), torch.empty_like(logits[0])
+    m.kernel_fn({"hidden_states": a, "router_logits": b}, st)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        torch.mul(b, 1.0, out=l)
+        torch.mul(a, 1.0, out=x)
+        out = m.kernel_fn({"hidden_states": x, "router_logits": l}, st)
+    got = []
+    for r, s in zip(rows, logits):
+        a.copy_(r)
+        b.copy_(s)
+        graph.replay()
+        got.append(out.clone())
+    for r, s, y in zip(rows, logits, got):
+        want, ids, tw = m.kernel_fn({"hidden_states": r, "router_logits": s}, st, return_routing=True)
+        assert torch.equal(y, want)
+        host = r.cpu().pin_memory()
+        m._forward(st, st["cfg"], st["lib"].lib, host.data_ptr(), None, ids.data_ptr(), tw.data_ptr(), out.data_ptr(), T)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
     assert m.read_status(st) == 0
 
 
