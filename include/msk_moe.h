@@ -140,7 +140,9 @@ int msk_moe_sort(const MskMoeCfg* cfg, const int32_t* topk_ids, int n_tokens, in
 /* ---- the routed-expert step (replaces okc_run, muse_moe_w4a16/cuda/moe.cu:2796-2881) ---- */
 
 /* Scratch needed by msk_moe_forward for up to cfg->max_tokens tokens. The carving depends
- * on cfg->max_tokens only, so every call must pass the cfg the workspace was sized with. */
+ * on cfg->max_tokens only, so every call must pass the cfg the workspace was sized with. (Where token_tile, decode_path,
+ * flat_shares or stop_after ask for a form, the room that only the FP4 kernel needs is left out; in a workspace without it, steps
+ * that would take that kernel run in the others.) */
 int msk_moe_workspace_bytes(const MskMoeCfg* cfg, size_t* host_bytes);
 
 /* Zero the control words of a workspace (status word, sort tables, unit and token tickets, grid and

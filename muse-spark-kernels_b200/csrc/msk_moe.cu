@@ -735,9 +735,12 @@ static double nv_even_bytes(const MskMoeCfg* c, int T) {
   return touched * 3.0 * c->hidden * c->inter * 0.5625;
 }
 
-// Whether a step runs in it; norms: MSK_NVF4_* bits. A form that the configuration asks for is always the asked one.
+// A form that the configuration asks for is always the asked one.
+static bool form_asked(const MskMoeCfg* c) { return c->token_tile != 0 || c->decode_path != 0 || c->flat_shares != 0 || c->stop_after != 0; }
+
+// Whether a step runs in it; norms: MSK_NVF4_* bits.
 static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, int norms) {
-  if (c->token_tile != 0 || c->decode_path != 0 || c->flat_shares != 0 || c->stop_after != 0 || p.grid > sm_count() || T > nv_max_tokens(c, T)) return false;
+  if (form_asked(c) || p.grid > sm_count() || T > nv_max_tokens(c, T)) return false;
   const bool all = c->local_count == c->n_experts, pre = (norms & MSK_NVF4_PRE_NORM) != 0, post = (norms & MSK_NVF4_POST_NORM) != 0;
   const bool many = c->n_experts >= NV_MANY_EXPERTS;
   if (T <= ONE_LAUNCH_MAX_TOKENS) {
@@ -749,7 +752,7 @@ static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, int norms) {
 
 // Workspace carving. Everything is sized for max_tokens with the worst plan.
 struct Carve {
-  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, nv_tiles, nv_img[2], total;
+  size_t status, trace, cnt, off, perm, inv, tickets, few_ctl, sort_blk, tile_ctr, inter, y, partial, xs, nv_tiles, nv_img[2], nv_end, total;
 };
 constexpr size_t TRACE_CTAS = 256;
 constexpr size_t TRACE_WORDS = TRACE_CTAS * 16 + 3 * 256;
@@ -788,7 +791,7 @@ static Carve carve(const MskMoeCfg* c, int T) {
   // tile hand-over between the gate/up and the down launch: per token tile the finished gate/up units and
   // the down units that have seen them all (two counters per tile, zero between steps)
   k.tile_ctr = o; o += round_up(2 * max_tiles(c, T) * 4, 256);
-  // the FP4 kernel, for the most tokens it takes: counters of its tiles (no more than it has groups of eight rows); its rows further down
+  // the FP4 kernel, for the most tokens it takes: counters of its tiles (no more than it has groups of eight rows)
   const size_t nv_rows = static_cast<size_t>(nv_max_tokens(c, T)) * c->top_k;
   const size_t nv_groups = nv_groups_bound(nv_rows, static_cast<size_t>(c->local_count));
   k.nv_tiles = o; o += round_up(nv_groups * NV_TILE_WORDS * 4, 256);
@@ -797,12 +800,16 @@ static Carve carve(const MskMoeCfg* c, int T) {
   k.y = o; o += round_up(R * c->hidden * 4, 256);
   k.partial = o; o += 2 * round_up(partial_floats(c) * 4, 256);  // one region per GEMM
   k.xs = o; o += round_up(R * c->hidden * 2, 256);  // F16 copy of the token rows ([T, H], or sorted [R, H] for wide token tiles)
-  // the FP4 kernel's split rows
+  // The FP4 kernel's split rows, 3.8 times their F16 bytes: where the pieces and the F16 rows lie, which its steps have no use for, and beyond
+  // them where there is less room (with a capacity of 8192 tokens there never is). Room that only they need is left out where a form is
+  // asked for, whose steps never run there; forward() looks whether it is there.
   const int nv_k[2] = {c->hidden, c->inter};
+  k.nv_end = k.partial;
   for (int i = 0; i < 2; ++i) {
-    k.nv_img[i] = o; o += round_up(nv_groups * (nv_k[i] / KS) * NV_GROUP_BYTES, 256);
+    k.nv_img[i] = k.nv_end;
+    k.nv_end += round_up(nv_groups * (nv_k[i] / KS) * NV_GROUP_BYTES, 256);
   }
-  k.total = o;
+  k.total = form_asked(c) ? o : std::max(o, k.nv_end);
   return k;
 }
 
@@ -1466,7 +1473,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
   const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
                          (host_x ? MSK_FEW_HOST_X : 0);
-  const bool nv = nv_takes(cfg, n_tokens, plan, (pre_norm_w != nullptr ? MSK_NVF4_PRE_NORM : 0) | (post_norm_w != nullptr ? MSK_NVF4_POST_NORM : 0));
+  const bool nv = k.nv_end <= workspace_bytes && nv_takes(cfg, n_tokens, plan, (pre_norm_w != nullptr ? MSK_NVF4_PRE_NORM : 0) | (post_norm_w != nullptr ? MSK_NVF4_POST_NORM : 0));
   if (plan.path == 0 && !(nv && cfg->local_count == cfg->n_experts) && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);

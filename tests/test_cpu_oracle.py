@@ -424,6 +424,30 @@ def test_workspace_init_covers_every_control_word():
     assert ws.value < 200 << 20      # the pieces of cut units take two slots per CTA, not a split-K buffer per unit
 
 
+def test_workspace_has_room_of_its_own_for_split_rows_only_where_they_need_it():
+    """The FP4 kernel's split rows lie where the F16 rows and the pieces of cut units would: nothing more for a large capacity, the
+    rest of them for a small one, and nothing where a form is asked for whose steps never take it."""
+    from muse_moe_w4a16 import _lib
+
+    lib = _lib.load()
+
+    def size(**shape):
+        ws = ctypes.c_size_t()
+        assert lib.msk_moe_workspace_bytes(ctypes.byref(_lib.MskMoeCfg(**dict(dict(local_start=0), **shape))), ctypes.byref(ws)) == 0
+        return ws.value
+
+    for shape in (_ONE, _RANK, dict(_RANK, hidden=7168, inter=2048)):
+        for form in (dict(token_tile=16), dict(decode_path=1), dict(flat_shares=1), dict(stop_after=1)):
+            assert size(max_tokens=8192, **shape) == size(max_tokens=8192, **dict(shape, **form))
+            assert size(max_tokens=64, **shape) > size(max_tokens=64, **dict(shape, **form))
+        # images: 15,744 bytes for eight rows x 256 K, at most a group more per expert than full ones
+        H, I, rows = shape["hidden"], shape["inter"], 64 * shape["top_k"]
+        groups = shape["local_count"] + (rows - shape["local_count"]) // 8
+        more = size(max_tokens=64, **shape) - size(max_tokens=64, token_tile=16, **shape)
+        assert more < groups * (H + I) // 256 * 15744
+    assert size(max_tokens=8192, **_ONE) < 1.853e9
+
+
 def test_module_refuses_cpu_tensors():
     import muse_moe_w4a16 as moe
     from muse_moe_w4a16 import inputs
