@@ -368,9 +368,9 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
                 "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if few.value else "moe_gemm_kernel<N,2>"),
                 "peak_source": peaks["source"] + " (burst copy)"}
     elif nvf4:
-        # both GEMMs in one launch: the touched experts' tiles, x read, its digits written and read (25/8 bytes a value), inter written, read
-        # and its digits written and read, y written
-        alg = mean_touched * (3 * I * H * 0.5625 + 8) + 2.0 * T * H + 6.25 * R * (H + I) + 4.0 * R * I + 4.0 * R * H
+        # both GEMMs in one launch: the touched experts' tiles, x read, inter written and read, y written (the split rows, 3.8 bytes a value
+        # each way, are the kernel's own and stay in L2 for the most part)
+        alg = mean_touched * (3 * I * H * 0.5625 + 8) + 2.0 * T * H + 4.0 * R * I + 4.0 * R * H
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": None,
