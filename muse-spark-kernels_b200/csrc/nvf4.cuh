@@ -6,9 +6,9 @@
 // blocks are the core matrices of an unswizzled K-major operand), only its scale bytes pass through registers into TMEM. No weight
 // is decoded, so the kernel keeps pace with memory: the tcgen05 kernel of gemm.cuh, which decodes to F16 and passes every half
 // stage through a TMEM slot, needs 1500 cycles and more for a stage that memory delivers in 1400, and power for it: long rows of
-// steps run into the card's limit, where its clock falls. 64 tokens, all of 128 experts (1.3 GB), both GEMMs: 229 us there, 200 here; a
-// row of whole steps 288 and 240 (both sides of the other sizes: nv_takes() in msk_moe.cu). Bound by memory, some 6.8 TB/s between the
-// first MMA and the last, and by the 10 us before it (tables, split of the token rows) and 6 after.
+// steps run into the card's limit, where its clock falls. 64 tokens, all of 128 experts (1.3 GB), both GEMMs: 230 us there, 208 here; a
+// row of whole steps 279 and 241 (both sides of the other sizes: nv_takes() in msk_moe.cu). Bound by memory, some 7.1 TB/s between the
+// first MMA and the last, and by the 11 to 13 us before it (tables, split of the token rows) and 4 after.
 //
 // Activations enter exactly as in the F16 kernels: every F16 value, whatever lies beside it (tested bit for bit). A token row becomes nine E2M1
 // rows of its own, the digits of a fixed-point number: in a block of 16 K an element is x = 2^u * (d0 + d1 / 8 + ... + d8 / 8^8), digits
@@ -65,7 +65,7 @@ __host__ __device__ constexpr int nv_level_at(int level) { return level == 0 ? 0
 constexpr int NV_LEVEL_BYTES = nv_level_at(1);             // of the first level, the widest
 constexpr int NV_GROUP_BYTES = nv_level_at(2) + nv_digits(2) * 1024 + 128;   // eight token rows x 256 K
 constexpr int NV_W_STAGES = 4, NV_S_STAGES = 2;            // rings: weights, scales in TMEM
-constexpr int NV_MARKS = 8;                                // stages whose MMAs have a barrier of their own
+constexpr int NV_MARKS = 8;                                // passes whose MMAs have a barrier of their own
 constexpr int NV_UNITS = 4;
 constexpr int NV_SPLIT_WARP = 4, NV_SPLIT_THREADS = NV_THREADS - NV_SPLIT_WARP * 32;
 constexpr int NV_MAX_BLOCKS = 512;                         // blocks of 16 K in a token row: H <= 8192
