@@ -1167,7 +1167,10 @@ def test_few_token_kernel_gives_up_cleanly_and_recovers(cuda_dev, T, post):
     _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 8, ctypes.byref(ptr)),
                "view")
     tile0 = ptr.value - st["workspace"].data_ptr() + 4352     # per-tile counters of the few-token paths
-    st["workspace"][tile0:tile0 + 4].fill_(255)               # -1: the tile's last unit will not complete it
+    # the second tile's: its units are dealt in the same round as the first one's, and its count is asked for behind a complete first one, by
+    # when some of them have been counted (the first tile's is now and then asked for before any has, and -1 passes for complete)
+    tile = tile0 + 4
+    st["workspace"][tile:tile + 4].fill_(255)                 # -1: the tile's last unit will not complete it
     m.kernel_fn(data, st)
     torch.cuda.synchronize()
     assert m.read_status(st) == 1
