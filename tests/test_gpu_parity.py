@@ -1154,7 +1154,8 @@ def test_few_token_kernel_gives_up_cleanly_and_recovers(cuda_dev, T, post):
     wait for that tile runs out (one second), the kernel comes back by itself with the time-out status, the
     context stays usable, and after reinit_workspace the state gives the clean bits again."""
     m, inputs, _lib, orc = _mods()
-    H, I, E, k = 1024, 2048, 16, 8     # every team has gate/up units to do before its first down unit
+    # every team has three gate/up units to do before its first down unit (with H = 1024 those of 64 CTAs have none, and ask at once)
+    H, I, E, k = 4096, 4096, 16, 8
     w = inputs.make_weights(H, I, E, 8, cuda_dev, post_norm=post)
     st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
     g = torch.Generator(device=cuda_dev).manual_seed(4)
@@ -1167,8 +1168,8 @@ def test_few_token_kernel_gives_up_cleanly_and_recovers(cuda_dev, T, post):
     _lib.check(st["lib"].lib.msk_moe_workspace_view(ctypes.byref(st["cfg"]), _lib.ptr(st["workspace"]), 8, ctypes.byref(ptr)),
                "view")
     tile0 = ptr.value - st["workspace"].data_ptr() + 4352     # per-tile counters of the few-token paths
-    # the second tile's: its units are dealt in the same round as the first one's, and its count is asked for behind a complete first one, by
-    # when some of them have been counted (the first tile's is now and then asked for before any has, and -1 passes for complete)
+    # the second tile's: its units are dealt in the first rounds, and its count is asked for behind a complete first one, by when some of them
+    # have been counted (-1 itself passes for complete)
     tile = tile0 + 4
     st["workspace"][tile:tile + 4].fill_(255)                 # -1: the tile's last unit will not complete it
     m.kernel_fn(data, st)
