@@ -32,7 +32,7 @@
 //   warps 4-7    scales: shared memory -> TMEM, each warp for its lane quarter (the hardware wants four copies);
 //   warps 8-11   epilogue: digits summed, SwiGLU / scale, rows to global memory;
 //   warp 3       counts stored gate/up units for their tiles;
-//   warps 12-15  split `inter`: pieces of eight rows x 256 columns of a token tile, dealt over the CTAs in the order of the tiles, as each tile's
+//   warps 12-15  split `inter`: pieces of two to eight rows x 256 columns of a token tile, dealt over the CTAs in the order of the tiles, as each tile's
 //                gate/up units are all stored. Whole tiles, split by the CTA that stored their last unit, kept a rank's 24-token step waiting
 //                for some 20 us.
 // Warps 4-15 first split the token rows, a row or a part of one per CTA at a time, while the first weights are on their way.
@@ -79,6 +79,10 @@ __host__ __device__ inline int nv_width(int rows) { return (rows + 7) >> 3; }
 // Groups that the image of an expert's rows takes: all tiles but the last have whole ones.
 constexpr int NV_GROUPS = NV_ROWS / 8;
 __host__ __device__ inline int nv_groups(int c) { return nv_width(c); }
+// Rows of a piece of inter (x 256 columns), as a power of two, given how many pieces eight rows would make: eight, or two while there are as
+// many warps as half of those to split them. Two rows take a warp 2 us, eight 7, for which the down units of a step of few tiles stood still
+// (a few experts taking most tokens, 12: 68.4 -> 65.5 us a step, 24: 83.6 -> 81.0; four rows in between gained nothing, 32: 89.9 -> 90.4).
+__device__ __forceinline__ int nv_piece_bits(int eights, int n_ctas) { return eights * 2 <= NV_CONV_WARPS * n_ctas ? 1 : 3; }
 // A bound on their sum over experts with `rows` rows in all: nv_groups(c) <= 1 + (c - 1) / 8.
 inline size_t nv_groups_bound(size_t rows, size_t experts) {
   const size_t e = rows < experts ? rows : experts;
@@ -89,7 +93,7 @@ inline size_t nv_groups_bound(size_t rows, size_t experts) {
 constexpr int NV_TILE_WORDS = 64;
 enum : int {
   NV_DONE = 0,     // stored gate/up units
-  NV_READY = 8,    // pieces of inter that are split
+  NV_READY = 8,    // pieces of inter that are split, of two rows each or four times that
   NV_SEEN = 16,    // down units that have fetched them all
   NV_MORE = 32,    // bit per K stage, a word for 32 of them: stages with a second level, a third level; token rows, then inter
   NV_MORE_INTER = NV_MORE + 2 * (NV_MAX_BLOCKS * 16 / KS / 32),
@@ -733,6 +737,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       const uint64_t keep = policy_evict_last();   // re-read by every pair of the expert
       uint32_t st = 0, bs = 0;
       int last_tile = -1;
+      const int n_stages = p.I / KS;
       bool ok = true, split = false;
       NvUnit u;
       while (ok && wait_unit(u, mbar_wait_inline)) {
@@ -746,7 +751,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         unsigned int* tile = p.tiles + u.tile * NV_TILE_WORDS;
         if (u.phase == 1) {
           if (u.tile != last_tile) {
-            if (!grid_counter_wait(tile + NV_READY, static_cast<unsigned>(u.width * (p.I / KS)), abortw)) break;
+            if (!grid_counter_wait(tile + NV_READY, static_cast<unsigned>(u.width * n_stages * 4), abortw)) break;
             fence_proxy_async_all();
             last_tile = u.tile;
           }
@@ -958,11 +963,11 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     }
   } else if (warp >= 12) {
     // ---------------------------------------------------------- split of inter
-    // A warp takes a piece: eight rows of a tile, 256 columns, half a warp to a row. Early tiles are split while later ones are still at their
-    // gate/up units, so the first down units wait for nothing.
-    const int pieces = p.I / KS, n = group_start[p.nloc] * pieces;
-    for (int i = static_cast<int>(blockIdx.x) + (warp - 12) * n_ctas; i < n; i += NV_CONV_WARPS * n_ctas) {
-      const int group = i / pieces, blk = (i - group * pieces) * 16 + (lane & 15);
+    // A warp takes a piece, half a warp to a row. Early tiles are split while later ones are still at their gate/up units, so the first down
+    // units wait for nothing.
+    const int n_stages = p.I / KS, eights = group_start[p.nloc] * n_stages, bits = nv_piece_bits(eights, n_ctas);
+    for (int i = static_cast<int>(blockIdx.x) + (warp - 12) * n_ctas; i < eights << (3 - bits); i += NV_CONV_WARPS * n_ctas) {
+      const int eight = i >> (3 - bits), group = eight / n_stages, blk = (eight - group * n_stages) * 16 + (lane & 15);
       int lo = 0, hi = p.nloc;                     // largest e with group_start[e] <= group
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -971,7 +976,8 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       NvUnit u;
       const int at_row = (group - group_start[lo]) * 8;
       set_tile(u, lo, at_row / nv_tile_rows(cnt_s[lo], nv_tiles(cnt_s[lo])));
-      const int first = (group - u.group) * 8;     // row of the tile
+      const int first = (group - u.group) * 8 + ((i << bits) & 7);   // row of the tile
+      if (first >= u.rows) continue;
       const bool go = lane != 0 || nv_tile_wait(p.tiles + u.tile * NV_TILE_WORDS + NV_DONE, static_cast<unsigned>(p.n_pairs[0]), abortw);
       if (!__all_sync(0xffffffffu, go)) break;
       __syncwarp();   // the vote orders no memory: the other lanes read rows that lane 0 has acquired
@@ -981,9 +987,9 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         v0 = __ldcg(src);
         v1 = __ldcg(src + 1);
       };
-      const int last = min(first + 8, u.rows);
+      const int last = min(first + (1 << bits), u.rows);
       unsigned any1 = 0u, any2 = 0u;
-      uint8_t* stage = p.img[1] + (static_cast<size_t>(u.group) * pieces + static_cast<size_t>(blk >> 4) * u.width) * NV_GROUP_BYTES;
+      uint8_t* stage = p.img[1] + (static_cast<size_t>(u.group) * n_stages + static_cast<size_t>(blk >> 4) * u.width) * NV_GROUP_BYTES;
       load(first + (lane >> 4));
 #pragma unroll 1
       for (int r0 = first; r0 < last; r0 += 2) {
@@ -1005,7 +1011,10 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       if (any1 != 0u && lane < 2 && (lane == 0 || any2 != 0u))
         atomicOr(p.tiles + u.tile * NV_TILE_WORDS + NV_MORE_INTER + (blk >> 9) * 2 + lane, 1u << ((blk >> 4) & 31));
       __syncwarp();
-      if (lane == 0) red_release_add(p.tiles + u.tile * NV_TILE_WORDS + NV_READY, 1u);   // (its readers put the fence between their acquire and their bulk copies)
+      // a piece counts as the two rows that it has, or four times that; the tile's last one for the rows behind it as well (the counter's
+      // readers put the fence between their acquire and their bulk copies)
+      const unsigned twos = bits == 3 ? 4u : first + 2 < u.rows ? 1u : 4u - ((first & 7) >> 1);
+      if (lane == 0) red_release_add(p.tiles + u.tile * NV_TILE_WORDS + NV_READY, twos);
     }
   }
 
