@@ -693,30 +693,31 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
   return p;
 }
 
-// The kernel on the FP4 tensor cores (nvf4.cuh). It streams weights at the pace of memory and pays some 5 us more in front of the first MMA, so it
-// gains with the bytes that a step streams: those of the experts that get a token, which the host does not know. Whole steps in us, the other
-// kernel / this one, in turn on one box; "uneven": a few experts taking most tokens (Zipf routes).
-// All of 128 experts (H4096 I1536 top-8, 10.6 MB each), near-even (uneven): 4 tokens 66 / 68 (54 / 56), 5: 76 / 74 (57 / 59), 6: 86 / 82 (61 / 61), 8:
-// 106 / 96 (64 / 64), 9: 117 / 102 (61 / 66), 12: 145 / 127 (65 / 69), 16: 179 / 151 (71 / 75), 20: 206 / 176 (77 / 79), 24: 222 / 187 (84 / 84), 64: 276 / 227
-// (137 / 115), 192 (12 rows an expert) 339 / 317 (283 / 252); 224: 310 / 332 (208 / 279), 256: 271 / 322 (220 / 310): beyond 12 rows an expert the other
-// one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one for 16. So uneven steps of 9
-// to 20 tokens lose 1 to 8 %, near-even ones, which stream twice the bytes, gain 12 to 18: the line stays at 6.
-// A rank (32 of 256, one row a token): H4096 I4096, two experts taking most, 4: 46 / 46, 6: 50 / 52, 8: 59 / 59, 12: 61 / 64, 16: 66 / 70, 24: 78 / 78, 26: 81 /
-// 81, 28: 86 / 82, 32: 94 / 88, 64: 136 / 115, 384: 317 / 267 (512: 225 / 290); H7168 I2048, even, 6: 51 / 53, 8: 56 / 58, 16: 74 / 74, 26: 88 / 85, 28: 92 / 88,
-// 64: 131 / 117, 384: 203 / 193.
-// Layers of less: experts of 4.4 MB and less (a small model, H2048 I1024 E64 top-4, down units of four K stages) 8: 39 / 40 (38 / 37), 24: 50 / 53 (36 / 42), 64: 58
-// / 65 (43 / 51); H2048 I1536 E64 (340 MB in all) 8: 43 / 46 (39 / 40), 24: 64 / 63 (43 / 49), 160: 83 / 92 (78 / 89); H2048 I2048 E64 (453 MB) 24: 77 / 72 (50 / 55),
-// 64: 94 / 87 (62 / 66), 160: 103 / 106 (98 / 103); 32 experts of H4096 I1536 (340 MB) 6: 53 / 57, 32: 73 / 74 (59 / 64). H4096 I1280 E128 would gain 7 to 18 %
-// near-even, and lose 4 uneven (24 tokens 80 / 83). (Fewer than 32 experts: 8 of H4096 I14336 16 tokens 164 / 144.)
+// The kernel on the FP4 tensor cores (nvf4.cuh). It streams weights at the pace of memory and pays some us more in front of the first MMA and
+// between the GEMMs, so it gains with the bytes that a step streams: those of the experts that get a token, which the host does not know. Whole
+// steps in us, the other kernel / this one, in turn on one box; "uneven": a few experts taking most tokens (Zipf routes).
+// All of 128 experts (H4096 I1536 top-8, 10.6 MB each), near-even (uneven): 4 tokens 65 / 69 (54 / 55), 5: 76 / 75 (56 / 57), 6: 87 / 82 (60 / 60), 8:
+// 105 / 95 (64 / 61), 9: 115 / 102 (60 / 62), 12: 147 / 125 (64 / 66), 16: 174 / 149 (71 / 72), 20: 200 / 170 (77 / 76), 24: 216 / 180 (84 / 81), 64: 262 / 224
+// (134 / 116), 192 (12 rows an expert) 339 / 305 (278 / 246); 224: 320 / 351 (191 / 285), 256: 325 / 382 (213 / 309): beyond 12 rows an expert the other
+// one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one for 16. Uneven steps of 9
+// to 16 tokens lose 1 to 3 %, near-even ones, which stream twice the bytes, gain 13 to 17: the line stays at 6.
+// A rank (32 of 256, one row a token): H4096 I4096, two experts taking most, 4: 45 / 46, 6: 50 / 49, 8: 59 / 58, 10: 59 / 62, 16: 66 / 67, 18: 69 / 69, 20: 70 / 69,
+// 24: 79 / 76, 28: 86 / 80, 64: 138 / 115, 384: 308 / 263 (512: 236 / 310); H7168 I2048, even, 4: 50 / 51, 6: 50 / 53, 8: 56 / 58, 16: 74 / 74, 18: 77 / 77, 20: 81 /
+// 79, 24: 83 / 80, 28: 91 / 88, 64: 128 / 114, 384: 201 / 171.
+// Layers of less: experts of 3.5 MB (a small model, H2048 I1024 E64 top-4, down units of four K stages) 8: 45 / 44 (38 / 35), 24: 54 / 55 (37 / 39), 64: 58
+// / 62 (44 / 47); H2048 I1536 E64 (340 MB in all) 8: 43 / 45 (39 / 38), 24: 64 / 62 (44 / 45), 160: 83 / 93 (78 / 89); H2048 I2048 E64 (453 MB) 24: 76 / 72 (50 / 51),
+// 64: 94 / 87 (63 / 67), 160: 103 / 107 (100 / 103); 32 experts of H4096 I1536 (340 MB) 6: 53 / 56 (46 / 44), 32: 71 / 71 (59 / 60). H4096 I1280 E128, 24: 161 / 146
+// (83 / 77), would gain. (Fewer than 32 experts: 8 of H4096 I14336 16 tokens 155 / 144.)
 // With an expert norm the others take an exchange or a launch more up to eight tokens, and this one, whose combine is a launch anyway, does not.
-// Post-expert norm, the 128 experts 3: 70 / 63 (56 / 57), 4: 73 / 71 (77 / 59), 8: 120 / 98 (99 / 66); the small model 4: 35 / 36 (41 / 34), 8: 44 / 42; a rank
-// 3: 40 / 45, 4: 51 / 46, 8: 65 / 59, H7168 3: 42 / 51, 4: 56 / 53, 8: 61 / 59. Pre-expert norm, the 128 experts 4: 77 / 69 (51 / 57), 5: 82 / 75 (61 / 59),
-// 8: 117 / 96 (67 / 63); H2048 I1536 E64 4: 35 / 41 (27 / 38), 6: 44 / 43 (32 / 40); 32 experts of H4096 I1536 6: 57 / 57 (42 / 47); a rank 4: 42 / 48, 8: 59 / 59, H7168 5: 50 / 54, 8: 58 / 59; from nine
-// tokens on the other one has a row copy in front as well: H2048 I1536 E64 9: 52 / 49 (38 / 41), 32: 79 / 67 (49 / 51).
-// Where the few-token kernel takes four tokens and more of a rank (both norms), it keeps them: 4: 46 / 48, 6: 53 / 55.
+// Post-expert norm, the 128 experts 3: 70 / 62 (56 / 56), 4: 74 / 70 (75 / 57), 8: 119 / 98 (100 / 63); the small model 4: 35 / 37 (38 / 33), 8: 44 / 41; a rank
+// 3: 41 / 45, 4: 50 / 47, 8: 66 / 58, H7168 3: 43 / 50, 4: 54 / 52, 8: 61 / 59. Pre-expert norm, the 128 experts 4: 77 / 69 (51 / 56), 5: 82 / 75 (61 / 58),
+// 8: 117 / 95 (68 / 61); H2048 I1536 E64 4: 35 / 40 (27 / 35), 6: 43 / 43 (32 / 37); 32 experts of H4096 I1536 6: 57 / 57 (42 / 45); a rank 4: 42 / 48, 8: 59 / 59, H7168
+// 5: 50 / 54, 8: 58 / 59; from nine tokens on the other one has a row copy in front as well: H2048 I1536 E64 9: 51 / 49 (37 / 40), 32: 79 / 68 (49 / 47), a
+// rank 12: 66 / 63, H7168 12: 75 / 65.
+// Where the few-token kernel takes four tokens and more of a rank (both norms), it keeps them: 4: 45 / 48, 6: 52 / 54.
 constexpr int NV_MIN_TOKENS = 6;
 constexpr int NV_MIN_NORM_TOKENS = 4;        // with an expert norm
-constexpr int NV_MIN_RANK_TOKENS = 28;       // of a rank that holds a part of the experts (with the post-expert norm: beyond the one-launch form's)
+constexpr int NV_MIN_RANK_TOKENS = 20;       // of a rank that holds a part of the experts (with the post-expert norm: beyond the one-launch form's)
 constexpr int NV_MAX_MEAN_ROWS = 12;
 constexpr int NV_MIN_INTER = 1536;
 // Bytes of near-even routes, where all of NV_MANY_EXPERTS experts or more are here: beyond the one-launch form's tokens, up to them, with the

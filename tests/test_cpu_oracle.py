@@ -373,7 +373,7 @@ _RANK = dict(hidden=4096, inter=4096, n_experts=256, local_count=32, top_k=8)
 
 @pytest.mark.parametrize("shape,norms,taken", [      # ranges of token counts: with no norm 0, the post-expert one 1, the pre-expert one 2, both 3
     (_ONE, 0, [(6, 192)]), (_ONE, 1, [(4, 192)]), (_ONE, 2, [(4, 192)]), (_ONE, 3, [(4, 192)]),
-    (_RANK, 0, [(28, 384)]), (_RANK, 1, [(4, 8), (28, 384)]), (_RANK, 2, [(28, 384)]), (_RANK, 3, [(4, 8), (28, 384)]),
+    (_RANK, 0, [(20, 384)]), (_RANK, 1, [(4, 8), (20, 384)]), (_RANK, 2, [(20, 384)]), (_RANK, 3, [(4, 8), (20, 384)]),
     (dict(_ONE, inter=1280), 0, []), (dict(_ONE, inter=1280), 1, []),
     (dict(_ONE, hidden=2048, n_experts=64, local_count=64, top_k=4), 0, []),                   # 340 MB in all
     (dict(_ONE, hidden=2048, n_experts=64, local_count=64, top_k=4), 1, [(4, 8)]),
