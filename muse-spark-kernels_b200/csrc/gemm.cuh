@@ -118,8 +118,8 @@ struct PhaseParams {
 };
 
 struct GemmParams {
-  CUtensorMap tmap_act[2][3];   // TMA_B only, per phase: [rows, K] f16, boxes 64 x (16 << i) up to 64 x N, 128-byte swizzle
-                                // (64-byte aligned: first member)
+  CUtensorMap tmap_act[2][3];   // TMA_B only, per phase: f16 rows as [K / 64][rows][64], boxes 4 x (16 << i) x 64 up to N rows, 128-byte
+                                // swizzle (64-byte aligned: first member)
   PhaseParams ph[2];         // [0] gate/up, [1] down; a single-phase launch uses its own entry only
   const __nv_bfloat16* post_norm_w;  // phase 1, nullable
   int32_t* cnt;              // [local_count]      sort tables in global memory: read here, or written by CTA 0

@@ -120,10 +120,9 @@
     }
     drain();
     } else if (lane == 0) {
-      // Wide token tiles: four boxes per K stage, rows row0.. of the sorted matrix, no higher than the tile's
-      // rows need (16, 32 or 64: a tensor map each). The copies of a stage stay four; only their bytes
-      // shrink. (Whole 32-row boxes put side by side, more copies per stage, were slower than full height.) A full
-      // box of 64 rows is 32 KB a stage beside 36 KB of weights.
+      // The 64-token tile: one copy per K stage, four sub-tiles of 64 K of the rows row0.. of the sorted matrix, no higher than the tile's
+      // rows need (16, 32 or 64: a tensor map each). A full stage of 64 rows is 32 KB beside 36 KB of weights. As four copies of 64 K
+      // the issue alone took about half of a stage's time.
       const uint64_t keep = policy_evict_last();  // token rows are re-read by every pair of the expert
       uint32_t it = 0;
       bool ok = true;
@@ -153,8 +152,7 @@
             if (!MSK_WAIT(&ctl.b_empty[slot], par ^ 1u, abortw)) { ok = false; break; }
             uint8_t* dstB = ring + slot * C::STAGE_BYTES + 2 * TILE_BYTES;
             mbar_arrive_expect_tx(&ctl.b_full[slot], static_cast<uint32_t>(4 * 64 * 2 * 16) << h);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) tma_load_2d(dstB + j * (N * 128), map, ks * KS + j * 64, ui.row0, &ctl.b_full[slot], keep);
+            tma_load_3d(dstB, map, 0, ui.row0, ks * 4, &ctl.b_full[slot], keep);
           }
         }
         if (!ok) break;

@@ -845,6 +845,15 @@ static int encode_act_map(CUtensorMap* map, const void* base, size_t rows, int K
   return encode_map(map, dtype, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// F16 rows as a tensor [K / 64][rows][64]: a box is a K stage of box_rows rows, four sub-tiles of 64 K one behind the other, so that
+// one copy fetches what four boxes of 64 K did.
+static int encode_stage_map(CUtensorMap* map, const void* base, size_t rows, int K, int box_rows) {
+  const cuuint64_t dims[3] = {64u, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 64)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, 128u};
+  const cuuint32_t box[3] = {64u, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(KS / 64)};
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
 // Experiment switch (environment variable MSK_FUSED_PLAIN): launch the one-launch kernel without the
 // cooperative attribute. Its grid never exceeds the SM count and it holds an SM per CTA, so its CTAs
 // are resident together in practice, and its waits are bounded either way.
@@ -916,8 +925,8 @@ static int launch_pair(PairParams& p, const __half* xs, size_t rows, int grid, c
     attr_set[dev] = true;
   }
   for (int i = 0; i < PAIR_MAPS; ++i) {
-    int e = encode_act_map(&p.tmap[0][i], xs, rows, p.K[0], 16 * (i + 1));
-    if (e == 0) e = encode_act_map(&p.tmap[1][i], p.inter, rows, p.K[1], 16 * (i + 1));
+    int e = encode_stage_map(&p.tmap[0][i], xs, rows, p.K[0], 16 * (i + 1));
+    if (e == 0) e = encode_stage_map(&p.tmap[1][i], p.inter, rows, p.K[1], 16 * (i + 1));
     if (e != 0) return e;
   }
   cudaLaunchConfig_t lc{};
@@ -1613,8 +1622,8 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     if (e != 0) return e;
     if (tma_b && plan.N != 128) {
       for (int i = 0; (16 << i) <= plan.N; ++i) {
-        e = encode_act_map(&p.tmap_act[0][i], xs, r_max, cfg->hidden, 16 << i);
-        if (e == 0) e = encode_act_map(&p.tmap_act[1][i], inter, r_max, cfg->inter, 16 << i);
+        e = encode_stage_map(&p.tmap_act[0][i], xs, r_max, cfg->hidden, 16 << i);
+        if (e == 0) e = encode_stage_map(&p.tmap_act[1][i], inter, r_max, cfg->inter, 16 << i);
         if (e != 0) return e;
       }
     }

@@ -12,8 +12,8 @@
 //
 // Per CTA (640 threads, one CTA per SM):
 //   warp 0        weight producer: half a K stage (18,432 contiguous bytes, layout.cuh) per bulk copy into a ring;
-//   warp 1        CTA 0: MMA issuer; both: TMEM allocation;
-//   warp 2        activations: four TMA boxes (64 K x half the tile's rows, 128-byte swizzle) per K stage; the copies of
+//   warp 1        CTA 0: MMA issuer (one thread); both: TMEM allocation;
+//   warp 2        activations (one thread): a TMA copy (4 x 64 K x half the tile's rows, 128-byte swizzle) per K stage; the copies of
 //                 both CTAs complete on CTA 0's barrier;
 //   warp 3        CTA 0: scheduler: draws units from a counter in global memory and hands them to both CTAs; both: counts
 //                 drained gate/up units for their token tile;
@@ -78,7 +78,7 @@ struct PairCfg {
 };
 
 struct PairParams {
-  CUtensorMap tmap[2][PAIR_MAPS];        // per phase: [rows, K] f16, boxes 64 x 16(i + 1), 128-byte swizzle
+  CUtensorMap tmap[2][PAIR_MAPS];        // per phase: f16 rows as [K / 64][rows][64], boxes 4 x 16(i + 1) x 64, 128-byte swizzle
   const uint8_t* w[2];                   // packed tiles
   const float* gs[2];
   __half* inter;                         // [R, I]
@@ -327,66 +327,61 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     }
   } else if (warp == 1) {
     // ----------------------------------------------------------- MMA issuer
-    if (rank == 0) {
+    if (rank == 0 && elect_one()) {                // one thread walks the whole loop (ptx.cuh, MSK_MMA_STEP)
       const uint64_t b_desc0 = smem_desc_kmajor_sw128(smem_u32(b_ring));   // slots and K steps advance its address field
       PairBuffers db;
       uint32_t st = 0;                             // K stage, through all units
       bool ready = false;                          // stage st was seen full while the one before was issued
       bool ok = true;
       PairUnit u;
-      while (ok && wait_unit(u, mbar_wait_warp)) {
-        __syncwarp();
-        if (lane == 0) done_unit();
+      while (ok && wait_unit(u, mbar_wait_inline)) {
+        done_unit();
         if (u.phase < 0) break;
         const uint32_t idesc = idesc_f16(FMT_F16, FMT_F16, 256, static_cast<uint32_t>(u.nmma));
         db.take(u.nmma);
-        if (db.uses(0) && !mbar_wait_warp(&ctl.d_empty[0], db.p0 ^ 1u, abortw)) { ok = false; break; }
-        if (db.uses(1) && !mbar_wait_warp(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) { ok = false; break; }
+        if (db.uses(0) && !mbar_wait_inline(&ctl.d_empty[0], db.p0 ^ 1u, abortw)) { ok = false; break; }
+        if (db.uses(1) && !mbar_wait_inline(&ctl.d_empty[1], db.p1 ^ 1u, abortw)) { ok = false; break; }
         const uint32_t d_tmem = tmem + db.buf * static_cast<uint32_t>(BH);
         tc_fence_after();
-        const uint64_t sub = static_cast<uint64_t>(db.wide ? C::B_SUB_BYTES : C::B_SUB_BYTES / 2) >> 4;
+        const uint32_t sub = static_cast<uint32_t>(u.nmma) * 4u;   // half of the rows, 128 bytes each, in units of 16 bytes
         for (int k = 0; k < p.K[u.phase]; k += KS) {
-          if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&ctl.full[st & 3u], (st >> 2) & 1u, abortw)) { ok = false; break; }
+          if (!ready && !mbar_wait_inline(&ctl.full[st & 3u], (st >> 2) & 1u, abortw)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sn = st + 1u, sl = (st & 1u) * 2u;
-          const uint32_t place = sl * C::B_SLOT_BYTES + (db.wide ? 0u : ((st >> 1) & 1u) * (C::B_SLOT_BYTES / 2));
+          const uint32_t place = sl * C::B_SLOT_BYTES + (db.wide ? 0u : ((st >> 1) & 1u) * C::B_SLOT_BYTES);
           ready = mma_stage_pair(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + (place >> 4), idesc, k > 0 ? 1u : 0u,
-                                 smem_u32(&ctl.empty[(st & 3u) * 2u]), smem_u32(&ctl.full[sn & 3u]), (sn >> 2) & 1u, sub,
-                                 (C::B_SLOT_BYTES >> 4) - sub);
+                                 smem_u32(&ctl.empty[(st & 3u) * 2u]), smem_u32(&ctl.full[sn & 3u]), (sn >> 2) & 1u, sub);
           st = sn;
         }
-        if (ok && elect_one()) {
+        if (ok) {
           if (db.uses(0)) tc_commit_pair(&ctl.d_full[0]);
           if (db.uses(1)) tc_commit_pair(&ctl.d_full[1]);
         }
-        __syncwarp();
       }
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------- activations
-    // (the whole warp walks the loop, one elected lane issues: addresses and coordinates stay in uniform registers)
+    // One thread, one wait and one copy a K stage: as a warp that elects a lane for four copies, each half a stage behind a wait of its
+    // own, this role took 850 cycles a stage beside the decode warps, and set the pace of tiles of few rows.
     const uint64_t keep = policy_evict_last();     // token rows are re-read by every pair of the expert
     uint32_t n = 0, wide_end = 0;                  // slot, through all units; the one behind the last wide tile's
     bool ok = true;
-    int last_tile = -1;
-    PairUnit u;
-    while (ok && wait_unit(u, mbar_wait_warp)) {
-      __syncwarp();
-      if (lane == 0) done_unit();
-      if (u.phase < 0) break;
-      const int half = u.nmma >> 1;
-      const CUtensorMap* map = &p.tmap[u.phase][half / 16 - 1];
-      const int row = u.row0 + static_cast<int>(rank) * half, K = p.K[u.phase];
-      const uint32_t bytes = static_cast<uint32_t>(half) * 256u * 2u * 2u;   // 256 K of both CTAs' rows
-      if (u.phase == 1 && p.first == 0) {
-        if (u.tile != last_tile) {
-          const bool seen = grid_counter_wait(p.tile_done + u.tile, 2u * static_cast<unsigned>(p.n_pairs[0]), abortw);
-          if (!__all_sync(0xffffffffu, seen)) { ok = false; break; }
-          fence_proxy_async_all();                 // ordinary stores of other SMs, about to be read by bulk copies
-          last_tile = u.tile;
-          __syncwarp();
-        }
-        if (lane == 0) {
+    if (elect_one()) {
+      int last_tile = -1;
+      PairUnit u;
+      while (ok && wait_unit(u, mbar_wait_inline)) {
+        done_unit();
+        if (u.phase < 0) break;
+        const int half = u.nmma >> 1;
+        const CUtensorMap* map = &p.tmap[u.phase][half / 16 - 1];
+        const int row = u.row0 + static_cast<int>(rank) * half, K = p.K[u.phase];
+        const uint32_t bytes = static_cast<uint32_t>(half) * 256u * 2u * 2u;   // 256 K of both CTAs' rows
+        if (u.phase == 1 && p.first == 0) {
+          if (u.tile != last_tile) {
+            if (!grid_counter_wait(p.tile_done + u.tile, 2u * static_cast<unsigned>(p.n_pairs[0]), abortw)) { ok = false; break; }
+            fence_proxy_async_all();               // ordinary stores of other SMs, about to be read by bulk copies
+            last_tile = u.tile;
+          }
           // the last CTA to have seen the count complete puts both counters back for the next launch
           const unsigned seen = atomicAdd(p.tile_seen + u.tile, 1u);
           if (seen == 2u * static_cast<unsigned>(p.n_pairs[1]) - 1u) {
@@ -394,26 +389,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             atomicExch(p.tile_seen + u.tile, 0u);
           }
         }
-      }
-      for (int k = 0; k < K; k += KS) {
-        // half a stage at a time, as its slots come back: the MMAs wait for these rows more than for the weights
-        const uint32_t bar = lead_bar(&ctl.full[(n >> 1) & 3u]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h, ++n) {
-          const uint32_t before = pair_b_waits_for(n, u.nmma, wide_end);   // (of the first slots: a barrier that nothing has completed, parity 1)
-          if (!mbar_wait_warp(&ctl.empty[before & 7u], (before >> 3) & 1u, abortw)) { ok = false; break; }
-          if (elect_one()) {
-            if (h == 0 && rank == 0) mbar_arrive_expect_tx(&ctl.full[(n >> 1) & 3u], bytes);
-            uint8_t* dst = b_ring + (n & 3u) * C::B_SLOT_BYTES + (half > BH / 2 ? 0u : ((n >> 2) & 1u) * (C::B_SLOT_BYTES / 2));
-            tma_load_2d_pair(dst, map, k + h * 128, row, bar, keep);
-            tma_load_2d_pair(dst + (half > BH / 2 ? C::B_SUB_BYTES : C::B_SUB_BYTES / 2), map, k + h * 128 + 64, row, bar, keep);
-          }
-          __syncwarp();
+        for (int k = 0; k < K; k += KS, n += 2) {
+          // both slots of the stage: MMAs are done in order, so the second one's barrier tells (of the first slots: a barrier that
+          // nothing has completed, parity 1)
+          const uint32_t before = pair_b_waits_for(n, u.nmma, wide_end) + 1u;
+          if (!mbar_wait_inline(&ctl.empty[before & 7u], (before >> 3) & 1u, abortw)) { ok = false; break; }
+          const uint32_t i = n >> 1;
+          if (rank == 0) mbar_arrive_expect_tx(&ctl.full[i & 3u], bytes);
+          uint8_t* dst = b_ring + (i & 1u) * (2 * C::B_SLOT_BYTES) + (half > BH / 2 ? 0u : ((i >> 1) & 1u) * C::B_SLOT_BYTES);
+          tma_load_3d_pair(dst, map, 0, row, k >> 6, lead_bar(&ctl.full[i & 3u]), keep);
         }
-        if (!ok) break;
+        if (half > BH / 2) wide_end = n;
       }
-      if (half > BH / 2) wide_end = n;
     }
+    __syncwarp();
+    ok = __all_sync(0xffffffffu, ok);
+    n = __reduce_max_sync(0xffffffffu, n);
     // the commits of the last slots arrive in this CTA's shared memory: it stays until they have
     for (int i = 0; ok && i < PAIR_MARKS; ++i) {
       --n;

@@ -262,6 +262,15 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, in
       "l"(tmap), "r"(c0), "r"(c1), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
+// The same from a tensor of three dimensions.
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar,
+                                            uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
 // L2 prefetch of a contiguous piece (16-byte aligned, a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_prefetch_l2(const void* gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
@@ -312,12 +321,13 @@ __device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// 2-D tiled TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair (a cluster address).
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, int c0, int c1, uint32_t bar, uint64_t policy) {
+// 3-D tiled TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair (a cluster address).
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint32_t bar,
+                                                 uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
-      "[%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_u32(smem_dst)),
-      "l"(tmap), "r"(c0), "r"(c1), "r"(bar), "l"(policy)
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(bar), "l"(policy)
       : "memory");
 }
 
@@ -377,58 +387,45 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
                "h"(static_cast<uint16_t>(3))
                : "memory");
 }
+// One MMA of a run over K: B lies `o` behind descriptor half `l` (units of 16 bytes; an address never carries out of the low half), A
+// `c` columns behind the first. By a single thread (elect_one() around the whole loop of an issuer): measured beside sixteen
+// decoding warps, an MMA of 32 columns issues every 16 cycles this way, every 50 to 70 where the warp elects a lane, issues and meets
+// again for each run.
+#define MSK_MMA_STEP(group, d, a, l, o, c, idesc, acc)                                                  \
+  "add.u32 x, " l ", " o ";\n\tmov.b64 b, {x, hi};\n\tadd.u32 c, " a ", " c ";\n\t"                       \
+  "tcgen05.mma.cta_group::" group ".kind::f16 [" d "], [c], b, " idesc ", " acc ";\n\t"
+
 // D[256 rows over both CTAs' TMEM, N] (+)= A[256 rows, 256] (128 rows in either TMEM) * B[N, 256] (N / 2 rows in either CTA): the
-// sixteen MMAs of a K stage (two slots) by one elected lane, and the commits that hand its slots back in both CTAs (empty_bar and
+// sixteen MMAs of a K stage (two slots) by one thread, and the commits that hand its slots back in both CTAs (empty_bar and
 // the barrier behind it). The answer of a probe of `next_full` (true: complete) is asked for before the MMAs and read behind them, so
-// that its latency hides behind the issue. b_desc: the first of four sub-tiles of 64 K; the second one of a slot lies `sub` behind the
-// first, the next slot's first `gap` behind that (in units of 16 bytes).
+// that its latency hides behind the issue. b_desc: the first of four sub-tiles of 64 K, which lie `sub` apart (units of 16 bytes).
 __device__ __forceinline__ bool mma_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
-                                               uint32_t empty_bar, uint32_t next_full, uint32_t parity, uint64_t sub, uint64_t gap) {
+                                               uint32_t empty_bar, uint32_t next_full, uint32_t parity, uint32_t sub) {
   uint32_t ok;
+#define MSK_PAIR_COMMIT(bar) "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [" bar "], %10;\n\t"
+#define MSK_PAIR_STEP(l, o, c, acc) MSK_MMA_STEP("2", "%1", "%2", l, o, c, "%4", acc)
   asm volatile(
-      "{\n\t.reg .pred q, e, acc, t;\n\t.reg .b64 b, d;\n\t.reg .b32 a;\n\t"
+      "{\n\t.reg .pred q, acc, t;\n\t.reg .b32 l0, l1, l2, l3, hi, second, x, c;\n\t.reg .b64 b;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 q, [%7], %8;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
       "setp.ne.b32 acc, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [%2], %3, %4, acc;\n\t"
-      "mov.b64 b, %3;\n\tadd.s64 d, b, 2;\n\tadd.u32 a, %2, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], %10;\n\t"
-      "add.s64 b, b, %11;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 b, b, %9;\n\tmov.b64 d, b;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.s64 d, d, 2;\n\tadd.u32 a, a, 8;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], [a], d, %4, t;\n\t"
-      "add.u32 a, %6, 8;\n\t"
-      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [a], %10;\n\t"
+      "mov.b64 {l0, hi}, %3;\n\tadd.u32 l1, l0, %9;\n\tadd.u32 l2, l1, %9;\n\tadd.u32 l3, l2, %9;\n\tadd.u32 second, %6, 8;\n\t"
+      MSK_PAIR_STEP("l0", "0", "0", "acc") MSK_PAIR_STEP("l0", "2", "8", "t")
+      MSK_PAIR_STEP("l0", "4", "16", "t") MSK_PAIR_STEP("l0", "6", "24", "t")
+      MSK_PAIR_STEP("l1", "0", "32", "t") MSK_PAIR_STEP("l1", "2", "40", "t")
+      MSK_PAIR_STEP("l1", "4", "48", "t") MSK_PAIR_STEP("l1", "6", "56", "t")
+      MSK_PAIR_COMMIT("%6")
+      MSK_PAIR_STEP("l2", "0", "64", "t") MSK_PAIR_STEP("l2", "2", "72", "t")
+      MSK_PAIR_STEP("l2", "4", "80", "t") MSK_PAIR_STEP("l2", "6", "88", "t")
+      MSK_PAIR_STEP("l3", "0", "96", "t") MSK_PAIR_STEP("l3", "2", "104", "t")
+      MSK_PAIR_STEP("l3", "4", "112", "t") MSK_PAIR_STEP("l3", "6", "120", "t")
+      MSK_PAIR_COMMIT("second")
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(ok)
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_full), "r"(parity),
-        "l"(sub), "h"(static_cast<uint16_t>(3)), "l"(gap)
+        "r"(sub), "h"(static_cast<uint16_t>(3))
       : "memory");
+#undef MSK_PAIR_STEP
+#undef MSK_PAIR_COMMIT
   return ok != 0;
 }
 
@@ -474,16 +471,26 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]; A: lane = row, one 32-bit column = two consecutive K elements.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem]; A: lane = row, one 32-bit column = two consecutive K elements. The eight MMAs of an A slot (128 K) by
+// one thread: B of K step j lies (j & 3) * STEP + (j >> 2) * sub behind b_desc (units of 16 bytes).
+template <int STEP>
+__device__ __forceinline__ void mma_slot_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                            uint32_t sub) {
+#define MSK_SLOT_STEP(l, o, c, acc) MSK_MMA_STEP("1", "%0", "%1", l, o, c, "%3", acc)
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred acc, t;\n\t.reg .b32 l0, l1, hi, x, c;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 acc, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "mov.b64 {l0, hi}, %2;\n\tadd.u32 l1, l0, %5;\n\t"
+      MSK_SLOT_STEP("l0", "0", "0", "acc") MSK_SLOT_STEP("l0", "%6", "8", "t")
+      MSK_SLOT_STEP("l0", "%7", "16", "t") MSK_SLOT_STEP("l0", "%8", "24", "t")
+      MSK_SLOT_STEP("l1", "0", "32", "t") MSK_SLOT_STEP("l1", "%6", "40", "t")
+      MSK_SLOT_STEP("l1", "%7", "48", "t") MSK_SLOT_STEP("l1", "%8", "56", "t")
+      "}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sub), "n"(STEP), "n"(2 * STEP), "n"(3 * STEP)
       : "memory");
+#undef MSK_SLOT_STEP
 }
+#undef MSK_MMA_STEP
 
 // 32 lanes x 32 bit, N consecutive columns per thread. The warp may only touch
 // TMEM lanes [32*(warp_id%4), +32); the lane base goes in bits 31..16 of taddr.
