@@ -925,8 +925,8 @@ static int launch_pair(PairParams& p, const __half* xs, size_t rows, int grid, c
     attr_set[dev] = true;
   }
   for (int i = 0; i < PAIR_MAPS; ++i) {
-    int e = encode_stage_map(&p.tmap[0][i], xs, rows, p.K[0], 16 * (i + 1));
-    if (e == 0) e = encode_stage_map(&p.tmap[1][i], p.inter, rows, p.K[1], 16 * (i + 1));
+    int e = encode_stage_map(&p.tmap[0][i], xs, rows, p.K[0], 8 * (i + 1));
+    if (e == 0) e = encode_stage_map(&p.tmap[1][i], p.inter, rows, p.K[1], 8 * (i + 1));
     if (e != 0) return e;
   }
   cudaLaunchConfig_t lc{};

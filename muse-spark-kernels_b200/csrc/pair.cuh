@@ -30,6 +30,10 @@
 // (pair_slots_before_drain), so the wait ends whatever part of the grid is resident. Which cluster computes a unit does not
 // change its bits.
 //
+// MMAs are as wide as a tile's rows in steps of sixteen (eight rows in either CTA); in steps of 32 a row of steps took, before / after:
+// 777 tokens at H4096 I1536 E128 422 / 411 us, 1500 tokens whose routes favour a few experts 619 / 607, 3012 skewed tokens of a rank 533 / 526,
+// 8192 tokens of one rank of eight, H7168 I2048, 733 / 712.
+//
 // Numerics as in gemm.cuh: the same products, FP32 accumulation along K, the same roundings (the same bits as its tiles).
 //
 // Measured (both GEMMs, us, against one CTA to a tile of up to 128 tokens, which this replaces): 8192 tokens of Zipf routes at
@@ -59,7 +63,7 @@ constexpr int PAIR_THREADS = 640;
 constexpr int PAIR_DQ_WARP = 4;          // first decode warp
 constexpr int PAIR_DQ_WARPS = 16;
 constexpr int PAIR_SLOT_COLS = PAIR_SLOT_K / 2;
-constexpr int PAIR_MAPS = 8;             // tensor maps per phase: boxes of 16, 32 .. 128 rows
+constexpr int PAIR_MAPS = 16;            // tensor maps per phase: boxes of 8, 16 .. 128 rows
 
 struct PairCfg {
   static constexpr int BH = PAIR_BH;
@@ -78,7 +82,7 @@ struct PairCfg {
 };
 
 struct PairParams {
-  CUtensorMap tmap[2][PAIR_MAPS];        // per phase: f16 rows as [K / 64][rows][64], boxes 4 x 16(i + 1) x 64, 128-byte swizzle
+  CUtensorMap tmap[2][PAIR_MAPS];        // per phase: f16 rows as [K / 64][rows][64], boxes 4 x 8(i + 1) x 64, 128-byte swizzle
   const uint8_t* w[2];                   // packed tiles
   const float* gs[2];
   __half* inter;                         // [R, I]
@@ -101,7 +105,7 @@ struct PairParams {
 struct alignas(16) PairUnit {              // written and read 16 bytes at a time
   int phase;                             // -1: no more units
   int expert, row0, rows, pair, tile;
-  int nmma;                              // rows rounded up to 32
+  int nmma;                              // rows rounded up to 16
   int pad_;
 };
 
@@ -146,7 +150,7 @@ struct PairBuffers {
 template <typename Release>
 __device__ __forceinline__ void pair_epilogue(const PairParams& p, const PairUnit& u, uint32_t d_tmem, int rank, int q, int part,
                                               int lane, Release release) {
-  const int nc = u.nmma >> 2, c0 = part * nc;
+  const int nc = ((u.nmma >> 2) + 15) & ~15, c0 = part * nc;   // whole steps of sixteen columns
   if (c0 >= u.rows) {
     release();
     return;
@@ -344,14 +348,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         const uint32_t d_tmem = tmem + db.buf * static_cast<uint32_t>(BH);
         tc_fence_after();
         const uint32_t sub = static_cast<uint32_t>(u.nmma) * 4u;   // half of the rows, 128 bytes each, in units of 16 bytes
-        for (int k = 0; k < p.K[u.phase]; k += KS) {
+        uint32_t accumulate = 0u;
+        for (int left = p.K[u.phase] / KS; left > 0; --left) {
           if (!ready && !mbar_wait_inline(&ctl.full[st & 3u], (st >> 2) & 1u, abortw)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sn = st + 1u, sl = (st & 1u) * 2u;
           const uint32_t place = sl * C::B_SLOT_BYTES + (db.wide ? 0u : ((st >> 1) & 1u) * C::B_SLOT_BYTES);
-          ready = mma_stage_pair(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + (place >> 4), idesc, k > 0 ? 1u : 0u,
+          ready = mma_stage_pair(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + (place >> 4), idesc, accumulate,
                                  smem_u32(&ctl.empty[(st & 3u) * 2u]), smem_u32(&ctl.full[sn & 3u]), (sn >> 2) & 1u, sub);
           st = sn;
+          accumulate = 1u;
         }
         if (ok) {
           if (db.uses(0)) tc_commit_pair(&ctl.d_full[0]);
@@ -373,7 +379,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         done_unit();
         if (u.phase < 0) break;
         const int half = u.nmma >> 1;
-        const CUtensorMap* map = &p.tmap[u.phase][half / 16 - 1];
+        const CUtensorMap* map = &p.tmap[u.phase][half / 8 - 1];
         const int row = u.row0 + static_cast<int>(rank) * half, K = p.K[u.phase];
         const uint32_t bytes = static_cast<uint32_t>(half) * 256u * 2u * 2u;   // 256 K of both CTAs' rows
         if (u.phase == 1 && p.first == 0) {
@@ -473,7 +479,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             const int per = pair_tile_rows(c, nt), at = (tile - tile_start[lo]) * per;
             const int rows = min(per, c - at);
             a = make_int4(phase, lo, off_s[lo] + at, rows);
-            b = make_int4(pair, tile, (rows + 31) & ~31, 0);
+            b = make_int4(pair, tile, (rows + 15) & ~15, 0);
           }
           const uint32_t s = i % PAIR_UNITS;
           const uint32_t par = ((i / PAIR_UNITS) & 1u) ^ 1u;   // of the unit whose place this one takes

@@ -536,6 +536,25 @@ def test_pair_kernel_hands_few_narrow_tiles_from_gate_up_to_down(cuda_dev, H, I,
     _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
+@pytest.mark.parametrize("H,I,counts", [(256, 256, [8, 9, 15, 16, 17, 24, 47, 48]), (512, 768, [49, 79, 80, 81, 111, 112, 113, 144]),
+                                        (768, 512, [145, 175, 176, 177, 209, 239, 240, 241])])
+def test_pair_kernel_at_every_width_of_its_mmas(cuda_dev, H, I, counts):
+    """MMAs are as wide as the tile's rows in steps of sixteen, half of them, eight at the least, in either CTA: rows around those
+    steps, narrow and wide tiles in turn."""
+    m, inputs, _lib, orc = _mods()
+    E, T = len(counts), 256
+    w = inputs.make_weights(H, I, E, 97, cuda_dev, post_norm=True)
+    st = m.prepare(w, n_experts=E, top_k=E, max_tokens=T, token_tile=128)
+    g = torch.Generator(device=cuda_dev).manual_seed(101)
+    ids = torch.stack([torch.where(torch.randperm(T, generator=g, device=cuda_dev) < c, e, -1) for e, c in enumerate(counts)], 1)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16),
+            "topk_ids": ids.to(torch.int32).contiguous(), "topk_weights": torch.rand((T, E), generator=g, device=cuda_dev)}
+    ref, parts = orc.moe_forward(data["hidden_states"], data["topk_ids"], data["topk_weights"], w, return_parts=True)
+    out = m.kernel_fn(data, st)
+    assert m.read_status(st) == 0
+    _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
 @pytest.mark.parametrize("E,k,nloc,T", [(8, 2, 8, 256), (128, 8, 4, 700)])
 def test_pair_kernel_by_default_on_a_handful_of_experts(cuda_dev, E, k, nloc, T):
     """The default plan takes the pair kernel by the mean rows per expert, also where only a handful of experts is there."""
