@@ -232,9 +232,6 @@ __global__ void __launch_bounds__(64) convert_rows_kernel(const __nv_bfloat16* _
 // Slots without a local route (inv < 0) are squeezed out first, keeping their order, so an expert-parallel rank
 // that owns one or two of a token's eight routes reads only those rows, and a token without any
 // local route only gets zeros. Bound by memory for many tokens (8192 tokens, eight rows each: 0.6 GB).
-constexpr int COMBINE_THREADS = 512;
-constexpr int COMBINE_MAX_F4 = 4;   // float4 per thread per row: H <= 8192
-constexpr int COMBINE_WIDE_TOKENS = 512;  // from here on two blocks per SM, two slots per group
 
 // Eight consecutive y values of a row, FP32 or BF16 (the pair kernel's), in registers while in flight.
 template <bool YB> struct YOct;
@@ -247,6 +244,9 @@ template <> struct YOct<false> {
   __device__ __forceinline__ void add_to(float (&acc)[8], float w) const {
     acc[0] += a.x * w; acc[1] += a.y * w; acc[2] += a.z * w; acc[3] += a.w * w;
     acc[4] += b.x * w; acc[5] += b.y * w; acc[6] += b.z * w; acc[7] += b.w * w;
+  }
+  __device__ __forceinline__ float squares() const {
+    return ((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w));
   }
 };
 template <> struct YOct<true> {
@@ -261,6 +261,16 @@ template <> struct YOct<true> {
       acc[2 * i] += __uint_as_float(v[i] << 16) * w;
       acc[2 * i + 1] += __uint_as_float(v[i] & 0xFFFF0000u) * w;
     }
+  }
+  __device__ __forceinline__ float squares() const {
+    const uint32_t v[4] = {a.x, a.y, a.z, a.w};
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float lo = __uint_as_float(v[i] << 16), hi = __uint_as_float(v[i] & 0xFFFF0000u);
+      s += lo * lo + hi * hi;
+    }
+    return s;
   }
 };
 
@@ -321,94 +331,50 @@ __global__ void __launch_bounds__(COMBINE_COLS_WARPS * 32)
   }
 }
 
-// With the post-expert norm: one block per token. The block sum of squares is a fixed shuffle tree followed by a
-// fixed-order sum of the warp partials, so the result does not depend on scheduling.
-// G = slots whose rows are loaded together (one memory latency per group instead of one per
-// slot; the sums still run in slot order). G = 4 for few tokens (latency), G = 2 with two blocks
-// per SM for many (one block's loads overlap the other's reduction and stores); BF16 rows need
-// half the registers while in flight, so they get G = 4 and two blocks per SM.
-// Four consecutive y values of a row as they sit in registers while their group is in flight:
-// FP32 (16 bytes) or BF16 (8 bytes, for the wide token tile), expanded when used.
-template <bool YB> struct YQuad;
-template <> struct YQuad<false> {
-  float4 v;
-  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void load(const float* y, size_t row_elems, int j) {
-    v = __ldcs(reinterpret_cast<const float4*>(y + row_elems) + j);
-  }
-  __device__ __forceinline__ float4 get() const { return v; }
-};
-template <> struct YQuad<true> {
-  uint2 b;
-  __device__ __forceinline__ void zero() { b = make_uint2(0u, 0u); }
-  __device__ __forceinline__ void load(const float* y, size_t row_elems, int j) {
-    b = __ldcs(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(y) + row_elems) + j);
-  }
-  __device__ __forceinline__ float4 get() const {
-    return make_float4(__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xFFFF0000u), __uint_as_float(b.y << 16),
-                       __uint_as_float(b.y & 0xFFFF0000u));
-  }
-};
-
-// NF4 = float4 slots per thread per row that the kernel is built for: 4 (H <= 8192) or 2 (H <= 4096, half
-// the registers per row in flight, which is what lets all eight rows of a token be loaded at once).
-template <int G, bool YB, int MINB, int NF4 = COMBINE_MAX_F4>
-__global__ void __launch_bounds__(COMBINE_THREADS, MINB)
+// With the post-expert norm: a block of TH threads per token, G rows in registers at a time (NO octets of columns a thread, H <= 8 * TH * NO). The sum of
+// squares of a row is a fixed shuffle tree followed by a fixed-order sum of the warps' parts, so the result does not depend on
+// scheduling; the sums run in slot order. Bound by latency (table, rows, reduction, each behind the other), so what counts is rows in flight on
+// an SM. Many tokens: blocks of 128 threads (256 beyond 4096 columns), five or four of them on an SM, where blocks of 512 left two tokens to
+// one: 3012 tokens with 1.6 local routes each 41 -> 18 us, 777 with eight 22 -> 16, 7000 149 -> 98. Few
+// tokens: 512 threads and as many rows at once as fit (64 tokens of eight 8 -> 6).
+constexpr int COMBINE_FEW_TOKENS = 256;
+constexpr int COMBINE_MAX_H = 8192;
+template <bool YB, int TH, int NO, int G, int MINB>
+__global__ void __launch_bounds__(TH, MINB)
     combine_norm_kernel(const float* y, const int32_t* inv, const float* tw, __nv_bfloat16* __restrict__ out, int H, int k,
                         float eps) {   // (y, inv and tw: as above)
-  constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
-  static_assert(G == 1 << LG, "two, four or eight rows together");
-  __shared__ __align__(16) float wsum[G][COMBINE_THREADS / 32];
-  __shared__ int s_q[MAX_TOP_K];
-  __shared__ float s_w[MAX_TOP_K];
-  __shared__ int s_n;
+  constexpr int NW = TH / 32, LG = G == 8 ? 3 : G == 4 ? 2 : 1;
+  static_assert(G == 1 << LG && NW % 4 == 0, "two, four or eight rows together");
+  __shared__ __align__(16) float part[2][G][NW];   // in turn: a group's parts are read while the next one's are written
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();  // y and inv come from the kernels before this one
-  if (warp == 0) {  // lane s takes slot s (k <= 16); a ballot keeps the order
-    const int q = lane < k ? inv[static_cast<size_t>(t) * k + lane] : -1;
-    const float w = lane < k ? tw[static_cast<size_t>(t) * k + lane] : 0.f;
-    const unsigned have = __ballot_sync(0xffffffffu, q >= 0);
-    if (q >= 0) {
-      const int at = __popc(have & ((1u << lane) - 1u));
-      s_q[at] = q;
-      s_w[at] = w;
-    }
-    if (lane == 0) s_n = __popc(have);
-  }
-  __syncthreads();
-  const int nv = s_n;
-  const int n4 = H / 4;  // float4 per row; thread tid owns indices i*512 + tid
-  float4 acc[NF4];
-#pragma unroll
-  for (int i = 0; i < NF4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < nv; s0 += G) {
-    int q[G];
-    float wgt[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const bool in = s0 + g < nv;
-      q[g] = in ? s_q[s0 + g] : -1;
-      wgt[g] = in ? s_w[s0 + g] : 0.f;
-    }
-    YQuad<YB> v[G][NF4];
-    float ss[G];
+  const int q = lane < k ? inv[static_cast<size_t>(t) * k + lane] : -1;
+  const float w = lane < k ? tw[static_cast<size_t>(t) * k + lane] : 0.f;
+  unsigned have = __ballot_sync(0xffffffffu, q >= 0);   // the same in every warp
+  float acc[NO][8] = {};
+  for (int turn = 0; have != 0u; turn ^= 1) {
+    YOct<YB> v[G][NO];
+    float wgt[G], ss[G];
+    const int n = min(__popc(have), G);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       ss[g] = 0.f;
-      const size_t r = static_cast<size_t>(q[g] < 0 ? 0 : q[g]) * H;
+      if (g < n) {
+        const int s = __ffs(have) - 1;
+        have &= have - 1u;
+        wgt[g] = __shfl_sync(0xffffffffu, w, s);
+        const size_t at = static_cast<size_t>(__shfl_sync(0xffffffffu, q, s)) * H;
 #pragma unroll
-      for (int i = 0; i < NF4; ++i) {
-        v[g][i].zero();
-        if (q[g] >= 0 && i * COMBINE_THREADS + tid < n4) v[g][i].load(y, r, i * COMBINE_THREADS + tid);
+        for (int c = 0; c < NO; ++c)
+          if ((c * TH + tid) * 8 < H) v[g][c].load(y, at + (c * TH + tid) * 8);
       }
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      if (s0 + g >= nv) continue;
+      if (g < n) {
 #pragma unroll
-      for (int i = 0; i < NF4; ++i) {
-        const float4 f = v[g][i].get();
-        ss[g] += f.x * f.x + f.y * f.y + f.z * f.z + f.w * f.w;
+        for (int c = 0; c < NO; ++c)
+          if ((c * TH + tid) * 8 < H) ss[g] += v[g][c].squares();
       }
     }
     // G sums over the warp at once: in each of the first steps a lane passes on half of its sums and keeps the other
@@ -425,41 +391,34 @@ __global__ void __launch_bounds__(COMBINE_THREADS, MINB)
     }
 #pragma unroll
     for (int r = 16 >> LG; r > 0; r >>= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], r);
-    if (s0 > 0) __syncthreads();  // wsum of the previous group fully read
-    if ((lane & ((32 >> LG) - 1)) == 0) wsum[lane >> (5 - LG)][warp] = ss[0];
+    if ((lane & ((32 >> LG) - 1)) == 0) part[turn][lane >> (5 - LG)][warp] = ss[0];
     __syncthreads();
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (s0 + g >= nv) continue;
-      float tot = 0.f;
+    for (int g = 0; g < G; ++g) {   // slot order
+      if (g < n) {
+        float tot = 0.f;
 #pragma unroll
-      for (int w = 0; w < COMBINE_THREADS / 128; ++w) {  // fixed order
-        const float4 f = reinterpret_cast<const float4*>(wsum[g])[w];
-        tot += f.x; tot += f.y; tot += f.z; tot += f.w;
-      }
-      wgt[g] *= rsqrtf(tot / static_cast<float>(H) + eps);
-    }
+        for (int i = 0; i < NW / 4; ++i) {  // fixed order
+          const float4 f = reinterpret_cast<const float4*>(part[turn][g])[i];
+          tot += f.x; tot += f.y; tot += f.z; tot += f.w;
+        }
+        wgt[g] *= rsqrtf(tot / static_cast<float>(H) + eps);
 #pragma unroll
-    for (int g = 0; g < G; ++g) {  // slot order within the group
-      if (q[g] < 0) continue;
-#pragma unroll
-      for (int i = 0; i < NF4; ++i) {
-        const float4 f = v[g][i].get();
-        acc[i].x += f.x * wgt[g]; acc[i].y += f.y * wgt[g];
-        acc[i].z += f.z * wgt[g]; acc[i].w += f.w * wgt[g];
+        for (int c = 0; c < NO; ++c)
+          if ((c * TH + tid) * 8 < H) v[g][c].add_to(acc[c], wgt[g]);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < NF4; ++i) {
-    if (i * COMBINE_THREADS + tid < n4) {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(acc[i].x, acc[i].y);
-      __nv_bfloat162 hi = __floats2bfloat162_rn(acc[i].z, acc[i].w);
-      uint2 pk;
-      pk.x = *reinterpret_cast<uint32_t*>(&lo);
-      pk.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(out + static_cast<size_t>(t) * H + (i * COMBINE_THREADS + tid) * 4) = pk;
+  for (int c = 0; c < NO; ++c) {
+    if ((c * TH + tid) * 8 >= H) break;
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(acc[c][2 * i], acc[c][2 * i + 1]);
+      o[i] = *reinterpret_cast<const uint32_t*>(&h);
     }
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * H + (c * TH + tid) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -583,7 +542,7 @@ static inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 static int check_cfg(const MskMoeCfg* c) {
   if (c == nullptr) return MSK_ERR_NULL;
   if (c->hidden <= 0 || c->inter <= 0 || c->hidden % 256 != 0 || c->inter % 256 != 0) return MSK_ERR_SHAPE;
-  if (c->hidden > COMBINE_THREADS * COMBINE_MAX_F4 * 4) return MSK_ERR_SHAPE;  // combine keeps a row in registers
+  if (c->hidden > COMBINE_MAX_H) return MSK_ERR_SHAPE;  // combine keeps a row in registers
   if (c->max_tokens < 0) return MSK_ERR_SHAPE;
   if (c->top_k < 1 || c->top_k > MAX_TOP_K) return MSK_ERR_SHAPE;
   if (c->local_count < 1 || c->local_count > MAX_LOCAL_EXPERTS) return MSK_ERR_SHAPE;
@@ -1404,8 +1363,8 @@ static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, con
   lc.numAttrs = 1;
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   const int H = static_cast<int>(cfg->hidden), k = static_cast<int>(cfg->top_k);
+  const bool few_local = static_cast<long long>(k) * cfg->local_count <= 2LL * cfg->n_experts;   // two or fewer of a token's routes expected
   if (!post_norm) {
-    const bool few_local = static_cast<long long>(k) * cfg->local_count <= 2LL * cfg->n_experts;   // two or fewer of a token's routes expected
     const int cols = few_local ? 1024 : 256;
     const long long items = static_cast<long long>(n_tokens) * ((H + cols - 1) / cols);
     lc.gridDim = dim3(static_cast<unsigned>((items + COMBINE_COLS_WARPS - 1) / COMBINE_COLS_WARPS));
@@ -1415,11 +1374,17 @@ static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, con
     return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, n_tokens, H, k));
   }
   lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
-  lc.blockDim = dim3(COMBINE_THREADS);
-  const bool wide = n_tokens >= COMBINE_WIDE_TOKENS;
-  const bool narrow_rows = H <= COMBINE_THREADS * 2 * 4;   // two float4 slots per thread hold a row
-  auto* kern = y_bf16 ? (narrow_rows ? combine_norm_kernel<8, true, 2, 2> : combine_norm_kernel<4, true, 2>)
-                      : (wide ? combine_norm_kernel<2, false, 2> : combine_norm_kernel<4, false, 1>);
+  const bool narrow = H <= 4096;
+  if (n_tokens < COMBINE_FEW_TOKENS) {
+    lc.blockDim = dim3(512);
+    auto* kern = y_bf16 ? (narrow ? combine_norm_kernel<true, 512, 1, 8, 1> : combine_norm_kernel<true, 512, 2, 8, 1>)
+                        : (narrow ? combine_norm_kernel<false, 512, 1, 8, 1> : combine_norm_kernel<false, 512, 2, 4, 1>);
+    return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, H, k, cfg->post_norm_eps));
+  }
+  lc.blockDim = dim3(narrow ? 128 : 256);
+  auto* kern = !y_bf16 ? (narrow ? combine_norm_kernel<false, 128, 4, 2, 4> : combine_norm_kernel<false, 256, 4, 2, 2>)
+               : few_local ? (narrow ? combine_norm_kernel<true, 128, 4, 2, 5> : combine_norm_kernel<true, 256, 4, 2, 3>)
+                           : (narrow ? combine_norm_kernel<true, 128, 4, 4, 4> : combine_norm_kernel<true, 256, 4, 4, 2>);
   return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, H, k, cfg->post_norm_eps));
 }
 
@@ -2000,7 +1965,7 @@ int msk_moe_attrs(int which, int token_tile, int* host_out) {
       }
       break;
     }
-    case 4: e = cudaFuncGetAttributes(&a, combine_norm_kernel<4, false, 1>); break;
+    case 4: e = cudaFuncGetAttributes(&a, combine_norm_kernel<false, 512, 1, 8, 1>); break;
     default: return MSK_ERR_SHAPE;
   }
   if (e != cudaSuccess) return static_cast<int>(e);

@@ -555,6 +555,29 @@ def test_pair_kernel_at_every_width_of_its_mmas(cuda_dev, H, I, counts):
     _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
+@pytest.mark.parametrize("H,T,k,tile,lo,nloc", [(4096, 255, 3, 16, 0, 12), (4096, 256, 9, 64, 0, 12), (4096, 256, 9, 128, 0, 12), (4352, 256, 3, 128, 4, 6),
+                                                (8192, 257, 5, 128, 0, 12), (8192, 256, 5, 16, 0, 12), (8192, 255, 5, 128, 0, 12), (8192, 20, 9, 16, 2, 9),
+                                                (256, 300, 16, 128, 0, 16), (256, 300, 2, 128, 3, 5)])
+def test_combine_with_the_norm_at_its_block_sizes(cuda_dev, H, T, k, tile, lo, nloc):
+    """The combine with the post-expert norm in each of its forms (few and many tokens, up to and beyond 4096 columns, FP32 and BF16
+    rows, few and many local routes), tokens without a local route among them."""
+    m, inputs, _lib, orc = _mods()
+    E = 16 if nloc == 16 else 12
+    w = inputs.make_weights(H, 256, nloc, 103, cuda_dev, post_norm=True)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T, local_start=lo, token_tile=tile)
+    g = torch.Generator(device=cuda_dev).manual_seed(107)
+    ids = torch.rand((T, E), generator=g, device=cuda_dev).topk(k, 1)[1].to(torch.int32)
+    ids[3] = ids[T - 1] = -1
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    tw = torch.rand((T, k), generator=g, device=cuda_dev)
+    out = m.kernel_fn({"hidden_states": x, "topk_ids": ids.contiguous(), "topk_weights": tw}, st)
+    torch.cuda.synchronize()
+    assert m.read_status(st) == 0
+    assert not out[3].any() and not out[T - 1].any()
+    ref, parts = orc.moe_forward(x, ids, tw, w, local_start=lo, return_parts=True)
+    _check_forward(out, ref, parts, m.workspace_views(st, T))
+
+
 @pytest.mark.parametrize("E,k,nloc,T", [(8, 2, 8, 256), (128, 8, 4, 700)])
 def test_pair_kernel_by_default_on_a_handful_of_experts(cuda_dev, E, k, nloc, T):
     """The default plan takes the pair kernel by the mean rows per expert, also where only a handful of experts is there."""
