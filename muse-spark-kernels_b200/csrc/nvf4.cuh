@@ -76,6 +76,10 @@ constexpr int NV_AHEAD = 8;                                // stages of the firs
 __host__ __device__ inline int nv_tiles(int c) { return (c + NV_ROWS - 1) / NV_ROWS; }
 __host__ __device__ inline int nv_tile_rows(int c, int n) { return n <= 1 ? c : ((c + n - 1) / n + 7) & ~7; }
 __host__ __device__ inline int nv_width(int rows) { return (rows + 7) >> 3; }
+// Rows that its image and its MMAs have room for: up to four rows take four. (The second level's two digits of four rows are the narrowest MMA; room for
+// twelve needs scale columns of their own and was 1 to 2 % slower.) With room for eight only, a row of steps in turn on one box, before / after: 8
+// tokens 106.4 / 103.7 us, 16: 163.8 / 159.2, 32: 214.9 / 209.9, 64: 242.6 / 238.2; fewer columns and token rows' bytes, and with them less power.
+__host__ __device__ inline int nv_room(int rows) { return rows <= 4 ? 4 : 8 * nv_width(rows); }
 // Groups that the image of an expert's rows takes: all tiles but the last have whole ones.
 constexpr int NV_GROUPS = NV_ROWS / 8;
 __host__ __device__ inline int nv_groups(int c) { return nv_width(c); }
@@ -137,7 +141,7 @@ struct NvCtrl {
   uint64_t u_full[NV_UNITS], u_empty[NV_UNITS];
   uint64_t stored[NV_UNITS];             // the epilogue has stored its values of a unit
   NvUnit unit[NV_UNITS];
-  uint4 route[MAX_TOP_K];                // of the token row that is split: place of its digits in the image, tile's width, tile, row in it
+  uint4 route[MAX_TOP_K];                // of the token row that is split: place of its digits in the image, its tile's room, tile, row in it
   float red[NV_SPLIT_THREADS / 32];
   int n_routes;
   uint32_t tmem_base;
@@ -148,7 +152,7 @@ struct NvCtrl {
 static_assert(sizeof(NvCtrl) <= 1024 && offsetof(NvCtrl, unit) % 16 == 0, "control block");
 
 constexpr int NV_LAST = 4;
-__host__ __device__ constexpr int nv_place_bytes(int width) { return (width * NV_LEVEL_BYTES + 1023) / 1024 * 1024; }
+__host__ __device__ constexpr int nv_place_bytes(int room) { return (room * (NV_LEVEL_BYTES / 8) + 1023) / 1024 * 1024; }
 
 struct NvCfg {
   static constexpr int TABLE_INTS = MAX_LOCAL_EXPERTS + 4;
@@ -157,7 +161,7 @@ struct NvCfg {
   static constexpr int B_RING = 76 * 1024;
   static constexpr int W_OFF = 0, B_OFF = NV_W_STAGES * STAGE_W_BYTES, CTL_OFF = B_OFF + B_RING, TABLE_OFF = CTL_OFF + 1024;
   static constexpr int SMEM_BYTES = TABLE_OFF + 4 * TABLE_INTS * 4;
-  static_assert(SMEM_BYTES <= 232448 && 4 * nv_place_bytes(NV_GROUPS) <= B_RING, "shared memory of a CTA");
+  static_assert(SMEM_BYTES <= 232448 && 4 * nv_place_bytes(NV_ROWS) <= B_RING, "shared memory of a CTA");
   // TMEM: accumulators of two tiles (digits x rows columns each; those of a tile of eight rows twice), two stages of scales
   static constexpr int D_WIDE = NV_PARTS * NV_ROWS, D_NARROW = NV_PARTS * 8;
   static constexpr int S_BASE = 2 * D_WIDE, S_COLS = 32, S_B = S_BASE + NV_S_STAGES * S_COLS;   // 4 x 4 columns per weight tile, 4 x 8 for the token rows
@@ -210,9 +214,9 @@ __device__ __forceinline__ bool mma_nvf4_stage(uint32_t d0, uint32_t d1, uint64_
 }
 #undef NV_MMA
 
-// ---- the split. Image of a tile (width W groups, K): per K stage of 256 and level, digits [9, 2 or 4][W][8 rows][128 bytes], the eight
-// 16-byte chunks of a row in the order of the 128-byte swizzle (chunk c of row r at c ^ r: a row's digit is one line to write), then
-// scales [8 W rows][16]; one contiguous copy a level, NV_GROUP_BYTES * W bytes a stage.
+// ---- the split. Image of a tile (room for R rows, K): per K stage of 256 and level, digits [9, 2 or 4][R rows][128 bytes], the eight
+// 16-byte chunks of a row in the order of the 128-byte swizzle (chunk c of row n = digit * R + r at c ^ (n & 7): a row's digit is one line to
+// write), then scales [R rows][16]; one contiguous copy a level, NV_GROUP_BYTES / 8 * R bytes a stage.
 __device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
 constexpr int NV_MAX_EXP = 14;   // of a block's unit: 65504 is below four of 2^14
 constexpr int NV_MIN_EXP = 0;    // its ninth digit is a step of 2^-24, the smallest there is
@@ -319,11 +323,12 @@ __device__ __forceinline__ void nv_split_block(const uint32_t (&h)[8], bool mine
 }
 
 // Where a row of a tile lies in a digit, a block's codes in its row, its scale in a level.
-__device__ __forceinline__ int nv_row_at(int slot) { return (slot >> 3) * 1024 + (slot & 7) * 128; }
-__device__ __forceinline__ int nv_code_at(int slot, int blk) { return ((((blk & 15) >> 1) ^ (slot & 7)) * 16) + (blk & 1) * 8; }
-__device__ __forceinline__ int nv_digit_at(int width, int level, int d) { return width * (nv_level_at(level) + d * 1024); }
-__device__ __forceinline__ int nv_scale_at(int width, int level, int slot, int blk) {
-  return nv_digit_at(width, level, nv_digits(level)) + slot * 16 + (blk & 15);
+__device__ __forceinline__ int nv_digit_at(int room, int level, int d) { return room * (nv_level_at(level) / 8 + d * 128); }
+__device__ __forceinline__ int nv_code_at(int room, int level, int d, int slot, int blk) {
+  return nv_digit_at(room, level, d) + slot * 128 + (((blk & 15) >> 1) ^ ((d * room + slot) & 7)) * 16 + (blk & 1) * 8;
+}
+__device__ __forceinline__ int nv_scale_at(int room, int level, int slot, int blk) {
+  return nv_digit_at(room, level, nv_digits(level)) + slot * 16 + (blk & 15);
 }
 
 // Which accumulators the units take in turn: tiles of up to eight rows one or the other, wider ones both (as PairBuffers).
@@ -517,7 +522,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
     if (lane == 0) {
       tile_start[p.nloc] = tiles;
       group_start[p.nloc] = groups;
-      ctl.b_bytes = nv_place_bytes(nv_width(max(1, min(most, NV_ROWS))));   // (no tile at all: places that nobody uses)
+      ctl.b_bytes = nv_place_bytes(nv_room(min(most, NV_ROWS)));   // (no tile at all: places that nobody uses)
       ctl.b_stages = min(NV_MARKS, C::B_RING / ctl.b_bytes);
     }
   }
@@ -569,9 +574,9 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         const unsigned have = __ballot_sync(0xffffffffu, q >= 0);
         if (q >= 0) {
           const int e = id - p.lo, c = cnt_s[e], per = nv_tile_rows(c, nv_tiles(c)), r = q - off_s[e], ti = r / per, slot = r - ti * per;
-          const int group = group_start[e] + ti * (per >> 3), width = nv_width(min(per, c - ti * per));
+          const int group = group_start[e] + ti * (per >> 3), room = nv_room(min(per, c - ti * per));
           ctl.route[__popc(have & ((1u << th) - 1u))] =
-              make_uint4(static_cast<uint32_t>(group * (p.H / KS) * NV_GROUP_BYTES), static_cast<uint32_t>(width),
+              make_uint4(static_cast<uint32_t>(group * (p.H / KS) * NV_GROUP_BYTES), static_cast<uint32_t>(room),
                          static_cast<uint32_t>(tile_start[e] + ti), static_cast<uint32_t>(slot));
         }
         if (th == 0) ctl.n_routes = __popc(have);
@@ -594,26 +599,25 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         const int third = j / by_route, r0 = j - third * by_route, b = stage * 16 + (lane & 15);
         const uint4 v0 = row_s[2 * b], v1 = row_s[2 * b + 1];
         const uint32_t g[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        auto at = [&](const uint4& to) { return p.img[0] + (to.x + to.y * static_cast<uint32_t>(stage * NV_GROUP_BYTES)); };
+        auto at = [&](const uint4& to) { return p.img[0] + (to.x + to.y * static_cast<uint32_t>(stage * (NV_GROUP_BYTES / 8))); };
         unsigned more[2];
         nv_split_block(g, first + (lane >> 4) < shares, NV_PARTS / by_digit, NV_PARTS / by_digit * (third + 1), third == 0, more[0], more[1],
             [&](uint32_t s0, uint32_t s1, uint32_t s2) {
 #pragma unroll 1
               for (int s = r0; s < n_routes; s += by_route) {
                 const uint4 to = ctl.route[s];
-                const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
+                const int room = static_cast<int>(to.y), slot = static_cast<int>(to.w);
                 uint8_t* img = at(to);
-                img[nv_scale_at(width, 0, slot, b)] = static_cast<uint8_t>(s0);
-                img[nv_scale_at(width, 1, slot, b)] = static_cast<uint8_t>(s1);
-                img[nv_scale_at(width, 2, slot, b)] = static_cast<uint8_t>(s2);
+                img[nv_scale_at(room, 0, slot, b)] = static_cast<uint8_t>(s0);
+                img[nv_scale_at(room, 1, slot, b)] = static_cast<uint8_t>(s1);
+                img[nv_scale_at(room, 2, slot, b)] = static_cast<uint8_t>(s2);
               }
             },
             [&](int level, int d, uint2 w) {
 #pragma unroll 1
               for (int s = r0; s < n_routes; s += by_route) {
                 const uint4 to = ctl.route[s];
-                const int width = static_cast<int>(to.y), slot = static_cast<int>(to.w);
-                *reinterpret_cast<uint2*>(at(to) + nv_digit_at(width, level, d) + nv_row_at(slot) + nv_code_at(slot, b)) = w;
+                *reinterpret_cast<uint2*>(at(to) + nv_code_at(static_cast<int>(to.y), level, d, static_cast<int>(to.w), b)) = w;
               }
             });
 #pragma unroll
@@ -715,10 +719,10 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
           if (st == 0u && lane == 0) MSK_TR(TR_FIRST_MMA);
           const int pass = ctl.b_pass[bs], level = pass & 3;
           last = static_cast<uint32_t>(pass & NV_LAST);
-          const uint32_t mark = st % NV_MARKS, rows = static_cast<uint32_t>(8 * u.width), first = static_cast<uint32_t>(nv_first(level)) * rows;
+          const uint32_t mark = st % NV_MARKS, rows = static_cast<uint32_t>(nv_room(u.rows)), first = static_cast<uint32_t>(nv_first(level)) * rows;
           ++st;
           ready = mma_nvf4_stage(d0 + first, d1 + first, a0 + ((ws * STAGE_W_BYTES) >> 4), b0 + ((bs * b_bytes) >> 4),
-                                 idesc_nvf4(static_cast<uint32_t>(nv_digits(level)) * rows), tmem + C::S_BASE + (wst % NV_S_STAGES) * C::S_COLS,
+                                 idesc_nvf4((static_cast<uint32_t>(nv_digits(level)) * rows + 7u) & ~7u), tmem + C::S_BASE + (wst % NV_S_STAGES) * C::S_COLS,
                                  tmem + C::S_B + ss * C::S_COLS, accumulate,
                                  smem_u32(&ctl.done[mark]), smem_u32(&ctl.w_done[ws]), last, smem_u32(&ctl.s_full[st % NV_S_STAGES]), (st / NV_S_STAGES) & 1u);
           accumulate = 1u;
@@ -756,11 +760,11 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
             last_tile = u.tile;
           }
         }
-        const int nst = p.K[u.phase] / KS;
+        const int nst = p.K[u.phase] / KS, room = nv_room(u.rows);
         const uint8_t* src = p.img[u.phase] + static_cast<size_t>(u.group) * nst * NV_GROUP_BYTES;
         const unsigned int* flags = tile + (u.phase == 0 ? NV_MORE : NV_MORE_INTER);
         unsigned int more1 = 0u, more2 = 0u;
-        for (int ks = 0; ok && ks < nst; ++ks, more1 >>= 1, more2 >>= 1, src += u.width * NV_GROUP_BYTES) {
+        for (int ks = 0; ok && ks < nst; ++ks, more1 >>= 1, more2 >>= 1, src += room * (NV_GROUP_BYTES / 8)) {
           if ((ks & 31) == 0) {
             more1 = __ldcg(flags + ks / 16);
             more2 = __ldcg(flags + ks / 16 + 1);
@@ -769,9 +773,9 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
             if ((level == 1 && (more1 & 1u) == 0u) || (level == 2 && (more2 & 1u) == 0u)) continue;
             const uint32_t before = st - b_stages;
             if (st >= b_stages && !mbar_wait_inline(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
-            const uint32_t bytes = static_cast<uint32_t>(u.width * (nv_digits(level) * 1024 + 128));
+            const uint32_t bytes = static_cast<uint32_t>(room * (nv_digits(level) * 128 + 16));
             mbar_arrive_expect_tx(&ctl.b_full[bs], bytes);
-            bulk_g2s(b_ring + bs * b_bytes, src + u.width * nv_level_at(level), bytes, &ctl.b_full[bs], keep);
+            bulk_g2s(b_ring + bs * b_bytes, src + nv_digit_at(room, level, 0), bytes, &ctl.b_full[bs], keep);
             const bool last = level == 2 || ((level == 1 || (more1 & 1u) == 0u) && (more2 & 1u) == 0u);
             ctl.b_pass[bs] = level | (last ? NV_LAST : 0);
             mbar_arrive(&ctl.b_full[bs]);
@@ -817,8 +821,9 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       if (u.phase < 0) break;
       const int nst = p.K[u.phase] / KS;
       // This lane's token row: column c of a stage's scales is that of the MMA's columns 32 c + lane, digit after digit of the tile's
-      // rows: with one or two groups of eight all columns are alike.
-      const uint32_t row_at = (lane % static_cast<uint32_t>(8 * u.width)) * 16u;
+      // rows: with room for four, eight or sixteen all columns are alike.
+      const int room = nv_room(u.rows);
+      const uint32_t row_at = static_cast<uint32_t>(lane & (room - 1)) * 16u;
       for (int ks = 0; ok && ks < nst; ++ks, ++wst) {
         const uint32_t ws = wst % NV_W_STAGES;
         if (!mbar_wait_warp(&ctl.w_full[ws], (wst / NV_W_STAGES) & 1u, abortw)) { ok = false; break; }
@@ -858,7 +863,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
           if (!mbar_wait_warp(&ctl.b_full[bs], bpar, abortw)) { ok = false; break; }
           const int pass = ctl.b_pass[bs];
           last = (pass & NV_LAST) != 0;
-          const uint8_t* sc = b_ring + bs * b_bytes + nv_digits(pass & 3) * 1024 * u.width;
+          const uint8_t* sc = b_ring + bs * b_bytes + nv_digits(pass & 3) * 128 * room;
           const uint4 v = *reinterpret_cast<const uint4*>(sc + row_at);
           const uint32_t before = st - NV_S_STAGES;
           if (st >= NV_S_STAGES && !mbar_wait_warp(&ctl.done[before % NV_MARKS], (before / NV_MARKS) & 1u, abortw)) { ok = false; break; }
@@ -907,6 +912,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       tc_fence_after();
       if (leader) { if (n_unit == 0u) MSK_TR(TR_FIRST_DFULL); MSK_TR(TR_LAST_DFULL); }
       const uint32_t d0 = tmem + quarter + db.col(), d1 = d0 + db.tile_cols();
+      const int room = nv_room(u.rows);
 #pragma unroll 1
       for (int c0 = 0; c0 < u.rows; c0 += 8) {
         const int left = u.rows - c0;
@@ -914,7 +920,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         {
           uint32_t v[NV_PARTS][8];
 #pragma unroll
-          for (int q = 0; q < NV_PARTS; ++q) tmem_ld8(d0 + q * 8 * u.width + c0, v[q]);
+          for (int q = 0; q < NV_PARTS; ++q) tmem_ld8(d0 + q * room + c0, v[q]);
           tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -923,7 +929,7 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
             for (int q = NV_PARTS - 2; q >= 0; --q) a0[j] = fmaf(a0[j], 0.125f, __uint_as_float(v[q][j]));
           }
 #pragma unroll
-          for (int q = 0; q < NV_PARTS; ++q) tmem_ld8(d1 + q * 8 * u.width + c0, v[q]);
+          for (int q = 0; q < NV_PARTS; ++q) tmem_ld8(d1 + q * room + c0, v[q]);
           tmem_wait_ld();
           if (left <= 8) {                         // the accumulators are read
             tc_fence_before();
@@ -989,7 +995,8 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
       };
       const int last = min(first + (1 << bits), u.rows);
       unsigned any1 = 0u, any2 = 0u;
-      uint8_t* stage = p.img[1] + (static_cast<size_t>(u.group) * n_stages + static_cast<size_t>(blk >> 4) * u.width) * NV_GROUP_BYTES;
+      const int room = nv_room(u.rows);
+      uint8_t* stage = p.img[1] + static_cast<size_t>(u.group) * n_stages * NV_GROUP_BYTES + static_cast<size_t>((blk >> 4) * room) * (NV_GROUP_BYTES / 8);
       load(first + (lane >> 4));
 #pragma unroll 1
       for (int r0 = first; r0 < last; r0 += 2) {
@@ -997,14 +1004,13 @@ __global__ void __launch_bounds__(NV_THREADS, 1) moe_nvf4_kernel(const __grid_co
         const uint32_t h8[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         load(slot + 2);                            // the next two rows, while these are split
         unsigned more1, more2;
-        uint8_t* at = stage + nv_row_at(slot) + nv_code_at(slot, blk);
         nv_split_block(h8, slot < last, NV_PARTS, NV_PARTS, true, more1, more2,
             [&](uint32_t s0, uint32_t s1, uint32_t s2) {
-              stage[nv_scale_at(u.width, 0, slot, blk)] = static_cast<uint8_t>(s0);
-              stage[nv_scale_at(u.width, 1, slot, blk)] = static_cast<uint8_t>(s1);
-              stage[nv_scale_at(u.width, 2, slot, blk)] = static_cast<uint8_t>(s2);
+              stage[nv_scale_at(room, 0, slot, blk)] = static_cast<uint8_t>(s0);
+              stage[nv_scale_at(room, 1, slot, blk)] = static_cast<uint8_t>(s1);
+              stage[nv_scale_at(room, 2, slot, blk)] = static_cast<uint8_t>(s2);
             },
-            [&](int level, int d, uint2 w) { *reinterpret_cast<uint2*>(at + nv_digit_at(u.width, level, d)) = w; });
+            [&](int level, int d, uint2 w) { *reinterpret_cast<uint2*>(stage + nv_code_at(room, level, d, slot, blk)) = w; });
         any1 |= more1;
         any2 |= more2;
       }

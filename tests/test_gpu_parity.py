@@ -1537,6 +1537,38 @@ def test_activations_enter_the_gemms_exactly(cuda_dev, tile):
     assert torch.equal(v["y"], want.float())
 
 
+@pytest.mark.parametrize("counts", [[1, 2, 3, 4, 5, 8, 9, 12], [4, 4, 4, 4, 4, 4, 4, 3], [17, 18, 19, 20, 4, 3, 2, 1]])
+def test_nvf4_tiles_with_room_for_four_rows_hold_every_level(cuda_dev, counts):
+    """Tiles of one to four rows, alone and behind whole ones, beside wider tiles: experts that hand their row through (gate x[0] = 32, up x[i] / 32),
+    rows with second and third levels of digits in every K stage; y and inter bit for bit, twice."""
+    m, inputs, _lib, orc = _mods()
+    H, E, k, T = 1536, 8, 1, sum(counts)
+    eye = torch.zeros((H, H), dtype=torch.uint8, device=cuda_dev)
+    eye.fill_diagonal_(2)                                         # E2M1 code of 1
+    gate = torch.zeros_like(eye)
+    gate[:, 0] = 2
+    pack = lambda c: (c[:, 0::2] | (c[:, 1::2] << 4)).expand(E, -1, -1).contiguous()  # noqa: E731
+    sf13 = torch.full((E, 2 * H, H // 16), 0x38, dtype=torch.uint8, device=cuda_dev)      # 1
+    sf13[:, H:] = 0x10                                            # 2^-5
+    one = torch.ones(E, device=cuda_dev)
+    w = {"w13": pack(torch.cat([gate, eye])), "w13_sf": sf13, "w13_gs": one, "w2": pack(eye),
+         "w2_sf": torch.full((E, H, H // 16), 0x38, dtype=torch.uint8, device=cuda_dev), "w2_gs": one}
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=T)
+    assert _nvf4_takes(st, T)
+    g = torch.Generator(device=cuda_dev).manual_seed(37)
+    x = _wide_rows(T, H, g, cuda_dev)
+    x[:, 0] = 32.0
+    d = {"hidden_states": x, "topk_ids": _ids_of_counts(counts, 0, k, cuda_dev), "topk_weights": torch.ones((T, k), device=cuda_dev)}
+    for _ in range(2):
+        m.kernel_fn(d, st)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0
+        v = m.workspace_views(st, T)
+        want = x.half()[v["perm"].long()]
+        assert torch.equal(v["inter"], want)
+        assert torch.equal(v["y"], want.float())
+
+
 @pytest.mark.parametrize("large", [1000.0, 20000.0])
 def test_nvf4_kernel_beside_large_channels_that_the_weights_ignore(cuda_dev, large):
     """Every sixteenth channel large, in the token rows and in inter, the others orders below, and weights of zero
