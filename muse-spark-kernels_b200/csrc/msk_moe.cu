@@ -47,11 +47,14 @@ __device__ __forceinline__ long long source_row(const RepackGeom& g, long long o
 // each of the eight rows and writes four full 128-byte lines, eight such steps (4 KB) in flight. The form
 // this replaces gave each thread one 16-byte piece with the rows running along the lanes (16 useful bytes
 // of every 32-byte sector on the source side): 128 experts of 4096 x 1536, both matrices, 535 us in and
-// 722 us back out.
+// 722 us back out. Blocks of eight warps on the way in, of one on the way out, where a warp's eight rows are pages of their own: both
+// matrices 426 us in, 423 out; with blocks of 32 / 64 / 128 / 256 / 512 / 1024 threads 428 / 430 / 430 / 426 / 431 / 457 in, 423 / 429 / 429 / 445 / 445 / 465 out
+// (what has to be read and written takes 416 at the rate of a copy).
+template <bool INVERSE> constexpr int REPACK_WARPS = INVERSE ? 1 : 8;
 template <bool INVERSE>
-__global__ void __launch_bounds__(256) repack_kernel(uint8_t* codes, uint8_t* sf, uint8_t* packed, RepackGeom g,
+__global__ void __launch_bounds__(REPACK_WARPS<INVERSE> * 32) repack_kernel(uint8_t* codes, uint8_t* sf, uint8_t* packed, RepackGeom g,
                                                      long long n_og) {
-  const long long og = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const long long og = static_cast<long long>(blockIdx.x) * REPACK_WARPS<INVERSE> + (threadIdx.x >> 5);
   if (og >= n_og) return;
   const int lane = threadIdx.x & 31, r = lane >> 2, c4 = lane & 3;
   const long long srow = source_row(g, og) + r;
@@ -1100,17 +1103,16 @@ static int repack_common(const MskMoeCfg* cfg, void* w13, void* w13_sf, void* w2
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const RepackGeom g13 = geom13(cfg), g2 = geom2(cfg);
   const long long n13 = n_og_of(cfg, g13), n2 = n_og_of(cfg, g2);
-  const unsigned b13 = static_cast<unsigned>((n13 + 7) / 8), b2 = static_cast<unsigned>((n2 + 7) / 8);
+  auto launch = [&](auto kern, int warps, void* codes, void* sf, void* packed, const RepackGeom& g, long long n) {
+    kern<<<static_cast<unsigned>((n + warps - 1) / warps), warps * 32, 0, st>>>(static_cast<uint8_t*>(codes), static_cast<uint8_t*>(sf),
+                                                                               static_cast<uint8_t*>(packed), g, n);
+  };
   if (!inverse) {
-    repack_kernel<false><<<b13, 256, 0, st>>>(static_cast<uint8_t*>(w13), static_cast<uint8_t*>(w13_sf),
-                                              static_cast<uint8_t*>(packed13), g13, n13);
-    repack_kernel<false><<<b2, 256, 0, st>>>(static_cast<uint8_t*>(w2), static_cast<uint8_t*>(w2_sf),
-                                             static_cast<uint8_t*>(packed2), g2, n2);
+    launch(repack_kernel<false>, REPACK_WARPS<false>, w13, w13_sf, packed13, g13, n13);
+    launch(repack_kernel<false>, REPACK_WARPS<false>, w2, w2_sf, packed2, g2, n2);
   } else {
-    repack_kernel<true><<<b13, 256, 0, st>>>(static_cast<uint8_t*>(w13), static_cast<uint8_t*>(w13_sf),
-                                             static_cast<uint8_t*>(packed13), g13, n13);
-    repack_kernel<true><<<b2, 256, 0, st>>>(static_cast<uint8_t*>(w2), static_cast<uint8_t*>(w2_sf),
-                                            static_cast<uint8_t*>(packed2), g2, n2);
+    launch(repack_kernel<true>, REPACK_WARPS<true>, w13, w13_sf, packed13, g13, n13);
+    launch(repack_kernel<true>, REPACK_WARPS<true>, w2, w2_sf, packed2, g2, n2);
   }
   return static_cast<int>(cudaGetLastError());
 }
