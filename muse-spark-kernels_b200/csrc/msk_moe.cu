@@ -603,16 +603,18 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     p.N = c->token_tile;
   } else {
     const double rpe = static_cast<double>(T) * c->top_k / c->n_experts;  // mean tokens per expert
-    // measured at H4096 I1536 E128 (us a step with 16 / 64-token tiles, near-even routing): T = 160 (rpe 10): 268 / 281;
-    // T = 192 (rpe 12): 313 / 302. 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
+    // 16 / 64-token tile (us, rows of steps): H2048 I1024 E64 near-even rpe 4 58.9 / 58.8, 6 61.1 / 59.8, 8 63.2 / 61.2, 12 68.9 / 63.0, a few experts
+    // taking most tokens 45.3 / 47.0, 51.9 / 51.4, 55.1 / 53.7, 67.0 / 59.6; H4096 I1024 E128 rpe 4 193 / 199 (105 / 90), 6 202 / 205, 8 210 / 208 (158 / 117), 12
+    // 238 / 215 (210 / 144); H4096 I1280 E128 rpe 6 247 / 250, 8 254 / 252. 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
     // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. Beyond: rpe 48 near-even
     // 406 / 464, 32 of 256 experts at H4096 I4096 255 / 289, a few experts taking most 456 / 420, the same at H2048 I1024 E64
     // 107 / 88; rpe 56 445 / 477, 279 / 295, 508 / 452, 114 / 95; rpe 64 near-even 566 / 505. At rpe 40 the 64-token tile loses 13 %
     // at worst and the pair kernel 18, at 48 it is 21 and 20. The 16-token tile is the
     // fastest per K stage and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The
     // host does not know the counts, and the less even they are the lower that line lies. The 32-token tile never wins at
-    // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh)
-    p.N = rpe <= 12 ? 16 : rpe <= 40 ? 64 : 128;
+    // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh). Where a path is asked for
+    // the narrow tile, which the paths are made for, stays up to 12.
+    p.N = rpe <= (c->decode_path == 0 ? 7 : 12) ? 16 : rpe <= 40 ? 64 : 128;
   }
   const long long rows = static_cast<long long>(T) * c->top_k;
   // Flat shares are an option, off by default: measured on B200 a cut unit's pieces cost about 6 us of
@@ -663,6 +665,9 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
 // (134 / 116), 192 (12 rows an expert) 339 / 305 (278 / 246); 224: 320 / 351 (191 / 285), 256: 325 / 382 (213 / 309): beyond 12 rows an expert the other
 // one is the 64-token tile, which streams the weights of an expert with many rows once for 64 of them, this one for 16. Uneven steps of 9
 // to 16 tokens lose 1 to 3 %, near-even ones, which stream twice the bytes, gain 13 to 17: the line stays at 6.
+// With the other kernel's issue by one thread and this one's room for four rows (64-token tile / this one, rows of steps) 64: 288 / 240 (123 / 135), 128: 296 / 272
+// (161 / 200), 160: 299 / 292 (182 / 235), 192: 304 / 316 (198 / 263), 256: 316 / 384 (230 / 323); a rank, two experts taking most, 100: 158 / 154, 200: 205 / 213, 384:
+// 242 / 281; H7168 I2048, even, 200: 171 / 159, 300: 176 / 175, 384: 178 / 192: near the line the other one has drawn level.
 // A rank (32 of 256, one row a token): H4096 I4096, two experts taking most, 4: 45 / 46, 6: 50 / 49, 8: 59 / 58, 10: 59 / 62, 16: 66 / 67, 18: 69 / 69, 20: 70 / 69,
 // 24: 79 / 76, 28: 86 / 80, 64: 138 / 115, 384: 308 / 263 (512: 236 / 310); H7168 I2048, even, 4: 50 / 51, 6: 50 / 53, 8: 56 / 58, 16: 74 / 74, 18: 77 / 77, 20: 81 /
 // 79, 24: 83 / 80, 28: 91 / 88, 64: 128 / 114, 384: 201 / 171.
