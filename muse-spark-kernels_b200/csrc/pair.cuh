@@ -106,7 +106,7 @@ struct alignas(16) PairUnit {              // written and read 16 bytes at a tim
   int phase;                             // -1: no more units
   int expert, row0, rows, pair, tile;
   int nmma;                              // rows rounded up to 16
-  int pad_;
+  int again;                             // its weights are read by other tiles of the expert as well
 };
 
 struct PairCtrl {
@@ -301,7 +301,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     if (!wait(&ctl.u_full[s], (ui / PAIR_UNITS) & 1u, abortw)) return false;
     const int4 x = *reinterpret_cast<const int4*>(&ctl.unit[s]), y = *(reinterpret_cast<const int4*>(&ctl.unit[s]) + 1);
     u.phase = x.x; u.expert = x.y; u.row0 = x.z; u.rows = x.w;
-    u.pair = y.x; u.tile = y.y; u.nmma = y.z;
+    u.pair = y.x; u.tile = y.y; u.nmma = y.z; u.again = y.w;
     ++ui;
     return true;
   };
@@ -310,7 +310,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
   if (warp == 0) {
     // ------------------------------------------------------- weight producer
     if (lane == 0) {
-      const uint64_t pol = policy_evict_first();
+      // Weights that one tile reads leave L2 first. Those of an expert with several tiles are read again within microseconds: first to leave
+      // as well, they came from memory for each tile (8192 tokens of Zipf routes 2436 -> 2366 us in a row of steps, evenly spread 2400 -> 2327, one rank
+      // of eight, H7168 I2048, 729 -> 716, 3012 skewed tokens of a rank 537 -> 527).
+      const uint64_t once = policy_evict_first(), several = policy_evict_normal();
       uint32_t ws = 0, wpar = 0;
       bool ok = true;
       PairUnit u;
@@ -319,6 +322,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
         if (u.phase < 0) break;
         const int nst = p.K[u.phase] / KS;
         const uint8_t* src = p.w[u.phase] + static_cast<size_t>(u.expert * p.n_pairs[u.phase] + u.pair) * nst * STAGE_W_BYTES + rank * TILE_BYTES;
+        const uint64_t pol = u.again != 0 ? several : once;
         for (int ks = 0; ks < nst; ++ks) {
           if (!mbar_wait_inline(&ctl.raw_empty[ws], wpar ^ 1u, abortw)) { ok = false; break; }
           mbar_arrive_expect_tx(&ctl.raw_full[ws], TILE_BYTES);
@@ -479,7 +483,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             const int per = pair_tile_rows(c, nt), at = (tile - tile_start[lo]) * per;
             const int rows = min(per, c - at);
             a = make_int4(phase, lo, off_s[lo] + at, rows);
-            b = make_int4(pair, tile, (rows + 15) & ~15, 0);
+            b = make_int4(pair, tile, (rows + 15) & ~15, nt > 1 ? 1 : 0);
           }
           const uint32_t s = i % PAIR_UNITS;
           const uint32_t par = ((i / PAIR_UNITS) & 1u) ^ 1u;   // of the unit whose place this one takes
