@@ -80,6 +80,7 @@ struct FewParams {
   unsigned int* tile_done;       // [tiles], zero between launches
   unsigned int* ctl;             // [0] CTAs that are done, [1] CTAs whose norm sums are written, [2] slices of xs written
   float* norm_part;              // [CTAs][rows]
+  float* logits_copy;            // [T][E], with share_x and logits in host memory: one CTA fetches them, all read its copy; else null
   unsigned long long* trace;
   float pre_eps, post_eps, route_scale;
   int H, I, T, E, k, lo, nloc, mode, route;
@@ -198,7 +199,7 @@ struct FewIter {
 // Top-k of one token by one warp: k rounds of two hardware warp reductions (largest orderable score, then the
 // lowest expert that has it), the weights as route_one_token forms them. Same ids and weights, bit for bit.
 template <int PER>
-__device__ __forceinline__ void few_route(const float* __restrict__ row, const float* __restrict__ bias, int* ids_s,
+__device__ __forceinline__ void few_route(const float* row, const float* __restrict__ bias, int* ids_s,
                                           float* tw_s, int E, int k, int mode, float scale, int lane) {
   uint32_t key[PER];
   float raw[PER];
@@ -207,7 +208,7 @@ __device__ __forceinline__ void few_route(const float* __restrict__ row, const f
     const int e = i * 32 + lane;
     key[i] = 0u;
     raw[i] = 0.f;
-    if (e < E) raw[i] = row[e];
+    if (e < E) raw[i] = __ldcg(row + e);   // (may be another CTA's copy)
   }
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
@@ -348,6 +349,11 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       const uint4 v = src[i];
       dst[i] = make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
     }
+    // The logits once over PCIe as well: 148 CTAs that fetched a row of 512 bytes each had it after 3 to 8.5 us, behind which
+    // their slices of the rows queued too. A step from and to pinned memory, 128 experts: 1 token 42.9 -> 39.4 us, 2 tokens
+    // 57.8 -> 53.4 us, together with the one warp that polls below.
+    if (p.logits_copy != nullptr && cta == n_ctas - 1)
+      for (int i = tid; i < p.T * p.E; i += FEW_THREADS) p.logits_copy[i] = p.logits[i];
     __threadfence();
   }
   __syncthreads();
@@ -356,8 +362,9 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
   if (warp < FEW_ROUTE_WARPS) {
     // ---- routing (a warp per token) and the stable sort (brute force: at most 128 entries)
     if (p.route == 1) {
+      if (p.logits_copy != nullptr) named_bar_sync(3, FEW_WARPS * 32);   // behind the wait below, of the warps that fetch the rows
       if (warp < p.T) {
-        const float* row = p.logits + static_cast<size_t>(warp) * p.E;
+        const float* row = (p.logits_copy != nullptr ? p.logits_copy : p.logits) + static_cast<size_t>(warp) * p.E;
         int* ids_s = ctl.ids + warp * p.k;
         float* tw_s = ctl.tw + warp * p.k;
         if (p.E <= 128) few_route<4>(row, p.bias, ids_s, tw_s, p.E, p.k, p.mode, p.route_scale, lane);
@@ -415,7 +422,11 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
     const int xw = warp - FEW_ROUTE_WARPS, wpr = p.T == 1 ? XW : p.T == 2 ? XW / 2 : 1;
     const int i_first = (xw % wpr) * 32 + lane, i_step = wpr * 32, n16 = p.H / 8;
     if (p.share_x) {
-      const bool go = warp_counter_wait(p.ctl + 2, static_cast<unsigned int>(n_ctas), abortw, lane);
+      // One warp polls, the others wait for it: with four of each of 148 CTAs on the counter's line, the counts behind which they
+      // wait came microseconds late.
+      if (xw == 0) warp_counter_wait(p.ctl + 2, static_cast<unsigned int>(n_ctas), abortw, lane);
+      named_bar_sync(3, p.logits_copy != nullptr ? FEW_WARPS * 32 : XW * 32);
+      const bool go = __all_sync(0xffffffffu, *abortw == 0);
       for (int t = xw / wpr; t < p.T && go; t += XW / wpr) {
         const uint4* src = reinterpret_cast<const uint4*>(p.xs + static_cast<size_t>(t) * p.H);
         uint4* dst = reinterpret_cast<uint4*>(xb + t * x_stride);
