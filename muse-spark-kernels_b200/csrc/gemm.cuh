@@ -7,7 +7,7 @@
 //   warps 1, 3   MMA issuers (one per tile of the pair): tcgen05.mma kind::f16, A from TMEM,
 //                B from shared memory, FP32 accumulators in TMEM; warp 1 owns the TMEM allocation;
 //   warp 2       activations: cp.async gather of the token rows of the tile (through the permutation for
-//                the gate/up GEMM) into the K-major core-matrix layout, or TMA boxes of sorted rows;
+//                the gate/up GEMM) into the K-major core-matrix layout, or a TMA copy of sorted rows a K stage;
 //   warps 4-7    epilogue (gemm_epilogue.inl): TMEM accumulators -> SwiGLU / scale -> global,
 //                or split-K partials;
 //   warps 8-23   dequant (gemm_dequant.inl): 2 tiles x 4 lane quarters x 2 K halves. A thread
@@ -84,7 +84,7 @@ struct GemmCfg {
   static constexpr int NSLOT = N <= 32 ? 3 : 2;
   static constexpr int SLOT_COLS = 64;
   static constexpr int A_GROUP_COLS = NSLOT * SLOT_COLS;
-  // Token tiles of 64 and more fetch the activation operand with TMA (2-D boxes of 64 K x 16 to N rows,
+  // Token tiles of 64 and more fetch the activation operand with TMA (a K stage of 16 to N rows a copy,
   // 128-byte swizzle) from rows that are contiguous in sorted order (the sorted F16 copy of the token
   // rows for the gate/up GEMM, `inter` for the down GEMM); narrower tiles gather rows through the
   // permutation with cp.async (gemm_gather.inl). Gathering the wide tiles' rows with cp.async as well

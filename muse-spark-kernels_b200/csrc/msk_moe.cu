@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(128) dequant_packed_kernel(const uint8_t* pack
 
 // --------------------------------------------------------------- row copy
 // F16 copy of the token rows, a block per token. With `inv` a row goes to each of its routes' places in sorted
-// (expert-major) order, xs[inv[t, s]] = f16(x[t]), so that wide token tiles can be fetched as plain 2-D TMA boxes (the
+// (expert-major) order, xs[inv[t, s]] = f16(x[t]), so that wide token tiles can be fetched as plain TMA boxes (the
 // reference's prefill path gathers rows into per-expert tiles, muse_prefill_layer/cuda/prefill.cu:1446-1608, fused with
 // its pre-expert norm); without it xs[t] = f16(x[t]), for the narrow token tiles that gather rows through the permutation.
 // F16 is the operand type of the MMA (layout.cuh).
