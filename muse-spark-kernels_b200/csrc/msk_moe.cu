@@ -584,6 +584,7 @@ static bool handover_env_off() {
 constexpr int MAX_CTAS = 512;
 constexpr int FLAT_MAX_ROWS = SMALL_SORT_MAX_ENTRIES;  // up to here the weight stream may be cut into equal shares
 constexpr int ONE_LAUNCH_MAX_TOKENS = 8;               // up to here the step is one launch by default
+constexpr int ONE_LAUNCH_NORM_TOKENS = 4;              // from here on it is not with the post-expert norm (forward_impl)
 constexpr int BOTH_GEMMS_MIN_TOKENS = 9;               // from here on (narrow tiles) both GEMMs share one launch by default
 
 struct Plan {
@@ -1494,6 +1495,14 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
 
+  // With the post-expert norm the one launch ends with tickets per token and a combine by whole CTAs; from four tokens on the sort, both
+  // GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
+  // 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2, with both norms 8: 48.8 / 44.6; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
+  // 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
+  if (plan.path == 0 && !nv && post_norm_w != nullptr && cfg->decode_path == 0 && n_tokens >= ONE_LAUNCH_NORM_TOKENS) {
+    plan.path = 4;
+    plan.both = true;
+  }
   if (!nv && plan.path != 1 && plan.path != 4) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
     p.route = logits != nullptr ? 1 : 2;

@@ -736,6 +736,37 @@ def test_host_mapped_step_reads_and_writes_pinned_host_memory(cuda_dev, T, route
     assert m.read_status(st) == 0
 
 
+@pytest.mark.parametrize("T", [3, 4, 8])
+@pytest.mark.parametrize("pre,ids", [(False, False), (True, False), (False, True)])
+def test_few_tokens_with_the_post_norm_around_the_end_of_the_one_launch(cuda_dev, T, pre, ids):
+    """Default steps on both sides of the line from which the post-expert norm takes launches of its own, against the oracle; from
+    the line on with the bits of that form when it is asked for."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1024, 512, 40, 5
+    w = inputs.make_weights(H, I, E, 64, cuda_dev, post_norm=True)
+    g = torch.Generator(device=cuda_dev).manual_seed(40 + T)
+    if pre:
+        w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
+    asked = m.prepare(w, n_experts=E, top_k=k, max_tokens=8, decode_path=4)
+    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+    lg = torch.randn((T, E), generator=g, device=cuda_dev)
+    if ids:
+        tw, top = torch.softmax(lg, dim=-1).topk(k, dim=-1)
+        data["topk_ids"], data["topk_weights"] = top.to(torch.int32).contiguous(), tw.contiguous()
+    else:
+        data["router_logits"] = lg
+    for _ in range(2):
+        got, same = m.kernel_fn(data, st), m.kernel_fn(data, asked)
+        assert _rel(got, same.float()) <= TOL
+        if T >= 4 and not pre:
+            assert torch.equal(got, same)
+    if not pre:
+        _, top, tw = m.kernel_fn(data, asked, return_routing=True)
+        assert _rel(got, orc.moe_forward(data["hidden_states"], top, tw, w).float()) <= TOL
+    assert m.read_status(st) == 0 and m.read_status(asked) == 0
+
+
 @pytest.mark.parametrize("T,E,k,nloc,H,host", [(1, 16, 8, 16, 256, "xl"), (2, 128, 8, 128, 1024, "xl"), (3, 130, 5, 130, 768, "xl"), (1, 512, 4, 256, 512, "xl"),
                                                (3, 512, 2, 40, 768, "xl"), (2, 16, 4, 16, 1024, "x"), (2, 16, 4, 16, 1024, "l")])
 def test_logits_in_host_memory_are_fetched_once_for_all_ctas(cuda_dev, T, E, k, nloc, H, host):
