@@ -1499,7 +1499,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   // GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
   // 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2, with both norms 8: 48.8 / 44.6; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
   // 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
-  if (plan.path == 0 && !nv && post_norm_w != nullptr && cfg->decode_path == 0 && n_tokens >= ONE_LAUNCH_NORM_TOKENS) {
+  // Rows in host memory: every CTA of the one launch reads the logits or ids over PCIe, the sort launch once, H2048 I1024 4: 50 - 53 / 39.0,
+  // 8: 65 / 46.8, given ids 8: 59 - 71 / 44.2; H4096 I1536 E128 4: 95 / 78.5, given ids 3: 71 - 76 / 62.2, 4: 92 - 98 / 73.
+  if (plan.path == 0 && !nv && cfg->decode_path == 0 && (host_x || (post_norm_w != nullptr && n_tokens >= ONE_LAUNCH_NORM_TOKENS))) {
     plan.path = 4;
     plan.both = true;
   }

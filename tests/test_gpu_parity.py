@@ -767,6 +767,32 @@ def test_few_tokens_with_the_post_norm_around_the_end_of_the_one_launch(cuda_dev
     assert m.read_status(st) == 0 and m.read_status(asked) == 0
 
 
+@pytest.mark.parametrize("T,routed", [(4, False), (7, True), (8, False)])
+def test_host_mapped_steps_of_a_few_tokens_without_a_norm(cuda_dev, T, routed):
+    """Steps from pinned memory that the few-token kernel leaves take launches of their own where those on device tensors take one:
+    the same units and the same order of sums, so the same bits."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k = 1024, 512, 40, 5
+    w = inputs.make_weights(H, I, E, 65, cuda_dev, post_norm=False)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
+    g = torch.Generator(device=cuda_dev).manual_seed(50 + T)
+    step = None
+    for _ in range(3):
+        d = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+        lg = torch.randn((T, E), generator=g, device=cuda_dev)
+        if routed:
+            tw, ids = torch.softmax(lg, dim=-1).topk(k, dim=-1)
+            d["topk_ids"], d["topk_weights"] = ids.to(torch.int32), tw.contiguous()
+        else:
+            d["router_logits"] = lg
+        host = {key: v.cpu() for key, v in d.items()}
+        step = step or m.HostMappedStep(st, host)
+        want, got = m.kernel_fn(d, st), step(host)
+        step.done.synchronize()
+        assert torch.equal(got, want.cpu())
+    assert m.read_status(st) == 0
+
+
 @pytest.mark.parametrize("T,E,k,nloc,H,host", [(1, 16, 8, 16, 256, "xl"), (2, 128, 8, 128, 1024, "xl"), (3, 130, 5, 130, 768, "xl"), (1, 512, 4, 256, 512, "xl"),
                                                (3, 512, 2, 40, 768, "xl"), (2, 16, 4, 16, 1024, "x"), (2, 16, 4, 16, 1024, "l")])
 def test_logits_in_host_memory_are_fetched_once_for_all_ctas(cuda_dev, T, E, k, nloc, H, host):
