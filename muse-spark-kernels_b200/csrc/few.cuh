@@ -81,6 +81,7 @@ struct FewParams {
   unsigned int* ctl;             // [0] CTAs that are done, [1] CTAs whose norm sums are written, [2] slices of xs written
   float* norm_part;              // [CTAs][rows]
   float* logits_copy;            // [T][E], with share_x and logits in host memory: one CTA fetches them, all read its copy; else null
+  int32_t* ids_copy;             // [T][k] ids, [T][k] weights behind them: the same where both are given
   unsigned long long* trace;
   float pre_eps, post_eps, route_scale;
   int H, I, T, E, k, lo, nloc, mode, route;
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
   const int n_entries = p.T * p.k;
   const int x_stride = p.H * 2 + 64;   // 64 bytes of skew: two rows of a quarter-warp in different banks
   volatile int* abortw = &ctl.abort_word;
+  const bool shared_routes = p.logits_copy != nullptr || p.ids_copy != nullptr;
 
   if (tid < FEW_TEAMS) ctl.mail[tid] = 0;
   if (tid == 0) {
@@ -351,9 +353,14 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
     }
     // The logits once over PCIe as well: 148 CTAs that fetched a row of 512 bytes each had it after 3 to 8.5 us, behind which
     // their slices of the rows queued too. A step from and to pinned memory, 128 experts: 1 token 42.9 -> 39.4 us, 2 tokens
-    // 57.8 -> 53.4 us, together with the one warp that polls below.
+    // 57.8 -> 53.4 us, together with the one warp that polls below. Given ids and weights in the same way: 1 token 43 - 50 -> 38.7 us, 2 tokens
+    // 60 - 65 -> 55.0 us.
     if (p.logits_copy != nullptr && cta == n_ctas - 1)
       for (int i = tid; i < p.T * p.E; i += FEW_THREADS) p.logits_copy[i] = p.logits[i];
+    if (p.ids_copy != nullptr && cta == n_ctas - 1 && tid < n_entries) {
+      p.ids_copy[tid] = p.ids_in[tid];
+      p.ids_copy[n_entries + tid] = __float_as_int(p.tw_in[tid]);
+    }
     __threadfence();
   }
   __syncthreads();
@@ -361,8 +368,8 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
 
   if (warp < FEW_ROUTE_WARPS) {
     // ---- routing (a warp per token) and the stable sort (brute force: at most 128 entries)
+    if (shared_routes) named_bar_sync(3, FEW_WARPS * 32);   // behind the wait below, of the warps that fetch the rows
     if (p.route == 1) {
-      if (p.logits_copy != nullptr) named_bar_sync(3, FEW_WARPS * 32);   // behind the wait below, of the warps that fetch the rows
       if (warp < p.T) {
         const float* row = (p.logits_copy != nullptr ? p.logits_copy : p.logits) + static_cast<size_t>(warp) * p.E;
         int* ids_s = ctl.ids + warp * p.k;
@@ -372,8 +379,8 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       }
       named_bar_sync(1, 256);
     } else if (tid < n_entries) {
-      ctl.ids[tid] = p.ids_in[tid];
-      ctl.tw[tid] = p.tw_in[tid];
+      ctl.ids[tid] = p.ids_copy != nullptr ? __ldcg(p.ids_copy + tid) : p.ids_in[tid];
+      ctl.tw[tid] = p.ids_copy != nullptr ? __int_as_float(__ldcg(p.ids_copy + n_entries + tid)) : p.tw_in[tid];
     }
     if (tid == 0) MSK_TR(TR_TOPK);
     int l = -1, key = 0x7fffffff, q = 0, r = 0, c = 0;
@@ -425,7 +432,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) moe_few_kernel(const __grid_co
       // One warp polls, the others wait for it: with four of each of 148 CTAs on the counter's line, the counts behind which they
       // wait came microseconds late.
       if (xw == 0) warp_counter_wait(p.ctl + 2, static_cast<unsigned int>(n_ctas), abortw, lane);
-      named_bar_sync(3, p.logits_copy != nullptr ? FEW_WARPS * 32 : XW * 32);
+      named_bar_sync(3, shared_routes ? FEW_WARPS * 32 : XW * 32);
       const bool go = __all_sync(0xffffffffu, *abortw == 0);
       for (int t = xw / wpr; t < p.T && go; t += XW / wpr) {
         const uint4* src = reinterpret_cast<const uint4*>(p.xs + static_cast<size_t>(t) * p.H);

@@ -1471,7 +1471,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     f.tile_done = reinterpret_cast<unsigned int*>(b + k.few_ctl + 4352);
     f.norm_part = partial; f.trace = trace;
     // (the second region of pieces, which this kernel has no use for: at least 128 KB, for 8 rows of up to 512 logits)
-    f.logits_copy = host_x && logits != nullptr && in_host_memory(logits) ? partial + round_up(partial_floats(cfg) * 4, 256) / 4 : nullptr;
+    float* copies = partial + round_up(partial_floats(cfg) * 4, 256) / 4;
+    f.logits_copy = host_x && logits != nullptr && in_host_memory(logits) ? copies : nullptr;
+    f.ids_copy = host_x && logits == nullptr && in_host_memory(topk_ids) && in_host_memory(topk_weights) ? reinterpret_cast<int32_t*>(copies) : nullptr;
     f.H = cfg->hidden; f.I = cfg->inter; f.T = n_tokens; f.E = cfg->n_experts; f.k = cfg->top_k;
     f.lo = cfg->local_start; f.nloc = cfg->local_count; f.mode = cfg->routing_mode; f.route_scale = cfg->route_scale;
     f.route = logits != nullptr ? 1 : 2;

@@ -794,19 +794,22 @@ def test_host_mapped_steps_of_a_few_tokens_without_a_norm(cuda_dev, T, routed):
 
 
 @pytest.mark.parametrize("T,E,k,nloc,H,host", [(1, 16, 8, 16, 256, "xl"), (2, 128, 8, 128, 1024, "xl"), (3, 130, 5, 130, 768, "xl"), (1, 512, 4, 256, 512, "xl"),
-                                               (3, 512, 2, 40, 768, "xl"), (2, 16, 4, 16, 1024, "x"), (2, 16, 4, 16, 1024, "l")])
-def test_logits_in_host_memory_are_fetched_once_for_all_ctas(cuda_dev, T, E, k, nloc, H, host):
-    """The few-token kernel with its rows and logits in pinned memory, one of them, both: routing and output are those on device
+                                               (3, 512, 2, 40, 768, "xl"), (2, 16, 4, 16, 1024, "x"), (2, 16, 4, 16, 1024, "l"),
+                                               (1, 16, 8, 16, 256, "xi"), (3, 130, 5, 130, 768, "xi"), (2, 512, 7, 40, 512, "xi"), (2, 16, 4, 16, 1024, "i")])
+def test_routes_in_host_memory_are_fetched_once_for_all_ctas(cuda_dev, T, E, k, nloc, H, host):
+    """The few-token kernel with its rows and logits, or given ids and weights, in pinned memory, one of them, both: routing and output are those on device
     tensors, bit for bit, from call to call (1 to 3 rows, rows that no warp's 32 lanes divide, the most experts, few of them local)."""
     m, inputs, _lib, orc = _mods()
     w = inputs.make_weights(H, 256, nloc, 63, cuda_dev, post_norm=True)
     st = m.prepare(w, n_experts=E, top_k=k, max_tokens=4)
     g = torch.Generator(device=cuda_dev).manual_seed(30 + T)
 
-    def run(x, logits):
-        out, ids = torch.empty((T, H), dtype=torch.bfloat16, device=cuda_dev), torch.empty((T, k), dtype=torch.int32, device=cuda_dev)
-        tw = torch.empty((T, k), device=cuda_dev)
-        m._forward(st, st["cfg"], st["lib"].lib, x.data_ptr(), logits.data_ptr(), ids.data_ptr(), tw.data_ptr(), out.data_ptr(), T)
+    def run(x, logits=None, ids=None, tw=None):
+        out = torch.empty((T, H), dtype=torch.bfloat16, device=cuda_dev)
+        if ids is None:
+            ids, tw = torch.empty((T, k), dtype=torch.int32, device=cuda_dev), torch.empty((T, k), device=cuda_dev)
+        m._forward(st, st["cfg"], st["lib"].lib, x.data_ptr(), None if logits is None else logits.data_ptr(), ids.data_ptr(), tw.data_ptr(),
+                   out.data_ptr(), T)
         torch.cuda.synchronize()
         return out, ids, tw
 
@@ -814,8 +817,13 @@ def test_logits_in_host_memory_are_fetched_once_for_all_ctas(cuda_dev, T, E, k, 
         x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
         logits = torch.randn((T, E), generator=g, device=cuda_dev)
         want = run(x, logits)
-        got = run(x.cpu().pin_memory() if "x" in host else x, logits.cpu().pin_memory() if "l" in host else logits)
-        assert all(torch.equal(u, v) for u, v in zip(got, want))
+        xh = x.cpu().pin_memory() if "x" in host else x
+        if "i" in host:
+            got = run(xh, None, want[1].cpu().pin_memory(), want[2].cpu().pin_memory())
+            assert torch.equal(got[0], want[0])
+        else:
+            got = run(xh, logits.cpu().pin_memory() if "l" in host else logits)
+            assert all(torch.equal(u, v) for u, v in zip(got, want))
     assert m.read_status(st) == 0
 
 
