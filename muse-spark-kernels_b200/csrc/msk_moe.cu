@@ -335,10 +335,11 @@ __global__ void __launch_bounds__(COMBINE_COLS_WARPS * 32)
 }
 
 // With the post-expert norm: a block of TH threads per token, G rows in registers at a time (NO octets of columns a thread, H <= 8 * TH * NO). The sum of
-// squares of a row is a fixed shuffle tree followed by a fixed-order sum of the warps' parts, so the result does not depend on
-// scheduling; the sums run in slot order. Bound by latency (table, rows, reduction, each behind the other), so what counts is rows in flight on
+// squares of a row is a fixed tree over every 1024 columns followed by the sum of those in column order, whatever
+// the block's size, so the result depends neither on scheduling nor on how many tokens a step has; the sums run in slot order. Bound by latency (table, rows, reduction, each behind the other), so what counts is rows in flight on
 // an SM. Many tokens: blocks of 128 threads (256 beyond 4096 columns), five or four of them on an SM, where blocks of 512 left two tokens to
-// one: 3012 tokens with 1.6 local routes each 41 -> 18 us, 777 with eight 22 -> 16, 7000 149 -> 98. Few
+// one: 3012 tokens with 1.6 local routes each 41 -> 18 us, 777 with eight 22 -> 16, 7000 149 -> 98. Up to 2048 columns two octets a
+// thread, which four leave half the block's threads without: 2000 tokens of four at 2048 columns 17 -> 13, 4000 of eight at 1024 39 -> 27. Few
 // tokens: 512 threads and as many rows at once as fit (64 tokens of eight 8 -> 6).
 constexpr int COMBINE_FEW_TOKENS = 256;
 constexpr int COMBINE_MAX_H = 8192;
@@ -346,10 +347,17 @@ template <bool YB, int TH, int NO, int G, int MINB>
 __global__ void __launch_bounds__(TH, MINB)
     combine_norm_kernel(const float* y, const int32_t* inv, const float* tw, __nv_bfloat16* __restrict__ out, int H, int k,
                         float eps) {   // (y, inv and tw: as above)
-  constexpr int NW = TH / 32, LG = G == 8 ? 3 : G == 4 ? 2 : 1;
-  static_assert(G == 1 << LG && NW % 4 == 0, "two, four or eight rows together");
+  // A run of 1024 columns is four quarters of 32 octets. Its squares are summed over the quarters, over eight neighbours and over the
+  // four groups of neighbours, each as a tree, then run after run: NO = 4 has the quarters of a run in a thread and the run in a warp,
+  // NO = 2 half of either, NO = 1 a quarter, and SUM_BITS are the lane bits of the same additions in the same order.
+  constexpr int CL = 4 / NO, JW = 32 / CL, NW = TH / 32, LG = G == 8 ? 3 : G == 4 ? 2 : 1;
+  constexpr int SUM_BITS[5] = {NO == 4 ? 4 : 16, NO == 4 ? 2 : NO == 2 ? 4 : 8, NO == 4 ? 1 : NO == 2 ? 2 : 4, NO == 4 ? 8 : NO == 2 ? 1 : 2,
+                               NO == 4 ? 16 : NO == 2 ? 8 : 1};
+  static_assert(G == 1 << LG && (NO == 1 || NO == 2 || NO == 4) && NW % 4 == 0, "two, four or eight rows together");
   __shared__ __align__(16) float part[2][G][NW];   // in turn: a group's parts are read while the next one's are written
-  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = ((warp / CL) * 128 + (lane / JW) * 32 + (warp % CL) * JW + lane % JW) * 8;   // column of the first octet
+  constexpr int STEP = CL * 256;                                                                 // to the next one
   pdl_wait();  // y and inv come from the kernels before this one
   const int q = lane < k ? inv[static_cast<size_t>(t) * k + lane] : -1;
   const float w = lane < k ? tw[static_cast<size_t>(t) * k + lane] : 0.f;
@@ -361,7 +369,6 @@ __global__ void __launch_bounds__(TH, MINB)
     const int n = min(__popc(have), G);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      ss[g] = 0.f;
       if (g < n) {
         const int s = __ffs(have) - 1;
         have &= have - 1u;
@@ -369,59 +376,73 @@ __global__ void __launch_bounds__(TH, MINB)
         const size_t at = static_cast<size_t>(__shfl_sync(0xffffffffu, q, s)) * H;
 #pragma unroll
         for (int c = 0; c < NO; ++c)
-          if ((c * TH + tid) * 8 < H) v[g][c].load(y, at + (c * TH + tid) * 8);
+          if (first + c * STEP < H) v[g][c].load(y, at + first + c * STEP);
       }
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
+      float sq[NO] = {};
       if (g < n) {
 #pragma unroll
         for (int c = 0; c < NO; ++c)
-          if ((c * TH + tid) * 8 < H) ss[g] += v[g][c].squares();
+          if (first + c * STEP < H) sq[c] = v[g][c].squares();
       }
+      ss[g] = NO == 1 ? sq[0] : NO == 2 ? sq[0] + sq[NO / 2] : (sq[0] + sq[NO / 2]) + (sq[NO / 4] + sq[NO - 1]);
     }
     // G sums over the warp at once: in each of the first steps a lane passes on half of its sums and keeps the other
-    // half (xor 16, 8, 4, 2, 1 for every sum, as in G separate trees, but in G + 4 - LG shuffles instead of 5 * G)
-    int o = 16;
+    // half (the same additions as in G separate trees, but in G + 4 - LG shuffles instead of 5 * G)
+    int mine = 0;   // whose sum this lane ends with
+    bool first_of = true;
 #pragma unroll
-    for (int h = G / 2; h >= 1; h >>= 1, o >>= 1) {
+    for (int b = 0; b < 5; ++b) {
+      const int o = SUM_BITS[b], h = G >> (b + 1);
       const bool up = (lane & o) != 0;
+      if (b < LG) {
+        mine = mine * 2 + (up ? 1 : 0);
 #pragma unroll
-      for (int g = 0; g < h; ++g) {
-        const float keep = up ? ss[g + h] : ss[g], send = up ? ss[g] : ss[g + h];
-        ss[g] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        for (int g = 0; g < h; ++g) {
+          const float keep = up ? ss[g + h] : ss[g], send = up ? ss[g] : ss[g + h];
+          ss[g] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      } else {
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+        first_of = first_of && !up;
       }
     }
-#pragma unroll
-    for (int r = 16 >> LG; r > 0; r >>= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], r);
-    if ((lane & ((32 >> LG) - 1)) == 0) part[turn][lane >> (5 - LG)][warp] = ss[0];
+    if (first_of) part[turn][mine][warp] = ss[0];
     __syncthreads();
 #pragma unroll
     for (int g = 0; g < G; ++g) {   // slot order
       if (g < n) {
         float tot = 0.f;
 #pragma unroll
-        for (int i = 0; i < NW / 4; ++i) {  // fixed order
+        for (int i = 0; i < NW / 4; ++i) {  // a run is one part, two or four
           const float4 f = reinterpret_cast<const float4*>(part[turn][g])[i];
-          tot += f.x; tot += f.y; tot += f.z; tot += f.w;
+          if (NO == 1) {
+            tot += (f.x + f.y) + (f.z + f.w);
+          } else if (NO == 2) {
+            tot += f.x + f.y; tot += f.z + f.w;
+          } else {
+            tot += f.x; tot += f.y; tot += f.z; tot += f.w;
+          }
         }
         wgt[g] *= rsqrtf(tot / static_cast<float>(H) + eps);
 #pragma unroll
         for (int c = 0; c < NO; ++c)
-          if ((c * TH + tid) * 8 < H) v[g][c].add_to(acc[c], wgt[g]);
+          if (first + c * STEP < H) v[g][c].add_to(acc[c], wgt[g]);
       }
     }
   }
 #pragma unroll
   for (int c = 0; c < NO; ++c) {
-    if ((c * TH + tid) * 8 >= H) break;
+    if (first + c * STEP >= H) break;
     uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const __nv_bfloat162 h = __floats2bfloat162_rn(acc[c][2 * i], acc[c][2 * i + 1]);
       o[i] = *reinterpret_cast<const uint32_t*>(&h);
     }
-    *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * H + (c * TH + tid) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * H + first + c * STEP) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -1382,7 +1403,7 @@ static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, con
     return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, n_tokens, H, k));
   }
   lc.gridDim = dim3(static_cast<unsigned>(n_tokens));
-  const bool narrow = H <= 4096;
+  const bool narrow = H <= 4096, short_rows = H <= 2048;
   if (n_tokens < COMBINE_FEW_TOKENS) {
     lc.blockDim = dim3(512);
     auto* kern = y_bf16 ? (narrow ? combine_norm_kernel<true, 512, 1, 8, 1> : combine_norm_kernel<true, 512, 2, 8, 1>)
@@ -1390,9 +1411,9 @@ static int launch_combine(const MskMoeCfg* cfg, bool y_bf16, const float* y, con
     return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, H, k, cfg->post_norm_eps));
   }
   lc.blockDim = dim3(narrow ? 128 : 256);
-  auto* kern = !y_bf16 ? (narrow ? combine_norm_kernel<false, 128, 4, 2, 4> : combine_norm_kernel<false, 256, 4, 2, 2>)
-               : few_local ? (narrow ? combine_norm_kernel<true, 128, 4, 2, 5> : combine_norm_kernel<true, 256, 4, 2, 3>)
-                           : (narrow ? combine_norm_kernel<true, 128, 4, 4, 4> : combine_norm_kernel<true, 256, 4, 4, 2>);
+  auto* kern = !y_bf16 ? (short_rows ? combine_norm_kernel<false, 128, 2, 4, 4> : narrow ? combine_norm_kernel<false, 128, 4, 2, 4> : combine_norm_kernel<false, 256, 4, 2, 2>)
+               : few_local ? (short_rows ? combine_norm_kernel<true, 128, 2, 2, 8> : narrow ? combine_norm_kernel<true, 128, 4, 2, 5> : combine_norm_kernel<true, 256, 4, 2, 3>)
+                           : (short_rows ? combine_norm_kernel<true, 128, 2, 4, 6> : narrow ? combine_norm_kernel<true, 128, 4, 4, 4> : combine_norm_kernel<true, 256, 4, 4, 2>);
   return static_cast<int>(cudaLaunchKernelEx(&lc, kern, y, inv, tw, o, H, k, cfg->post_norm_eps));
 }
 

@@ -578,6 +578,25 @@ def test_combine_with_the_norm_at_its_block_sizes(cuda_dev, H, T, k, tile, lo, n
     _check_forward(out, ref, parts, m.workspace_views(st, T))
 
 
+@pytest.mark.parametrize("H,k,tile,lo,nloc", [(4096, 3, 16, 0, 12), (3840, 9, 64, 0, 12), (2048, 9, 64, 0, 12), (1024, 9, 128, 0, 12), (1536, 3, 128, 4, 6), (4096, 3, 128, 4, 6),
+                                              (8192, 3, 16, 0, 12), (4352, 9, 128, 0, 12), (7168, 3, 128, 4, 6)])
+def test_combine_with_the_norm_gives_a_token_the_same_bits_in_steps_of_any_size(cuda_dev, H, k, tile, lo, nloc):
+    """The blocks of the combine with the post-expert norm are smaller from 256 tokens on: a row's squares are summed in the same order all the
+    same, so that with one token tile a token's output does not change with the tokens beside it."""
+    m, inputs, _lib, _ = _mods()
+    E, T = 12, 257
+    st = m.prepare(inputs.make_weights(H, 256, nloc, 109, cuda_dev, post_norm=True), n_experts=E, top_k=k, max_tokens=T, local_start=lo, token_tile=tile)
+    g = torch.Generator(device=cuda_dev).manual_seed(113)
+    ids = torch.rand((T, E), generator=g, device=cuda_dev).topk(k, 1)[1].to(torch.int32)
+    x = torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)
+    tw = torch.rand((T, k), generator=g, device=cuda_dev)
+    step = lambda n: m.kernel_fn({"hidden_states": x[:n], "topk_ids": ids[:n].contiguous(), "topk_weights": tw[:n].contiguous()}, st)  # noqa: E731
+    most = step(T)
+    for n in (9, 40, 255, 256):
+        assert torch.equal(step(n), most[:n]), n
+    assert m.read_status(st) == 0
+
+
 @pytest.mark.parametrize("E,k,nloc,T", [(8, 2, 8, 256), (128, 8, 4, 700)])
 def test_pair_kernel_by_default_on_a_handful_of_experts(cuda_dev, E, k, nloc, T):
     """The default plan takes the pair kernel by the mean rows per expert, also where only a handful of experts is there."""
