@@ -24,7 +24,6 @@ with the step; the reference sweeps by reading for that reason), and the steps c
 pool of different routings.
 """
 import argparse
-import ctypes
 import json
 import math
 import os
@@ -348,24 +347,21 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     mean_touched = sum(touched[i % POOL] for i in range(n_prof)) / n_prof
     R = T * k
     plan = moe.plan(state, T)
-    few, nvf4 = ctypes.c_int(0), ctypes.c_int(0)
-    state["lib"].lib.msk_moe_few_fits(ctypes.byref(state["cfg"]), T, 1, ctypes.byref(few))   # (timed with given ids)
-    state["lib"].lib.msk_moe_nvf4_takes(ctypes.byref(state["cfg"]), T, int(state["post_norm_w"] is not None) + 2 * int(state["pre_norm_w"] is not None), ctypes.byref(nvf4))
-    nvf4 = bool(nvf4.value) and not few.value
-    one_launch = plan[1] == 0 and T <= 32 and R <= 256 and not nvf4
-    # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine
-    both_gemms = plan[1] == 4 or (plan[0] == 64 and not plan[2] and state["cfg"].decode_path != 1)
-    pair = plan[0] == 128 and state["cfg"].decode_path != 1     # both GEMMs in one launch on pairs of SMs
+    form = moe.step_form(state, T, given_ids=True)   # (timed with given ids)
+    few, nvf4 = form == "few-token kernel", form == "FP4 kernel"
+    one_launch = few or form == "one launch"
+    pair = plan[0] == 128 and form == "both GEMMs"   # on pairs of SMs
+    both_gemms = form == "both GEMMs" and not pair   # sort launch(es), [64-token tile: row copy,] both GEMMs in one launch, combine
     step_bytes = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(steps)) / steps
     step_flops = inputs.algorithmic_flops(H, I, R)
     if one_launch:
         alg = sum(inputs.algorithmic_bytes(H, I, E, k, T, touched[i % POOL]) for i in range(n_prof)) / n_prof
         achieved = alg / (k_ms[2] * 1e-3) / 1e9
-        ratio = NCU_TRAFFIC_RATIO["moe_few_kernel" if few.value else "moe_gemm_kernel<N,2> T8"]
+        ratio = NCU_TRAFFIC_RATIO["moe_few_kernel" if few else "moe_gemm_kernel<N,2> T8"]
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": alg * ratio,
                 "traffic_source": "ncu dram bytes of the kernel's 32-expert capture / its algorithmic bytes (%.2f), scaled" % ratio,
-                "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if few.value else "moe_gemm_kernel<N,2>"),
+                "kernel": "%s (whole step in one launch)" % ("moe_few_kernel" if few else "moe_gemm_kernel<N,2>"),
                 "peak_source": peaks["source"] + " (burst copy)"}
     elif nvf4:
         # both GEMMs in one launch: the touched experts' tiles, x read, inter written and read, y written (the split rows, 3.8 bytes a value
@@ -413,7 +409,7 @@ def measure(moe, inputs, state, spec, steps, warmup, peaks, dev, flush_fn, with_
     sec = total_ms / steps * 1e-3
     if one_launch:
         launches = 1
-    elif plan[1] == 2 and T <= 32 and R <= 256:
+    elif form == "folded":
         launches = 3      # row copy, gate/up kernel (routes, sorts), down kernel (combines)
     elif nvf4:            # top-k and sort (one launch up to 32 tokens, two beyond), both GEMMs, combine
         launches = 3 if T <= 32 else 4

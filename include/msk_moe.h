@@ -70,7 +70,7 @@ typedef struct MskMoeCfg {
   int32_t no_pdl;        /* non-zero: launches are not chained with programmatic dependent launch (the reference's
                             okc_set_pdl(0), muse_moe_w4a16/cuda/moe.cu:2348,2565) */
   int32_t token_tile;    /* MMA N (tokens per tile): 16/32/64/128; 0 = chosen from the mean rows per expert
-                            (up to 12: 16, up to 40: 64, beyond: 128). 128 stands for the kernel on pairs of SMs,
+                            (up to 7, or 12 with decode_path set: 16, up to 40: 64, beyond: 128). 128 stands for the kernel on pairs of SMs,
                             whose tiles hold up to 256 rows; it rounds num_ctas up to an even number */
   int32_t max_tokens;    /* token capacity the workspace is sized for (msk_moe_forward rejects more) */
   int32_t trace;         /* non-zero: the GEMM kernels stamp %globaltimer per CTA into the workspace (view 6) */
@@ -220,9 +220,10 @@ int msk_moe_forward_static(const MskMoeCfg* cfg, const void* packed13, const voi
  * Allocates nothing; not for the timed path. No counterpart in the reference. */
 int msk_moe_static_status(int* host_status, void* stream);
 
-/* The launch plan msk_moe_forward uses for n_tokens: host_out[4] = token tile N, path (as
+/* The launch plan that the configuration and n_tokens give: host_out[4] = token tile N, path (as
  * MskMoeCfg.decode_path; 1 or 4 beyond a few tokens), 1 when the weight stream is cut into equal
- * shares (else whole units), persistent grid size. The reference picks its build by
+ * shares (else whole units), persistent grid size. What a step really runs in depends on its inputs
+ * and norms as well: msk_moe_step_form. The reference picks its build by
  * token count the same way (muse_moe_w4a16/py/03_kernel_fn.py:33-40). */
 int msk_moe_plan(const MskMoeCfg* cfg, int n_tokens, int* host_out);
 
@@ -240,6 +241,17 @@ int msk_moe_few_fits(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_f
 #define MSK_NVF4_POST_NORM 1
 #define MSK_NVF4_PRE_NORM 2
 int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_takes);
+
+/* The form that a step of n_tokens runs in (msk_moe_forward*, not msk_moe_forward_static), *host_form = MSK_FORM_*. inputs: MSK_FEW_* bits and
+ * the ones below. No GPU needed. No counterpart in the reference. */
+#define MSK_STEP_POST_NORM 8      /* post_norm_w is given */
+#define MSK_FORM_ONE_LAUNCH 0     /* routing, sort, both GEMMs and combine in the tcgen05 kernel */
+#define MSK_FORM_CHAIN 1          /* sort, [row copy,] gate/up GEMM, down GEMM, combine */
+#define MSK_FORM_FOLDED 2         /* row copy, gate/up GEMM that routes and sorts, down GEMM that combines */
+#define MSK_FORM_BOTH_GEMMS 4     /* sort, [row copy,] both GEMMs in one launch, combine */
+#define MSK_FORM_FEW 5            /* the few-token kernel: one launch */
+#define MSK_FORM_NVF4 6           /* sort, both GEMMs in the FP4 kernel, combine */
+int msk_moe_step_form(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_form);
 
 /* How the GEMM kernels deal their work (host-side twin of the device code, a test hook): the pieces
  * that CTA `cta` of `shares` gets from n_base base units of n_stages K stages each. flat == 0: whole

@@ -605,7 +605,7 @@ static bool handover_env_off() {
 constexpr int MAX_CTAS = 512;
 constexpr int FLAT_MAX_ROWS = SMALL_SORT_MAX_ENTRIES;  // up to here the weight stream may be cut into equal shares
 constexpr int ONE_LAUNCH_MAX_TOKENS = 8;               // up to here the step is one launch by default
-constexpr int ONE_LAUNCH_NORM_TOKENS = 4;              // from here on it is not with the post-expert norm (forward_impl)
+constexpr int ONE_LAUNCH_NORM_TOKENS = 4;              // from here on it is not with the post-expert norm (step_form)
 constexpr int BOTH_GEMMS_MIN_TOKENS = 9;               // from here on (narrow tiles) both GEMMs share one launch by default
 
 struct Plan {
@@ -1028,6 +1028,28 @@ static bool few_takes(const MskMoeCfg* c, int T, int inputs, int grid, FewPlan* 
   const double rows = static_cast<double>(T) * c->top_k * c->local_count / c->n_experts;
   const int most = pre ? (host ? 0 : c->hidden <= 4096 && rows <= 24 ? 6 : 4) : host && rows > 16 ? 2 : 3;
   return T <= most && few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
+}
+
+// The form that a step runs in, MSK_FORM_*, and with the few-token kernel its plan; inputs: MSK_FEW_* and MSK_STEP_* bits. nv_room: whether
+// the workspace has room for the FP4 kernel's split rows.
+// With the post-expert norm the one launch ends with tickets per token and a combine by whole CTAs; from four tokens on the sort, both
+// GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
+// 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2, with both norms 8: 48.8 / 44.6; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
+// 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
+// Rows in host memory: every CTA of the one launch reads the logits or ids over PCIe, the sort launch once, H2048 I1024 4: 50 - 53 / 39.0,
+// 8: 65 / 46.8, given ids 8: 59 - 71 / 44.2; H4096 I1536 E128 4: 95 / 78.5, given ids 3: 71 - 76 / 62.2, 4: 92 - 98 / 73.
+static int step_form(const MskMoeCfg* c, int T, const Plan& p, int inputs, bool nv_room, FewPlan* few) {
+  const bool pre = (inputs & MSK_FEW_PRE_NORM) != 0, post = (inputs & MSK_STEP_POST_NORM) != 0, host_x = (inputs & MSK_FEW_HOST_X) != 0;
+  const bool nv = nv_room && nv_takes(c, T, p, (pre ? MSK_NVF4_PRE_NORM : 0) | (post ? MSK_NVF4_POST_NORM : 0));
+  if (p.path == 0 && !(nv && c->local_count == c->n_experts) && few_takes(c, T, inputs, p.grid, few)) return MSK_FORM_FEW;
+  if (nv) return MSK_FORM_NVF4;
+  if (p.path == 2) return MSK_FORM_FOLDED;
+  if (p.path == 0) {
+    if (c->decode_path == 0 && (host_x || (post && T >= ONE_LAUNCH_NORM_TOKENS))) return pre ? MSK_FORM_CHAIN : MSK_FORM_BOTH_GEMMS;
+    return pre ? MSK_FORM_FOLDED : MSK_FORM_ONE_LAUNCH;   // (the pre-expert norm needs a kernel in front of the GEMMs)
+  }
+  if (p.N == 128) return c->decode_path == 1 || c->stop_after == 2 ? MSK_FORM_CHAIN : MSK_FORM_BOTH_GEMMS;
+  return p.both && (p.N == 64 || !pre) ? MSK_FORM_BOTH_GEMMS : MSK_FORM_CHAIN;   // narrow tiles: the pre-expert norm needs the row-copy kernel
 }
 
 static bool in_host_memory(const void* p) {   // page-locked, or pageable where the device can read that
@@ -1475,10 +1497,11 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   p.eps = cfg->post_norm_eps;
   FewPlan few;
   const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
-  const int few_inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
-                         (host_x ? MSK_FEW_HOST_X : 0);
-  const bool nv = k.nv_end <= workspace_bytes && nv_takes(cfg, n_tokens, plan, (pre_norm_w != nullptr ? MSK_NVF4_PRE_NORM : 0) | (post_norm_w != nullptr ? MSK_NVF4_POST_NORM : 0));
-  if (plan.path == 0 && !(nv && cfg->local_count == cfg->n_experts) && few_takes(cfg, n_tokens, few_inputs, plan.grid, &few)) {
+  const int inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
+                     (host_x ? MSK_FEW_HOST_X : 0) | (post_norm_w != nullptr ? MSK_STEP_POST_NORM : 0);
+  const int form = step_form(cfg, n_tokens, plan, inputs, k.nv_end <= workspace_bytes, &few);
+  const bool nv = form == MSK_FORM_NVF4;
+  if (form == MSK_FORM_FEW) {
     FewParams f{};
     f.w13 = static_cast<const uint8_t*>(packed13); f.w2 = static_cast<const uint8_t*>(packed2);
     f.gs13 = gs13; f.gs2 = gs2;
@@ -1518,17 +1541,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   g2.tickets = tickets + round_up(ticket_ints(cfg, cfg->max_tokens) * 4, 256) / 4;
   g2.K = cfg->inter; g2.out_ld = cfg->hidden; g2.n_pairs = cfg->hidden / 256;
 
-  // With the post-expert norm the one launch ends with tickets per token and a combine by whole CTAs; from four tokens on the sort, both
-  // GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
-  // 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2, with both norms 8: 48.8 / 44.6; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
-  // 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
-  // Rows in host memory: every CTA of the one launch reads the logits or ids over PCIe, the sort launch once, H2048 I1024 4: 50 - 53 / 39.0,
-  // 8: 65 / 46.8, given ids 8: 59 - 71 / 44.2; H4096 I1536 E128 4: 95 / 78.5, given ids 3: 71 - 76 / 62.2, 4: 92 - 98 / 73.
-  if (plan.path == 0 && !nv && cfg->decode_path == 0 && (host_x || (post_norm_w != nullptr && n_tokens >= ONE_LAUNCH_NORM_TOKENS))) {
-    plan.path = 4;
-    plan.both = true;
-  }
-  if (!nv && plan.path != 1 && plan.path != 4) {
+  if (form == MSK_FORM_ONE_LAUNCH || form == MSK_FORM_FOLDED) {
     // ---- few tokens: the GEMM kernels route, sort and combine themselves
     p.route = logits != nullptr ? 1 : 2;
     p.logits = logits; p.bias = bias; p.ids_in = topk_ids; p.ids_out = ids_out; p.tw_out = tw_out;
@@ -1541,7 +1554,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     p.tile_seen = p.tile_done + 384;
     p.x_bf16 = static_cast<const __nv_bfloat16*>(x);
     if (ev) { cudaEventRecord(ev[0], st); cudaEventRecord(ev[1], st); }
-    if (plan.path == 0 && pre_norm_w == nullptr) {
+    if (form == MSK_FORM_ONE_LAUNCH) {
       if (ev) cudaEventRecord(ev[5], st);
       const int e1 = launch_gemm_fused(plan.N, p, plan.grid, st);
       if (ev) { cudaEventRecord(ev[2], st); cudaEventRecord(ev[3], st); cudaEventRecord(ev[4], st); }
@@ -1590,7 +1603,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   int e = 0;
   // narrow token tiles read an F16 copy of x; for few tokens the sorting CTA makes it
   const bool tma_b = !nv && plan.N >= 64;  // GemmCfg<N>::TMA_B
-  const bool both_gemms = !nv && plan.both && (tma_b || pre_norm_w == nullptr);   // narrow tiles: the pre-expert norm needs the row-copy kernel
+  const bool both_gemms = form == MSK_FORM_BOTH_GEMMS;   // (N = 128: the pair kernel)
   const bool convert_in_sort = !nv && !tma_b && !both_gemms && n_tokens <= FUSED_ROUTE_MAX_TOKENS;
   const __nv_bfloat16* xin = convert_in_sort ? static_cast<const __nv_bfloat16*>(x) : nullptr;
   __half* xh_in_sort = convert_in_sort ? xs : nullptr;
@@ -1666,7 +1679,7 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
     q.tile_seen = q.tile_done + max_tiles(cfg, cfg->max_tokens);
     q.K[0] = g13.K; q.K[1] = g2.K; q.n_pairs[0] = g13.n_pairs; q.n_pairs[1] = g2.n_pairs;
     q.nloc = cfg->local_count; q.H = cfg->hidden; q.I = cfg->inter;
-    const bool split = cfg->decode_path == 1 || cfg->stop_after == 2;
+    const bool split = form == MSK_FORM_CHAIN;
     q.first = 0; q.last = split ? 0 : 1;
     e = launch_pair(q, xs, r_max, plan.grid, st, pdl);
     if (e != 0) return e;
@@ -1968,6 +1981,16 @@ int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_
   if (!host_takes) return MSK_ERR_NULL;
   if (n_tokens < 1) return MSK_ERR_SHAPE;
   *host_takes = nv_takes(cfg, n_tokens, make_plan(cfg, n_tokens), norms) ? 1 : 0;
+  return MSK_OK;
+}
+
+int msk_moe_step_form(const MskMoeCfg* cfg, int n_tokens, int inputs, int* host_form) {
+  const int rc = check_cfg(cfg);
+  if (rc != MSK_OK) return rc;
+  if (!host_form) return MSK_ERR_NULL;
+  if (n_tokens < 1) return MSK_ERR_SHAPE;
+  FewPlan f;
+  *host_form = step_form(cfg, n_tokens, make_plan(cfg, n_tokens), inputs, true, &f);
   return MSK_OK;
 }
 

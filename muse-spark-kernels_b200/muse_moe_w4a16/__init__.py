@@ -460,10 +460,22 @@ def kernel_fn_timed(data, state):
 
 
 def plan(state, T):
-    """(token tile N, path, flat shares, grid) that kernel_fn uses for T tokens (see msk_moe_plan)."""
+    """(token tile N, path, flat shares, grid) that the configuration gives for T tokens (see msk_moe_plan; what a step runs in,
+    which its inputs and norms decide with it, is step_form)."""
     out = (ctypes.c_int * 4)()
     _lib.check(state["lib"].lib.msk_moe_plan(ctypes.byref(state["cfg"]), T, out), "msk_moe_plan")
     return tuple(out)
+
+
+FORMS = {0: "one launch", 1: "chain", 2: "folded", 4: "both GEMMs", 5: "few-token kernel", 6: "FP4 kernel"}
+
+
+def step_form(state, T, given_ids=False):
+    """Which of FORMS kernel_fn runs T tokens in (see msk_moe_step_form), from router logits or given ids and weights."""
+    form = ctypes.c_int(0)
+    inputs = int(given_ids) + 2 * int(state.get("pre_norm_w") is not None) + 8 * int(state["post_norm_w"] is not None)
+    _lib.check(state["lib"].lib.msk_moe_step_form(ctypes.byref(state["cfg"]), T, inputs, ctypes.byref(form)), "msk_moe_step_form")
+    return FORMS[form.value]
 
 
 def export_weights(state):

@@ -81,6 +81,7 @@ SIGNATURES = {
     "msk_moe_plan": [_CFG, ctypes.c_int, _INTP],
     "msk_moe_few_fits": [_CFG, ctypes.c_int, ctypes.c_int, _INTP],
     "msk_moe_nvf4_takes": [_CFG, ctypes.c_int, ctypes.c_int, _INTP],
+    "msk_moe_step_form": [_CFG, ctypes.c_int, ctypes.c_int, _INTP],
     "msk_moe_share_pieces": [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                              _INTP, ctypes.c_int, _INTP],
     "msk_moe_workspace_view": [_CFG, _P, ctypes.c_int, ctypes.POINTER(_P)],

@@ -397,6 +397,43 @@ def test_fp4_kernel_is_taken_where_it_was_measured_faster(shape, norms, taken):
     assert got == [T for a, b in taken for T in range(a, b + 1)]
 
 
+_SMALL = dict(hidden=2048, inter=1024, n_experts=64, local_count=64, top_k=4)
+_GIVEN, _PRE, _HOST_X, _POST = 1, 2, 4, 8                                # inputs of msk_moe_step_form
+_ONE_LAUNCH, _CHAIN, _FOLDED, _BOTH, _FEW, _NVF4 = 0, 1, 2, 4, 5, 6      # what it answers
+
+
+@pytest.mark.parametrize("shape,inputs,forms", [     # (first token count, form), each up to the next one
+    (_SMALL, 0, [(1, _FEW), (4, _ONE_LAUNCH), (9, _BOTH)]), (_SMALL, _GIVEN, [(1, _FEW), (4, _ONE_LAUNCH), (9, _BOTH)]),
+    (_SMALL, _POST, [(1, _FEW), (4, _BOTH)]), (_SMALL, _HOST_X, [(1, _FEW), (4, _BOTH)]), (_SMALL, _HOST_X | _POST, [(1, _FEW), (4, _BOTH)]),
+    (_SMALL, _PRE, [(1, _FEW), (7, _FOLDED), (9, _CHAIN), (113, _BOTH)]),          # (narrow tiles to 7 rows an expert, row copy in front of them)
+    (_SMALL, _PRE | _POST, [(1, _FEW), (7, _CHAIN), (113, _BOTH)]),
+    (_ONE, 0, [(1, _FEW), (4, _ONE_LAUNCH), (6, _NVF4), (193, _BOTH)]), (_ONE, _POST, [(1, _FEW), (4, _NVF4), (193, _BOTH)]),
+    (_ONE, _HOST_X, [(1, _FEW), (3, _BOTH), (6, _NVF4), (193, _BOTH)]),
+    (_RANK, 0, [(1, _FEW), (4, _ONE_LAUNCH), (9, _BOTH), (20, _NVF4), (385, _BOTH)]),
+    (_RANK, _PRE | _POST, [(1, _FEW), (7, _NVF4), (9, _CHAIN), (20, _NVF4), (385, _BOTH)]),
+    (dict(_SMALL, decode_path=3), _POST, [(1, _FEW), (4, _ONE_LAUNCH), (33, _CHAIN), (193, _BOTH)]),
+    (dict(_SMALL, decode_path=3), _PRE | _POST, [(1, _FEW), (7, _FOLDED), (33, _CHAIN), (193, _BOTH)]),
+    (dict(_SMALL, decode_path=2), _POST, [(1, _FOLDED), (33, _CHAIN), (193, _BOTH)]),
+    (dict(_SMALL, decode_path=1), _POST, [(1, _CHAIN)]), (dict(_SMALL, decode_path=4), _POST, [(1, _BOTH)]),
+    (dict(_SMALL, num_ctas=256), 0, [(1, _FOLDED), (9, _CHAIN), (641, _BOTH)])])
+def test_step_form_names_what_a_step_runs_in(shape, inputs, forms):
+    """Both sides of every line between the forms, by the function that launches them: four tokens with the post-expert norm, rows in host
+    memory, the end of the narrow tile (7 rows an expert, 12 where a path is asked for), the FP4 and the few-token kernel."""
+    from muse_moe_w4a16 import _lib
+
+    cfg = _lib.MskMoeCfg(**dict(dict(local_start=0, max_tokens=1024), **shape))
+    want = {}
+    for first, form in forms:
+        want.update({T: form for T in range(first, 1025)})
+    got = {}
+    for T in range(1, 1025):
+        form = ctypes.c_int(-1)
+        # (rows in host memory make a difference up to eight tokens only)
+        assert _lib.load().msk_moe_step_form(ctypes.byref(cfg), T, inputs & ~(_HOST_X if T > 8 else 0), ctypes.byref(form)) == 0
+        got[T] = form.value
+    assert got == want, [(T, got[T], want[T]) for T in got if got[T] != want[T]][:5]
+
+
 def test_workspace_init_covers_every_control_word():
     """msk_moe_workspace_init zeroes everything in front of `inter`: the status word, the sort tables,
     both ticket regions, the control words of the few-token paths (token tickets, grid and tile
