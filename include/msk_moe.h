@@ -245,6 +245,7 @@ int msk_moe_nvf4_takes(const MskMoeCfg* cfg, int n_tokens, int norms, int* host_
 /* The form that a step of n_tokens runs in (msk_moe_forward*, not msk_moe_forward_static), *host_form = MSK_FORM_*. inputs: MSK_FEW_* bits and
  * the ones below. No GPU needed. No counterpart in the reference. */
 #define MSK_STEP_POST_NORM 8      /* post_norm_w is given */
+#define MSK_STEP_HOST_ROUTES 16   /* the logits, or the given ids and weights, lie in host memory (as x: MSK_FEW_HOST_X) */
 #define MSK_FORM_ONE_LAUNCH 0     /* routing, sort, both GEMMs and combine in the tcgen05 kernel */
 #define MSK_FORM_CHAIN 1          /* sort, [row copy,] gate/up GEMM, down GEMM, combine */
 #define MSK_FORM_FOLDED 2         /* row copy, gate/up GEMM that routes and sorts, down GEMM that combines */

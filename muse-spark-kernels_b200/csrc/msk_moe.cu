@@ -1030,11 +1030,31 @@ static bool few_takes(const MskMoeCfg* c, int T, int inputs, int grid, FewPlan* 
   return T <= most && few_plan(c, T, (inputs & MSK_FEW_GIVEN_IDS) != 0, grid, f);
 }
 
+// With the pre-expert norm the other forms have a kernel in front of the GEMMs: the folded form (a row copy by many CTAs, then routes in every CTA
+// of both GEMMs) or the chain (a sort launch whose one CTA norms the rows as well, and a combine: a launch more, and nothing that grows with the routes
+// but the combine). The chain takes the steps with the post-expert norm that have local routes enough, from five tokens on (few_takes() has those
+// below). Folded / chain, us, rows of steps, local routes a token:
+//   given ids: a half, H2048 I1024, 8: 26 / 31; one, H2048 8: 29 / 31, H7168 I1280 5: 49 / 52, 8: 55 / 58; two, H2048 8: 34.4 / 32.3, H4096 I1024 48 / 46.5, of less
+// than 40 MB of weights H1024 I512 24.5 / 26.1, H2048 I512 29.5 / 29.7; four, H2048 I1024 46 / 43;
+//   logits, which every CTA ranks: 64 experts 31.4 / 33.7 (one), 37 / 35.5 (two); 128, H4096 I1024 one 47 / 43, I512 43 / 41; 256, H7168 60 / 55 .. 73 / 62.
+// Rows in host memory and routes on the device (many CTAs fetch the rows faster than one): one route, H7168 4: 50 / 70, 8: 59 / 95; four, H2048 8: 44.4 / 46.7; eight,
+// H4096 I1024 6: 79 / 79, 8: 104 / 92. Routes in host memory too, which the folded form fetches once a CTA (35 to 70 us for one step from
+// run to run): eight 1: 41 - 55 / 52, 3: 71 - 110 / 70, 8: 115 - 165 / 95; four 3: 35 - 69 / 41, 8: 65 - 87 / 51; one, H7168 2: 49 - 102 / 70, 8: 88 - 155 / 107.
+static bool chain_with_pre_norm(const MskMoeCfg* c, int T, int inputs) {
+  const bool host_x = (inputs & MSK_FEW_HOST_X) != 0;
+  const double mean = static_cast<double>(c->top_k) * c->local_count / c->n_experts;   // local routes of a token
+  if (host_x && (inputs & MSK_STEP_HOST_ROUTES) != 0) return mean > 2.0 && T >= 3;
+  if ((inputs & MSK_STEP_POST_NORM) == 0 || T <= ONE_LAUNCH_NORM_TOKENS) return false;
+  if (host_x) return mean > 4.0;
+  return mean > 2.0 || (mean == 2.0 && T * mean * 3.0 * c->hidden * c->inter * 0.5625 >= 40e6) ||
+         ((inputs & MSK_FEW_GIVEN_IDS) == 0 && c->n_experts >= 128 && mean >= 1.0);
+}
+
 // The form that a step runs in, MSK_FORM_*, and with the few-token kernel its plan; inputs: MSK_FEW_* and MSK_STEP_* bits. nv_room: whether
 // the workspace has room for the FP4 kernel's split rows.
 // With the post-expert norm the one launch ends with tickets per token and a combine by whole CTAs; from four tokens on the sort, both
 // GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
-// 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2, with both norms 8: 48.8 / 44.6; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
+// 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
 // 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
 // Rows in host memory: every CTA of the one launch reads the logits or ids over PCIe, the sort launch once, H2048 I1024 4: 50 - 53 / 39.0,
 // 8: 65 / 46.8, given ids 8: 59 - 71 / 44.2; H4096 I1536 E128 4: 95 / 78.5, given ids 3: 71 - 76 / 62.2, 4: 92 - 98 / 73.
@@ -1045,8 +1065,8 @@ static int step_form(const MskMoeCfg* c, int T, const Plan& p, int inputs, bool 
   if (nv) return MSK_FORM_NVF4;
   if (p.path == 2) return MSK_FORM_FOLDED;
   if (p.path == 0) {
-    if (c->decode_path == 0 && (host_x || (post && T >= ONE_LAUNCH_NORM_TOKENS))) return pre ? MSK_FORM_CHAIN : MSK_FORM_BOTH_GEMMS;
-    return pre ? MSK_FORM_FOLDED : MSK_FORM_ONE_LAUNCH;   // (the pre-expert norm needs a kernel in front of the GEMMs)
+    if (pre) return c->decode_path == 0 && chain_with_pre_norm(c, T, inputs) ? MSK_FORM_CHAIN : MSK_FORM_FOLDED;
+    return c->decode_path == 0 && (host_x || (post && T >= ONE_LAUNCH_NORM_TOKENS)) ? MSK_FORM_BOTH_GEMMS : MSK_FORM_ONE_LAUNCH;
   }
   if (p.N == 128) return c->decode_path == 1 || c->stop_after == 2 ? MSK_FORM_CHAIN : MSK_FORM_BOTH_GEMMS;
   return p.both && (p.N == 64 || !pre) ? MSK_FORM_BOTH_GEMMS : MSK_FORM_CHAIN;   // narrow tiles: the pre-expert norm needs the row-copy kernel
@@ -1497,8 +1517,9 @@ static int forward_impl(const MskMoeCfg* cfg, const void* packed13, const void* 
   p.eps = cfg->post_norm_eps;
   FewPlan few;
   const bool host_x = plan.path == 0 && n_tokens <= FEW_TOKENS && in_host_memory(x);
+  const bool host_routes = host_x && pre_norm_w != nullptr && in_host_memory(logits != nullptr ? static_cast<const void*>(logits) : topk_ids);
   const int inputs = (logits == nullptr ? MSK_FEW_GIVEN_IDS : 0) | (pre_norm_w != nullptr ? MSK_FEW_PRE_NORM : 0) |
-                     (host_x ? MSK_FEW_HOST_X : 0) | (post_norm_w != nullptr ? MSK_STEP_POST_NORM : 0);
+                     (host_x ? MSK_FEW_HOST_X : 0) | (post_norm_w != nullptr ? MSK_STEP_POST_NORM : 0) | (host_routes ? MSK_STEP_HOST_ROUTES : 0);
   const int form = step_form(cfg, n_tokens, plan, inputs, k.nv_end <= workspace_bytes, &few);
   const bool nv = form == MSK_FORM_NVF4;
   if (form == MSK_FORM_FEW) {

@@ -398,7 +398,7 @@ def test_fp4_kernel_is_taken_where_it_was_measured_faster(shape, norms, taken):
 
 
 _SMALL = dict(hidden=2048, inter=1024, n_experts=64, local_count=64, top_k=4)
-_GIVEN, _PRE, _HOST_X, _POST = 1, 2, 4, 8                                # inputs of msk_moe_step_form
+_GIVEN, _PRE, _HOST_X, _POST, _HOST_ROUTES = 1, 2, 4, 8, 16                              # inputs of msk_moe_step_form
 _ONE_LAUNCH, _CHAIN, _FOLDED, _BOTH, _FEW, _NVF4 = 0, 1, 2, 4, 5, 6      # what it answers
 
 
@@ -407,6 +407,17 @@ _ONE_LAUNCH, _CHAIN, _FOLDED, _BOTH, _FEW, _NVF4 = 0, 1, 2, 4, 5, 6      # what 
     (_SMALL, _POST, [(1, _FEW), (4, _BOTH)]), (_SMALL, _HOST_X, [(1, _FEW), (4, _BOTH)]), (_SMALL, _HOST_X | _POST, [(1, _FEW), (4, _BOTH)]),
     (_SMALL, _PRE, [(1, _FEW), (7, _FOLDED), (9, _CHAIN), (113, _BOTH)]),          # (narrow tiles to 7 rows an expert, row copy in front of them)
     (_SMALL, _PRE | _POST, [(1, _FEW), (7, _CHAIN), (113, _BOTH)]),
+    # both norms: the chain from five tokens on, with more than two local routes a token, two of 40 MB, one behind the top-k of 128 experts
+    (dict(_SMALL, local_count=16), _PRE | _POST, [(1, _FEW), (7, _FOLDED), (9, _CHAIN), (113, _BOTH)]),
+    (dict(_SMALL, local_count=32), _PRE | _POST, [(1, _FEW), (7, _CHAIN), (113, _BOTH)]),
+    (dict(_SMALL, local_count=32, inter=768), _PRE | _POST, [(1, _FEW), (7, _FOLDED), (8, _CHAIN), (113, _BOTH)]),
+    (dict(_SMALL, hidden=7168, n_experts=256, local_count=32, top_k=8), _PRE | _POST, [(1, _FEW), (5, _CHAIN), (225, _BOTH)]),
+    (dict(_SMALL, hidden=7168, n_experts=256, local_count=32, top_k=8), _GIVEN | _PRE | _POST, [(1, _FEW), (5, _FOLDED), (9, _CHAIN), (225, _BOTH)]),
+    # rows in host memory, routes on the device or there as well
+    (_SMALL, _HOST_X | _PRE | _POST, [(1, _FOLDED), (9, _CHAIN), (113, _BOTH)]), (_SMALL, _HOST_X | _PRE, [(1, _FOLDED), (9, _CHAIN), (113, _BOTH)]),
+    (dict(_SMALL, top_k=8), _HOST_X | _PRE | _POST, [(1, _FOLDED), (5, _CHAIN), (57, _BOTH)]),
+    (_SMALL, _HOST_X | _HOST_ROUTES | _PRE, [(1, _FOLDED), (3, _CHAIN), (113, _BOTH)]),
+    (dict(_SMALL, local_count=32), _HOST_X | _HOST_ROUTES | _GIVEN | _PRE | _POST, [(1, _FOLDED), (9, _CHAIN), (113, _BOTH)]),
     (_ONE, 0, [(1, _FEW), (4, _ONE_LAUNCH), (6, _NVF4), (193, _BOTH)]), (_ONE, _POST, [(1, _FEW), (4, _NVF4), (193, _BOTH)]),
     (_ONE, _HOST_X, [(1, _FEW), (3, _BOTH), (6, _NVF4), (193, _BOTH)]),
     (_RANK, 0, [(1, _FEW), (4, _ONE_LAUNCH), (9, _BOTH), (20, _NVF4), (385, _BOTH)]),
@@ -429,7 +440,7 @@ def test_step_form_names_what_a_step_runs_in(shape, inputs, forms):
     for T in range(1, 1025):
         form = ctypes.c_int(-1)
         # (rows in host memory make a difference up to eight tokens only)
-        assert _lib.load().msk_moe_step_form(ctypes.byref(cfg), T, inputs & ~(_HOST_X if T > 8 else 0), ctypes.byref(form)) == 0
+        assert _lib.load().msk_moe_step_form(ctypes.byref(cfg), T, inputs & ~(_HOST_X | _HOST_ROUTES if T > 8 else 0), ctypes.byref(form)) == 0
         got[T] = form.value
     assert got == want, [(T, got[T], want[T]) for T in got if got[T] != want[T]][:5]
 
