@@ -70,7 +70,7 @@ typedef struct MskMoeCfg {
   int32_t no_pdl;        /* non-zero: launches are not chained with programmatic dependent launch (the reference's
                             okc_set_pdl(0), muse_moe_w4a16/cuda/moe.cu:2348,2565) */
   int32_t token_tile;    /* MMA N (tokens per tile): 16/32/64/128; 0 = chosen from the mean rows per expert
-                            (up to 7, or 12 with decode_path set: 16, up to 40: 64, beyond: 128). 128 stands for the kernel on pairs of SMs,
+                            (up to 7, or 12 with decode_path, flat_shares or stop_after set: 16, up to 40: 64, beyond: 128). 128 stands for the kernel on pairs of SMs,
                             whose tiles hold up to 256 rows; it rounds num_ctas up to an even number */
   int32_t max_tokens;    /* token capacity the workspace is sized for (msk_moe_forward rejects more) */
   int32_t trace;         /* non-zero: the GEMM kernels stamp %globaltimer per CTA into the workspace (view 6) */

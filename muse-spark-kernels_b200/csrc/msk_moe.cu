@@ -616,6 +616,9 @@ struct Plan {
   bool both;     // both GEMMs in one launch: path 4, and the 64-token tile of path 1
 };
 
+// A form that the configuration asks for is always the asked one.
+static bool form_asked(const MskMoeCfg* c) { return c->token_tile != 0 || c->decode_path != 0 || c->flat_shares != 0 || c->stop_after != 0; }
+
 static Plan make_plan(const MskMoeCfg* c, int T) {
   Plan p;
   p.grid = c->num_ctas > 0 ? std::min(c->num_ctas, MAX_CTAS) : DEFAULT_CTAS;
@@ -627,16 +630,17 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     const double rpe = static_cast<double>(T) * c->top_k / c->n_experts;  // mean tokens per expert
     // 16 / 64-token tile (us, rows of steps): H2048 I1024 E64 near-even rpe 4 58.9 / 58.8, 6 61.1 / 59.8, 8 63.2 / 61.2, 12 68.9 / 63.0, a few experts
     // taking most tokens 45.3 / 47.0, 51.9 / 51.4, 55.1 / 53.7, 67.0 / 59.6; H4096 I1024 E128 rpe 4 193 / 199 (105 / 90), 6 202 / 205, 8 210 / 208 (158 / 117), 12
-    // 238 / 215 (210 / 144); H4096 I1280 E128 rpe 6 247 / 250, 8 254 / 252. 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
+    // 238 / 215 (210 / 144); H4096 I1280 E128 rpe 6 247 / 250, 8 254 / 252. Few narrow experts, top-2 of 8, rpe 7.25 / 8 / 10 / 12: H4096 I1024 41.2 / 39.2, 41.3 /
+    // 39.2, 41.4 / 39.3, 43.2 / 39.3 (43.3 / 41.4, 43.3 / 42.2, 43.3 / 43.4, 43.3 / 44.9); H1024 I512 28.9 / 27.1 .. 29.0 / 28.8 (29.0 / 28.8 .. 29.1 / 31.0). 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
     // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. Beyond: rpe 48 near-even
     // 406 / 464, 32 of 256 experts at H4096 I4096 255 / 289, a few experts taking most 456 / 420, the same at H2048 I1024 E64
     // 107 / 88; rpe 56 445 / 477, 279 / 295, 508 / 452, 114 / 95; rpe 64 near-even 566 / 505. At rpe 40 the 64-token tile loses 13 %
     // at worst and the pair kernel 18, at 48 it is 21 and 20. The 16-token tile is the
     // fastest per K stage and wins while most experts fit one tile; the 64-token tile wins while most fit one of those. The
     // host does not know the counts, and the less even they are the lower that line lies. The 32-token tile never wins at
-    // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh). Where a path is asked for
-    // the narrow tile, which the paths are made for, stays up to 12.
-    p.N = rpe <= (c->decode_path == 0 ? 7 : 12) ? 16 : rpe <= 40 ? 64 : 128;
+    // these shapes (it stays selectable with cfg.token_tile). 128 stands for the pair kernel (pair.cuh). Where a path, flat shares or
+    // a part of the step is asked for, the narrow tile, which those are made for, stays up to 12.
+    p.N = rpe <= (form_asked(c) ? 12 : 7) ? 16 : rpe <= 40 ? 64 : 128;
   }
   const long long rows = static_cast<long long>(T) * c->top_k;
   // Flat shares are an option, off by default: measured on B200 a cut unit's pieces cost about 6 us of
@@ -724,9 +728,6 @@ static double nv_even_bytes(const MskMoeCfg* c, int T) {
   const double touched = c->n_experts * (1.0 - std::pow(1.0 - static_cast<double>(c->top_k) / c->n_experts, T));
   return touched * 3.0 * c->hidden * c->inter * 0.5625;
 }
-
-// A form that the configuration asks for is always the asked one.
-static bool form_asked(const MskMoeCfg* c) { return c->token_tile != 0 || c->decode_path != 0 || c->flat_shares != 0 || c->stop_after != 0; }
 
 // Whether a step runs in it; norms: MSK_NVF4_* bits.
 static bool nv_takes(const MskMoeCfg* c, int T, const Plan& p, int norms) {

@@ -307,6 +307,19 @@ def test_plan_is_a_function_of_the_configuration_only():
     assert lib.msk_moe_plan(ctypes.byref(cfg), 64, plan) == 0 and tuple(plan) == (16, 1, 0, 37)
 
 
+@pytest.mark.parametrize("asked,T,plan", [({}, 28, (16, 0)), ({}, 29, (64, 0)), (dict(flat_shares=1), 29, (16, 1)), (dict(flat_shares=1), 48, (16, 1)),
+                                          (dict(flat_shares=1), 49, (64, 1)), (dict(stop_after=1), 48, (16, 0)), (dict(stop_after=3), 49, (64, 0)),
+                                          (dict(decode_path=1), 48, (16, 0))])
+def test_a_form_that_is_asked_for_keeps_the_narrow_tile(asked, T, plan):
+    """From 7 rows an expert on the default tile is 64; paths, flat shares and parts of the step, asked for, keep the 16-token tile to 12."""
+    from muse_moe_w4a16 import _lib
+
+    cfg = _lib.MskMoeCfg(**dict(dict(hidden=2048, inter=1024, n_experts=16, local_start=0, local_count=16, top_k=4, max_tokens=64), **asked))
+    out = (ctypes.c_int * 4)()
+    assert _lib.load().msk_moe_plan(ctypes.byref(cfg), T, out) == 0
+    assert (out[0], out[2]) == plan
+
+
 def _few_fits(T, inputs=0, **shape):
     from muse_moe_w4a16 import _lib
 
