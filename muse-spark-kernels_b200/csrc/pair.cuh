@@ -41,8 +41,8 @@
 // 462 -> 444; 777 tokens, 49 rows an expert, 397 -> 369. Bound by the hand-over of the K stages of the rings (activation rows and A
 // slots come back, are refilled over L2 and by the decode warps, 1100 cycles a stage at the least) and, with full tiles, by the MMAs
 // and the power limit; the tensor core also stands still while an accumulator of more than 128 columns is drained.
-// Two K stages of token rows are in flight with tiles of more than 128 rows; narrower ones, which fill half of a place, have four
-// (pair_b_waits_for). With two for all, the loads of 64 to 96 rows an expert, evenly spread, were up to 4 % behind the kernel replaced:
+// Two K stages of token rows are in flight with tiles of more than 128 rows; narrower ones, which take one of a stage's two places, have four
+// (pair_b_place). With two for all, the loads of 64 to 96 rows an expert, evenly spread, were up to 4 % behind the kernel replaced:
 // whole steps at H4096 I1536 E128 with that kernel / two stages / four, 64 rows 468 / 471 / 458 us, 80 rows 552 / 560 / 541, 96
 // rows 565 / 586 / 572; 32 of 256 experts at H7168 I2048, 80 rows 305 / 313 / 300, 128 rows 387 / 374 / 364.
 #pragma once
@@ -357,7 +357,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
           if (!ready && !mbar_wait_inline(&ctl.full[st & 3u], (st >> 2) & 1u, abortw)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sn = st + 1u, sl = (st & 1u) * 2u;
-          const uint32_t place = sl * C::B_SLOT_BYTES + (db.wide ? 0u : ((st >> 1) & 1u) * C::B_SLOT_BYTES);
+          const uint32_t place = pair_b_place(st, u.nmma) * C::B_SLOT_BYTES;
           ready = mma_stage_pair(d_tmem, tmem + C::A_BASE + sl * PAIR_SLOT_COLS, b_desc0 + (place >> 4), idesc, accumulate,
                                  smem_u32(&ctl.empty[(st & 3u) * 2u]), smem_u32(&ctl.full[sn & 3u]), (sn >> 2) & 1u, sub);
           st = sn;
@@ -374,7 +374,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
     // One thread, one wait and one copy a K stage: as a warp that elects a lane for four copies, each half a stage behind a wait of its
     // own, this role took 850 cycles a stage beside the decode warps, and set the pace of tiles of few rows.
     const uint64_t keep = policy_evict_last();     // token rows are re-read by every pair of the expert
-    uint32_t n = 0, wide_end = 0;                  // slot, through all units; the one behind the last wide tile's
+    uint32_t st = 0, wide_end = 0;                 // K stage, through all units; the one behind the last wide tile's
     bool ok = true;
     if (elect_one()) {
       int last_tile = -1;
@@ -399,22 +399,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             atomicExch(p.tile_seen + u.tile, 0u);
           }
         }
-        for (int k = 0; k < K; k += KS, n += 2) {
-          // both slots of the stage: MMAs are done in order, so the second one's barrier tells (of the first slots: a barrier that
-          // nothing has completed, parity 1)
-          const uint32_t before = pair_b_waits_for(n, u.nmma, wide_end) + 1u;
+        for (int k = 0; k < K; k += KS, ++st) {
+          const uint32_t before = pair_b_waits_for(st, u.nmma, wide_end);   // (of the first stages: a barrier that nothing has completed, parity 1)
           if (!mbar_wait_inline(&ctl.empty[before & 7u], (before >> 3) & 1u, abortw)) { ok = false; break; }
-          const uint32_t i = n >> 1;
-          if (rank == 0) mbar_arrive_expect_tx(&ctl.full[i & 3u], bytes);
-          uint8_t* dst = b_ring + (i & 1u) * (2 * C::B_SLOT_BYTES) + (half > BH / 2 ? 0u : ((i >> 1) & 1u) * C::B_SLOT_BYTES);
-          tma_load_3d_pair(dst, map, 0, row, k >> 6, lead_bar(&ctl.full[i & 3u]), keep);
+          if (rank == 0) mbar_arrive_expect_tx(&ctl.full[st & 3u], bytes);
+          tma_load_3d_pair(b_ring + pair_b_place(st, u.nmma) * C::B_SLOT_BYTES, map, 0, row, k >> 6, lead_bar(&ctl.full[st & 3u]), keep);
         }
-        if (half > BH / 2) wide_end = n;
+        if (u.nmma > BH) wide_end = st;
       }
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok);
-    n = __reduce_max_sync(0xffffffffu, n);
+    uint32_t n = 2u * __reduce_max_sync(0xffffffffu, st);
     // the commits of the last slots arrive in this CTA's shared memory: it stays until they have
     for (int i = 0; ok && i < PAIR_MARKS; ++i) {
       --n;
@@ -483,7 +479,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) moe
             const int per = pair_tile_rows(c, nt), at = (tile - tile_start[lo]) * per;
             const int rows = min(per, c - at);
             a = make_int4(phase, lo, off_s[lo] + at, rows);
-            b = make_int4(pair, tile, (rows + 15) & ~15, nt > 1 ? 1 : 0);
+            b = make_int4(pair, tile, pair_cols(rows), nt > 1 ? 1 : 0);
           }
           const uint32_t s = i % PAIR_UNITS;
           const uint32_t par = ((i / PAIR_UNITS) & 1u) ^ 1u;   // of the unit whose place this one takes

@@ -13,8 +13,8 @@ namespace msk {
 
 constexpr int PAIR_BH = 128;             // most token rows a CTA holds of a tile; columns of an accumulator buffer
 constexpr int PAIR_SLOT_K = 128;         // K of an A / B slot
-constexpr int PAIR_NSLOT = 4;            // A slots; B slots of PAIR_BH rows
-constexpr int PAIR_MARKS = 2 * PAIR_NSLOT;   // slots whose MMAs have their own barrier; B slots of PAIR_BH / 2 rows
+constexpr int PAIR_NSLOT = 4;            // A slots; places of token rows, each PAIR_SLOT_K of PAIR_BH rows in either CTA
+constexpr int PAIR_MARKS = 2 * PAIR_NSLOT;   // slots whose MMAs have their own barrier
 constexpr int PAIR_GROUPS = 4;           // of decode warps: group g fills the slots g, g + PAIR_GROUPS, ... of the list of all slots
 constexpr int PAIR_NST = 5;              // weight stages
 constexpr int PAIR_UNITS = 4;            // units handed out ahead of their use
@@ -23,11 +23,20 @@ constexpr int PAIR_UNITS = 4;            // units handed out ahead of their use
 // is never empty: a share is below its limit only while the limit exceeds c / n by more than the rounding).
 MSK_HOST_DEVICE inline int pair_tile_rows(int c, int n) { return ((c + n - 1) / n + 31) & ~31; }
 
-// The slot whose MMAs have to be done before token rows are copied into slot n: the last one that used any of its bytes. A
-// tile of up to PAIR_BH rows (half of them in either CTA) fills half a place of the ring and alternates between the halves, so that its
-// rows are fetched twice as many slots ahead; `wide_end`: the number behind the last slot of a wider tile.
-MSK_HOST_DEVICE inline unsigned pair_b_waits_for(unsigned n, int cols, unsigned wide_end) {
-  return cols <= PAIR_BH && n >= wide_end + PAIR_NSLOT ? n - PAIR_MARKS : n - PAIR_NSLOT;
+// Columns of the MMAs of a tile with `rows` rows, half of them (eight at the least) from either CTA.
+MSK_HOST_DEVICE inline int pair_cols(int rows) { return (rows + 15) & ~15; }
+
+// Token rows come a K stage at a time: the two slots 2 * stage and 2 * stage + 1, numbered through all units. Where a stage lies: a tile of more than
+// PAIR_BH columns takes two places, this one and the next; a narrower one (half of its rows are PAIR_BH / 2 at the most) takes one, in
+// turn with the other of the pair, so that its rows are fetched four stages ahead instead of two.
+MSK_HOST_DEVICE inline unsigned pair_b_place(unsigned stage, int cols) {
+  return (stage & 1u) * 2u + (cols > PAIR_BH ? 0u : (stage >> 1) & 1u);
+}
+
+// The slot whose MMAs have to be done before the rows of a stage are copied: the second one of the last stage that used any of its bytes
+// (MMAs are done in order). `wide_end`: the number behind the last stage of a tile of more than PAIR_BH columns.
+MSK_HOST_DEVICE inline unsigned pair_b_waits_for(unsigned stage, int cols, unsigned wide_end) {
+  return 2u * (cols <= PAIR_BH && stage >= wide_end + 2u ? stage - 4u : stage - 2u) + 1u;
 }
 
 // Slots of its next unit that a decode warp fills before it drains the unit it owes (phase 0 gate/up, 1 down; cols: columns

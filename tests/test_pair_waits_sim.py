@@ -1,5 +1,5 @@
 """The waits of the pair kernel (csrc/pair.cuh), replayed on the CPU: per cluster the scheduler, the weight producer, the
-activation warp, the MMA issuer and the four groups of decode warps, each walking the units it is handed in the order of the
+activations, the MMA issuer and the four groups of decode warps, each walking the units it is handed in the order of the
 kernel and standing still until what it waits for has happened. Units are drawn from one counter by clusters that run at
 different speeds or start late. Ring sizes and the rule when accumulators are drained are compiled from the kernel's own
 header (csrc/pair_sched.h). Checked: every cluster reaches the end of the list, for any number of token tiles, any reduction
@@ -11,6 +11,7 @@ one stands for both."""
 import ctypes
 import os
 import random
+import re
 import subprocess
 
 import pytest
@@ -25,7 +26,9 @@ def sched(tmp_path_factory):
     src, so = d / "shim.cpp", d / "shim.so"
     src.write_text('#include "pair_sched.h"\nextern "C" {\n'
                    "int tile_rows(int c, int n) { return msk::pair_tile_rows(c, n); }\n"
-                   "int b_waits_for(int n, int c, int w) { return (int)msk::pair_b_waits_for(n, c, w); }\n"
+                   "int b_waits_for(int s, int c, int w) { return (int)msk::pair_b_waits_for(s, c, w); }\n"
+                   "int b_place(int s, int c) { return (int)msk::pair_b_place(s, c); }\n"
+                   "int cols(int rows) { return msk::pair_cols(rows); }\n"
                    "int before_drain(int a, int b, int c, int d) { return msk::pair_slots_before_drain(a, b, c, d); }\n"
                    + "".join(f"int c_{n}() {{ return msk::{n}; }}\n" for n in NAMES) + "}\n")
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", str(so), str(src)], check=True)
@@ -43,7 +46,7 @@ class Cluster:
         self.announced = 0              # units whose stores were announced (or need not be)
         self.done = False
         self.act_unit = self.act_slots = 0              # activations: unit walked, slots filled,
-        self.wide_end = 0                               # number behind the last slot of a wide tile
+        self.wide_end = 0                               # number behind the last stage of a wide tile
         self.raw_unit = self.raw_stages = 0             # weights: unit walked, stages issued
         self.mma_unit = self.mma_slots = 0              # MMAs: unit walked, slots read and handed back
         G = c["PAIR_GROUPS"]
@@ -104,13 +107,13 @@ class Cluster:
         phase, tile, cols, nsl = self.units[self.act_unit]
         if phase == 1 and self.act_slots == self.first[self.act_unit] and not self.deal.complete(tile):
             return False
-        if self.b_waits_for(self.act_slots, cols, self.wide_end) >= self.mma_slots:
+        if self.b_waits_for(self.act_slots // 2, cols, self.wide_end) >= self.mma_slots:
             return False
-        self.act_slots += 1
+        self.act_slots += 2                             # a stage, two slots, at a time
         if self.act_slots == self.first[self.act_unit] + nsl:
             self.act_unit += 1
             if cols > self.c["PAIR_BH"]:
-                self.wide_end = self.act_slots
+                self.wide_end = self.act_slots // 2
         return True
 
     def mma(self):
@@ -235,7 +238,7 @@ def _constants(sched):
 
 def _tiles(kind, n, seed):
     rng = random.Random(seed)
-    return [{"narrow": 64, "wide": 256}.get(kind) or rng.choice((32, 64, 96, 128, 160, 256)) for _ in range(n)]
+    return [{"narrow": 64, "wide": 256}.get(kind) or rng.choice((16, 48, 64, 112, 128, 144, 240, 256)) for _ in range(n)]
 
 
 @pytest.mark.parametrize("H,inter,clusters", [(4096, 256, 74), (4096, 512, 74), (4096, 768, 74), (4096, 1536, 74), (4096, 4096, 74),
@@ -259,28 +262,55 @@ def test_the_model_sees_a_drain_behind_the_down_units_mmas(sched, H, inter, clus
     assert not all(ends(c, old_rule(c), sched.b_waits_for, [64] * tiles, H, inter, clusters, seed) for seed in range(seeds))
 
 
-def test_token_rows_overwrite_only_what_the_mmas_have_read(sched):
-    """The ring of token rows, byte by byte: a slot of a wide tile takes a whole place, one of a narrow tile the half that the place's
-    slot before did not take (the addresses of the activation warp). Every slot that last used a byte is, by number, at or before
-    the one the copy waits for; MMAs are done in order."""
-    c = _constants(sched)
-    N = c["PAIR_NSLOT"]
+def overwrites_only_read_rows(c, sched, waits_for):
+    """The ring of token rows, place by place, over units of random widths: whether, when a stage's copy starts, the MMAs of every stage that
+    last used one of its places are done (MMAs are done in order), and the barrier waited for has not come round again."""
     for seed in range(40):
         rng = random.Random(seed)
-        user = [[-1, -1] for _ in range(N)]
-        n = wide_end = 0
+        user = [-1] * c["PAIR_NSLOT"]
+        stage = wide_end = 0
         for _ in range(60):
-            wide = rng.random() < (0.5, 0.1, 0.9)[seed % 3]
-            for _ in range(2 * rng.choice((1, 1, 2, 3, 5, 8))):
-                halves = (0, 1) if wide else ((n // N) % 2,)
-                waits = sched.b_waits_for(n, 2 * c["PAIR_BH"] if wide else c["PAIR_BH"], wide_end)
-                assert max(user[n % N][h] for h in halves) <= max(waits, -1) and waits < n
-                assert waits >= n - c["PAIR_MARKS"]      # the barrier of that slot has not come round again
-                for h in halves:
-                    user[n % N][h] = n
-                n += 1
+            cols = sched.cols(rng.randint(129, 256) if rng.random() < (0.5, 0.1, 0.9)[seed % 3] else rng.randint(1, 128))
+            wide = cols > c["PAIR_BH"]
+            for _ in range(rng.choice((1, 1, 2, 3, 5, 8))):
+                at = sched.b_place(stage, cols)
+                places = (at, at + 1) if wide else (at,)
+                # the four sub-tiles of 64 K, 128 bytes a row, fit what the stage takes
+                assert places[-1] < c["PAIR_NSLOT"] and 4 * 128 * (cols // 2) <= len(places) * c["PAIR_BH"] * 2 * c["PAIR_SLOT_K"]
+                waits = waits_for(stage, cols, wide_end)
+                if max(user[p] for p in places) >= 0 and 2 * max(user[p] for p in places) + 1 > waits:
+                    return False
+                if not 2 * stage - c["PAIR_MARKS"] <= waits < 2 * stage:
+                    return False
+                for p in places:
+                    user[p] = stage
+                stage += 1
             if wide:
-                wide_end = n
+                wide_end = stage
+    return True
+
+
+def test_token_rows_overwrite_only_what_the_mmas_have_read(sched):
+    """With the places and the waits of the kernel's own header; and the replay sees waits that are too short."""
+    c = _constants(sched)
+    assert overwrites_only_read_rows(c, sched, sched.b_waits_for)
+    narrow = lambda cols: cols <= c["PAIR_BH"]  # noqa: E731
+    assert not overwrites_only_read_rows(c, sched, lambda s, cols, w: 2 * (s - (4 if narrow(cols) else 2)) + 1)     # no regard to wide tiles before
+    assert not overwrites_only_read_rows(c, sched, lambda s, cols, w: sched.b_waits_for(s, cols, w) - 1)             # a stage's first slot
+    assert not overwrites_only_read_rows(c, sched, lambda s, cols, w: sched.b_waits_for(s, cols, max(w - 1, 0)))     # a stage too early
+
+
+def test_the_kernel_takes_places_and_waits_from_the_header():
+    """Copies and MMAs both ask pair_b_place, and the copies wait for pair_b_waits_for as it stands."""
+    src = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "pair.cuh")).read())
+    assert len(re.findall(r"\bpair_b_place\(st, u\.nmma\) \* C::B_SLOT_BYTES", src)) == src.count("pair_b_place(") == 2
+    assert re.findall(r"before = (pair_b_waits_for\([^;]*);\s*if \(!mbar_wait_inline\(&ctl\.empty\[before & 7u\], \(before >> 3\) & 1u", src) == ["pair_b_waits_for(st, u.nmma, wide_end)"]
+
+
+def test_columns_are_whole_rows_of_either_cta(sched):
+    for rows in range(1, 257):
+        cols = sched.cols(rows)
+        assert rows <= cols < rows + 16 and cols % 16 == 0 and cols <= 256
 
 
 def test_tile_rows_share_an_expert_evenly(sched):
