@@ -768,21 +768,25 @@ def test_few_tokens_with_the_post_norm_around_the_end_of_the_one_launch(cuda_dev
         w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
     st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8)
     asked = m.prepare(w, n_experts=E, top_k=k, max_tokens=8, decode_path=4)
-    data = {"hidden_states": torch.randn((T, H), generator=g, device=cuda_dev).to(torch.bfloat16)}
+    data = {"hidden_states": (torch.randn((T, H), generator=g, device=cuda_dev) * 3.0).to(torch.bfloat16)}
     lg = torch.randn((T, E), generator=g, device=cuda_dev)
     if ids:
         tw, top = torch.softmax(lg, dim=-1).topk(k, dim=-1)
         data["topk_ids"], data["topk_weights"] = top.to(torch.int32).contiguous(), tw.contiguous()
     else:
         data["router_logits"] = lg
+    form = m.step_form(st, T, given_ids=ids)
+    assert form == ("few-token kernel" if T == 3 or (pre and T == 4) else "chain" if pre else "both GEMMs")
     for _ in range(2):
-        got, same = m.kernel_fn(data, st), m.kernel_fn(data, asked)
-        assert _rel(got, same.float()) <= TOL
-        if T >= 4 and not pre:
-            assert torch.equal(got, same)
-    if not pre:
-        _, top, tw = m.kernel_fn(data, asked, return_routing=True)
-        assert _rel(got, orc.moe_forward(data["hidden_states"], top, tw, w).float()) <= TOL
+        same = m.kernel_fn(data, asked)
+        got, top, tw = m.kernel_fn(data, st, return_routing=True)
+        ref, parts = orc.moe_forward(data["hidden_states"], top, tw, w, return_parts=True)
+        _check_forward(got, ref, parts, m.workspace_views(st, T))
+        assert torch.equal(got, same) if form != "few-token kernel" else _rel(got, same.float()) <= TOL
+        if not ids:
+            assert torch.equal(top.cpu(), orc.route_topk(lg.cpu(), k)[0])
+    if pre:      # the norm is not a no-op here
+        assert _rel(got, orc.moe_forward(data["hidden_states"], top, tw, {n: v for n, v in w.items() if n != "pre_norm_w"}).float()) > 0.05
     assert m.read_status(st) == 0 and m.read_status(asked) == 0
 
 
