@@ -880,6 +880,42 @@ def test_pinned_token_rows_through_the_c_interface(cuda_dev, T, pre):
         assert any(torch.equal(words[int(a):int(a) + row.numel()], row) for a in at)
 
 
+@pytest.mark.parametrize("T,nloc,host,post", [(2, 16, "x", False), (8, 16, "x", True), (3, 16, "xr", False), (8, 16, "xr", True), (8, 8, "xr", True),
+                                              (8, 4, "", True), (8, 16, "", True), (7, 16, "r", True)])
+@pytest.mark.parametrize("given", [False, True])
+def test_few_tokens_with_the_pre_norm_in_the_chain_and_folded(cuda_dev, T, nloc, host, post, given):
+    """Rows (x) and routes (r) on the device or in pinned memory, few and many local routes: both forms that steps with the pre-expert norm
+    take beyond the few-token kernel, against the oracle, tables and routing included, twice on one state."""
+    m, inputs, _lib, orc = _mods()
+    H, I, E, k, lo = 1280, 512, 16, 4, 16 - nloc
+    w = inputs.make_weights(H, I, nloc, 57, cuda_dev, post_norm=post)
+    g = torch.Generator(device=cuda_dev).manual_seed(60 + T)
+    w["pre_norm_w"] = (torch.randn((H,), generator=g, device=cuda_dev) * 0.1).to(torch.bfloat16)
+    st = m.prepare(w, n_experts=E, top_k=k, max_tokens=8, local_start=lo)
+    place = lambda t, what: t.cpu().pin_memory() if what in host else t  # noqa: E731
+    forms = set()
+    for _ in range(2):
+        x = (torch.randn((T, H), generator=g, device=cuda_dev) * 3.0).to(torch.bfloat16)
+        lg = torch.randn((T, E), generator=g, device=cuda_dev)
+        rid, _ = orc.route_topk(lg.cpu(), k)
+        tw, ids = torch.empty((T, k), device=cuda_dev), torch.empty((T, k), dtype=torch.int32, device=cuda_dev)
+        if given:
+            tw, ids = torch.softmax(lg, dim=-1).topk(k, dim=-1)
+            ids, tw = place(ids.to(torch.int32).contiguous(), "r"), place(tw.contiguous(), "r")
+        xp, lp = place(x, "x"), None if given else place(lg, "r")
+        out = torch.empty((T, H), dtype=torch.bfloat16, device=cuda_dev)
+        m._forward(st, st["cfg"], st["lib"].lib, xp.data_ptr(), None if given else lp.data_ptr(), ids.data_ptr(), tw.data_ptr(), out.data_ptr(), T)
+        torch.cuda.synchronize()
+        assert m.read_status(st) == 0 and torch.equal(ids.cpu(), rid)
+        ref, parts = orc.moe_forward(x, ids.to(cuda_dev), tw.to(cuda_dev), w, local_start=lo, return_parts=True)
+        _check_forward(out, ref, parts, m.workspace_views(st, T))
+        form = ctypes.c_int(0)
+        bits = int(given) + 2 + 4 * ("x" in host) + 8 * post + 16 * (host == "xr")
+        assert st["lib"].lib.msk_moe_step_form(ctypes.byref(st["cfg"]), T, bits, ctypes.byref(form)) == 0
+        forms.add(form.value)
+    assert forms == {1 if nloc == 16 and host != "x" else 2}
+
+
 @pytest.mark.parametrize("T,tile", [(9, 0), (40, 0), (100, 16), (100, 32), (260, 32)])
 def test_both_gemms_in_one_launch_behind_the_sort_gives_the_chain_bits(cuda_dev, T, tile):
     """decode_path = 4 (sort launches, then the gate/up and the down GEMM in one cooperative launch that
