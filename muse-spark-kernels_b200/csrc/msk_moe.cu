@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(COMBINE_COLS_WARPS * 32)
 // an SM. Many tokens: blocks of 128 threads (256 beyond 4096 columns), five or four of them on an SM, where blocks of 512 left two tokens to
 // one: 3012 tokens with 1.6 local routes each 41 -> 18 us, 777 with eight 22 -> 16, 7000 149 -> 98. Up to 2048 columns two octets a
 // thread, which four leave half the block's threads without: 2000 tokens of four at 2048 columns 17 -> 13, 4000 of eight at 1024 39 -> 27. Few
-// tokens: 512 threads and as many rows at once as fit (64 tokens of eight 8 -> 6).
+// tokens: 512 threads and as many rows at once as fit (64 tokens of eight 8 -> 6). Every warp reads the table for itself; where given weights lie in
+// pinned memory that is no slower than one warp's read that the others wait for (whole steps from pinned rows, ids and weights, H2048 I1024, 16 / 24 / 48 tokens,
+// that form / this: 53.6 / 51.7, 59.9 / 58.6, 67.6 / 66.0).
 constexpr int COMBINE_FEW_TOKENS = 256;
 constexpr int COMBINE_MAX_H = 8192;
 template <bool YB, int TH, int NO, int G, int MINB>
@@ -693,7 +695,9 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
 // to 16 tokens lose 1 to 3 %, near-even ones, which stream twice the bytes, gain 13 to 17: the line stays at 6.
 // With the other kernel's issue by one thread and this one's room for four rows (64-token tile / this one, rows of steps) 64: 288 / 240 (123 / 135), 128: 296 / 272
 // (161 / 200), 160: 299 / 292 (182 / 235), 192: 304 / 316 (198 / 263), 256: 316 / 384 (230 / 323); a rank, two experts taking most, 100: 158 / 154, 200: 205 / 213, 384:
-// 242 / 281; H7168 I2048, even, 200: 171 / 159, 300: 176 / 175, 384: 178 / 192: near the line the other one has drawn level.
+// 242 / 281; H7168 I2048, even, 200: 171 / 159, 300: 176 / 175, 384: 178 / 192. By these this one gains 9 % at eight rows an expert of near-even routes and 2 % at
+// ten, loses 4 % at twelve, and loses 24, 29 and 33 % there where a few experts take most; a rank's skewed steps lose 4 % at six rows and 16 at twelve, its even ones 8 at twelve. The line at
+// twelve is the one of before those two changes and is later than they would have it: six to eight rows, or the counts, which the host does not know.
 // A rank (32 of 256, one row a token): H4096 I4096, two experts taking most, 4: 45 / 46, 6: 50 / 49, 8: 59 / 58, 10: 59 / 62, 16: 66 / 67, 18: 69 / 69, 20: 70 / 69,
 // 24: 79 / 76, 28: 86 / 80, 64: 138 / 115, 384: 308 / 263 (512: 236 / 310); H7168 I2048, even, 4: 50 / 51, 6: 50 / 53, 8: 56 / 58, 16: 74 / 74, 18: 77 / 77, 20: 81 /
 // 79, 24: 83 / 80, 28: 91 / 88, 64: 128 / 114, 384: 201 / 171.

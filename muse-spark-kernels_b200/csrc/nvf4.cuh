@@ -156,7 +156,8 @@ __host__ __device__ constexpr int nv_place_bytes(int room) { return (room * (NV_
 
 struct NvCfg {
   static constexpr int TABLE_INTS = MAX_LOCAL_EXPERTS + 4;
-  // The ring of token rows has places for the widest tile of the launch (whole swizzle atoms of 1 KB): 4 or 7 of them. (Places of each pass's
+  // The ring of token rows has places for the widest tile of the launch (whole swizzle atoms of 1 KB): 4 of them, 7 where no tile has more than eight rows, 8 (as
+  // many as there are marks) where none has more than four. (Places of each pass's
   // own size, more of them: 1 % slower; three of them, and three stages of weights ahead: 2 %.)
   static constexpr int B_RING = 76 * 1024;
   static constexpr int W_OFF = 0, B_OFF = NV_W_STAGES * STAGE_W_BYTES, CTL_OFF = B_OFF + B_RING, TABLE_OFF = CTL_OFF + 1024;

@@ -30,7 +30,10 @@
 // (pair_slots_before_drain), so the wait ends whatever part of the grid is resident. Which cluster computes a unit does not
 // change its bits.
 //
-// MMAs are as wide as a tile's rows in steps of sixteen (eight rows in either CTA); in steps of 32 a row of steps took, before / after:
+// MMAs are as wide as a tile's rows in steps of sixteen (eight rows in either CTA). kind::f16 with cta_group::2 and M = 256 takes N from 16
+// to 256 in steps of 16, whichever memory A lies in: the check of tcgen05 operations in CUTLASS's CuTe DSL (MmaOp in cute/nvgpu/tcgen05/mma.py, which cites
+// the PTX manual's section; its exceptions are 8-bit operands) makes no difference between them. Its C++ wrapper for A in tensor memory asserts
+// 32, the one for A in shared memory 16. Every width is compared with the oracle (tests). In steps of 32 a row of steps took, before / after:
 // 777 tokens at H4096 I1536 E128 422 / 411 us, 1500 tokens whose routes favour a few experts 619 / 607, 3012 skewed tokens of a rank 533 / 526,
 // 8192 tokens of one rank of eight, H7168 I2048, 733 / 712.
 //

@@ -362,7 +362,7 @@ class HostMappedStep:
     straight into a pinned host tensor, so a step that starts and ends on the host has no copy
     launches around the kernel at all. At a few tokens the copies are a quarter of the step (launches
     of several microseconds each around a 45 us kernel); the reads they replace are 8 KB per token
-    once, plus the logits row every CTA needs, and cost one PCIe round trip.
+    once, plus the logits, or the given ids and weights, once as well, and cost one PCIe round trip.
 
     step(data) copies data's host tensors into a pinned block, replays the graph captured over that
     block on the current stream and returns the pinned output tensor of that block; it holds this
