@@ -61,7 +61,8 @@ typedef struct MskMoeCfg {
   int32_t decode_path;   /* steps of few tokens (n_tokens <= 32, n_tokens * top_k <= 256, token tile <= 32):
                             0 = chosen by token count (one launch up to 8 tokens, the chain beyond; the step
                             itself leaves the one launch from 4 tokens with the post-expert norm, and with
-                            rows in host memory, for form 4),
+                            rows in host memory, for form 4, and with the pre-expert norm for 2 or 1:
+                            msk_moe_step_form),
                             1 = the chain of launches used for many tokens,
                             2 = row copy, gate/up kernel that routes and sorts, down kernel that combines,
                             3 = one launch (routing, sort, both GEMMs and the combine in one kernel);

@@ -1060,7 +1060,7 @@ static bool chain_with_pre_norm(const MskMoeCfg* c, int T, int inputs) {
 // With the post-expert norm the one launch ends with tickets per token and a combine by whole CTAs; from four tokens on the sort, both
 // GEMMs and the combine as launches of their own are faster (one launch / those, us, rows of steps): H2048 I1024 E64 top-4 4: 35.6 /
 // 33.7, 5: 36.6 / 34.6, 6: 42.5 / 38.2, 8: 46.2 / 40.2; a rank of H4096 I4096 4: 41.7 / 39.5, 8: 52.0 /
-// 49.6. Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
+// 49.6; 8 of 64 experts of H2048 I1024 8: 31.8 / 29.1 (two launches more are 1.3 us where no route is local: 12.5 / 13.8). Without the norm, whose tickets are per token and columns: 4: 31.4 / 32.8, 8: 39.7 / 39.2, H4096 I1536 E128 5: 78.6 / 80.0.
 // Rows in host memory: every CTA of the one launch reads the logits or ids over PCIe, the sort launch once, H2048 I1024 4: 50 - 53 / 39.0,
 // 8: 65 / 46.8, given ids 8: 59 - 71 / 44.2; H4096 I1536 E128 4: 95 / 78.5, given ids 3: 71 - 76 / 62.2, 4: 92 - 98 / 73.
 static int step_form(const MskMoeCfg* c, int T, const Plan& p, int inputs, bool nv_room, FewPlan* few) {
