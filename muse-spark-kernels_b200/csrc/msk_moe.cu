@@ -633,7 +633,7 @@ static Plan make_plan(const MskMoeCfg* c, int T) {
     // 16 / 64-token tile (us, rows of steps): H2048 I1024 E64 near-even rpe 4 58.9 / 58.8, 6 61.1 / 59.8, 8 63.2 / 61.2, 12 68.9 / 63.0, a few experts
     // taking most tokens 45.3 / 47.0, 51.9 / 51.4, 55.1 / 53.7, 67.0 / 59.6; H4096 I1024 E128 rpe 4 193 / 199 (105 / 90), 6 202 / 205, 8 210 / 208 (158 / 117), 12
     // 238 / 215 (210 / 144); H4096 I1280 E128 rpe 6 247 / 250, 8 254 / 252. Few narrow experts, top-2 of 8, rpe 7.25 / 8 / 10 / 12: H4096 I1024 41.2 / 39.2, 41.3 /
-    // 39.2, 41.4 / 39.3, 43.2 / 39.3 (43.3 / 41.4, 43.3 / 42.2, 43.3 / 43.4, 43.3 / 44.9); H1024 I512 28.9 / 27.1 .. 29.0 / 28.8 (29.0 / 28.8 .. 29.1 / 31.0). 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
+    // 39.2, 41.4 / 39.3, 43.2 / 39.3 (43.3 / 41.4, 43.3 / 42.2, 43.3 / 43.4, 43.3 / 44.9); H1024 I512 28.9 / 27.1 .. 29.0 / 28.8 (29.0 / 28.8 .. 29.1 / 31.0); a rank, 16 of 64 of H2048 I1024, rpe 9 / 12 34.1 / 32.4, 34.5 / 33.9 (36.5 / 38.2, 36.9 / 39.7). 64-token tile / pair kernel: T = 384 (rpe 24) 297 / 341, T = 512 319 / 362, T = 640
     // (rpe 40) 343 / 389; with a few experts taking most tokens 252 / 245, 311 / 287, 359 / 330. Beyond: rpe 48 near-even
     // 406 / 464, 32 of 256 experts at H4096 I4096 255 / 289, a few experts taking most 456 / 420, the same at H2048 I1024 E64
     // 107 / 88; rpe 56 445 / 477, 279 / 295, 508 / 452, 114 / 95; rpe 64 near-even 566 / 505. At rpe 40 the 64-token tile loses 13 %
